@@ -1,0 +1,399 @@
+// Attention of single tokens in the latent space on the tensor cores: all heads of a token read the same cached rows
+// [latent of RANK numbers | rotated key part of ROT], so a block takes 16 or 32 heads of one token and a run of its keys,
+// and every row it brings in serves all of them.
+//
+// A block (eight warps) walks its run 32 rows at a time; the rows come in with cp.async, STAGES tiles deep.  Per tile:
+//   S = Q K^T   four groups of warps take a quarter of the row's 576 numbers each (144: nine steps of mma.sync m16n8k16) and
+//               leave their partial scores in shared memory; the queries stay in registers for the whole run;
+//   softmax     a thread adds the quarters of a few scores of one head, in float32, and keeps the head's maximum and sum;
+//   O += P V    every warp takes 64 of the 512 value columns.
+// S of the next tile is computed together with P V of this one, so that the tensor cores wait for the softmax only.
+// Queries and weights are float32 and stay so: each goes in as three bfloat16 terms whose sum is the number to its last bit
+// (8 + 8 + 8 bits), against rows that are bfloat16 to begin with, so every product is exact and sums are float32.  A block
+// that shares a token's keys with others leaves maximum, sum and unscaled result for the merge kernel.
+//
+// What bounds it: the tensor cores' legacy path (three terms: 108 + 96 instructions a warp and tile, 1,024 multiply-adds a
+// clock and SM; busy 48 % of the time).  The kernel on the CUDA cores beside it (latent_attention_rows_kernel, still used for
+// other sizes) reads every row once for each pair of heads: 16 tokens of 32 heads over up to 3,500 keys took it 401 us, this
+// one 47; 8 tokens of 16 heads over a window of 1,024 take 9.
+#include "common.cuh"
+
+#include <cfloat>
+
+namespace {
+
+constexpr int RANK = 512, ROT = 64, D = RANK + ROT;
+constexpr int WARPS = 8, THREADS = 32 * WARPS;
+constexpr int QUARTERS = 4, STEPS = D / 16 / QUARTERS;   // steps of 16 numbers a group of warps takes of a row
+constexpr int PITCH = D + 8;                             // elements from row to row: an odd number of 16-byte pieces
+constexpr int MAX_SPLITS = 32;
+static_assert(D % (16 * QUARTERS) == 0 && RANK == 64 * WARPS, "shares of the warps");
+
+// HEADS 32: the two halves of the block take 16 heads each.  HEADS 16: they take the two halves of a tile's keys.
+template <int HEADS>
+struct LatentShape {
+  static constexpr int MG = HEADS / 16;
+  static constexpr int KT = 32, STAGES = 4;
+  static constexpr int SPT = HEADS * KT / THREADS;  // scores a thread has in the softmax
+  static constexpr int S_PITCH = KT + 8, P_PITCH = KT + 8;
+  static constexpr int TILE_BYTES = KT * PITCH * 2;
+  static constexpr int S_OFF = STAGES * TILE_BYTES;
+  static constexpr int P_OFF = S_OFF + QUARTERS * HEADS * S_PITCH * 4;
+  static constexpr int A_OFF = P_OFF + 3 * HEADS * P_PITCH * 2;   // per head: the factor of this tile, at the end the sum
+  static constexpr int L_OFF = A_OFF + HEADS * 4;                 // per stage and row: whether the row counts
+  static constexpr int BYTES = L_OFF + STAGES * KT * 4;
+  static_assert(KT == 4 * WARPS && KT % SPT == 0, "rows of a tile");
+};
+
+__device__ __forceinline__ void latent_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void latent_ldmatrix(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void latent_ldmatrix_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void latent_copy16(uint32_t dst, const void* src, bool there) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+
+// (x, y) as three pairs of bfloat16, the largest term first; the sum of a number's terms is the number
+__device__ __forceinline__ void three_terms(float x, float y, uint32_t (&out)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 t = __floats2bfloat162_rn(x, y);
+    out[i] = *reinterpret_cast<const uint32_t*>(&t);
+    const float2 f = __bfloat1622float2(t);
+    x -= f.x;
+    y -= f.y;
+  }
+}
+
+template <int HEADS>
+__global__ void __launch_bounds__(THREADS, 1)
+latent_attention_mma_kernel(const float* __restrict__ q_lat, const __nv_bfloat16* __restrict__ cache, const int32_t* __restrict__ table,
+                            int table_width, const int32_t* __restrict__ positions, const int32_t* __restrict__ token_item,
+                            const float* __restrict__ gate, __nv_bfloat16* __restrict__ out, float* __restrict__ partial, int heads,
+                            int page_size, int num_pages, int window, float scale, const float* __restrict__ sink) {
+  using Sh = LatentShape<HEADS>;
+  constexpr int KT = Sh::KT, MG = Sh::MG;
+  extern __shared__ __align__(16) unsigned char latent_smem[];
+  float* scores = reinterpret_cast<float*>(latent_smem + Sh::S_OFF);
+  uint32_t* weights = reinterpret_cast<uint32_t*>(latent_smem + Sh::P_OFF);
+  float* factors = reinterpret_cast<float*>(latent_smem + Sh::A_OFF);
+  int* counts = reinterpret_cast<int*>(latent_smem + Sh::L_OFF);
+  const uint32_t tiles_at = (uint32_t)__cvta_generic_to_shared(latent_smem);
+  const uint32_t weights_at = tiles_at + Sh::P_OFF;
+  pdl_trigger();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int groups = heads / HEADS;
+  const int t = blockIdx.x / groups, h0 = (blockIdx.x - t * groups) * HEADS;
+  const int splits = gridDim.y, split = blockIdx.y;
+  const int p = positions[t];
+  const int32_t* pages = table + (size_t)token_item[t] * table_width;
+  const int lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
+  const int all = (p - lo + KT) / KT;                    // tiles of the token's keys, and this block's run of them
+  const int per = (all + splits - 1) / splits;
+  const int first = lo + split * per * KT;
+  const int end = min(p + 1, first + per * KT);
+  const int ntiles = max(0, (end - first + KT - 1) / KT);
+
+  // A warp brings in four neighbouring rows of a tile; where they lie is looked up one tile earlier (lane r: row r), so that
+  // the copies never wait for the page table.
+  constexpr int MINE = KT / WARPS;
+  auto look_up = [&](int i) -> long long {
+    const int key = first + i * KT + warp * MINE + (lane & (MINE - 1));
+    if (i >= ntiles || key >= end) return -1;
+    const int page = pages[key / page_size];
+    return page >= 0 && page < num_pages ? ((long long)page * page_size + key % page_size) * D : -1;
+  };
+  auto bring = [&](int i, long long rows) {
+    const int stage = i % Sh::STAGES;
+    if (i < ntiles) {
+      if (lane < MINE) counts[stage * KT + warp * MINE + lane] = rows >= 0;
+#pragma unroll
+      for (int j = 0; j < MINE; ++j) {
+        const long long at = __shfl_sync(0xffffffffu, rows, j);
+        const __nv_bfloat16* src = cache + (at < 0 ? 0 : at);
+        const uint32_t dst = tiles_at + stage * Sh::TILE_BYTES + (warp * MINE + j) * PITCH * 2;
+#pragma unroll
+        for (int c = 0; c < D / 8; c += 32)
+          if (c + lane < D / 8) latent_copy16(dst + (c + lane) * 16, src + (c + lane) * 8, at >= 0);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < Sh::STAGES - 1; ++i) bring(i, look_up(i));
+  long long next_rows = look_up(Sh::STAGES - 1);
+
+  const int quarter = warp & 3, half = warp >> 2;        // half: of the heads (32) or of a tile's keys (16)
+  const int gr = lane >> 2, gc = 2 * (lane & 3);
+  uint32_t q[STEPS][3][4];
+  {
+    const float* rows = q_lat + ((size_t)t * heads + h0 + (MG == 2 ? 16 * half : 0) + gr) * D + quarter * STEPS * 16 + gc;
+#pragma unroll
+    for (int k = 0; k < STEPS; ++k) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 x = *reinterpret_cast<const float2*>(rows + (size_t)(j & 1) * 8 * D + k * 16 + (j >> 1) * 8);
+        uint32_t terms[3];
+        three_terms(x.x, x.y, terms);
+#pragma unroll
+        for (int e = 0; e < 3; ++e) q[k][e][j] = terms[e];
+      }
+    }
+  }
+  float o[MG][8][4];
+#pragma unroll
+  for (int m = 0; m < MG; ++m)
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[m][n][e] = 0.f;
+  // the softmax's share of a thread: SPT neighbouring keys of one head
+  constexpr int SPT = Sh::SPT, PER_HEAD = KT / SPT;
+  const int head = threadIdx.x / PER_HEAD, key_at = (threadIdx.x % PER_HEAD) * SPT;
+  float m_run = -FLT_MAX, l_run = 0.f;
+
+  auto products = [&](int i) {  // this warp's share of the scores of tile i
+    constexpr int NT = MG == 2 ? KT / 8 : KT / 16;
+    const uint32_t tile = tiles_at + (i % Sh::STAGES) * Sh::TILE_BYTES;
+    const int key0 = MG == 2 ? 0 : KT / 2 * half;
+    float s[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
+    const uint32_t at = tile + ((key0 + (lane & 7) + 8 * (lane >> 4)) * PITCH + quarter * STEPS * 16 + 8 * ((lane >> 3) & 1)) * 2;
+#pragma unroll
+    for (int k = 0; k < STEPS; ++k) {
+#pragma unroll
+      for (int n = 0; n < NT; n += 2) {
+        uint32_t b[4];
+        latent_ldmatrix(b, at + (n * 8 * PITCH + k * 16) * 2);
+#pragma unroll
+        for (int e = 2; e >= 0; --e) {
+          latent_mma(s[n], q[k][e], b[0], b[1]);
+          latent_mma(s[n + 1], q[k][e], b[2], b[3]);
+        }
+      }
+    }
+    float* dst = scores + (quarter * HEADS + (MG == 2 ? 16 * half : 0) + gr) * Sh::S_PITCH + key0 + gc;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      *reinterpret_cast<float2*>(dst + n * 8) = make_float2(s[n][0], s[n][1]);
+      *reinterpret_cast<float2*>(dst + 8 * Sh::S_PITCH + n * 8) = make_float2(s[n][2], s[n][3]);
+    }
+  };
+
+  asm volatile("cp.async.wait_group %0;" ::"n"(Sh::STAGES - 2) : "memory");
+  __syncthreads();
+  if (ntiles > 0) products(0);
+  for (int i = 0; i < ntiles; ++i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(Sh::STAGES - 3) : "memory");
+    __syncthreads();  // the scores of tile i are there, tile i + 1 too, and everybody has left the stage of tile i - 1
+    bring(i + Sh::STAGES - 1, next_rows);
+    next_rows = look_up(i + Sh::STAGES);
+    {
+      float s[SPT];
+#pragma unroll
+      for (int j = 0; j < SPT; ++j) s[j] = 0.f;
+      bool on[SPT];
+#pragma unroll
+      for (int j = 0; j < SPT; j += 2) {
+#pragma unroll
+        for (int e = 0; e < QUARTERS; ++e) {
+          const float2 part = *reinterpret_cast<const float2*>(scores + (e * HEADS + head) * Sh::S_PITCH + key_at + j);
+          s[j] += part.x;
+          s[j + 1] += part.y;
+        }
+        const int2 live = *reinterpret_cast<const int2*>(counts + (i % Sh::STAGES) * KT + key_at + j);
+        on[j] = live.x != 0;
+        on[j + 1] = live.y != 0;
+      }
+      float m_new = m_run;
+#pragma unroll
+      for (int e = 0; e < SPT; ++e) {
+        s[e] *= scale;
+        if (on[e]) m_new = fmaxf(m_new, s[e]);
+      }
+#pragma unroll
+      for (int off = 1; off < PER_HEAD; off <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, off));
+      const float alpha = expf(m_run - m_new);  // first tile: exp(-huge) = 0; no key that counts so far: 1, of nothing
+      float w[SPT], add = 0.f;
+#pragma unroll
+      for (int e = 0; e < SPT; ++e) {
+        w[e] = on[e] ? expf(s[e] - m_new) : 0.f;
+        add += w[e];
+      }
+      l_run = fmaf(l_run, alpha, add);
+      m_run = m_new;
+#pragma unroll
+      for (int j = 0; j < SPT; j += 2) {
+        uint32_t a[3];
+        three_terms(w[j], w[j + 1], a);
+#pragma unroll
+        for (int e = 0; e < 3; ++e) weights[((e * HEADS + head) * Sh::P_PITCH + key_at + j) / 2] = a[e];
+      }
+      if (key_at == 0) factors[head] = alpha;
+    }
+    __syncthreads();
+    if (i + 1 < ntiles) products(i + 1);
+    {
+      const uint32_t tile = tiles_at + (i % Sh::STAGES) * Sh::TILE_BYTES;
+#pragma unroll
+      for (int m = 0; m < MG; ++m) {
+        const float f0 = factors[16 * m + gr], f1 = factors[16 * m + gr + 8];
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+          o[m][n][0] *= f0; o[m][n][1] *= f0;
+          o[m][n][2] *= f1; o[m][n][3] *= f1;
+        }
+      }
+      const uint32_t at = tile + ((lane & 15) * PITCH + 64 * warp + 8 * (lane >> 4)) * 2;
+      const uint32_t wat = weights_at + ((lane & 15) * Sh::P_PITCH + 8 * (lane >> 4)) * 2;
+#pragma unroll
+      for (int k = 0; k < KT / 16; ++k) {
+        uint32_t a[MG][3][4];
+#pragma unroll
+        for (int m = 0; m < MG; ++m)
+#pragma unroll
+          for (int e = 0; e < 3; ++e) latent_ldmatrix(a[m][e], wat + ((e * HEADS + 16 * m) * Sh::P_PITCH + k * 16) * 2);
+#pragma unroll
+        for (int n = 0; n < 8; n += 2) {
+          uint32_t b[4];
+          latent_ldmatrix_trans(b, at + (k * 16 * PITCH + n * 8) * 2);
+#pragma unroll
+          for (int e = 2; e >= 0; --e)
+#pragma unroll
+            for (int m = 0; m < MG; ++m) {
+              latent_mma(o[m][n], a[m][e], b[0], b[1]);
+              latent_mma(o[m][n + 1], a[m][e], b[2], b[3]);
+            }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int off = 1; off < PER_HEAD; off <<= 1) l_run += __shfl_xor_sync(0xffffffffu, l_run, off);
+  if (splits > 1) {
+    float* mine = partial + (((size_t)t * heads + h0) * splits + split) * (RANK + 2);
+    if (key_at == 0) *reinterpret_cast<float2*>(mine + (size_t)head * splits * (RANK + 2)) = make_float2(m_run, l_run);
+#pragma unroll
+    for (int m = 0; m < MG; ++m)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        float* row = mine + (size_t)(16 * m + gr + 8 * r) * splits * (RANK + 2) + 2 + 64 * warp + gc;
+#pragma unroll
+        for (int n = 0; n < 8; ++n) *reinterpret_cast<float2*>(row + n * 8) = make_float2(o[m][n][2 * r], o[m][n][2 * r + 1]);
+      }
+    return;
+  }
+  __syncthreads();  // the last tile's factors have been read
+  if (key_at == 0) {
+    float by = 1.f / l_run;
+    if (sink) {
+      const float sk = sink[h0 + head], top = fmaxf(m_run, sk), down = expf(m_run - top);
+      by = down / fmaf(l_run, down, expf(sk - top));
+    }
+    factors[head] = by * (gate ? gate[(size_t)t * heads + h0 + head] : 1.f);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < MG; ++m)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int h = 16 * m + gr + 8 * r;
+      const float f = factors[h];
+      __nv_bfloat16* row = out + ((size_t)t * heads + h0 + h) * RANK + 64 * warp + gc;
+#pragma unroll
+      for (int n = 0; n < 8; ++n) *reinterpret_cast<__nv_bfloat162*>(row + n * 8) = __floats2bfloat162_rn(o[m][n][2 * r] * f, o[m][n][2 * r + 1] * f);
+    }
+}
+
+// A block per (token, head): the shares of the blocks that split its keys, in split order.
+__global__ void __launch_bounds__(RANK / 4)
+latent_attention_mma_merge_kernel(const float* __restrict__ partial, const float* __restrict__ gate, __nv_bfloat16* __restrict__ out,
+                                  int splits, const float* __restrict__ sink, int heads) {
+  __shared__ float by[MAX_SPLITS];
+  pdl_trigger();
+  pdl_wait();
+  const size_t unit = blockIdx.x;
+  const float* mine = partial + unit * splits * (RANK + 2);
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {
+    const float2 ml = lane < splits ? *reinterpret_cast<const float2*>(mine + (size_t)lane * (RANK + 2)) : make_float2(-FLT_MAX, 0.f);
+    const float sk = sink ? sink[unit % heads] : -FLT_MAX;
+    const float top = fmaxf(warp_max(ml.x), sk);
+    const float f = ml.y > 0.f ? expf(ml.x - top) : 0.f;
+    const float sum = warp_sum(ml.y * f) + (sink ? expf(sk - top) : 0.f);
+    by[lane] = f * (gate ? gate[unit] : 1.f) / sum;
+  }
+  __syncthreads();
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  const float* src = mine + 2 + 4 * threadIdx.x;  // rows start on 8 bytes
+#pragma unroll 4
+  for (int s = 0; s < splits; ++s) {
+    const float2 a = *reinterpret_cast<const float2*>(src + (size_t)s * (RANK + 2)), b = *reinterpret_cast<const float2*>(src + (size_t)s * (RANK + 2) + 2);
+    const float f = by[s];
+    v[0] = fmaf(a.x, f, v[0]); v[1] = fmaf(a.y, f, v[1]);
+    v[2] = fmaf(b.x, f, v[2]); v[3] = fmaf(b.y, f, v[3]);
+  }
+  __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+  *reinterpret_cast<uint2*>(out + unit * RANK + 4 * threadIdx.x) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+}
+
+template <int HEADS>
+int launch_latent_mma(const float* q, const __nv_bfloat16* cache, const int32_t* table, int width, const int32_t* positions,
+                      const int32_t* token_item, const float* gate, __nv_bfloat16* out, float* partial, int T, int heads, int page_size,
+                      int num_pages, int window, float scale, int splits, const float* sink, cudaStream_t stream) {
+  static PsbPerDevice configured;
+  if (!configured.get()) {
+    if (cudaFuncSetAttribute(latent_attention_mma_kernel<HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, LatentShape<HEADS>::BYTES) != cudaSuccess)
+      PSB_REFUSE("latent_attention_mma: cannot raise the shared-memory limit");
+    configured.set();
+  }
+  psb_launch(latent_attention_mma_kernel<HEADS>, dim3((unsigned)(T * (heads / HEADS)), splits), dim3(THREADS), (size_t)LatentShape<HEADS>::BYTES,
+             stream, q, cache, table, width, positions, token_item, gate, out, partial, heads, page_size, num_pages, window, scale, sink);
+  PSB_LAUNCH_CHECK("latent_attention_mma");
+  return 0;
+}
+
+}  // namespace
+
+// (rank, rot, heads) -> heads a block takes of a token, 0 if the kernel is not built for the sizes
+PSB_API int psb_latent_attention_mma_heads(int rank, int rot, int heads) {
+  if (rank != RANK || rot != ROT || heads < 1) return 0;
+  return heads % 32 == 0 ? 32 : heads % 16 == 0 ? 16 : 0;
+}
+
+// bfloat16 cache and output, float32 queries [T, heads, RANK + ROT]; ``splits`` (1..32) blocks share a token's keys, with
+// ``partial`` float32 [T, heads, splits, RANK + 2] as their meeting place.
+PSB_API int psb_latent_attention_mma(const void* q_lat, const void* cache, const void* table, int table_width, const void* positions,
+                                     const void* token_item, const void* gate, void* out, int T, int heads, int rank, int rot, int page_size,
+                                     int num_pages, int window, float scale, int splits, void* partial, const void* sink, cudaStream_t stream) {
+  const int per_block = psb_latent_attention_mma_heads(rank, rot, heads);
+  if (!per_block || T < 0) PSB_REFUSE("latent_attention_mma: not built for T=%d heads=%d rank=%d rot=%d", T, heads, rank, rot);
+  if (page_size < 1 || num_pages < 1 || table_width < 1) PSB_REFUSE("latent_attention_mma: bad paging (page_size=%d pages=%d width=%d)", page_size, num_pages, table_width);
+  if (window < 0) PSB_REFUSE("latent_attention_mma: negative window");
+  if (splits < 1 || splits > MAX_SPLITS || (splits > 1 && !partial)) PSB_REFUSE("latent_attention_mma: 1 to %d splits (with their scratch), not %d", MAX_SPLITS, splits);
+  if (((uintptr_t)cache | (uintptr_t)q_lat | (uintptr_t)out | (uintptr_t)partial) & 15) PSB_REFUSE("latent_attention_mma: queries, cache, scratch and output must be 16-byte aligned");
+  if (T == 0) return 0;
+  if ((long long)T * heads > 0x7fffffffLL) PSB_REFUSE("latent_attention_mma: batch too large");
+  auto launch = per_block == 32 ? launch_latent_mma<32> : launch_latent_mma<16>;
+  const int status = launch((const float*)q_lat, (const __nv_bfloat16*)cache, (const int32_t*)table, table_width, (const int32_t*)positions,
+                            (const int32_t*)token_item, (const float*)gate, (__nv_bfloat16*)out, (float*)partial, T, heads, page_size,
+                            num_pages, window, scale, splits, (const float*)sink, stream);
+  if (status) return status;
+  if (splits > 1) {
+    psb_launch(latent_attention_mma_merge_kernel, dim3((unsigned)(T * heads)), dim3(RANK / 4), 0, stream, (const float*)partial,
+               (const float*)gate, (__nv_bfloat16*)out, splits, (const float*)sink, heads);
+    PSB_LAUNCH_CHECK("latent_attention_mma_merge");
+  }
+  return 0;
+}

@@ -739,14 +739,21 @@ def latent_attention(q_lat: torch.Tensor, cache: torch.Tensor, table: torch.Tens
 # rounds of 410: 105 -> 86 us a layer).
 ROWS_BLOCK_SHARE = 96      # what a block costs beyond its keys, in keys
 ROWS_KEYS_PER_SPLIT = 128  # no block of that kernel is given fewer keys than this by splitting
+# The tensor-core kernel (rows of 512 + 64 numbers, heads in groups of 16 or 32): a block's queries and its unscaled result
+# cost about what 64 keys do, and up to 32 blocks may share a token's keys.  Down to the shortest walks it is ahead of the
+# kernel that reads rows side by side (32 tokens of 32 heads over up to 100 keys: 17 us).
+LATENT_MMA = True
+LATENT_MMA_BLOCK_SHARE = 64
+LATENT_MMA_KEYS_PER_SPLIT = 64
 
 
-def _rows_splits(blocks: int, keys: int, slots: int) -> int:
+def _rows_splits(blocks: int, keys: int, slots: int, most: int = 8, least_keys: int = ROWS_KEYS_PER_SPLIT,
+                 share: int = ROWS_BLOCK_SHARE) -> int:
     best, best_cost = 1, None
-    for s in range(1, 9):
-        if s > 1 and keys // s < ROWS_KEYS_PER_SPLIT:
+    for s in range(1, most + 1):
+        if s > 1 and keys // s < least_keys:
             break
-        cost = -(-blocks * s // slots) * (keys / s + ROWS_BLOCK_SHARE)
+        cost = -(-blocks * s // slots) * (keys / s + share)
         if best_cost is None or cost < best_cost:
             best, best_cost = s, cost
     return best
@@ -758,6 +765,19 @@ def _latent_attention_walk(q_lat, cache, table, positions, token_item, gate, out
     longest sequence), for the choice of how many blocks share a (token, head)."""
     t, heads, d = q_lat.shape
     hp, splits, partial = 1, 1, None
+    per_block = 0
+    if LATENT_MMA and cache.dtype == torch.bfloat16 and out.dtype == torch.bfloat16:
+        per_block = lib().psb_latent_attention_mma_heads(rank, d - rank, heads)
+    if per_block and q_lat.data_ptr() % 16 == 0 and cache.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0:
+        from .tensorcore import _sms
+        splits = _rows_splits(t * heads // per_block, key_hint, _sms(q_lat.device), 32, LATENT_MMA_KEYS_PER_SPLIT, LATENT_MMA_BLOCK_SHARE)
+        if splits > 1:
+            partial = torch.empty((t, heads, splits, rank + 2), dtype=torch.float32, device=q_lat.device)
+        check(lib().psb_latent_attention_mma(q_lat.data_ptr(), cache.data_ptr(), table.data_ptr(), table.shape[1], positions.data_ptr(),
+                                             token_item.data_ptr(), _ptr(gate), out.data_ptr(), t, heads, rank, d - rank, page_size,
+                                             cache.shape[0], int(window or 0), float(scale), splits, _ptr(partial), _ptr(sink), _stream()),
+              "latent_attention")
+        return
     if lib().psb_latent_attention_rows_supported(_code(cache, "cache entry"), rank, d - rank):
         if heads % 2 == 0 and d <= 768:
             hp = 2  # two heads of a token share a block and every row it loads

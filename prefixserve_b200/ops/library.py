@@ -147,6 +147,11 @@ _SIGNATURES: dict[str, list] = {
     # (cache_dtype, rank, rot) -> 1 if the kernel that reads rows side by side takes the case
     "psb_latent_attention_rows_supported": [I, I, I],
     "psb_latent_attention_max_rank": [],
+    # (rank, rot, heads) -> heads a block of the tensor-core kernel takes, 0 if it is not built for the sizes
+    "psb_latent_attention_mma_heads": [I, I, I],
+    # (q_lat, cache, table, table_width, positions, token_item, gate, out, T, heads, rank, rot, page_size, num_pages, window,
+    #  scale, splits, partial, sink, stream)
+    "psb_latent_attention_mma": [P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, F, I, P, P, P],
     # (cache, dtype, table, table_width, positions, token_item, band, values2, t0, n, KP, D, rank, page_size, num_pages, window, stream)
     "psb_latent_band_gather": [P, I, P, I, P, P, P, P, I, I, I, I, I, I, I, I, P],
     # (x float32, hi, lo, total, stream)

@@ -498,7 +498,7 @@ template <int D, int V>  // key and value sizes rounded up to 64 or 128
 __global__ void __launch_bounds__(MMA_WARPS * 32, 2)
 attention_biased_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kv,
                             const int32_t* __restrict__ table, int table_width, const int32_t* __restrict__ positions,
-                            const int32_t* __restrict__ item_start, int items, int min_tokens, const float* __restrict__ bias,
+                            const int32_t* __restrict__ item_start, int items, int min_tokens, int max_tokens, const float* __restrict__ bias,
                             const float* __restrict__ sink, __nv_bfloat16* __restrict__ out, int hq, int hkv, int dim, int vdim,
                             int page_size, int window, int chunk, int reach, float scale, int keep_first, int heads_here, const RowsTail tail) {
   extern __shared__ __align__(16) unsigned char mma_raw[];
@@ -507,7 +507,7 @@ attention_biased_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
   int item = -1, t0 = 0, tiles = 0;
   for (int i = 0; i < items; ++i) {
     const int n = item_start[i + 1] - item_start[i];
-    if (n >= min_tokens) tiles += (n + tile_tokens - 1) / tile_tokens;
+    if (n >= min_tokens && n <= max_tokens) tiles += (n + tile_tokens - 1) / tile_tokens;
   }
   int at = tiles - 1 - (int)blockIdx.y;
   if (chunk >= 2 * tile_tokens && items == 1) {  // (the launch has blocks for this): the late tiles of every chunk, then the ones before them
@@ -517,7 +517,7 @@ attention_biased_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
   }
   for (int i = 0, left = at; i < items && left >= 0; ++i) {
     const int a = item_start[i], n = item_start[i + 1] - a;
-    if (n < min_tokens) continue;
+    if (n < min_tokens || n > max_tokens) continue;
     const int mine = (n + tile_tokens - 1) / tile_tokens;
     if (left < mine) { item = i; t0 = a + left * tile_tokens; break; }
     left -= mine;
@@ -1073,14 +1073,14 @@ PSB_API int psb_attention_biased_mma_supported(int hq, int hkv, int dim, int vdi
   return hq >= 1 && hkv >= 1 && hq % hkv == 0 && dim >= 8 && dim <= 128 && dim % 8 == 0 && vdim >= 8 && vdim <= 128 && vdim % 8 == 0 ? 1 : 0;
 }
 
-// The tensor-core kernel over every portion of at least ``min_tokens`` tokens (bfloat16; grid sized by an upper bound on
+// The tensor-core kernel over every portion of ``min_tokens`` to ``max_tokens`` tokens (bfloat16; grid sized by an upper bound on
 // the tiles).  Other tokens are left untouched.
-// (q, kv, table, table_width, positions, item_start, items, T, min_tokens, bias, sink, out, hq, hkv, dim, vdim,
+// (q, kv, table, table_width, positions, item_start, items, T, min_tokens, max_tokens, bias, sink, out, hq, hkv, dim, vdim,
 //  page_size, window, chunk, reach, scale, keep_first, gate, ldg, ldo, out_scale, softcap, stream)
 PSB_API int psb_attention_biased_mma(const void* q, const void* kv, const void* table, int table_width, const void* positions,
-                                     const void* item_start, int items, int T, int min_tokens, const void* bias, const void* sink,
-                                     void* out, int hq, int hkv, int dim, int vdim, int page_size, int window, int chunk, int reach,
-                                     float scale, int keep_first, const void* gate, long long ldg, long long ldo, float out_scale,
+                                     const void* item_start, int items, int T, int min_tokens, int max_tokens, const void* bias,
+                                     const void* sink, void* out, int hq, int hkv, int dim, int vdim, int page_size, int window, int chunk,
+                                     int reach, float scale, int keep_first, const void* gate, long long ldg, long long ldo, float out_scale,
                                      float softcap, cudaStream_t stream) {
   if (ldo < (long long)hq * vdim || ldo % 2 || ((uintptr_t)out & 3) || (gate && ldg < (long long)hq * vdim) || softcap < 0.f)
     PSB_REFUSE("attention_biased_mma: bad output or gate rows, or a negative cap");
@@ -1107,7 +1107,7 @@ PSB_API int psb_attention_biased_mma(const void* q, const void* kv, const void* 
     }                                                                                                                          \
     psb_launch(attention_biased_mma_kernel<D_, V_>, grid, dim3(MMA_WARPS * 32), smem, stream, (const __nv_bfloat16*)q,          \
                (const __nv_bfloat16*)kv, (const int32_t*)table, table_width, (const int32_t*)positions,                        \
-               (const int32_t*)item_start, items, min_tokens, (const float*)bias, (const float*)sink, (__nv_bfloat16*)out, hq,  \
+               (const int32_t*)item_start, items, min_tokens, max_tokens, (const float*)bias, (const float*)sink, (__nv_bfloat16*)out, hq,  \
                hkv, dim, vdim, page_size, window, chunk, reach, scale, keep_first, heads_here, tail);                          \
   } while (0)
   if (dim <= 64 && vdim <= 64) MMA_CASE(64, 64);

@@ -912,6 +912,30 @@ BIASED_MMA = True            # ... the tensor-core one where the sizes allow (mu
 # The tensor-core kernel also takes single tokens and short portions: its blocks bring keys and values in with wide,
 # coalesced loads of all threads, which is what a decode step is bound by (the rows of its tile that have no token idle).
 BIASED_MMA_MIN_TOKENS = 1
+# Heads of 128 in bfloat16: portions from this many tokens on go to the kernel on tcgen05, whose tiles hold 128 tokens of a head
+# (two portions of 64 and 51 tokens behind 1,500 keys, 32 heads: 26 us; the shorter one alone on mma.sync 99)
+ROWS_TCGEN05 = True
+ROWS_TCGEN05_MIN_TOKENS = 16
+# Its CTAs take whole rounds over the SMs; the units of a last round that is not full are cut into up to this many ranges of keys.
+# In blocks of 64 keys: what a CTA costs beside its blocks, and the kernel that joins the ranges.
+ROWS_TCGEN05_RANGES = 8
+ROWS_TCGEN05_CTA_COST = 3
+ROWS_TCGEN05_MERGE_COST = 3
+
+
+def _rows_ranges(units: int, blocks: int, device) -> tuple[int, int]:
+    """(units that are one CTA's, ranges of keys each of the others is cut into) for units of about so many blocks."""
+    from .tensorcore import _sms
+    sms = _sms(device)
+    rest = units % sms
+    if rest == 0:
+        return units, 1
+    cost = {s: -(-rest * s // sms) * (-(-blocks // s) + ROWS_TCGEN05_CTA_COST) + (ROWS_TCGEN05_MERGE_COST if s > 1 else 0)
+            for s in range(1, ROWS_TCGEN05_RANGES + 1) if s == 1 or blocks >= 2 * s}
+    best = min(cost, key=lambda s: (cost[s], s))
+    return (units, 1) if best == 1 else (units - rest, best)
+
+
 # Steps in which every item is a single token: the kernel that walks the keys, with the runs of a (token, head) shared out
 # among up to 16 blocks and a merge kernel behind them (a step of 8 tokens is 128 blocks of one warp's work each otherwise,
 # every one of them a chain of a thousand keys).  BIASED_BLOCKS_WANTED blocks keep every SM busy; no share below 128 keys.
@@ -1022,12 +1046,45 @@ def attention_over_rows(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, 
                                          _ptr(bias), _ptr(sink), out.data_ptr(), t, num_heads, num_kv_heads, dim, vdim,
                                          page_size, win, chk, reach, float(scale), item_start.data_ptr(),
                                          least if tiled else 0, keep_first, None, 1, *tail, _stream()), "attention_biased")
-    if tiled:
-        entry = lib().psb_attention_biased_mma if on_tensor_cores else lib().psb_attention_biased_tiles
-        check(entry(q.data_ptr(), kv.data_ptr(), table.data_ptr(), table.shape[1], positions.data_ptr(), item_start.data_ptr(),
-                    ctx.num_items, t, least, _ptr(bias), _ptr(sink), out.data_ptr(), num_heads, num_kv_heads, dim,
-                    vdim, page_size, win, chk, reach, float(scale), keep_first, *tail, _stream()),
-              "attention_biased_mma" if on_tensor_cores else "attention_biased_tiles")
+    if tiled and on_tensor_cores:
+        most = 0x7fffffff  # tokens of the longest portion left to the kernel on mma.sync
+        if (ROWS_TCGEN05 and ctx.max_new_tokens >= ROWS_TCGEN05_MIN_TOKENS and ldo % 8 == 0 and out.data_ptr() % 16 == 0
+                and (gate is None or (ldg % 8 == 0 and gate.data_ptr() % 16 == 0))
+                and bool(lib().psb_attention_rows_tcgen05_supported(num_heads, num_kv_heads, dim, vdim, page_size, 1 if softcap else 0,
+                                                                    0 if bias is None else 1))):
+            most = ROWS_TCGEN05_MIN_TOKENS - 1
+            items = getattr(ctx, "items", None)
+            if items is None:
+                tiles, others = t // 128 + ctx.num_items, ctx.num_items > 1
+            else:
+                lens = [it.end - it.start for it in items]
+                tiles, others = sum(-(-n // 128) for n in lens if n > most), min(lens) <= most
+            keys = int((getattr(ctx, "extras", None) or {}).get("static_kv_len") or ctx.max_kv_len)
+            span = min(keys, win + keep_first + 128 if win else keys, chk + 128 if chk else keys)
+            units = tiles * (num_heads // lib().psb_attention_rows_tcgen05_heads(num_heads, num_kv_heads))
+            whole, ranges = _rows_ranges(units, -(-span // 64), q.device)
+            part_o = part_ml = None
+            if whole < units:
+                part_o = torch.empty((units - whole, ranges, 256, 128), dtype=torch.float32, device=q.device)
+                part_ml = torch.empty((units - whole, ranges, 256, 2), dtype=torch.float32, device=q.device)
+            check(lib().psb_attention_rows_tcgen05(q.data_ptr(), kv.data_ptr(), kv.shape[0], table.data_ptr(), table.shape[1],
+                                                   positions.data_ptr(), item_start.data_ptr(), ctx.num_items, t, ROWS_TCGEN05_MIN_TOKENS,
+                                                   tiles, _ptr(bias), _ptr(sink), out.data_ptr(), num_heads, num_kv_heads,
+                                                   dim, vdim, page_size, win, chk, reach, float(scale), keep_first, *tail, whole, ranges,
+                                                   _ptr(part_o), _ptr(part_ml), _stream()),
+                  "attention_rows_tcgen05")
+        else:
+            others = True
+        if others:
+            check(lib().psb_attention_biased_mma(q.data_ptr(), kv.data_ptr(), table.data_ptr(), table.shape[1], positions.data_ptr(),
+                                                 item_start.data_ptr(), ctx.num_items, t, least, most, _ptr(bias), _ptr(sink), out.data_ptr(),
+                                                 num_heads, num_kv_heads, dim, vdim, page_size, win, chk, reach, float(scale), keep_first,
+                                                 *tail, _stream()), "attention_biased_mma")
+    elif tiled:
+        check(lib().psb_attention_biased_tiles(q.data_ptr(), kv.data_ptr(), table.data_ptr(), table.shape[1], positions.data_ptr(),
+                                               item_start.data_ptr(), ctx.num_items, t, least, _ptr(bias), _ptr(sink), out.data_ptr(),
+                                               num_heads, num_kv_heads, dim, vdim, page_size, win, chk, reach, float(scale), keep_first,
+                                               *tail, _stream()), "attention_biased_tiles")
     return out
 
 

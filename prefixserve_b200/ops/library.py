@@ -185,7 +185,16 @@ _SIGNATURES: dict[str, list] = {
     #  page_size, window, chunk, reach, scale, stream)
     "psb_attention_biased_tiles": [P, P, P, I, P, P, I, I, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, L, L, F, F, P],
     "psb_attention_biased_mma_supported": [I, I, I, I],
-    "psb_attention_biased_mma": [P, P, P, I, P, P, I, I, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, L, L, F, F, P],
+    # the same with max_tokens behind min_tokens
+    "psb_attention_biased_mma": [P, P, P, I, P, P, I, I, I, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, L, L, F, F, P],
+    # (hq, hkv, dim, vdim, page_size, capped, biased) -> 1 if the tcgen05 kernel over rows takes them
+    "psb_attention_rows_tcgen05_supported": [I, I, I, I, I, I, I],
+    # (hq, hkv) -> query heads a unit of it takes
+    "psb_attention_rows_tcgen05_heads": [I, I],
+    # (q, kv, num_pages, table, table_width, positions, item_start, items, T, min_tokens, tiles, bias, sink, out, hq, hkv, dim, vdim,
+    #  page_size, window, chunk, reach, scale, keep_first, gate, ldg, ldo, out_scale, softcap, whole, ranges, part_o, part_ml, stream)
+    "psb_attention_rows_tcgen05": [P, P, L, P, I, P, P, I, I, I, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, L, L, F, F, I, I, P, P, P],
+    "psb_attention_rows_tcgen05_status": [],
     "psb_delta_max_taps": [],
     # (proj, dtype, ld, beta_at, ba, decay, taps, a_log, dt_bias, state, positions, token_item, item_start, slots, qkv_out, bd_out, T,
     #  G, H, dim, vdim, K, num_slots, slot_floats, stream)
@@ -327,9 +336,10 @@ def tcgen05_status() -> int:
     """0 unless a bounded wait inside a tcgen05 kernel ever gave up (then its results are void). Synchronises.
 
     The product's code sits in the low byte, prefill attention's in the next, the TMA-fed decode attention's in the
-    third, the few-row product's in the fourth."""
+    third, the few-row product's in the fourth, prefill attention's over rows in the fifth."""
     return (int(lib().psb_tcgen05_status()) | (int(lib().psb_attention_tcgen05_status()) << 8)
-            | (int(lib().psb_attention_decode_tma_status()) << 16) | (int(lib().psb_gemm_fewrows_status()) << 24))
+            | (int(lib().psb_attention_decode_tma_status()) << 16) | (int(lib().psb_gemm_fewrows_status()) << 24)
+            | (int(lib().psb_attention_rows_tcgen05_status()) << 32))
 
 
 def declare(name: str, argtypes: list) -> None:

@@ -1,0 +1,110 @@
+"""Prompt portions' attention over cache rows on tcgen05 against the same in float64: every mask, a cap on scores near and far
+from it, a distance bias with a short reach, kept first keys that lie in the window's own blocks, in blocks of their own and
+across several, sinks and gates; portions at the edges of tiles of 128 tokens and of blocks of 64 keys, whole and cut into
+ranges of keys; pages that nobody has written or that have been given back (NaN, and no number in the table)."""
+
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+D = 128
+
+
+def step(lengths, starts):
+    positions, item_of, offsets = [], [], [0]
+    for i, (n, s) in enumerate(zip(lengths, starts)):
+        positions += range(s, s + n)
+        item_of += [i] * n
+        offsets.append(offsets[-1] + n)
+    dev = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    return types.SimpleNamespace(positions=dev(positions), token_item=dev(item_of), item_start=dev(offsets), num_items=len(lengths),
+                                 max_new_tokens=max(lengths), max_kv_len=max(n + s for n, s in zip(lengths, starts)), extras={})
+
+
+def seen_keys(i, keys, window, chunk, keep):
+    j = torch.arange(keys)
+    seen = j <= i
+    if window:
+        seen &= (i - j < window) | (j < keep)
+    if chunk:
+        seen &= j // chunk == i // chunk
+    return seen
+
+
+@pytest.mark.parametrize("hq,hkv,page,options", [
+    (4, 1, 16, dict(window=200)),
+    (4, 2, 16, dict(window=None)),
+    (3, 1, 8, dict(window=1)),
+    (2, 2, 64, dict(window=65, sink=True, gate=True)),
+    (4, 2, 16, dict(window=100, softcap=3.0, gate=True)),
+    (4, 2, 32, dict(window=300, softcap=500.0, gate=True, out_scale=-0.5)),
+    (4, 1, 16, dict(window=90, keep=4, sink=True)),
+    (2, 1, 16, dict(window=64, keep=70)),
+    (2, 1, 8, dict(window=200, keep=130, sink=True)),
+    (4, 2, 16, dict(chunk=256, bias=256, sink=True)),
+    (2, 1, 16, dict(chunk=100, bias=30)),
+    (2, 1, 16, dict(window=5000, bias=4600)),
+])
+@pytest.mark.parametrize("ranges", [1, 8])
+def test_portions(hq, hkv, page, options, ranges, monkeypatch):
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import kernels, library
+    monkeypatch.setattr(kernels, "ROWS_TCGEN05_RANGES", ranges)   # every unit a CTA's, or cut into ranges of keys where that pays
+    window, chunk, keep = options.get("window"), options.get("chunk"), options.get("keep", 0)
+    far = options.get("bias", 0) > 4096   # distances beyond those whose bias the kernel keeps at hand
+    lengths, starts = ([200], [4500]) if far else ([64, 300, 1, 129, 20, 256], [0, 331, 500, 1000, 7, 60])
+    g = torch.Generator().manual_seed(hq + page + len(options))
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    ctx, t = step(lengths, starts), sum(lengths)
+    held = [n + s for n, s in zip(lengths, starts)]
+    need = [-(-n // page) for n in held]
+    ids = torch.randperm(sum(need), generator=g).tolist()
+    table = torch.full((len(held), max(need)), -1, dtype=torch.int32)
+    kv = torch.full((sum(need), 1, hkv, page, 2 * D), float("nan"), dtype=torch.bfloat16)
+    rows = [rnd(n, hkv, 2 * D).bfloat16() for n in held]
+    for i, n in enumerate(held):
+        # what the portion's first token can see and everything behind it; other pages have been given back
+        first = seen_keys(starts[i], n, window, chunk, keep)
+        first[starts[i]:] = True
+        for j in range(need[i]):
+            if first[j * page: (j + 1) * page].any():
+                table[i, j] = pid = ids.pop()
+                part = rows[i][j * page: (j + 1) * page]
+                kv[pid, 0, :, : len(part)] = part.transpose(0, 1)
+    q = rnd(t, hq, D).bfloat16()
+    sink = 2.0 * rnd(hq) if options.get("sink") else None
+    bias = rnd(hq, options["bias"]) if "bias" in options else None
+    gate = rnd(t, hq * D + 16).bfloat16() if options.get("gate") else None
+    wide = torch.full((t, hq * D + 24), 7.0, dtype=torch.bfloat16, device="cuda")
+    dev = lambda x: None if x is None else x.cuda()
+    before = library.launch_counts.copy()
+    out = ops.attention_over_rows(q.cuda(), kv.cuda(), table.cuda(), ctx, num_heads=hq, num_kv_heads=hkv, dim=D, vdim=D, page_size=page, scale=0.2,
+                                  window=window, chunk=chunk, keep_first=keep, bias=dev(bias), sink=dev(sink), softcap=options.get("softcap"),
+                                  gate=None if gate is None else gate.cuda()[:, 8: 8 + hq * D], out_scale=options.get("out_scale", 1.0),
+                                  out=wide[:, 8: 8 + hq * D])
+    taken = library.launch_counts - before
+    assert taken["attention_rows_tcgen05"] == 1 and taken["attention_biased_mma"] == (0 if far else 1)
+    assert bool((wide[:, :8] == 7.0).all()) and bool((wide[:, 8 + hq * D:] == 7.0).all())
+    got, at = out.cpu().double().view(t, hq, D), 0
+    for i, (n, s) in enumerate(zip(lengths, starts)):
+        keys, values = (x.cuda().double().repeat_interleave(hq // hkv, 1) for x in (rows[i][..., :D], rows[i][..., D:]))
+        scores = torch.einsum("thd,jhd->thj", q[at: at + n].cuda().double(), keys) * 0.2
+        if options.get("softcap"):
+            scores = options["softcap"] * torch.tanh(scores / options["softcap"])
+        if bias is not None:
+            dist = (torch.arange(s, s + n)[:, None] - torch.arange(held[i])[None]).clamp(0, options["bias"] - 1)
+            scores = scores + bias.cuda().double()[:, dist.cuda()].transpose(0, 1)
+        mask = torch.stack([seen_keys(s + r, held[i], window, chunk, keep) for r in range(n)]).cuda()
+        scores = scores.masked_fill(~mask[:, None], float("-inf"))
+        if sink is not None:
+            scores = torch.cat([scores, sink.cuda().double()[None, :, None].expand(n, hq, 1)], -1)
+        want = torch.einsum("thj,jhd->thd", torch.softmax(scores, -1)[..., : held[i]], values).cpu() * options.get("out_scale", 1.0)
+        if gate is not None:
+            want = want * torch.sigmoid(gate[at: at + n, 8: 8 + hq * D].double().view(n, hq, D))
+        # rounding of the result to bfloat16 (2^-9); weights to 16 bits (2^-17 of values up to 5) and float32 scores up to 100
+        assert ((got[at: at + n] - want).abs() <= 2.0 ** -8 * want.abs() + 3e-4).all(), (i, n, s, (got[at: at + n] - want).abs().max())
+        at += n
+    assert library.tcgen05_status() == 0

@@ -22,6 +22,9 @@
 // per request also brings the slot's convolution inputs up to date (the last K-1 rows of the projection, or what
 // was there before, moved up, when the portion is shorter).
 //
+// Portions of a few dozen tokens and more of the usual sizes go through the kernels of delta_chunks.cu instead, which need
+// neither the single steps nor:
+//
 // delta_cross_kernel (a warp per token and head): q.k, and k.k' and q.k' with the key of the token before.
 //
 // channel_delta_rule_kernel: the same rule with a decay per head and key channel, g [T, H, dim], which multiplies the rows
@@ -32,14 +35,11 @@
 // the compute type for the output projection.
 //
 // Slot layout (float32): [K-1, C] convolution inputs, oldest first (C = 2 G dim + H vdim), then S as [H, dim, vdim].
-#include "common.cuh"
+#include "delta_common.cuh"
 
 namespace {
 
-constexpr int MAX_TAPS = 16;
-// Per token and head the recurrence is handed five numbers, [T, BD, H]: beta, decay, and three dot products that do
-// not depend on the state: q.k of the token, and k.k' and q.k' with the key k' of the token before it in the portion.
-constexpr int BD = 5;
+using namespace delta;
 
 __device__ __forceinline__ float softplusf_(float x) { return log1pf(expf(-fabsf(x))) + fmaxf(x, 0.f); }
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + expf(-x)); }
@@ -256,41 +256,6 @@ delta_cross_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ to
 
 constexpr int RULE_WARPS = 4;
 
-__device__ __forceinline__ void copy_async4(float* dst, const float* src) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy_async16(float* dst, const float* src) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy_async_wait() {
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-}
-
-// One block per request, at the end of its portion: the slot's convolution inputs, which are the K-1 positions before the
-// next token (the portion's last rows, or what was there before, moved up, when the portion is shorter).
-template <typename T>
-__device__ __forceinline__ void keep_conv_inputs(const T* __restrict__ proj, long long P, float* __restrict__ base, int t0, int t1,
-                                                 int C, int K) {
-  if (K <= 1 || t1 <= t0) return;
-  const int n = t1 - t0;
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    float keep[MAX_TAPS];
-#pragma unroll
-    for (int k = 0; k < MAX_TAPS; ++k) {
-      if (k >= K - 1) break;
-      const int back = K - 1 - k;  // this row is the input ``back`` positions before the next token
-      keep[k] = back <= n ? to_float<T>(proj[(size_t)(t1 - back) * P + c]) : base[(size_t)(k + n) * C + c];
-    }
-#pragma unroll
-    for (int k = 0; k < MAX_TAPS; ++k) {
-      if (k >= K - 1) break;
-      base[(size_t)k * C + c] = keep[k];
-    }
-  }
-}
-
 // PER: numbers of a column one lane holds; R: lanes per column.  R * PER >= dim.  What the tokens of a stage bring
 // (queries, keys, the block's value columns, beta, decay) is copied into shared memory one stage ahead of the
 // arithmetic (cp.async into the other of two buffers), so the chain from token to token never waits for memory.
@@ -305,7 +270,7 @@ __global__ void __launch_bounds__(RULE_WARPS * 32)
 delta_rule_kernel(const float* __restrict__ qkv, const float* __restrict__ bd, const T* __restrict__ proj,
                   float* __restrict__ state, const int32_t* __restrict__ item_start, const int32_t* __restrict__ slots,
                   float* __restrict__ o, int G, int H, int dim, int vdim, int K, int num_slots, size_t slot_floats,
-                  int stage_tokens) {
+                  int stage_tokens, int max_tokens) {
   extern __shared__ __align__(16) float staged[];  // [2][stage_tokens][W]
   constexpr int COLS = 32 / R;  // columns a warp holds
   constexpr int RP = R * PER, BC = RULE_WARPS * COLS, W = (2 * RP + BC + BD + 3) / 4 * 4;
@@ -322,6 +287,7 @@ delta_rule_kernel(const float* __restrict__ qkv, const float* __restrict__ bd, c
   const bool wide = dim % 4 == 0 && C % 4 == 0 && (((uintptr_t)qkv) & 15) == 0;
   pdl_wait();
   const int t0 = item_start[item], t1 = item_start[item + 1];
+  if (t1 - t0 > max_tokens) return;  // a portion of the kernels that work in chunks
   int slot = slots[item];
   slot = slot < 0 ? 0 : (slot >= num_slots ? num_slots - 1 : slot);
   float* base = state + (size_t)slot * slot_floats;
@@ -975,13 +941,13 @@ delta_finish_kernel(const float* __restrict__ o, const T* __restrict__ proj, con
 template <typename T, int PER, int R>
 void launch_rule(dim3 grid, cudaStream_t stream, const float* qkv, const float* bd, const T* proj, float* state,
                  const int32_t* item_start, const int32_t* slots, float* o, int G, int H, int dim, int vdim, int K,
-                 int num_slots, size_t slot_floats) {
+                 int num_slots, size_t slot_floats, int max_tokens) {
   constexpr int W = (2 * R * PER + RULE_WARPS * (32 / R) + BD + 3) / 4 * 4;
   // two buffers within the 48 KB a kernel has without asking: 16 tokens a stage for keys up to 128 numbers, 4 beyond
   const int stage_tokens = 2 * 16 * W * (int)sizeof(float) <= 48 * 1024 ? 16 : 4;
   static_assert(2 * 4 * W * sizeof(float) <= 48 * 1024, "a stage of four tokens fits the default shared memory twice");
   psb_launch(delta_rule_kernel<T, PER, R>, grid, dim3(RULE_WARPS * 32), (size_t)2 * stage_tokens * W * sizeof(float), stream, qkv,
-             bd, proj, state, item_start, slots, o, G, H, dim, vdim, K, num_slots, slot_floats, stage_tokens);
+             bd, proj, state, item_start, slots, o, G, H, dim, vdim, K, num_slots, slot_floats, stage_tokens, max_tokens);
 }
 
 }  // namespace
@@ -991,11 +957,11 @@ PSB_API int psb_delta_max_taps() { return MAX_TAPS; }
 // ``ba`` null: the write strengths' pre-activations are the projection's columns beta_at .. beta_at + H - 1 and the decays come
 // from elsewhere; ``decay`` (float32 [T, H, dim] or null) then goes into the products with the key of the token before.
 // (proj, dtype, ld, beta_at, ba, decay, taps, a_log, dt_bias, state, positions, token_item, item_start, slots, qkv_out, bd_out, T, G,
-//  H, dim, vdim, K, num_slots, slot_floats, stream)
+//  H, dim, vdim, K, num_slots, slot_floats, cross, stream); ``cross`` 0: no token goes through a kernel that reads those products
 PSB_API int psb_delta_prepare(const void* proj, int dtype, long long ld, int beta_at, const void* ba, const void* decay,
                               const void* taps, const void* a_log, const void* dt_bias, const void* state, const void* positions, const void* token_item,
                               const void* item_start, const void* slots, void* qkv, void* bd, int T, int G, int H, int dim,
-                              int vdim, int K, int num_slots, long long slot_floats, cudaStream_t stream) {
+                              int vdim, int K, int num_slots, long long slot_floats, int cross, cudaStream_t stream) {
   if (T < 0 || G < 1 || H < 1 || H % G || dim < 1 || vdim < 1) PSB_REFUSE("delta_prepare: bad sizes G=%d H=%d dim=%d vdim=%d", G, H, dim, vdim);
   if (K < 1 || K > MAX_TAPS) PSB_REFUSE("delta_prepare: %d taps are outside [1, %d]", K, MAX_TAPS);
   const long long C = 2LL * G * dim + (long long)H * vdim;
@@ -1024,7 +990,7 @@ PSB_API int psb_delta_prepare(const void* proj, int dtype, long long ld, int bet
     }
   });
   PSB_LAUNCH_CHECK("delta_prepare");
-  if (!ba && !decay) return 0;  // the chunked form makes its own products
+  if (!cross || (!ba && !decay)) return 0;  // the chunked forms make their own products
   const long long units = (long long)T * H;
   psb_launch(delta_cross_kernel, dim3((unsigned)((units + 3) / 4)), dim3(128), 0, stream, (const float*)qkv, (const int32_t*)token_item,
              (const int32_t*)item_start, (float*)bd, units, G, H, dim, vdim, (const float*)decay);
@@ -1032,12 +998,13 @@ PSB_API int psb_delta_prepare(const void* proj, int dtype, long long ld, int bet
   return 0;
 }
 
-// (qkv, bd, proj, dtype, state, item_start, slots, o_out, items, G, H, dim, vdim, K, num_slots, slot_floats, lanes, stream)
+// (qkv, bd, proj, dtype, state, item_start, slots, o_out, items, G, H, dim, vdim, K, num_slots, slot_floats, lanes, max_tokens,
+//  stream).  Portions of more than ``max_tokens`` tokens, and their slots, are left untouched.
 // ``lanes``: lanes of a warp that share a column of the state (4: a warp reads whole sectors of the state, for steps
 // of single tokens; 16 or 32: short chains per token and more warps, for long portions).
 PSB_API int psb_delta_rule(const void* qkv, const void* bd, const void* proj, int dtype, void* state, const void* item_start,
                            const void* slots, void* o, int items, int G, int H, int dim, int vdim, int K, int num_slots,
-                           long long slot_floats, int lanes, cudaStream_t stream) {
+                           long long slot_floats, int lanes, int max_tokens, cudaStream_t stream) {
   if (items < 0 || G < 1 || H < 1 || H % G || dim < 1 || vdim < 1) PSB_REFUSE("delta_rule: bad sizes G=%d H=%d dim=%d vdim=%d", G, H, dim, vdim);
   if (K < 1 || K > MAX_TAPS) PSB_REFUSE("delta_rule: %d taps are outside [1, %d]", K, MAX_TAPS);
   if (lanes != 4 && lanes != 16 && lanes != 32) PSB_REFUSE("delta_rule: %d lanes a column is not built (4, 16 or 32)", lanes);
@@ -1050,7 +1017,7 @@ PSB_API int psb_delta_rule(const void* qkv, const void* bd, const void* proj, in
 #define RULE(PER_, R_)                                                                                                \
   launch_rule<T_, PER_, R_>(grid, stream, (const float*)qkv, (const float*)bd, (const T_*)proj, (float*)state,       \
                             (const int32_t*)item_start, (const int32_t*)slots, (float*)o, G, H, dim, vdim, K, num_slots, \
-                            (size_t)slot_floats)
+                            (size_t)slot_floats, max_tokens)
   PSB_DISPATCH_DTYPE(dtype, T_, {
     if (lanes == 4) {
       if (per <= 4) RULE(4, 4);

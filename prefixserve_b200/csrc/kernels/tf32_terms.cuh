@@ -1,0 +1,56 @@
+// Products of float32 numbers on the tensor cores.
+//
+// mma.sync m16n8k8 multiplies numbers of 11 bits.  A float32 number enters as hi (rounded to nearest) + lo (22 bits), and a product as
+// hi hi + hi lo + lo hi.  The sums of the hi hi products leave the tensor cores after every eight terms and are added up in float32
+// with rounding to nearest, since the instruction cuts its sums off instead of rounding them.
+#pragma once
+#include "common.cuh"
+
+namespace terms {
+
+struct Split {
+  uint32_t hi, lo;
+};
+__device__ __forceinline__ Split split(float x) {
+  const uint32_t hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+  return {hi, __float_as_uint(x - __uint_as_float(hi))};  // (the instruction does not look at lo's last 13 bits)
+}
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const float (&c)[4]) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
+}
+// One step of eight terms: sum += hi hi (rounded to nearest), small += hi lo + lo hi.
+struct Sum {
+  float sum[4] = {}, small[2][4] = {};
+  __device__ __forceinline__ void step(const uint32_t (&ah)[4], const uint32_t (&al)[4], Split b0, Split b1) {
+    const float zero[4] = {};
+    float d[4];
+    mma_tf32(d, ah, b0.hi, b1.hi, zero);
+    mma_tf32(small[0], ah, b0.lo, b1.lo, small[0]);
+    mma_tf32(small[1], al, b0.hi, b1.hi, small[1]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sum[e] += d[e];
+  }
+  // the right operand's numbers are of eleven bits or fewer themselves (bfloat16)
+  __device__ __forceinline__ void step(const uint32_t (&ah)[4], const uint32_t (&al)[4], float b0, float b1) {
+    const float zero[4] = {};
+    float d[4];
+    mma_tf32(d, ah, __float_as_uint(b0), __float_as_uint(b1), zero);
+    mma_tf32(small[1], al, __float_as_uint(b0), __float_as_uint(b1), small[1]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sum[e] += d[e];
+  }
+  __device__ __forceinline__ float total(int e) const { return sum[e] + (small[0][e] + small[1][e]); }
+};
+// a fragment of the left operand: this lane's number, ``down`` for the row eight further, ``along`` for the place four further
+__device__ __forceinline__ void load_rows(const float* a, int down, int along, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const Split v = split(a[(e & 1) * down + (e >> 1) * along]);
+    hi[e] = v.hi;
+    lo[e] = v.lo;
+  }
+}
+
+}  // namespace terms

@@ -1092,6 +1092,19 @@ DELTA_LONG_PORTION = 32  # steps whose longest portion has this many tokens take
 DELTA_LONG_LANES = 16   # measured: 32 lanes (a column a warp) took 807 us for a 2,048-token portion with 16 heads of 128 x 128, 16 lanes 716
 
 
+# Portions of this many tokens take the form that works 32 tokens at a time (keys of up to 128 numbers).  Width 2,048, one portion of 47
+# tokens: 41 us token by token; of 48: 21 in chunks.
+DELTA_CHUNKED = 40
+
+
+def _has_portions_below(ctx, tokens: int) -> bool:
+    """Whether a step with a portion of at least ``tokens`` tokens has shorter ones as well (True where the host does not know)."""
+    items = getattr(ctx, "items", None)
+    if items is None:
+        return ctx.num_items > 1
+    return any(it.end - it.start < tokens for it in items)
+
+
 def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
                gain: torch.Tensor, state: torch.Tensor, ctx, *, groups: int, heads: int, dim: int, vdim: int, eps: float) -> torch.Tensor:
     """The gated delta rule over every portion of the step.  proj [T, 2*groups*dim + 2*heads*vdim] (queries, keys,
@@ -1111,6 +1124,10 @@ def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: 
         if x.dtype != torch.float32 or x.numel() != n or not x.is_cuda or not x.is_contiguous():
             raise KernelError(f"delta rule: {what} must be float32 with {n} numbers on the device")
     dev = proj.device
+    # Long portions go in chunks; what is left, if anything can be, token by token.  Which of the two a portion takes depends on
+    # its own length only.
+    record = int(lib().psb_delta_chunk_record(dim, vdim)) if ctx.max_new_tokens >= DELTA_CHUNKED else 0
+    short = not record or _has_portions_below(ctx, DELTA_CHUNKED)
     qkv = torch.empty((t, c), dtype=torch.float32, device=dev)
     bd = torch.empty((t, 5 * heads), dtype=torch.float32, device=dev)   # beta, decay and three state-free dot products per head
     positions, token_item = _i32(ctx.positions, "positions"), _i32(ctx.token_item, "token-to-item map")
@@ -1118,12 +1135,22 @@ def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: 
     check(lib().psb_delta_prepare(proj.data_ptr(), _code(proj, "projection output"), proj.shape[1], 0, ba.data_ptr(), None, taps.data_ptr(), a_log.data_ptr(),
                                   dt_bias.data_ptr(), state.data_ptr(), positions.data_ptr(), token_item.data_ptr(),
                                   item_start.data_ptr(), slots.data_ptr(), qkv.data_ptr(), bd.data_ptr(), t, groups, heads, dim, vdim,
-                                  k, state.shape[0], slot_floats, _stream()), "delta_prepare")
+                                  k, state.shape[0], slot_floats, 1 if short else 0, _stream()), "delta_prepare")
     o = torch.empty((t, heads, vdim), dtype=torch.float32, device=dev)
-    lanes = DELTA_LONG_LANES if ctx.max_new_tokens >= DELTA_LONG_PORTION and dim >= DELTA_LONG_LANES else 4
-    check(lib().psb_delta_rule(qkv.data_ptr(), bd.data_ptr(), proj.data_ptr(), _code(proj, "projection output"), state.data_ptr(),
-                               item_start.data_ptr(), slots.data_ptr(), o.data_ptr(), ctx.num_items, groups, heads, dim, vdim, k,
-                               state.shape[0], slot_floats, lanes, _stream()), "delta_rule")
+    most = 0x7fffffff  # tokens of the longest portion left to the kernel that goes token by token
+    if record:
+        most = DELTA_CHUNKED - 1
+        chunks = t // lib().psb_delta_chunk_tokens() + ctx.num_items
+        records = torch.empty((chunks, heads, record), dtype=torch.float32, device=dev)
+        check(lib().psb_delta_chunks(qkv.data_ptr(), bd.data_ptr(), proj.data_ptr(), _code(proj, "projection output"), proj.shape[1],
+                                     state.data_ptr(), item_start.data_ptr(), slots.data_ptr(), records.data_ptr(), o.data_ptr(),
+                                     ctx.num_items, chunks, DELTA_CHUNKED, groups, heads, dim, vdim, k, state.shape[0], slot_floats,
+                                     _stream()), "delta_chunks")
+    if short:
+        lanes = DELTA_LONG_LANES if min(ctx.max_new_tokens, most) >= DELTA_LONG_PORTION and dim >= DELTA_LONG_LANES else 4
+        check(lib().psb_delta_rule(qkv.data_ptr(), bd.data_ptr(), proj.data_ptr(), _code(proj, "projection output"), state.data_ptr(),
+                                   item_start.data_ptr(), slots.data_ptr(), o.data_ptr(), ctx.num_items, groups, heads, dim, vdim, k,
+                                   state.shape[0], slot_floats, lanes, most, _stream()), "delta_rule")
     out = torch.empty((t, heads * vdim), dtype=proj.dtype, device=dev)
     check(lib().psb_delta_finish(o.data_ptr(), proj.data_ptr(), _code(proj, "projection output"), gain.data_ptr(), out.data_ptr(), t,
                                  groups, heads, dim, vdim, float(eps), _stream()), "delta_finish")
@@ -1412,7 +1439,7 @@ def channel_delta_rule(proj: torch.Tensor, beta_at: int, decay: torch.Tensor, ta
     check(lib().psb_delta_prepare(proj.data_ptr(), code, ld, beta_at, None, None if record else decay.data_ptr(), taps.data_ptr(), None, None,
                                   state.data_ptr(), _i32(ctx.positions, "positions").data_ptr(),
                                   _i32(ctx.token_item, "token-to-item map").data_ptr(), item_start.data_ptr(), slots.data_ptr(),
-                                  qkv.data_ptr(), bd.data_ptr(), t, groups, heads, dim, vdim, k, state.shape[0], slot_floats, _stream()),
+                                  qkv.data_ptr(), bd.data_ptr(), t, groups, heads, dim, vdim, k, state.shape[0], slot_floats, 1, _stream()),
           "delta_prepare")
     o = torch.empty((t, heads, vdim), dtype=torch.float32, device=dev)
     if record:

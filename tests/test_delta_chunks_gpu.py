@@ -1,0 +1,80 @@
+"""The gated delta rule over long portions, which works 32 tokens at a time, against the recurrence in float64: portions at and
+around multiples of a chunk beside short ones and single tokens, one after the other from carried states, keys and values of
+fewer numbers than the kernels' runs, tokens that forget everything and tokens that forget nothing."""
+
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def step(lengths, starts):
+    positions, item_of, offsets = [], [], [0]
+    for i, (n, s) in enumerate(zip(lengths, starts)):
+        positions += range(s, s + n)
+        item_of += [i] * n
+        offsets.append(offsets[-1] + n)
+    dev = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    return types.SimpleNamespace(positions=dev(positions), token_item=dev(item_of), item_start=dev(offsets),
+                                 slots=dev(list(range(len(lengths)))[::-1]), num_items=len(lengths), max_new_tokens=max(lengths))
+
+
+def conv_silu(p, taps, before, start):
+    k = taps.shape[1]
+    before = torch.stack([r if start - (k - 1) + i >= 0 else torch.zeros_like(r) for i, r in enumerate(before)]) if k > 1 else before
+    x = torch.cat([before, p])
+    return torch.nn.functional.silu(sum(x[j: j + p.shape[0]] * taps[:, j] for j in range(k))), x[len(x) - (k - 1):]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("groups, heads, dim, vdim, taps", [(2, 4, 128, 128, 4), (1, 3, 100, 36, 2), (1, 1, 4, 4, 1), (3, 3, 64, 20, 4)])
+def test_long_portions(dtype, groups, heads, dim, vdim, taps):
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import kernels, library
+    assert kernels.DELTA_CHUNKED == 40
+    g = torch.Generator(device="cuda").manual_seed(dim + vdim)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    c = 2 * groups * dim + heads * vdim
+    unit = lambda x: x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6)
+    conv, gain = 0.6 * rnd(c, taps), 1 + 0.1 * rnd(vdim)
+    a_log, dt_bias = rnd(heads) - 1, rnd(heads) - 1
+    state = 0.3 * rnd(7, (taps - 1) * c + heads * dim * vdim)
+    exact = state.double()
+    lengths, starts = [40, 64, 1, 97, 33, 39, 160], [0, 5, 9, 2, 0, 1, 100]
+    for turn in range(2):
+        ctx, t = step(lengths, starts), sum(lengths)
+        proj, ba = rnd(t, c + heads * vdim).to(dtype), rnd(t, 2 * heads)
+        ba[::7, heads:] = 1e4     # decay 0
+        ba[3::11, heads:] = -1e4  # decay 1
+        ba[5::13, :heads] = 1e4   # written in full
+        before = library.launch_counts.copy()
+        out = ops.delta_rule(proj, ba, conv, a_log, dt_bias, gain, state, ctx, groups=groups, heads=heads, dim=dim, vdim=vdim, eps=1e-5)
+        taken = library.launch_counts - before
+        assert taken["delta_chunks"] == 1 and taken["delta_rule"] == 1
+        at = 0
+        for i, (n, s) in enumerate(zip(lengths, starts)):
+            slot = len(lengths) - 1 - i
+            p = proj[at: at + n].double()
+            u, tail = conv_silu(p[:, :c], conv.double(), exact[slot, : (taps - 1) * c].view(taps - 1, c), s)
+            q, k = (unit(u[:, a: a + groups * dim].view(n, groups, dim)).repeat_interleave(heads // groups, 1) for a in (0, groups * dim))
+            v = u[:, 2 * groups * dim:].view(n, heads, vdim)
+            beta = torch.sigmoid(ba[at: at + n, :heads].double())
+            decay = torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(ba[at: at + n, heads:].double() + dt_bias.double()))
+            m, o = exact[slot, (taps - 1) * c:].view(heads, dim, vdim), []
+            for j in range(n):
+                m = m * decay[j, :, None, None]
+                m = m + k[j, :, :, None] * (beta[j, :, None] * (v[j] - torch.einsum("hd,hdv->hv", k[j], m)))[:, None]
+                o.append(torch.einsum("hd,hdv->hv", q[j] * dim ** -0.5, m))
+            o = torch.stack(o)
+            want = o / torch.sqrt((o * o).mean(-1, keepdim=True) + 1e-5) * gain.double() * torch.nn.functional.silu(p[:, c:]).view(n, heads, vdim)
+            exact[slot, : (taps - 1) * c], exact[slot, (taps - 1) * c:] = tail.reshape(-1), m.reshape(-1)
+            got = out[at: at + n].double().view(n, heads, vdim)
+            # float32 sums of up to 128 products of numbers around one, divided by a root mean square that may be small; the
+            # result in the compute type
+            tol = 1e-4 + (0 if dtype == torch.float32 else 2.0 ** -8) * want.abs()
+            assert ((got - want).abs() <= tol).all(), (turn, i, (got - want).abs().max())
+            at += n
+        assert torch.allclose(state.double(), exact, atol=2e-5), (turn, (state.double() - exact).abs().max())
+        starts = [s + n for s, n in zip(starts, lengths)]

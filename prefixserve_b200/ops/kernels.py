@@ -944,6 +944,11 @@ BIASED_BLOCKS_WANTED = 2368
 # ... and of bfloat16 ones whose sizes its tensor-core kernel takes: blocks of (token, key/value head, share of the keys) to aim at
 ROWS_SINGLE = True
 ROWS_BLOCKS_WANTED = 592
+# ... and heads of 128, at most eight to a key/value head: the kernel fed by the TMA unit.  Its blocks cost, beside their keys, about
+# what ROWS_DECODE_BLOCK_SHARE keys do.
+ROWS_DECODE = True
+ROWS_DECODE_KEYS_PER_SPLIT = 128
+ROWS_DECODE_BLOCK_SHARE = 128
 
 
 def biased_attention(qkv: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, ctx, *, num_heads: int, num_kv_heads: int,
@@ -1020,6 +1025,20 @@ def attention_over_rows(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, 
             keys = min(keys, chk)
         if (both16 and ROWS_SINGLE and kv.data_ptr() % 16 == 0 and q.data_ptr() % 4 == 0
                 and bool(lib().psb_attention_rows_single_supported(num_heads, num_kv_heads, dim, vdim))):
+            if (ROWS_DECODE and kv.data_ptr() % 16 == 0
+                    and bool(lib().psb_attention_rows_decode_supported(num_heads, num_kv_heads, dim, vdim, page_size))):
+                from .tensorcore import _sms
+                splits = _rows_splits(t * num_kv_heads, keys, lib().psb_attention_rows_decode_blocks() * _sms(q.device), 16,
+                                      ROWS_DECODE_KEYS_PER_SPLIT, ROWS_DECODE_BLOCK_SHARE)
+                partial = torch.empty((t, num_heads, splits, vdim + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
+                check(lib().psb_attention_rows_decode(q.data_ptr(), kv.data_ptr(), kv.shape[0], table.data_ptr(), table.shape[1],
+                                                      positions.data_ptr(), token_item.data_ptr(), _ptr(bias), _ptr(sink), out.data_ptr(), t,
+                                                      num_heads, num_kv_heads, dim, vdim, page_size, win, chk, reach, float(scale), keep_first,
+                                                      _ptr(partial), splits, *tail, _stream()), "attention_rows_single")
+                if splits > 1:
+                    check(lib().psb_attention_rows_merge(partial.data_ptr(), _ptr(sink), out.data_ptr(), t, num_heads, vdim, splits, *tail[:4],
+                                                         _stream()), "attention_rows_merge")
+                return out
             blocks = t * num_kv_heads * -(-(num_heads // num_kv_heads) // 16)
             splits = max(1, min(16, -(-ROWS_BLOCKS_WANTED // max(blocks, 1)), keys // 128))
             partial = torch.empty((t, num_heads, splits, vdim + 2), dtype=torch.float32, device=q.device) if splits > 1 else None

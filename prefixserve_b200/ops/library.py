@@ -195,6 +195,15 @@ _SIGNATURES: dict[str, list] = {
     #  page_size, window, chunk, reach, scale, keep_first, gate, ldg, ldo, out_scale, softcap, whole, ranges, part_o, part_ml, stream)
     "psb_attention_rows_tcgen05": [P, P, L, P, I, P, P, I, I, I, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P, L, L, F, F, I, I, P, P, P],
     "psb_attention_rows_tcgen05_status": [],
+    # (hq, hkv, dim, vdim, page_size) -> 1 if the TMA-fed kernel for single tokens takes them; () -> its blocks an SM holds
+    "psb_attention_rows_decode_supported": [I, I, I, I, I],
+    "psb_attention_rows_decode_blocks": [],
+    # (q, kv, num_pages, table, table_width, positions, token_item, bias, sink, out, T, hq, hkv, dim, vdim, page_size, window, chunk, reach,
+    #  scale, keep_first, partial, splits, gate, ldg, ldo, out_scale, softcap, stream)
+    "psb_attention_rows_decode": [P, P, L, P, I, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P, I, P, L, L, F, F, P],
+    "psb_attention_rows_decode_status": [],
+    # (partial, sink, out, T, hq, vdim, splits, gate, ldg, ldo, out_scale, stream)
+    "psb_attention_rows_merge": [P, P, P, I, I, I, I, P, L, L, F, P],
     "psb_delta_max_taps": [],
     # (proj, dtype, ld, beta_at, ba, decay, taps, a_log, dt_bias, state, positions, token_item, item_start, slots, qkv_out, bd_out, T,
     #  G, H, dim, vdim, K, num_slots, slot_floats, stream)
@@ -342,10 +351,11 @@ def tcgen05_status() -> int:
     """0 unless a bounded wait inside a tcgen05 kernel ever gave up (then its results are void). Synchronises.
 
     The product's code sits in the low byte, prefill attention's in the next, the TMA-fed decode attention's in the
-    third, the few-row product's in the fourth, prefill attention's over rows in the fifth."""
+    third, the few-row product's in the fourth, prefill attention's over rows in the fifth,
+    decode attention's over rows in the sixth."""
     return (int(lib().psb_tcgen05_status()) | (int(lib().psb_attention_tcgen05_status()) << 8)
             | (int(lib().psb_attention_decode_tma_status()) << 16) | (int(lib().psb_gemm_fewrows_status()) << 24)
-            | (int(lib().psb_attention_rows_tcgen05_status()) << 32))
+            | (int(lib().psb_attention_rows_tcgen05_status()) << 32) | (int(lib().psb_attention_rows_decode_status()) << 40))
 
 
 def declare(name: str, argtypes: list) -> None:

@@ -128,20 +128,20 @@ delta_chunk_kernel(const float* __restrict__ qkv, const float* __restrict__ bd, 
     float* out = records + ((size_t)blockIdx.x * H + h) * RECORD;
     const float* mine = bd + (size_t)(t0 + min(lane, n - 1)) * BD * H + h;
     const float beta = lane < n ? mine[0] : 0.f, decay = lane < n ? mine[H] : 1.f;
-    float run = 1.f, before = 1.f, behind = 1.f;  // lane j: products over the tokens between j and i, up to j, behind j
+    Product run, before, behind;  // lane j: products over the tokens between j and i, up to j, behind j
 #pragma unroll
     for (int i = 0; i < CHUNK; ++i) {
       const float d = __shfl_sync(0xffffffffu, decay, i);
-      if (i <= lane) before *= d;
+      if (i <= lane) before.times(d);
       if (i > lane) {
-        run *= d;
-        behind *= d;
+        run.times(d);
+        behind.times(d);
       }
-      as[warp][i][lane] = i > lane ? run * kk[i][lane] : 0.f;
-      out[B_AT + i * CHUNK + lane] = i >= lane ? run * qk[i][lane] : 0.f;
+      as[warp][i][lane] = i > lane ? run.value() * kk[i][lane] : 0.f;
+      out[B_AT + i * CHUNK + lane] = i >= lane ? run.value() * qk[i][lane] : 0.f;
     }
-    out[C_AT + lane] = before;
-    out[R_AT + lane] = behind;
+    out[C_AT + lane] = before.value();
+    out[R_AT + lane] = behind.value();
     __syncwarp();
     float w[CHUNK];  // lane j: column j of W
 #pragma unroll

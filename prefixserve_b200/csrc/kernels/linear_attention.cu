@@ -17,7 +17,8 @@
 //   linear_attention_kernel<.., true>   every chunk but a portion's last: A [dim] and B [dim, vdim] from a zero state;
 //   linear_attention_starts_kernel      per portion, chunk by chunk: the state every chunk starts from (over B);
 //   linear_attention_kernel<.., false>  every chunk from its start, with read-outs; the last one leaves the slot's state.
-// A portion of one chunk takes the last kernel alone, from and to the slot.
+// A portion of one chunk takes the last kernel alone, from and to the slot.  Long portions of the usual sizes go through the kernels of
+// linear_attention_chunks.cu instead.
 //
 // normed_readout_kernel (a warp per token and head): o / sqrt(mean(o^2) + eps) * gain[vdim] * gate, rounded to the compute
 // type; the gate is read as it is, through silu or through a sigmoid; the gain is shared by the heads or each head has its own.
@@ -35,10 +36,11 @@ __device__ __forceinline__ void la_commit() { asm volatile("cp.async.commit_grou
 __device__ __forceinline__ void la_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // The chunk a block works on: chunks are numbered through the step's items in order.  False beyond the last.
-__device__ __forceinline__ bool find_chunk(const int32_t* __restrict__ item_start, int items, int chunk, int at, int& item, int& t0,
-                                           int& t1, bool& only, bool& last) {
+__device__ __forceinline__ bool find_chunk(const int32_t* __restrict__ item_start, int items, int chunk, int max_tokens, int at, int& item,
+                                           int& t0, int& t1, bool& only, bool& last) {
   for (int i = 0; i < items; ++i) {
     const int a = item_start[i], b = item_start[i + 1];
+    if (b - a > max_tokens) continue;
     const int n = (b - a + chunk - 1) / chunk;
     if (at < n) {
       item = i;
@@ -91,7 +93,7 @@ __global__ void __launch_bounds__(LA_WARPS * 32)
 linear_attention_kernel(const T* __restrict__ proj, long long ld, const float* __restrict__ alpha, float* __restrict__ state,
                         long long slot_floats, const int32_t* __restrict__ item_start, const int32_t* __restrict__ slots,
                         float* __restrict__ local_b, float* __restrict__ local_a, float* __restrict__ o, int items, int H, int dim,
-                        int vdim, int num_slots, int chunk, float scale) {
+                        int vdim, int num_slots, int chunk, int max_tokens, float scale) {
   using Z = LaSizes<T, PER, R, NC>;
   constexpr int RP = Z::RP, BC = Z::BC, EPP = 16 / (int)sizeof(T);  // EPP: elements of a 16-byte piece
   extern __shared__ __align__(16) unsigned char staged[];  // [2][LA_STAGE] tokens; zeros beyond dim and vdim
@@ -99,7 +101,7 @@ linear_attention_kernel(const T* __restrict__ proj, long long ld, const float* _
   pdl_wait();
   int item, t0, t1;
   bool only, last;
-  if (!find_chunk(item_start, items, chunk, blockIdx.z, item, t0, t1, only, last)) return;
+  if (!find_chunk(item_start, items, chunk, max_tokens, blockIdx.z, item, t0, t1, only, last)) return;
   if (LOCAL && last) return;
   const int h = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane % R;
@@ -332,11 +334,12 @@ normed_readout_kernel(const float* __restrict__ o, const TG* __restrict__ gate, 
 }  // namespace
 
 // (proj, dtype, ld, alpha, state, slot_floats, item_start, slots, local_b, local_a, o, items, chunks, H, dim, vdim, num_slots,
-//  chunk, scale, stream).  ``chunks``: blocks to launch, at least the number of chunks of the step's portions; local_b
+//  chunk, max_tokens, scale, stream).  Portions of more than ``max_tokens`` tokens, and their slots, are left untouched (with local_b,
+// none may be).  ``chunks``: blocks to launch, at least the number of chunks of the step's portions; local_b
 // [chunks, H, dim, vdim] and local_a [chunks, H, dim] float32 are scratch, null when no portion is longer than a chunk.
 PSB_API int psb_linear_attention(const void* proj, int dtype, long long ld, const void* alpha, void* state, long long slot_floats,
                                  const void* item_start, const void* slots, void* local_b, void* local_a, void* o, int items,
-                                 int chunks, int H, int dim, int vdim, int num_slots, int chunk, float scale, cudaStream_t stream) {
+                                 int chunks, int H, int dim, int vdim, int num_slots, int chunk, int max_tokens, float scale, cudaStream_t stream) {
   if (items < 0 || H < 1 || dim < 1 || vdim < 1 || chunk < 1 || num_slots < 1) PSB_REFUSE("linear_attention: bad sizes H=%d dim=%d vdim=%d", H, dim, vdim);
   if (ld < 2LL * H * dim + (long long)H * vdim) PSB_REFUSE("linear_attention: row stride %lld is shorter than the row", ld);
   if (slot_floats < (long long)H * dim * vdim) PSB_REFUSE("linear_attention: a slot of %lld numbers does not hold the state", slot_floats);
@@ -363,7 +366,7 @@ PSB_API int psb_linear_attention(const void* proj, int dtype, long long ld, cons
     if (local_b) {                                                                                                                \
       psb_launch(local, grid, dim3(LA_WARPS * 32), smem, stream, (const T*)proj, ld, (const float*)alpha, (float*)state,          \
                  slot_floats, (const int32_t*)item_start, (const int32_t*)slots, (float*)local_b, (float*)local_a, (float*)o,     \
-                 items, H, dim, vdim, num_slots, chunk, scale);                                                                   \
+                 items, H, dim, vdim, num_slots, chunk, max_tokens, scale);                                                       \
       PSB_LAUNCH_CHECK("linear_attention");                                                                                       \
       const long long per = (long long)H * dim * vdim;                                                                            \
       psb_launch(linear_attention_starts_kernel, dim3((unsigned)((per + 255) / 256), items), dim3(256), 0, stream,                \
@@ -373,7 +376,7 @@ PSB_API int psb_linear_attention(const void* proj, int dtype, long long ld, cons
     }                                                                                                                             \
     psb_launch(whole, grid, dim3(LA_WARPS * 32), smem, stream, (const T*)proj, ld, (const float*)alpha, (float*)state,            \
                slot_floats, (const int32_t*)item_start, (const int32_t*)slots, (float*)local_b, (float*)local_a, (float*)o,       \
-               items, H, dim, vdim, num_slots, chunk, scale);                                                                     \
+               items, H, dim, vdim, num_slots, chunk, max_tokens, scale);                                                           \
     PSB_LAUNCH_CHECK("linear_attention");                                                                                         \
   } while (0)
   PSB_DISPATCH_DTYPE(dtype, T, {

@@ -15,34 +15,50 @@ __device__ __forceinline__ Split split(float x) {
   const uint32_t hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
   return {hi, __float_as_uint(x - __uint_as_float(hi))};  // (the instruction does not look at lo's last 13 bits)
 }
+// ... with half of lo's last place added, so that what the instruction cuts off is centred; of a product, without rounding it first
+__device__ __forceinline__ Split split_centred(float x, float factor = 1.f) {
+  const uint32_t hi = (__float_as_uint(x * factor) + 0x1000u) & 0xffffe000u;
+  return {hi, __float_as_uint(fmaf(x, factor, -__uint_as_float(hi)) * (1.f + 0x1.6p-12f))};
+}
 __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const float (&c)[4]) {
   asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
                : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
 }
-// One step of eight terms: sum += hi hi (rounded to nearest), small += hi lo + lo hi.
-struct Sum {
-  float sum[4] = {}, small[2][4] = {};
-  __device__ __forceinline__ void step(const uint32_t (&ah)[4], const uint32_t (&al)[4], Split b0, Split b1) {
+// One step of eight terms: sum += hi hi (rounded to nearest), small += hi lo + lo hi.  Long sums go in several chains, which lose less.
+template <int CHAINS>
+struct Sums {
+  float sum[CHAINS][4] = {}, small[2][4] = {};
+  __device__ __forceinline__ void step(const uint32_t (&ah)[4], const uint32_t (&al)[4], Split b0, Split b1, int chain = 0) {
     const float zero[4] = {};
     float d[4];
     mma_tf32(d, ah, b0.hi, b1.hi, zero);
     mma_tf32(small[0], ah, b0.lo, b1.lo, small[0]);
     mma_tf32(small[1], al, b0.hi, b1.hi, small[1]);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) sum[e] += d[e];
+    for (int e = 0; e < 4; ++e) sum[chain][e] += d[e];
   }
   // the right operand's numbers are of eleven bits or fewer themselves (bfloat16)
-  __device__ __forceinline__ void step(const uint32_t (&ah)[4], const uint32_t (&al)[4], float b0, float b1) {
+  __device__ __forceinline__ void step(const uint32_t (&ah)[4], const uint32_t (&al)[4], float b0, float b1, int chain = 0) {
     const float zero[4] = {};
     float d[4];
     mma_tf32(d, ah, __float_as_uint(b0), __float_as_uint(b1), zero);
     mma_tf32(small[1], al, __float_as_uint(b0), __float_as_uint(b1), small[1]);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) sum[e] += d[e];
+    for (int e = 0; e < 4; ++e) sum[chain][e] += d[e];
   }
-  __device__ __forceinline__ float total(int e) const { return sum[e] + (small[0][e] + small[1][e]); }
+  __device__ __forceinline__ float total(int e) const {
+    float s[CHAINS];
+#pragma unroll
+    for (int c = 0; c < CHAINS; ++c) s[c] = sum[c][e];
+#pragma unroll
+    for (int n = CHAINS / 2; n > 0; n >>= 1)
+#pragma unroll
+      for (int c = 0; c < n; ++c) s[c] += s[c + n];
+    return s[0] + (small[0][e] + small[1][e]);
+  }
 };
+using Sum = Sums<1>;
 // a fragment of the left operand: this lane's number, ``down`` for the row eight further, ``along`` for the place four further
 __device__ __forceinline__ void load_rows(const float* a, int down, int along, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
 #pragma unroll
@@ -52,5 +68,16 @@ __device__ __forceinline__ void load_rows(const float* a, int down, int along, u
     lo[e] = v.lo;
   }
 }
+
+// A running product of decays with what its roundings lose carried along, rounded once where it is read.
+struct Product {
+  float hi = 1.f, lo = 0.f;
+  __device__ __forceinline__ void times(float a) {
+    const float p = hi * a;
+    lo = fmaf(lo, a, fmaf(hi, a, -p));
+    hi = p;
+  }
+  __device__ __forceinline__ float value() const { return hi + lo; }
+};
 
 }  // namespace terms

@@ -1327,7 +1327,12 @@ def low_rank(a: torch.Tensor, w: torch.Tensor, function: str, *, bias: torch.Ten
     return out
 
 
-LINEAR_ATTENTION_CHUNK = 64  # steps whose longest portion exceeds two of these cut their portions into chunks that run side by side
+# Steps with a portion of LINEAR_CHUNKED tokens take the kernels that work 64 tokens at a time on the tensor cores, where the sizes are
+# theirs, for portions of LINEAR_SHORT tokens and more; shorter ones go token by token beside them (30 us for one chunk against 29 for 64
+# tokens one by one and 44 for 100, 16 heads of 128; and up to 14 us for what stays).  In other steps a longest portion of more than two
+# LINEAR_ATTENTION_CHUNK cuts the portions into chunks that go token by token side by side.
+LINEAR_CHUNKED, LINEAR_SHORT = 96, 32
+LINEAR_ATTENTION_CHUNK = 64
 
 
 def linear_attention(proj: torch.Tensor, alpha: torch.Tensor, state: torch.Tensor, ctx, *, heads: int, dim: int, vdim: int) -> torch.Tensor:
@@ -1343,7 +1348,22 @@ def linear_attention(proj: torch.Tensor, alpha: torch.Tensor, state: torch.Tenso
     stride = _slot_rows(state, heads * dim * vdim, "linear attention state")
     dev = proj.device
     o = torch.empty((t, heads, vdim), dtype=torch.float32, device=dev)
-    chunked = ctx.max_new_tokens > 2 * LINEAR_ATTENTION_CHUNK
+    ld = int(proj.stride(0)) if t > 1 else max(int(proj.stride(0)), proj.shape[1])
+    most = 0x7fffffff  # tokens of the longest portion left to the kernels that go token by token
+    if (ctx.max_new_tokens >= LINEAR_CHUNKED and proj.dtype == torch.bfloat16 and ld % 4 == 0 and stride % 4 == 0
+            and proj.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0 and alpha.data_ptr() % 16 == 0
+            and bool(lib().psb_linear_chunks_supported(dim, vdim))):
+        most = LINEAR_SHORT - 1
+        chunks = t // lib().psb_linear_chunk_tokens() + ctx.num_items
+        local_b = torch.empty((chunks, heads, dim, vdim), dtype=torch.float32, device=dev)
+        local_a = torch.empty((chunks, heads, dim), dtype=torch.float32, device=dev)
+        check(lib().psb_linear_chunks(proj.data_ptr(), ld, alpha.data_ptr(), state.data_ptr(), stride,
+                                      _i32(ctx.item_start, "item offsets").data_ptr(), _i32(ctx.slots, "slots").data_ptr(), local_b.data_ptr(),
+                                      local_a.data_ptr(), o.data_ptr(), ctx.num_items, chunks, LINEAR_SHORT, heads, dim, vdim,
+                                      state.shape[0], dim ** -0.5, _stream()), "linear_attention_chunks")
+        if not _has_portions_below(ctx, LINEAR_SHORT):
+            return o
+    chunked = most > LINEAR_SHORT and ctx.max_new_tokens > 2 * LINEAR_ATTENTION_CHUNK
     chunk = LINEAR_ATTENTION_CHUNK if chunked else max(t, 1)
     chunks = ctx.num_items
     local_b = local_a = None
@@ -1351,10 +1371,10 @@ def linear_attention(proj: torch.Tensor, alpha: torch.Tensor, state: torch.Tenso
         chunks = t // chunk + ctx.num_items
         local_b = torch.empty((chunks, heads, dim, vdim), dtype=torch.float32, device=dev)
         local_a = torch.empty((chunks, heads, dim), dtype=torch.float32, device=dev)
-    check(lib().psb_linear_attention(proj.data_ptr(), _code(proj, "projection output"), int(proj.stride(0)) if t > 1 else max(int(proj.stride(0)), proj.shape[1]),
+    check(lib().psb_linear_attention(proj.data_ptr(), _code(proj, "projection output"), ld,
                                      alpha.data_ptr(), state.data_ptr(), stride, _i32(ctx.item_start, "item offsets").data_ptr(),
                                      _i32(ctx.slots, "slots").data_ptr(), _ptr(local_b), _ptr(local_a), o.data_ptr(), ctx.num_items,
-                                     chunks, heads, dim, vdim, state.shape[0], chunk, dim ** -0.5, _stream()), "linear_attention")
+                                     chunks, heads, dim, vdim, state.shape[0], chunk, most, dim ** -0.5, _stream()), "linear_attention")
     return o
 
 

@@ -1,0 +1,54 @@
+"""Gated linear attention over long portions, 64 tokens at a time, against the recurrence in float64: portions at and around multiples of
+a chunk and of its runs of 16 tokens beside short ones and single tokens, one after the other from carried states, keys and values of
+fewer numbers than the kernels' tiles, channels that forget everything and channels that forget nothing, rows and slots that are runs of
+wider ones.  (Projections in float32 stay with the kernels that go token by token.)"""
+
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads, dim, vdim", [(2, 128, 128), (3, 100, 36), (1, 4, 4), (2, 64, 96)])
+def test_long_portions(dtype, heads, dim, vdim):
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import kernels, library
+    assert kernels.LINEAR_CHUNKED <= 193 and kernels.LINEAR_SHORT == 32
+    g = torch.Generator(device="cuda").manual_seed(dim + vdim)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    lengths = [64, 65, 1, 127, 31, 32, 63, 193]
+    dev = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    offsets = [0]
+    for n in lengths:
+        offsets.append(offsets[-1] + n)
+    ctx = types.SimpleNamespace(item_start=dev(offsets), slots=dev(list(range(len(lengths)))[::-1]), num_items=len(lengths), max_new_tokens=max(lengths))
+    held = rnd(len(lengths), heads * dim * vdim + 8)
+    state = held[:, : heads * dim * vdim]
+    exact, t, width = state.double().clone(), sum(lengths), heads * (2 * dim + vdim)
+    for turn in range(2):
+        wide = rnd(t, width + 12).to(dtype)
+        alpha = torch.sigmoid(rnd(t, heads * dim)) ** (1 / 4)
+        alpha[5::9, ::3] = 0.0
+        alpha[::4, 1::5] = 1.0
+        before = library.launch_counts.copy()
+        out = ops.linear_attention(wide[:, : width + 8], alpha, state, ctx, heads=heads, dim=dim, vdim=vdim)
+        taken = library.launch_counts - before
+        assert taken["linear_attention_chunks"] == (dtype == torch.bfloat16) and taken["linear_attention"] == 1
+        for i, n in enumerate(lengths):
+            run, slot = slice(offsets[i], offsets[i] + n), len(lengths) - 1 - i
+            p = wide[run].double()
+            q, k = (p[:, a: a + heads * dim].view(n, heads, dim) for a in (0, heads * dim))
+            v, a = p[:, 2 * heads * dim: width].view(n, heads, vdim), alpha[run].double().view(n, heads, dim, 1)
+            m, o = exact[slot].view(heads, dim, vdim), []
+            for j in range(n):
+                m = a[j] * m + k[j, :, :, None] * v[j, :, None]
+                o.append(torch.einsum("hd,hdv->hv", q[j], m) * dim ** -0.5)
+            exact[slot] = m.reshape(-1)
+            # float32 sums of some hundred products of numbers around one
+            err = (out[run].double() - torch.stack(o)).abs().max()
+            assert err <= 2e-5 * max(1.0, float(torch.stack(o).abs().max())), (turn, i, err)
+        assert torch.allclose(state.double(), exact, rtol=1e-5, atol=2e-5), (turn, (state.double() - exact).abs().max())
+        assert state.data_ptr() == held.data_ptr()

@@ -1111,9 +1111,10 @@ DELTA_LONG_PORTION = 32  # steps whose longest portion has this many tokens take
 DELTA_LONG_LANES = 16   # measured: 32 lanes (a column a warp) took 807 us for a 2,048-token portion with 16 heads of 128 x 128, 16 lanes 716
 
 
-# Portions of this many tokens take the form that works 32 tokens at a time (keys of up to 128 numbers).  Width 2,048, one portion of 47
-# tokens: 41 us token by token; of 48: 21 in chunks.
-DELTA_CHUNKED = 40
+# Portions of this many tokens take the form that works 32 tokens at a time (keys of up to 128 numbers).  All four kernels, 16 heads over 8
+# groups of 128: one portion of 8 tokens 25 us in chunks and 37 token by token, of 32 tokens 28 and 44; three of 24 and fewer 37 and 63.
+# (Portions on both sides of the line pay for both: 8, 6 and 5 tokens 58 us instead of 41.)
+DELTA_CHUNKED = 8
 
 
 def _has_portions_below(ctx, tokens: int) -> bool:

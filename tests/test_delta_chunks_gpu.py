@@ -33,7 +33,7 @@ def conv_silu(p, taps, before, start):
 def test_long_portions(dtype, groups, heads, dim, vdim, taps):
     from prefixserve_b200 import ops
     from prefixserve_b200.ops import kernels, library
-    assert kernels.DELTA_CHUNKED == 40
+    assert kernels.DELTA_CHUNKED == 8
     g = torch.Generator(device="cuda").manual_seed(dim + vdim)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
     c = 2 * groups * dim + heads * vdim
@@ -42,7 +42,7 @@ def test_long_portions(dtype, groups, heads, dim, vdim, taps):
     a_log, dt_bias = rnd(heads) - 1, rnd(heads) - 1
     state = 0.3 * rnd(7, (taps - 1) * c + heads * dim * vdim)
     exact = state.double()
-    lengths, starts = [40, 64, 1, 97, 33, 39, 160], [0, 5, 9, 2, 0, 1, 100]
+    lengths, starts = [8, 64, 1, 97, 33, 7, 160], [0, 5, 9, 2, 0, 1, 100]
     for turn in range(2):
         ctx, t = step(lengths, starts), sum(lengths)
         proj, ba = rnd(t, c + heads * vdim).to(dtype), rnd(t, 2 * heads)

@@ -1,6 +1,6 @@
 """The gated delta rule over long portions, which works 32 tokens at a time, against the recurrence in float64: portions at and
 around multiples of a chunk beside short ones and single tokens, one after the other from carried states, keys and values of
-fewer numbers than the kernels' runs, tokens that forget everything and tokens that forget nothing."""
+fewer numbers than the kernels' runs (and enough of them for the wide kernels around the rule), tokens that forget everything and tokens that forget nothing."""
 
 import types
 
@@ -29,7 +29,7 @@ def conv_silu(p, taps, before, start):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("groups, heads, dim, vdim, taps", [(2, 4, 128, 128, 4), (1, 3, 100, 36, 2), (1, 1, 4, 4, 1), (3, 3, 64, 20, 4)])
+@pytest.mark.parametrize("groups, heads, dim, vdim, taps", [(2, 4, 128, 128, 4), (2, 6, 100, 36, 2), (1, 1, 4, 4, 1), (3, 3, 64, 20, 4), (1, 34, 8, 12, 3)])
 def test_long_portions(dtype, groups, heads, dim, vdim, taps):
     from prefixserve_b200 import ops
     from prefixserve_b200.ops import kernels, library

@@ -31,11 +31,12 @@
 // reads (``row_weight``, by row: the first product is linear, so the weight may as well multiply its sums) and one otherwise.
 //
 // moe_mma_kernel: the same product for bfloat16 operands on the tensor cores (mma.sync m16n8k16, float32 sums).
-// moe_fewrows_kernel: the same for steps with no more than four rows an expert on average (see there).
+// moe_fewrows_kernel: the same for steps with no more than eight rows an expert on average (see there).
 //
 // moe_combine_kernel: out[t] = sum over slots of weight[t, slot] * Y[pair_row[t, slot]]  (+ sigmoid(gate[t]) *
 // shared[t] for a shared expert that every token uses), float32 sums in slot order, rounded to the compute type; without
 // weights the rows are added as they are.
+#include <algorithm>
 #include <cfloat>
 
 #include "common.cuh"
@@ -394,32 +395,96 @@ moe_mma_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restr
   }
 }
 
-// A handful of rows per expert (decoding): what matters is that every chosen expert's matrix is read once, as fast as
-// memory gives it.  A block takes one expert and a slab of 32 output columns; the expert's rows (four at a time) lie in
-// shared memory as bfloat16; a warp takes four of the columns in turn, its lanes along K with 16-byte loads of the
-// weight rows, four sums per column finished by butterflies.  An expert without rows costs its blocks one look-up.
-constexpr int FEW_ROWS = 4, FEW_WARPS = 8, FEW_COLS = 32;  // four rows at a time: few registers, three blocks an SM
+// Some rows per expert (decoding): what matters is that every chosen expert's matrix is read once, as fast as memory gives it.
+// The work is cut into units of an expert, eight of its rows and a slab of 32 output columns; two blocks an SM take equal runs of
+// units, expert by expert, so that rows are staged once per expert and no block is left over at the end.  In a unit a warp takes 16
+// columns and every fourth 128 of K.  mma.sync m16n8k16 with the weights as the left operand: which k an instruction's places stand
+// for is free as long as both operands agree, so a lane's 16 bytes of a weight row, and the same 16 of a token's, are the places of two
+// instructions, straight out of memory.  A warp asks for its next 128 of K, and at the end of a unit for the next unit's first ones,
+// before it works on the ones it has.  The four shares of K are added up in shared memory, in order.
+//
+// Bound by memory.  12 tokens of 4 of 32 gated experts (4,096 in and out, 2,048 between): 142 and 81 us, 5.8 TB/s of the matrices.  A
+// block per expert and slab on the CUDA cores, four rows at a time, took 199 and 121; a block per expert and slab with these products
+// 158 and 97 (too few turns a block to keep memory busy, and a last round of blocks).
+constexpr int FEW_ROWS = 8, FEW_WARPS = 8, FEW_COLS = 32, FEW_SHARES = 4, FEW_STEPS = 4, FEW_TURN = 32 * FEW_STEPS;
+// Up to so many pairs an expert on average: all of the layer at 4,096 and 45 tokens (5.6 an expert) 327 us and 829 with moe_mma_kernel,
+// at 2,048 and 63 tokens (7.9) 126 and 234.
+constexpr int FEW_PAIRS = 8;
+constexpr int FEW_SMEM = 192 * 1024;
+// rows lie half a line off one another, so that a lane's pieces meet every bank once
+__host__ __device__ constexpr int few_pitch(int K) { return (K + 63) / 64 * 64 + 32; }
+
+__device__ __forceinline__ void few_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
 
 template <typename TC>
-__global__ void __launch_bounds__(FEW_WARPS * 32, 3)
+__global__ void __launch_bounds__(FEW_WARPS * 32, 2)
 moe_fewrows_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ W, TC* __restrict__ C,
-                   const int32_t* __restrict__ offsets, const int32_t* __restrict__ row_pair, int N, int K, int top, int gather,
-                   int act, int glu, const GluClip clip, const float* __restrict__ row_weight) {
+                   const int32_t* __restrict__ offsets, const int32_t* __restrict__ row_pair, int E, int N, int K, int top, int gather,
+                   int act, int glu, const GluClip clip, const float* __restrict__ row_weight, int rows_at_once) {
   extern __shared__ __align__(16) unsigned char few_smem[];
-  __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(few_smem);  // [FEW_ROWS][K]
+  __shared__ float shares[2][FEW_WARPS][FEW_ROWS][16];
+  __shared__ int32_t passes[MAX_EXPERTS * (1 + FEW_PAIRS * 2 / FEW_ROWS)];  // expert and first row of every pass over a matrix
+  __shared__ int passes_n;
+  static_assert(FEW_ROWS % 2 == 0, "rows_at_once is all or half of them");
+  __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(few_smem);  // [rows_at_once][pitch]
   pdl_trigger();
-  const int expert = blockIdx.y, n0 = blockIdx.x * FEW_COLS;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const __nv_bfloat16* We = W + (size_t)expert * N * K;
+  const int pitch = few_pitch(K);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, tg = lane & 3;
+  const int share = warp & (FEW_SHARES - 1);
   pdl_wait();
-  const int row0 = offsets[expert], row1 = offsets[expert + 1];
-  for (int r0 = row0; r0 < row1; r0 += FEW_ROWS) {
-    const int m = min(FEW_ROWS, row1 - r0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < FEW_ROWS * (K / 8); i += blockDim.x) {
-      const int r = i / (K / 8), c = i - r * (K / 8);
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (r < m) {
+  if (warp == 0) {
+    int at = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane, a = e < E ? offsets[e] : 0, n = e < E ? offsets[e + 1] - a : 0;
+      const int mine = (n + rows_at_once - 1) / rows_at_once;
+      int sum = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int below = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += below;
+      }
+      for (int p = 0; p < mine; ++p) passes[at + sum - mine + p] = e | (p * rows_at_once) << 9;
+      at += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (lane == 0) passes_n = at;
+  }
+  __syncthreads();
+  const int slabs = (N + FEW_COLS - 1) / FEW_COLS;
+  const long long units = (long long)passes_n * slabs;
+  const int first = (int)(units * blockIdx.x / gridDim.x), last = (int)(units * (blockIdx.x + 1) / gridDim.x);
+  if (first >= last) return;
+  const __nv_bfloat16 *w0, *w1;  // this lane's two weight rows of the unit
+  auto aim = [&](int unit) {
+    const int e = passes[unit / slabs] & (MAX_EXPERTS - 1), n1 = unit % slabs * FEW_COLS + warp / FEW_SHARES * 16;
+    w0 = W + ((size_t)e * N + min(N - 1, n1 + gr)) * K;
+    w1 = W + ((size_t)e * N + min(N - 1, n1 + gr + 8)) * K;
+  };
+  auto fetch = [&](int k0, uint4 (&x)[FEW_STEPS][2]) {
+#pragma unroll
+    for (int u = 0; u < FEW_STEPS; ++u) {
+      const int k = k0 + 32 * u + 8 * tg;
+      x[u][0] = k < K ? __ldg(reinterpret_cast<const uint4*>(w0 + k)) : make_uint4(0, 0, 0, 0);
+      x[u][1] = k < K ? __ldg(reinterpret_cast<const uint4*>(w1 + k)) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  uint4 now[FEW_STEPS][2], next[FEW_STEPS][2];
+  aim(first);
+  fetch(share * FEW_TURN, now);
+  int staged = -1, r0 = 0, m = 0;
+  for (int unit = first; unit < last; ++unit) {
+    const int pass = unit / slabs, n0 = unit % slabs * FEW_COLS;
+    if (pass != staged) {  // (everybody is through with the rows that lie there: the barrier of the unit before)
+      staged = pass;
+      const int e = passes[pass] & (MAX_EXPERTS - 1);
+      r0 = offsets[e] + (passes[pass] >> 9);
+      m = min(rows_at_once, offsets[e + 1] - r0);
+      for (int i = threadIdx.x; i < m * (K / 8); i += blockDim.x) {
+        const int r = i / (K / 8), c = i - r * (K / 8);
+        uint4 v = make_uint4(0, 0, 0, 0);
         const int pair = row_pair[r0 + r];
         const int src = pair < 0 ? -1 : (gather ? pair / top : r0 + r);
         if (src >= 0) {
@@ -430,58 +495,46 @@ moe_fewrows_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __r
             v = reinterpret_cast<const uint4*>(A + (size_t)src * K)[c];
           }
         }
+        *reinterpret_cast<uint4*>(rows + (size_t)r * pitch + 8 * c) = v;
       }
-      reinterpret_cast<uint4*>(rows)[i] = v;
+      __syncthreads();
     }
+    float acc[2][4] = {};
+    const __nv_bfloat16* mine = rows + (size_t)min(gr, m - 1) * pitch;  // (a row that is not there: its sums are not used)
+    for (int k0 = share * FEW_TURN; k0 < K; k0 += FEW_SHARES * FEW_TURN) {
+      const bool over = k0 + FEW_SHARES * FEW_TURN >= K;
+      if (over && unit + 1 < last) aim(unit + 1);
+      fetch(!over ? k0 + FEW_SHARES * FEW_TURN : unit + 1 < last ? share * FEW_TURN : K, next);
+#pragma unroll
+      for (int u = 0; u < FEW_STEPS; ++u) {
+        const int k = k0 + 32 * u + 8 * tg;
+        const uint4 b = k < K ? *reinterpret_cast<const uint4*>(mine + k) : make_uint4(0, 0, 0, 0);
+        const uint4 a = now[u][0], e = now[u][1];
+        few_mma(acc[0], a.x, e.x, a.y, e.y, b.x, b.y);
+        few_mma(acc[1], a.z, e.z, a.w, e.w, b.z, b.w);
+      }
+#pragma unroll
+      for (int u = 0; u < FEW_STEPS; ++u) {
+        now[u][0] = next[u][0];
+        now[u][1] = next[u][1];
+      }
+    }
+    auto& buf = shares[unit & 1];
+#pragma unroll
+    for (int x = 0; x < 4; ++x)  // columns gr and gr + 8, rows 2 tg and 2 tg + 1
+      buf[warp][2 * tg + (x & 1)][gr + 8 * (x >> 1)] = acc[0][x] + acc[1][x];
     __syncthreads();
-    // a warp's four columns side by side: their pieces of the weight rows are asked for together
-    constexpr int NC = FEW_COLS / FEW_WARPS;
-    const uint4* wrow[NC];
+    {
+      const int r = threadIdx.x / FEW_COLS, n = threadIdx.x % FEW_COLS, at = n / 16 * FEW_SHARES;
+      float v = 0.f;
 #pragma unroll
-    for (int j = 0; j < NC; ++j) wrow[j] = reinterpret_cast<const uint4*>(We + (size_t)min(N - 1, n0 + warp + j * FEW_WARPS) * K);
-    float acc[NC][FEW_ROWS];
-#pragma unroll
-    for (int j = 0; j < NC; ++j)
-#pragma unroll
-      for (int r = 0; r < FEW_ROWS; ++r) acc[j][r] = 0.f;
-#pragma unroll 2
-    for (int c = lane; c < K / 8; c += 32) {
-      uint4 wraw[NC];
-#pragma unroll
-      for (int j = 0; j < NC; ++j) wraw[j] = wrow[j][c];
-      float2 af[FEW_ROWS][4];
-#pragma unroll
-      for (int r = 0; r < FEW_ROWS; ++r) {
-        const uint4 araw = reinterpret_cast<const uint4*>(rows + (size_t)r * K)[c];
-        const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&araw);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) af[r][q] = __bfloat1622float2(a2[q]);
-      }
-#pragma unroll
-      for (int j = 0; j < NC; ++j) {
-        const __nv_bfloat162* w2 = reinterpret_cast<const __nv_bfloat162*>(&wraw[j]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float2 wf = __bfloat1622float2(w2[q]);
-#pragma unroll
-          for (int r = 0; r < FEW_ROWS; ++r) {
-            acc[j][r] = fmaf(af[r][q].x, wf.x, acc[j][r]);
-            acc[j][r] = fmaf(af[r][q].y, wf.y, acc[j][r]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < NC; ++j) {
-      const int n = n0 + warp + j * FEW_WARPS;
-#pragma unroll
-      for (int r = 0; r < FEW_ROWS; ++r) {
-        const float v = warp_sum(acc[j][r]);
-        if (lane == 0 && r < m && n < N) C[(size_t)(r0 + r) * N + n] = from_float<TC>(moe_act(v, act));
-      }
+      for (int q = 0; q < FEW_SHARES; ++q) v += buf[at + q][r][n % 16];
+      if (r < m && n0 + n < N) C[(size_t)(r0 + r) * N + n0 + n] = from_float<TC>(moe_act(v, act));
     }
   }
 }
+static_assert(FEW_WARPS * 32 == FEW_ROWS * FEW_COLS && FEW_WARPS == FEW_SHARES * FEW_COLS / 16, "a thread an output");
+static_assert(MAX_EXPERTS == 1 << 9, "an expert is nine bits of a pass");
 
 PsbPerDevice fewrows_attr[2];
 
@@ -628,21 +681,26 @@ PSB_API int psb_moe_gemm(const void* a, int a_dtype, const void* w, int w_dtype,
   const long long row_tiles = (pairs + TILE - 1) / TILE + E;
   if (row_tiles > 65535) PSB_REFUSE("moe_gemm: too many rows for one launch");
   const dim3 grid((N + TILE - 1) / TILE, (unsigned)row_tiles);
-  const size_t few_smem = (size_t)FEW_ROWS * K * sizeof(__nv_bfloat16);
+  const size_t few_row = few_pitch(K) * sizeof(__nv_bfloat16);
+  const int few_rows = FEW_ROWS * few_row <= FEW_SMEM ? FEW_ROWS : FEW_ROWS / 2;
+  const size_t few_smem = few_rows * few_row;
   if (a_dtype == PSB_BF16 && w_dtype == PSB_BF16 && K % 8 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0 &&
-      pairs <= FEW_ROWS * E && few_smem <= 192 * 1024 && E <= 65535) {
-    // no more rows than four an expert on average: stream every used expert's matrix once
-    const dim3 few_grid((N + FEW_COLS - 1) / FEW_COLS, E);
+      pairs <= FEW_PAIRS * E && few_smem <= FEW_SMEM) {
+    int device = 0, sms = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const dim3 few_grid(2 * std::max(sms, 1));
     PSB_DISPATCH_DTYPE(c_dtype, TC, {
       auto kernel = moe_fewrows_kernel<TC>;
       PsbPerDevice& done = fewrows_attr[c_dtype == PSB_F32 ? 0 : 1];
-      if (few_smem > 48 * 1024 && !done.get()) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024) != cudaSuccess)
+      if (!done.get()) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM) != cudaSuccess)
           PSB_REFUSE("moe_gemm: cannot raise the shared-memory limit");
         done.set();
       }
       psb_launch(kernel, few_grid, dim3(FEW_WARPS * 32), few_smem, stream, (const __nv_bfloat16*)a, (const __nv_bfloat16*)w, (TC*)c,
-                 (const int32_t*)offsets, (const int32_t*)row_pair, N, K, top, gather, act, glu, clip, (const float*)row_weight);
+                 (const int32_t*)offsets, (const int32_t*)row_pair, E, N, K, top, gather, act, glu, clip, (const float*)row_weight,
+                 few_rows);
     });
     PSB_LAUNCH_CHECK("moe_gemm");
     return 0;

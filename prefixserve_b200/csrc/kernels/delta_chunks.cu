@@ -1,4 +1,7 @@
-// The gated delta rule over long portions, 32 tokens at a time, float32 throughout.
+// The gated delta rule over long portions of bfloat16 projections, 32 tokens at a time, float32 throughout.
+//
+// Read-outs come out at 2.0e-7 of their size from float64 and states as from the token-by-token kernel, whose read-outs lie at 1.7e-7:
+// nothing beside the rounding to bfloat16 that follows, but float32 projections stay with that kernel.
 //
 // Within a chunk, with g_l the decays, c_i = g_1 .. g_i (from the chunk's start up to token i), r_j = g_(j+1) .. g_32 and S the
 // state before the chunk, the writes u_i of its tokens are the rows of
@@ -39,8 +42,6 @@ constexpr int CHAIN_THREADS = 512, CHUNK_THREADS = 128;
 
 // a chunk's record of a head: W, B [32][32], c, r [32]
 constexpr int W_AT = 0, B_AT = CHUNK * CHUNK, C_AT = 2 * CHUNK * CHUNK, R_AT = C_AT + CHUNK, RECORD = R_AT + CHUNK;
-// ... with decays per channel: W, B, c_32 [RP], then K c, Q c and K r [32][RP]
-constexpr int KC_AT = C_AT + RP, QC_AT = KC_AT + CHUNK * RP, KRR_AT = QC_AT + CHUNK * RP, CHANNEL_RECORD = KRR_AT + CHUNK * RP;
 
 __device__ __forceinline__ bool find_chunk(const int32_t* __restrict__ item_start, int items, int min_tokens, int at, int& t0, int& n) {
   for (int i = 0; i < items; ++i) {
@@ -165,13 +166,10 @@ delta_chunk_kernel(const float* __restrict__ qkv, const float* __restrict__ bd, 
 }
 
 // ---- the chain, on the tensor cores, operands in two terms (tf32_terms.cuh) ---------------------------------------------
-// CHANNEL: decays per key channel; the record then holds K and Q times c, K times r and c_32 themselves.
-template <bool CHANNEL>
 struct ChainShape {
-  static constexpr int K_AT = 0, Q_AT = K_AT + CHUNK * KP, KR_AT = CHANNEL ? Q_AT + CHUNK * KP : K_AT;
-  static constexpr int SW_AT = (CHANNEL ? KR_AT : Q_AT) + CHUNK * KP, V_AT = SW_AT + CHUNK * TP;
+  static constexpr int K_AT = 0, Q_AT = K_AT + CHUNK * KP, SW_AT = Q_AT + CHUNK * KP, V_AT = SW_AT + CHUNK * TP;
   static constexpr int STAGE = V_AT + CHUNK * CP;                          // floats of a stage
-  static constexpr int B_SIZE = CHUNK * TP + RP;                           // B, then c and r or c_32: read one chunk longer than the rest
+  static constexpr int B_SIZE = CHUNK * TP + 2 * CHUNK;                    // B, then c and r: read one chunk longer than the rest
   static constexpr int RING_AT = 2 * STAGE, S_AT = RING_AT + 3 * B_SIZE;   // the state in (hi, lo) pairs
   static constexpr int UU_AT = S_AT + RP * 2 * SP, U_AT = UU_AT + CHUNK * 2 * SP;  // U times r in (hi, lo) pairs; U of two chunks
   static constexpr int PART_AT = U_AT + 2 * CHUNK * CP, FLOATS = PART_AT + 2 * 4 * 2 * CHUNK * CP;  // quarters of [K; Q] S, of two chunks
@@ -185,12 +183,11 @@ __device__ __forceinline__ Split load_split(const float* at) {
   const uint2 v = *reinterpret_cast<const uint2*>(at);
   return {v.x, v.y};
 }
-template <typename T, bool CHANNEL>
 __global__ void __launch_bounds__(CHAIN_THREADS, 1)
-delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ records, const T* __restrict__ proj, long long P,
+delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ records, const __nv_bfloat16* __restrict__ proj, long long P,
                    float* __restrict__ state, const int32_t* __restrict__ item_start, const int32_t* __restrict__ slots,
                    float* __restrict__ o, int min_tokens, int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats) {
-  using Sh = ChainShape<CHANNEL>;
+  using Sh = ChainShape;
   extern __shared__ __align__(16) float chain[];
   float *st = chain + Sh::S_AT, *uu = chain + Sh::UU_AT;
   const int C = 2 * G * dim + H * vdim;
@@ -211,25 +208,18 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
   slot = slot < 0 ? 0 : (slot >= num_slots ? num_slots - 1 : slot);
   float* base = state + (size_t)slot * slot_floats;
   float* S = base + (size_t)(K - 1) * C + (size_t)h * dim * vdim;
-  constexpr int REC = CHANNEL ? CHANNEL_RECORD : RECORD;
 
   auto stage = [&](int c, int thread, int threads) {
     float *buf = chain + (c & 1) * Sh::STAGE, *ring = chain + Sh::RING_AT + c % 3 * Sh::B_SIZE;
     const int ts = t0 + c * CHUNK, n = min(CHUNK, t1 - ts);
     const float* rows = qkv + (size_t)ts * C;
-    const float* record = records + ((size_t)(first + c) * H + h) * REC;
+    const float* record = records + ((size_t)(first + c) * H + h) * RECORD;
     for (int i = thread; i < CHUNK * RP / 4; i += threads) {
       const int t = i / (RP / 4), d = (i % (RP / 4)) * 4;
-      if constexpr (CHANNEL) {
-        copy_async16(buf + Sh::K_AT + t * KP + d, record + KC_AT + t * RP + d);
-        copy_async16(buf + Sh::Q_AT + t * KP + d, record + QC_AT + t * RP + d);
-        copy_async16(buf + Sh::KR_AT + t * KP + d, record + KRR_AT + t * RP + d);
-      } else {
-        const bool there = t < n && d < dim;
-        const float* src = rows + (there ? (size_t)t * C + d : 0) + (size_t)g * dim;
-        copy_async16_or_zero(buf + Sh::K_AT + t * KP + d, src + (size_t)G * dim, there);
-        copy_async16_or_zero(buf + Sh::Q_AT + t * KP + d, src, there);
-      }
+      const bool there = t < n && d < dim;
+      const float* src = rows + (there ? (size_t)t * C + d : 0) + (size_t)g * dim;
+      copy_async16_or_zero(buf + Sh::K_AT + t * KP + d, src + (size_t)G * dim, there);
+      copy_async16_or_zero(buf + Sh::Q_AT + t * KP + d, src, there);
     }
     for (int i = thread; i < CHUNK * CHUNK / 4; i += threads) {
       const int row = i / (CHUNK / 4), piece = (i % (CHUNK / 4)) * 4;
@@ -241,7 +231,7 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
       const bool there = t < n && col0 + v < vdim;
       copy_async16_or_zero(buf + Sh::V_AT + t * CP + v, rows + (there ? (size_t)t * C + 2 * (size_t)G * dim + (size_t)h * vdim + col0 + v : 0), there);
     }
-    for (int i = thread; i < (CHANNEL ? RP : 2 * CHUNK) / 4; i += threads)  // c and r, or c_32
+    for (int i = thread; i < 2 * CHUNK / 4; i += threads)  // c and r
       copy_async16(ring + CHUNK * TP + 4 * i, record + C_AT + 4 * i);
   };
   auto part_of = [&](int c) { return chain + Sh::PART_AT + (c & 1) * 4 * 2 * CHUNK * CP; };
@@ -270,7 +260,7 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
         v.x += p.x;
         v.y += p.y;
       }
-      const float ci = CHANNEL ? 1.f : ring[CHUNK * TP + i0 + 8 * r];
+      const float ci = ring[CHUNK * TP + i0 + 8 * r];
       if (t < t1 && col < vdim)
         *reinterpret_cast<float2*>(o + ((size_t)t * H + h) * vdim + col) = make_float2(fmaf(ci, v.x, y.total(2 * r)), fmaf(ci, v.y, y.total(2 * r + 1)));
     }
@@ -328,14 +318,14 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
         for (int e = 0; e < 2; ++e) {
           const int i = (8 * k + 4 * e) * CP;
           const float y = (part[i] + part[2 * CHUNK * CP + i]) + (part[4 * CHUNK * CP + i] + part[6 * CHUNK * CP + i]);
-          x[e] = split(fmaf(CHANNEL ? -1.f : -ring[CHUNK * TP + 8 * k + 4 * e + tg], y, v[i]));
+          x[e] = split(fmaf(-ring[CHUNK * TP + 8 * k + 4 * e + tg], y, v[i]));
         }
         u.step(ah, al, x[0], x[1]);
       }
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int i = i0 + 8 * r, col = uc + 2 * tg;
-        const float ri = CHANNEL ? 1.f : ring[CHUNK * TP + CHUNK + i];
+        const float ri = ring[CHUNK * TP + CHUNK + i];
         *reinterpret_cast<float2*>(u_of(c) + i * CP + col) = make_float2(u.total(2 * r), u.total(2 * r + 1));
         store_split(uu + (i * SP + col) * 2, u.total(2 * r) * ri, u.total(2 * r + 1) * ri);
       }
@@ -347,7 +337,7 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
     __syncthreads();
     {
       Sum d;
-      const float* a = buf + Sh::KR_AT + tg * KP + d0;
+      const float* a = buf + Sh::K_AT + tg * KP + d0;
       const float* b = uu + (tg * SP + 8 * (warp & 1) + gr) * 2;
 #pragma unroll
       for (int k = 0; k < CHUNK / 8; ++k) {
@@ -355,9 +345,9 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
         load_rows(a + 8 * k * KP, 8, 4 * KP, ah, al);
         d.step(ah, al, load_split(b + 8 * k * SP * 2), load_split(b + (8 * k + 4) * SP * 2));
       }
-      const float cc[2] = {ring[CHUNK * TP + (CHANNEL ? d0 : CHUNK - 1)], ring[CHUNK * TP + (CHANNEL ? d0 + 8 : CHUNK - 1)]};
+      const float all = ring[CHUNK * TP + CHUNK - 1];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) s[e] = fmaf(cc[e >> 1], s[e], d.total(e));
+      for (int e = 0; e < 4; ++e) s[e] = fmaf(all, s[e], d.total(e));
       store_split(st + (d0 * SP + sc) * 2, s[0], s[1]);
       store_split(st + ((d0 + 8) * SP + sc) * 2, s[2], s[3]);
     }
@@ -369,24 +359,7 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
     const int d = d0 + 8 * (e >> 1), col = col0 + sc + (e & 1);
     if (d < dim && col < vdim) S[(size_t)d * vdim + col] = s[e];
   }
-  if (blockIdx.x == 0 && h == 0) keep_conv_inputs<T>(proj, P, base, t0, t1, C, K);
-}
-
-template <typename T, bool CHANNEL>
-int launch_chain(const float* qkv, const float* records, const T* proj, long long ld, float* state, const int32_t* item_start,
-                 const int32_t* slots, float* o, int items, int min_tokens, int G, int H, int dim, int vdim, int K, int num_slots,
-                 long long slot_floats, cudaStream_t stream) {
-  constexpr int bytes = ChainShape<CHANNEL>::FLOATS * (int)sizeof(float);
-  static PsbPerDevice configured;
-  if (!configured.get()) {
-    if (cudaFuncSetAttribute(delta_chain_kernel<T, CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
-      PSB_REFUSE("delta_chunks: cannot raise the shared-memory limit");
-    configured.set();
-  }
-  psb_launch(delta_chain_kernel<T, CHANNEL>, dim3((vdim + COLS - 1) / COLS, H, items), dim3(CHAIN_THREADS), (size_t)bytes, stream, qkv, records,
-             proj, ld, state, item_start, slots, o, min_tokens, G, H, dim, vdim, K, num_slots, slot_floats);
-  PSB_LAUNCH_CHECK("delta_chain");
-  return 0;
+  if (blockIdx.x == 0 && h == 0) keep_conv_inputs<__nv_bfloat16>(proj, P, base, t0, t1, C, K);
 }
 
 }  // namespace
@@ -401,9 +374,9 @@ PSB_API int psb_delta_chunk_tokens() { return CHUNK; }
 
 // The rule over every portion of at least ``min_tokens`` tokens, from what psb_delta_prepare left; other tokens, and the slots of
 // other portions, are left untouched.  records [chunks, H, RECORD] float32, chunks at least the number of these portions' chunks.
-// (qkv, bd, proj, dtype, ld, state, item_start, slots, records, o_out, items, chunks, min_tokens, G, H, dim, vdim, K, num_slots,
+// (qkv, bd, proj bfloat16, ld, state, item_start, slots, records, o_out, items, chunks, min_tokens, G, H, dim, vdim, K, num_slots,
 //  slot_floats, stream)
-PSB_API int psb_delta_chunks(const void* qkv, const void* bd, const void* proj, int dtype, long long ld, void* state, const void* item_start,
+PSB_API int psb_delta_chunks(const void* qkv, const void* bd, const void* proj, long long ld, void* state, const void* item_start,
                              const void* slots, void* records, void* o, int items, int chunks, int min_tokens, int G, int H, int dim, int vdim,
                              int K, int num_slots, long long slot_floats, cudaStream_t stream) {
   if (items < 0 || G < 1 || H < 1 || H % G || !psb_delta_chunk_record(dim, vdim)) PSB_REFUSE("delta_chunks: bad sizes G=%d H=%d dim=%d vdim=%d", G, H, dim, vdim);
@@ -413,12 +386,19 @@ PSB_API int psb_delta_chunks(const void* qkv, const void* bd, const void* proj, 
   if (H > 65535 || items > 65535 || chunks < 0) PSB_REFUSE("delta_chunks: too many heads or requests for one launch");
   if (((uintptr_t)qkv | (uintptr_t)records) & 15) PSB_REFUSE("delta_chunks: operands must be 16-byte aligned");
   if (items == 0 || chunks == 0) return 0;
+  constexpr int bytes = ChainShape::FLOATS * (int)sizeof(float);
+  static PsbPerDevice configured;
+  if (!configured.get()) {
+    if (cudaFuncSetAttribute(delta_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+      PSB_REFUSE("delta_chunks: cannot raise the shared-memory limit");
+    configured.set();
+  }
   psb_launch(delta_chunk_kernel, dim3(chunks, G), dim3(CHUNK_THREADS), 0, stream, (const float*)qkv, (const float*)bd, (const int32_t*)item_start,
              (float*)records, items, min_tokens, G, H, dim, vdim);
   PSB_LAUNCH_CHECK("delta_chunk");
-  PSB_DISPATCH_DTYPE(dtype, T_, {
-    return launch_chain<T_, false>((const float*)qkv, (const float*)records, (const T_*)proj, ld, (float*)state, (const int32_t*)item_start,
-                                   (const int32_t*)slots, (float*)o, items, min_tokens, G, H, dim, vdim, K, num_slots, slot_floats, stream);
-  });
+  psb_launch(delta_chain_kernel, dim3((vdim + COLS - 1) / COLS, H, items), dim3(CHAIN_THREADS), (size_t)bytes, stream, (const float*)qkv,
+             (const float*)records, (const __nv_bfloat16*)proj, ld, (float*)state, (const int32_t*)item_start, (const int32_t*)slots, (float*)o,
+             min_tokens, G, H, dim, vdim, K, num_slots, slot_floats);
+  PSB_LAUNCH_CHECK("delta_chain");
   return 0;
 }

@@ -1111,7 +1111,7 @@ DELTA_LONG_PORTION = 32  # steps whose longest portion has this many tokens take
 DELTA_LONG_LANES = 16   # measured: 32 lanes (a column a warp) took 807 us for a 2,048-token portion with 16 heads of 128 x 128, 16 lanes 716
 
 
-# Portions of this many tokens take the form that works 32 tokens at a time (keys of up to 128 numbers).  All four kernels, 16 heads over 8
+# Portions of this many tokens in bfloat16 take the form that works 32 tokens at a time (keys of up to 128 numbers).  All four kernels, 16 heads over 8
 # groups of 128: one portion of 8 tokens 25 us in chunks and 37 token by token, of 32 tokens 28 and 44; three of 24 and fewer 37 and 63.
 # (Portions on both sides of the line pay for both: 8, 6 and 5 tokens 58 us instead of 41.)
 DELTA_CHUNKED = 8
@@ -1146,7 +1146,7 @@ def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: 
     dev = proj.device
     # Long portions go in chunks; what is left, if anything can be, token by token.  Which of the two a portion takes depends on
     # its own length only.
-    record = int(lib().psb_delta_chunk_record(dim, vdim)) if ctx.max_new_tokens >= DELTA_CHUNKED else 0
+    record = int(lib().psb_delta_chunk_record(dim, vdim)) if proj.dtype == torch.bfloat16 and ctx.max_new_tokens >= DELTA_CHUNKED else 0
     short = not record or _has_portions_below(ctx, DELTA_CHUNKED)
     qkv = torch.empty((t, c), dtype=torch.float32, device=dev)
     bd = torch.empty((t, 5 * heads), dtype=torch.float32, device=dev)   # beta, decay and three state-free dot products per head
@@ -1162,7 +1162,7 @@ def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: 
         most = DELTA_CHUNKED - 1
         chunks = t // lib().psb_delta_chunk_tokens() + ctx.num_items
         records = torch.empty((chunks, heads, record), dtype=torch.float32, device=dev)
-        check(lib().psb_delta_chunks(qkv.data_ptr(), bd.data_ptr(), proj.data_ptr(), _code(proj, "projection output"), proj.shape[1],
+        check(lib().psb_delta_chunks(qkv.data_ptr(), bd.data_ptr(), proj.data_ptr(), proj.shape[1],
                                      state.data_ptr(), item_start.data_ptr(), slots.data_ptr(), records.data_ptr(), o.data_ptr(),
                                      ctx.num_items, chunks, DELTA_CHUNKED, groups, heads, dim, vdim, k, state.shape[0], slot_floats,
                                      _stream()), "delta_chunks")

@@ -52,7 +52,7 @@ def test_long_portions(dtype, groups, heads, dim, vdim, taps):
         before = library.launch_counts.copy()
         out = ops.delta_rule(proj, ba, conv, a_log, dt_bias, gain, state, ctx, groups=groups, heads=heads, dim=dim, vdim=vdim, eps=1e-5)
         taken = library.launch_counts - before
-        assert taken["delta_chunks"] == 1 and taken["delta_rule"] == 1
+        assert taken["delta_chunks"] == (dtype == torch.bfloat16) and taken["delta_rule"] == 1
         at = 0
         for i, (n, s) in enumerate(zip(lengths, starts)):
             slot = len(lengths) - 1 - i

@@ -749,12 +749,13 @@ LATENT_MMA_KEYS_PER_SPLIT = 64
 
 def _rows_splits(blocks: int, keys: int, slots: int, most: int = 8, least_keys: int = ROWS_KEYS_PER_SPLIT,
                  share: int = ROWS_BLOCK_SHARE) -> int:
-    best, best_cost = 1, None
-    for s in range(1, most + 1):
-        if s > 1 and keys // s < least_keys:
-            break
+    most = max(1, min(most, keys // least_keys))
+    if blocks * most <= slots:  # one round of blocks whatever the number
+        return most
+    best, best_cost = 1, -(-blocks // slots) * (keys + share)
+    for s in range(2, most + 1):
         cost = -(-blocks * s // slots) * (keys / s + share)
-        if best_cost is None or cost < best_cost:
+        if cost < best_cost:
             best, best_cost = s, cost
     return best
 
@@ -769,8 +770,9 @@ def _latent_attention_walk(q_lat, cache, table, positions, token_item, gate, out
     if LATENT_MMA and cache.dtype == torch.bfloat16 and out.dtype == torch.bfloat16:
         per_block = lib().psb_latent_attention_mma_heads(rank, d - rank, heads)
     if per_block and q_lat.data_ptr() % 16 == 0 and cache.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0:
-        from .tensorcore import _sms
-        splits = _rows_splits(t * heads // per_block, key_hint, _sms(q_lat.device), 32, LATENT_MMA_KEYS_PER_SPLIT, LATENT_MMA_BLOCK_SHARE)
+        if key_hint >= 2 * LATENT_MMA_KEYS_PER_SPLIT:
+            from .tensorcore import _sms
+            splits = _rows_splits(t * heads // per_block, key_hint, _sms(q_lat.device), 32, LATENT_MMA_KEYS_PER_SPLIT, LATENT_MMA_BLOCK_SHARE)
         if splits > 1:
             partial = torch.empty((t, heads, splits, rank + 2), dtype=torch.float32, device=q_lat.device)
         check(lib().psb_latent_attention_mma(q_lat.data_ptr(), cache.data_ptr(), table.data_ptr(), table.shape[1], positions.data_ptr(),
@@ -946,7 +948,10 @@ ROWS_SINGLE = True
 ROWS_BLOCKS_WANTED = 592
 # ... and heads of 128, at most eight to a key/value head: the kernel fed by the TMA unit.  Its blocks cost, beside their keys, about
 # what ROWS_DECODE_BLOCK_SHARE keys do.
+# Below so many (key/value head, key) pairs a step's rows are read in 12 us or less by either kernel, and the host takes longer to issue
+# one than that; the other kernel is issued with less (two tokens of 16 heads over 413 keys: 25 us a call instead of 36).
 ROWS_DECODE = True
+ROWS_DECODE_LEAST = 1 << 17
 ROWS_DECODE_KEYS_PER_SPLIT = 128
 ROWS_DECODE_BLOCK_SHARE = 128
 
@@ -1025,7 +1030,7 @@ def attention_over_rows(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, 
             keys = min(keys, chk)
         if (both16 and ROWS_SINGLE and kv.data_ptr() % 16 == 0 and q.data_ptr() % 4 == 0
                 and bool(lib().psb_attention_rows_single_supported(num_heads, num_kv_heads, dim, vdim))):
-            if (ROWS_DECODE and kv.data_ptr() % 16 == 0
+            if (ROWS_DECODE and t * num_kv_heads * keys >= ROWS_DECODE_LEAST
                     and bool(lib().psb_attention_rows_decode_supported(num_heads, num_kv_heads, dim, vdim, page_size))):
                 from .tensorcore import _sms
                 splits = _rows_splits(t * num_kv_heads, keys, lib().psb_attention_rows_decode_blocks() * _sms(q.device), 16,

@@ -39,6 +39,7 @@ def test_single_tokens(hq, hkv, page, options, least, monkeypatch):
     from prefixserve_b200.ops import kernels, library
     monkeypatch.setattr(kernels, "ROWS_DECODE_KEYS_PER_SPLIT", least)   # one share, a few, as many as there may be
     monkeypatch.setattr(kernels, "ROWS_DECODE_BLOCK_SHARE", 1)
+    monkeypatch.setattr(kernels, "ROWS_DECODE_LEAST", 0)
     window, chunk, keep = options.get("window"), options.get("chunk"), options.get("keep", 0)
     positions = [0, 15, 16, 63, 99, 255, 256, 700, 1500]
     g = torch.Generator().manual_seed(hq + page + len(options))

@@ -672,6 +672,8 @@ PSB_API int psb_attention_rows_tcgen05(const void* q, const void* kv, long long 
                                        int window, int chunk, int reach, float scale, int keep_first, const void* gate, long long ldg,
                                        long long ldo, float out_scale, float softcap, int whole, int ranges, void* part_o,
                                        void* part_ml, cudaStream_t stream) {
+  // (the largest raw score stands for the largest scaled one, and the cap's vote is on their size)
+  if (!(scale > 0.f)) PSB_REFUSE("attention_rows_tcgen05: scores are multiplied by a positive scale, not %g", scale);
   if (softcap < 0.f || !psb_attention_rows_tcgen05_supported(hq, hkv, dim, vdim, page_size, softcap > 0.f, bias != nullptr))
     PSB_REFUSE("attention_rows_tcgen05: %d heads over %d of %d and %d in pages of %d are not taken", hq, hkv, dim, vdim, page_size);
   if (ldo < (long long)hq * D || ldo % 8 || (gate && (ldg < (long long)hq * D || ldg % 8))) PSB_REFUSE("attention_rows_tcgen05: bad output or gate rows");

@@ -1072,7 +1072,7 @@ def attention_over_rows(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, 
                                          least if tiled else 0, keep_first, None, 1, *tail, _stream()), "attention_biased")
     if tiled and on_tensor_cores:
         most = 0x7fffffff  # tokens of the longest portion left to the kernel on mma.sync
-        if (ROWS_TCGEN05 and ctx.max_new_tokens >= ROWS_TCGEN05_MIN_TOKENS and ldo % 8 == 0 and out.data_ptr() % 16 == 0
+        if (ROWS_TCGEN05 and ctx.max_new_tokens >= ROWS_TCGEN05_MIN_TOKENS and scale > 0 and ldo % 8 == 0 and out.data_ptr() % 16 == 0
                 and (gate is None or (ldg % 8 == 0 and gate.data_ptr() % 16 == 0))
                 and bool(lib().psb_attention_rows_tcgen05_supported(num_heads, num_kv_heads, dim, vdim, page_size, 1 if softcap else 0,
                                                                     0 if bias is None else 1))):

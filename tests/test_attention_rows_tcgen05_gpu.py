@@ -108,3 +108,43 @@ def test_portions(hq, hkv, page, options, ranges, monkeypatch):
         assert ((got[at: at + n] - want).abs() <= 2.0 ** -8 * want.abs() + 3e-4).all(), (i, n, s, (got[at: at + n] - want).abs().max())
         at += n
     assert library.tcgen05_status() == 0
+
+
+def own_rows(lengths, starts, hq, hkv, seed=5):
+    """A step of portions with their queries and, in consecutive pages, keys and values."""
+    g = torch.Generator().manual_seed(seed)
+    held = [n + s for n, s in zip(lengths, starts)]
+    width = -(-max(held) // 16)
+    table = torch.arange(len(held) * width, dtype=torch.int32).view(len(held), width)
+    q = torch.randn(sum(lengths), hq, D, generator=g).bfloat16()
+    kv = torch.randn(len(held) * width, 1, hkv, 16, 2 * D, generator=g).bfloat16()
+    return step(lengths, starts), q.cuda(), kv.cuda(), table.cuda()
+
+
+def exact_rows(q, kv, table, lengths, starts, hq, hkv, scale, softcap=None):
+    out, at = [], 0
+    for i, (n, s) in enumerate(zip(lengths, starts)):
+        rows = kv[table[i].long()][:, 0].transpose(1, 2).reshape(-1, hkv, 2 * D)[: n + s].double().repeat_interleave(hq // hkv, 1)
+        scores = torch.einsum("thd,jhd->thj", q[at: at + n].double(), rows[..., :D]) * scale
+        if softcap:
+            scores = softcap * torch.tanh(scores / softcap)
+        seen = torch.arange(n + s, device="cuda")[None] <= torch.arange(s, s + n, device="cuda")[:, None]
+        out.append(torch.einsum("thj,jhd->thd", torch.softmax(scores.masked_fill(~seen[:, None], float("-inf")), -1), rows[..., D:]).flatten(1))
+        at += n
+    return torch.cat(out)
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+@pytest.mark.parametrize("softcap", [None, 3.0])
+def test_scales_that_are_not_positive(scale, softcap):
+    """They turn the order of the scores around (or make them equal): such calls stay with the kernel on mma.sync."""
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import library
+    lengths, starts = [150, 20], [30, 0]
+    ctx, q, kv, table = own_rows(lengths, starts, 4, 2)
+    before = library.launch_counts.copy()
+    out = ops.attention_over_rows(q, kv, table, ctx, num_heads=4, num_kv_heads=2, dim=D, vdim=D, page_size=16, scale=scale, softcap=softcap)
+    assert (library.launch_counts - before)["attention_rows_tcgen05"] == 0
+    want = exact_rows(q, kv, table, lengths, starts, 4, 2, scale, softcap)
+    # as in test_portions
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 3e-4).all()

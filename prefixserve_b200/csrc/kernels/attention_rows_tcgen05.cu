@@ -349,7 +349,7 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
     const int r = quarter * 32 + lane;
     if (t < ntiles) {
       const bool valid = r < n;
-      const int pr = min(p_first + r, p_last);  // an absent row computes what the last one sees; nobody stores it
+      const int pr = min(p_first + r, p_last);  // an absent row (its query is another request's, or zeros) is masked as the last one; nobody stores it
       const int low = low_of(pr), head = h0 + t;
       const float cap = args.softcap * PSB_LOG2E, rate = MODE == CAPPED ? args.scale / args.softcap : 0.f;
       const float factor = args.scale * PSB_LOG2E;
@@ -387,8 +387,20 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
         const int key0 = base_of(i);
         const uint32_t s_addr = lane_addr + (seq_of(i) % NB) * KB;
         const bool need_mask = kept ? key0 + KB > args.keep_first : (key0 + KB - 1 > p_first || key0 < low_last);
+        // (without kept blocks of their own the kept keys lie inside the ordinary blocks)
+        const int first = kept ? 0 : low, last = kept ? args.keep_first - 1 : pr, also = kept || kept_blocks ? 0 : args.keep_first;
+        auto masked = [&](int key) { return key > last || (key < first && key >= also); };
         tmem_ld_wait();
         if constexpr (MODE == CAPPED) {
+          // Only scores that count have a say in the form: those of masked keys (later ones, rows of a page that nobody has written)
+          // and of rows behind the portion (another request's queries) do not, or a result would depend on them.
+          if (need_mask || !valid) {
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc)
+#pragma unroll
+              for (int k = 0; k < 32; ++k)
+                if (!valid || masked(key0 + cc * 32 + k)) sv[cc][k] = 0.f;
+          }
           float top = 0.f;
 #pragma unroll
           for (int cc = 0; cc < 2; ++cc)
@@ -431,13 +443,9 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
         for (int cc = 0; cc < 2; ++cc) {
           float(&x)[32] = sv[cc];
           if (need_mask) {
-            // (without kept blocks of their own the kept keys lie inside the ordinary blocks)
-            const int first = kept ? 0 : low, last = kept ? args.keep_first - 1 : pr, also = kept || kept_blocks ? 0 : args.keep_first;
 #pragma unroll
-            for (int k = 0; k < 32; ++k) {
-              const int key = key0 + cc * 32 + k;
-              if (key > last || (key < first && key >= also)) x[k] = -INFINITY;
-            }
+            for (int k = 0; k < 32; ++k)
+              if (masked(key0 + cc * 32 + k)) x[k] = -INFINITY;
           }
 #pragma unroll
           for (int k = 0; k < 32; k += 8) {

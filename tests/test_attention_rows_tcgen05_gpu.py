@@ -148,3 +148,27 @@ def test_scales_that_are_not_positive(scale, softcap):
     want = exact_rows(q, kv, table, lengths, starts, 4, 2, scale, softcap)
     # as in test_portions
     assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 3e-4).all()
+
+
+def test_capped_scores_do_not_depend_on_what_does_not_count():
+    """The form of the cap is chosen by the scores of a run of rows: small ones here.  What lies behind a sequence's end in its last
+    page, the keys of later tokens, keys in front of the window and the request that follows must not change a bit."""
+    from prefixserve_b200 import ops
+    lengths, starts, hq, hkv, window = [100, 40], [120, 3], 4, 2, 90
+    ctx, q, kv, table = own_rows(lengths, starts, hq, hkv)
+    q[:100] *= 0.05
+    before = torch.arange(220, device="cuda") < 120 + 1 - window   # out of the first token's window, in a block it reads
+
+    def first_portion(garbage):
+        mine, queries = kv.clone(), q.clone()
+        queries[100:] = garbage * queries[100:]
+        rows = mine[table[0].long()]                   # [pages, 1, hkv, 16, 2 D]
+        flat = rows.transpose(1, 3).reshape(-1, hkv, 2 * D)
+        flat[220:] = garbage
+        flat[:220][before] *= garbage
+        mine[table[0].long()] = flat.view(-1, 16, hkv, 1, 2 * D).transpose(1, 3)
+        out = ops.attention_over_rows(queries, mine, table, ctx, num_heads=hq, num_kv_heads=hkv, dim=D, vdim=D, page_size=16, scale=0.1,
+                                      softcap=20.0, window=window)
+        return out[:100]
+
+    assert torch.equal(first_portion(1.0), first_portion(400.0))

@@ -146,6 +146,12 @@ __device__ __forceinline__ uint64_t capped_pair(uint64_t x, uint64_t rate, uint6
 }
 __device__ __forceinline__ float capped_far(float x, float rate2, float cap) { return fmaf(-2.f * cap, __fdividef(1.f, exp2f(x * rate2) + 1.f), cap); }
 
+// the output gate's factors of two neighbouring columns, with expf and a true division (as in attention_biased.cu): the quick forms
+// lose bits, and give 0 where 1 + exp(-g) is beyond 2^126
+__device__ __forceinline__ float2 gates_of(uint32_t pair) {
+  return make_float2(1.f / (1.f + expf(-__uint_as_float(pair << 16))), 1.f / (1.f + expf(-__uint_as_float(pair & 0xffff0000u))));
+}
+
 // status codes: 1 producer, 2 MMA, 3 softmax
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -574,8 +580,9 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
               for (int w = 0; w < 4; ++w) {
                 float a = __uint_as_float(v[k * 8 + 2 * w]) * inv, b = __uint_as_float(v[k * 8 + 2 * w + 1]) * inv;
                 if (gates) {
-                  a = __fdividef(a, 1.f + __expf(-__uint_as_float(gw[w] << 16)));
-                  b = __fdividef(b, 1.f + __expf(-__uint_as_float(gw[w] & 0xffff0000u)));
+                  const float2 f = gates_of(gw[w]);
+                  a *= f.x;
+                  b *= f.y;
                 }
                 packed[w] = pack2(a, b);
               }
@@ -637,8 +644,9 @@ attention_rows_merge_kernel(const RowsArgs args) {
     const uint32_t gw[2] = {g.x, g.y};
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      acc[2 * e] = __fdividef(acc[2 * e], 1.f + __expf(-__uint_as_float(gw[e] << 16)));
-      acc[2 * e + 1] = __fdividef(acc[2 * e + 1], 1.f + __expf(-__uint_as_float(gw[e] & 0xffff0000u)));
+      const float2 f = gates_of(gw[e]);
+      acc[2 * e] *= f.x;
+      acc[2 * e + 1] *= f.y;
     }
   }
   *reinterpret_cast<uint2*>(args.out + (size_t)(t0 + r) * args.ldo + (size_t)head * D + 4 * lane) = make_uint2(pack2(acc[0], acc[1]), pack2(acc[2], acc[3]));

@@ -172,3 +172,19 @@ def test_capped_scores_do_not_depend_on_what_does_not_count():
         return out[:100]
 
     assert torch.equal(first_portion(1.0), first_portion(400.0))
+
+
+@pytest.mark.parametrize("ranges", [1, 8])
+def test_gates_far_out(ranges, monkeypatch):
+    """Gates between -87.4 and -88.7, where 1 + exp(-gate) lies beyond 2^126, make a value of 2^100 one of about 10^-8, not 0."""
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import kernels
+    monkeypatch.setattr(kernels, "ROWS_TCGEN05_RANGES", ranges)
+    lengths, starts, hq, hkv = [60], [400], 2, 1
+    ctx, q, kv, table = own_rows(lengths, starts, hq, hkv)
+    kv[..., D:] = 2.0 ** 100
+    gate = torch.linspace(-88.7, -87.4, 60, device="cuda")[:, None].expand(60, hq * D).contiguous().bfloat16()
+    out = ops.attention_over_rows(q, kv, table, ctx, num_heads=hq, num_kv_heads=hkv, dim=D, vdim=D, page_size=16, scale=0.1, gate=gate)
+    want = 2.0 ** 100 * torch.sigmoid(gate.double())
+    # the result in bfloat16; a factor below the smallest normal number (2^-126) keeps at least 20 bits
+    assert (gate.double() > -88.8).all() and ((out.double() / want - 1).abs() <= 2.0 ** -8 + 2.0 ** -16).all()

@@ -70,7 +70,7 @@ struct RowsArgs {
   const __nv_bfloat16* gate;
   __nv_bfloat16* out;
   long long ldg, ldo;
-  float *part_o, *part_ml;  // of a unit cut into ranges: [unit - whole, range, tile, row] results of D numbers / (exponent, sum)
+  float *part_o, *part_ml;  // of a unit cut into ranges: [unit - whole, range, head, row] results of D numbers / (exponent, sum)
   int table_width, items, min_tokens, hq, hkv, heads_here, page_shift, window, chunk, reach, keep_first;
   int whole, ranges;        // units before ``whole`` are a CTA's, later ones ``ranges`` CTAs'
   float scale, softcap, out_scale;
@@ -538,7 +538,7 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
       }
       if (ok && cut) {
         fence_after();
-        const size_t slot = (((size_t)(unit - args.whole) * args.ranges + range) * TILES + t) * TILE_M + r;
+        const size_t slot = (((size_t)(unit - args.whole) * args.ranges + range) * ntiles + t) * TILE_M + r;
         const bool some = nblk > 0 && m_run != -INFINITY;
         *reinterpret_cast<float2*>(args.part_ml + slot * 2) = make_float2(some ? m_run * c : -INFINITY, some ? l_run : 0.f);
         if (nblk > 0) {
@@ -620,8 +620,8 @@ attention_rows_merge_kernel(const RowsArgs args) {
   unit_tokens(args, args.whole + rest, item, t0, n, h0);
   if (r >= n) return;
   const int head = h0 + t;
-  const size_t slot0 = ((size_t)rest * args.ranges * TILES + t) * TILE_M + r;  // ranges lie TILES * TILE_M further on
-  const size_t step = (size_t)TILES * TILE_M;
+  const size_t step = (size_t)args.heads_here * TILE_M;  // from range to range
+  const size_t slot0 = (size_t)rest * args.ranges * step + (size_t)t * TILE_M + r;
   const float2 ml = lane < args.ranges ? *reinterpret_cast<const float2*>(args.part_ml + (slot0 + lane * step) * 2) : make_float2(-INFINITY, 0.f);
   const float s2 = args.sink ? args.sink[head] * PSB_LOG2E : -INFINITY;
   const float top = fmaxf(warp_max(ml.x), s2);
@@ -678,8 +678,8 @@ PSB_API int psb_attention_rows_tcgen05_heads(int hq, int hkv) { return hkv > 0 &
 
 // Every portion of at least ``min_tokens`` tokens; other tokens are left untouched.  ``tiles``: at least the number of runs of
 // 128 tokens these portions make up.  A unit is such a run for psb_attention_rows_tcgen05_heads() heads; the first ``whole`` of
-// them, or all (whole < 0), are a CTA's each and the others ``ranges`` CTAs', with part_o float32 [units - whole, ranges, 256, 128]
-// and part_ml [.., 256, 2] as their scratch.
+// them, or all (whole < 0), are a CTA's each and the others ``ranges`` CTAs', with part_o float32 [units - whole, ranges, heads * 128, 128]
+// and part_ml [.., heads * 128, 2] as their scratch.
 // (q, kv, num_pages, table, table_width, positions, item_start, items, T, min_tokens, tiles, bias, sink, out, hq, hkv, dim, vdim,
 //  page_size, window, chunk, reach, scale, keep_first, gate, ldg, ldo, out_scale, softcap, whole, ranges, part_o, part_ml, stream)
 PSB_API int psb_attention_rows_tcgen05(const void* q, const void* kv, long long num_pages, const void* table, int table_width,

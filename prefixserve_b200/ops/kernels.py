@@ -1085,12 +1085,13 @@ def attention_over_rows(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, 
                 tiles, others = sum(-(-n // 128) for n in lens if n > most), min(lens) <= most
             keys = int((getattr(ctx, "extras", None) or {}).get("static_kv_len") or ctx.max_kv_len)
             span = min(keys, win + keep_first + 128 if win else keys, chk + 128 if chk else keys)
-            units = tiles * (num_heads // lib().psb_attention_rows_tcgen05_heads(num_heads, num_kv_heads))
+            together = lib().psb_attention_rows_tcgen05_heads(num_heads, num_kv_heads)
+            units = tiles * (num_heads // together)
             whole, ranges = _rows_ranges(units, -(-span // 64), q.device)
             part_o = part_ml = None
             if whole < units:
-                part_o = torch.empty((units - whole, ranges, 256, 128), dtype=torch.float32, device=q.device)
-                part_ml = torch.empty((units - whole, ranges, 256, 2), dtype=torch.float32, device=q.device)
+                part_o = torch.empty((units - whole, ranges, 128 * together, 128), dtype=torch.float32, device=q.device)
+                part_ml = torch.empty((units - whole, ranges, 128 * together, 2), dtype=torch.float32, device=q.device)
             check(lib().psb_attention_rows_tcgen05(q.data_ptr(), kv.data_ptr(), kv.shape[0], table.data_ptr(), table.shape[1],
                                                    positions.data_ptr(), item_start.data_ptr(), ctx.num_items, t, ROWS_TCGEN05_MIN_TOKENS,
                                                    tiles, _ptr(bias), _ptr(sink), out.data_ptr(), num_heads, num_kv_heads,

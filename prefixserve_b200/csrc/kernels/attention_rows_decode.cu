@@ -166,7 +166,10 @@ attention_rows_decode_kernel(const __grid_constant__ CUtensorMap map_kv, const D
         const int row = 8 * (e >> 1) + 2 * tg + (e & 1);
         float v = s[e >> 1][e & 1];
         v = args.softcap > 0.f ? quick_cap(v, rate, cap) : v * factor;
-        if (bias) v += bias[max(0, min(p - key0 - row, args.reach - 1))] * PSB_LOG2E;
+        if (bias) {  // (the lowest finite bias stays finite in powers of two: keys that all have it weigh the same)
+          const float b = bias[max(0, min(p - key0 - row, args.reach - 1))];
+          v += b == -INFINITY ? b : fmaxf(b * PSB_LOG2E, -FLT_MAX);
+        }
         if (row < from || row >= upto) v = -INFINITY;
         x[e] = v;
         top = fmaxf(top, v);

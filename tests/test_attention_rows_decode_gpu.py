@@ -90,3 +90,31 @@ def test_single_tokens(hq, hkv, page, options, least, monkeypatch):
         # rounding of the result to bfloat16 (2^-9); weights to 16 bits (2^-17 of values up to 5) and float32 scores up to 100
         assert ((got[i] - want).abs() <= 2.0 ** -8 * want.abs() + 3e-4).all(), (i, p, (got[i] - want).abs().max())
     assert library.tcgen05_status() == 0
+
+
+@pytest.mark.parametrize("least", [1 << 20, 16])
+def test_the_lowest_bias_is_finite(least, monkeypatch):
+    """A distance bias of the type's lowest value masks a key beside others; keys that all have it weigh the same."""
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import kernels
+    monkeypatch.setattr(kernels, "ROWS_DECODE_KEYS_PER_SPLIT", least)
+    monkeypatch.setattr(kernels, "ROWS_DECODE_BLOCK_SHARE", 1)
+    monkeypatch.setattr(kernels, "ROWS_DECODE_LEAST", 0)
+    positions, heads = [0, 40, 199], 4
+    g = torch.Generator().manual_seed(3)
+    kv = torch.randn(3 * 13, 1, 1, 16, 2 * D, generator=g).bfloat16()
+    table = torch.arange(3 * 13, dtype=torch.int32).view(3, 13)
+    q = torch.randn(3, heads, D, generator=g).bfloat16()
+    bias = torch.randn(heads, 300, generator=g)
+    bias[1] = bias[2, 50:] = bias[3, :30] = torch.finfo(torch.float32).min
+    dev = lambda x: torch.tensor(x, dtype=torch.int32).cuda()
+    ctx = types.SimpleNamespace(positions=dev(positions), token_item=dev([0, 1, 2]), item_start=dev([0, 1, 2, 3]), num_items=3, max_new_tokens=1,
+                                max_kv_len=200, extras={})
+    out = ops.attention_over_rows(q.cuda(), kv.cuda(), table.cuda(), ctx, num_heads=heads, num_kv_heads=1, dim=D, vdim=D, page_size=16, scale=0.1,
+                                  bias=bias.cuda()).cpu().double().view(3, heads, D)
+    for i, p in enumerate(positions):
+        rows = kv[table[i].long()].reshape(-1, 2 * D)[: p + 1].double()
+        scores = q[i].double() @ rows[:, :D].t() * 0.1 + bias.double()[:, p - torch.arange(p + 1)]
+        want = torch.softmax(scores, 1) @ rows[:, D:]
+        # as in test_single_tokens
+        assert ((out[i] - want).abs() <= 2.0 ** -8 * want.abs() + 3e-4).all(), (i, p)

@@ -925,6 +925,26 @@ ROWS_TCGEN05_CTA_COST = 3
 ROWS_TCGEN05_MERGE_COST = 3
 
 
+def _portion_lengths(ctx) -> list[int] | None:
+    """New tokens of every request of the step; None where the host does not hold the requests (no list, or an empty one).
+
+    Captured steps may look here: a capture is keyed by its requests' lengths, in order."""
+    items = getattr(ctx, "items", None)
+    return [it.end - it.start for it in items] if items else None
+
+
+def _has_portions_below(ctx, tokens: int) -> bool:
+    """Whether a step with a portion of at least ``tokens`` tokens has shorter ones as well (True where the host does not know)."""
+    lengths = _portion_lengths(ctx)
+    return ctx.num_items > 1 if lengths is None else min(lengths) < tokens
+
+
+def _portion_tiles(ctx, t: int, tokens: int, tile: int) -> int:
+    """Runs of ``tile`` tokens that the portions of at least ``tokens`` tokens make up, at least (the step has ``t`` tokens)."""
+    lengths = _portion_lengths(ctx)
+    return t // tile + ctx.num_items if lengths is None else sum(-(-n // tile) for n in lengths if n >= tokens)
+
+
 def _rows_ranges(units: int, blocks: int, device) -> tuple[int, int]:
     """(units that are one CTA's, ranges of keys each of the others is cut into) for units of about so many blocks."""
     from .tensorcore import _sms
@@ -1077,12 +1097,7 @@ def attention_over_rows(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, 
                 and bool(lib().psb_attention_rows_tcgen05_supported(num_heads, num_kv_heads, dim, vdim, page_size, 1 if softcap else 0,
                                                                     0 if bias is None else 1))):
             most = ROWS_TCGEN05_MIN_TOKENS - 1
-            items = getattr(ctx, "items", None)
-            if items is None:
-                tiles, others = t // 128 + ctx.num_items, ctx.num_items > 1
-            else:
-                lens = [it.end - it.start for it in items]
-                tiles, others = sum(-(-n // 128) for n in lens if n > most), min(lens) <= most
+            tiles, others = _portion_tiles(ctx, t, most + 1, 128), _has_portions_below(ctx, most + 1)
             keys = int((getattr(ctx, "extras", None) or {}).get("static_kv_len") or ctx.max_kv_len)
             span = min(keys, win + keep_first + 128 if win else keys, chk + 128 if chk else keys)
             together = lib().psb_attention_rows_tcgen05_heads(num_heads, num_kv_heads)
@@ -1121,14 +1136,6 @@ DELTA_LONG_LANES = 16   # measured: 32 lanes (a column a warp) took 807 us for a
 # groups of 128: one portion of 8 tokens 25 us in chunks and 37 token by token, of 32 tokens 28 and 44; three of 24 and fewer 37 and 63.
 # (Portions on both sides of the line pay for both: 8, 6 and 5 tokens 58 us instead of 41.)
 DELTA_CHUNKED = 8
-
-
-def _has_portions_below(ctx, tokens: int) -> bool:
-    """Whether a step with a portion of at least ``tokens`` tokens has shorter ones as well (True where the host does not know)."""
-    items = getattr(ctx, "items", None)
-    if items is None:
-        return ctx.num_items > 1
-    return any(it.end - it.start < tokens for it in items)
 
 
 def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,

@@ -414,10 +414,12 @@ constexpr int FEW_SMEM = 192 * 1024;
 // rows lie half a line off one another, so that a lane's pieces meet every bank once
 __host__ __device__ constexpr int few_pitch(int K) { return (K + 63) / 64 * 64 + 32; }
 
-__device__ __forceinline__ void few_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// 16 terms of each sum.  The instruction cuts its sums off instead of rounding them, so what it makes of a turn's terms is added up
+// outside, in pairs, and turns after one another.
+__device__ __forceinline__ void few_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 template <typename TC>
@@ -499,20 +501,27 @@ moe_fewrows_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __r
       }
       __syncthreads();
     }
-    float acc[2][4] = {};
+    float acc[4] = {};
     const __nv_bfloat16* mine = rows + (size_t)min(gr, m - 1) * pitch;  // (a row that is not there: its sums are not used)
     for (int k0 = share * FEW_TURN; k0 < K; k0 += FEW_SHARES * FEW_TURN) {
       const bool over = k0 + FEW_SHARES * FEW_TURN >= K;
       if (over && unit + 1 < last) aim(unit + 1);
       fetch(!over ? k0 + FEW_SHARES * FEW_TURN : unit + 1 < last ? share * FEW_TURN : K, next);
+      static_assert(FEW_STEPS == 4, "pairs of pairs");
+      float part[2][4];
 #pragma unroll
       for (int u = 0; u < FEW_STEPS; ++u) {
         const int k = k0 + 32 * u + 8 * tg;
         const uint4 b = k < K ? *reinterpret_cast<const uint4*>(mine + k) : make_uint4(0, 0, 0, 0);
         const uint4 a = now[u][0], e = now[u][1];
-        few_mma(acc[0], a.x, e.x, a.y, e.y, b.x, b.y);
-        few_mma(acc[1], a.z, e.z, a.w, e.w, b.z, b.w);
+        float d0[4], d1[4];
+        few_mma(d0, a.x, e.x, a.y, e.y, b.x, b.y);
+        few_mma(d1, a.z, e.z, a.w, e.w, b.z, b.w);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) part[u / 2][x] = u % 2 ? part[u / 2][x] + (d0[x] + d1[x]) : d0[x] + d1[x];
       }
+#pragma unroll
+      for (int x = 0; x < 4; ++x) acc[x] += part[0][x] + part[1][x];
 #pragma unroll
       for (int u = 0; u < FEW_STEPS; ++u) {
         now[u][0] = next[u][0];
@@ -522,7 +531,7 @@ moe_fewrows_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __r
     auto& buf = shares[unit & 1];
 #pragma unroll
     for (int x = 0; x < 4; ++x)  // columns gr and gr + 8, rows 2 tg and 2 tg + 1
-      buf[warp][2 * tg + (x & 1)][gr + 8 * (x >> 1)] = acc[0][x] + acc[1][x];
+      buf[warp][2 * tg + (x & 1)][gr + 8 * (x >> 1)] = acc[x];
     __syncthreads();
     {
       const int r = threadIdx.x / FEW_COLS, n = threadIdx.x % FEW_COLS, at = n / 16 * FEW_SHARES;

@@ -36,3 +36,24 @@ def test_few_rows(h, ff, glu):
     want = torch.einsum("tp,tpn,tphn->th", weight.double(), mid, picked)
     bound = torch.einsum("tp,tpn,tphn->th", weight.double(), spread + 1e-6 * (1 + mid.abs()), picked.abs()) + 1e-6
     assert ((out.double() - want).abs() <= bound).all(), ((out.double() - want).abs() / bound).max()
+
+
+@pytest.mark.parametrize("ff", [4096, 12296])
+def test_sums_are_rounded_not_cut_off(ff):
+    """Sums of positive terms: what an accumulator cuts off at every step would add up to a bias.  The first product picks a column,
+    so that the second one's operands are exact."""
+    from prefixserve_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(ff)
+    h, experts, t = 256, 6, 20
+    x = torch.zeros(t, h, device="cuda", dtype=torch.bfloat16)
+    x[:, 0] = 1.0
+    up = torch.rand(experts, ff, h, generator=g, device="cuda").to(torch.bfloat16)
+    down = torch.rand(experts, h, ff, generator=g, device="cuda").to(torch.bfloat16)
+    chosen = torch.randint(experts, (t, 1), generator=g, device="cuda").to(torch.int32)
+    out = ops.moe_experts(x, chosen, torch.ones(t, 1, device="cuda"), up, down, activation=None, out_dtype=torch.float32)
+    e = chosen[:, 0].long()
+    want = torch.einsum("tp,thp->th", up[e, :, 0].double(), down[e].double())
+    off = out.double() / want - 1
+    # float32 sums rounded to nearest err on both sides; an instruction cuts less than 2^-23 of its own 16 terms off
+    assert off.mean().abs() <= 2.0 ** -23, off.mean()
+    assert off.abs().max() <= (ff / 128 + 8) * 2.0 ** -24, off.abs().max()

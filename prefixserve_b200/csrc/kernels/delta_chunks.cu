@@ -19,6 +19,8 @@
 //                        V - .. and W (..) by four warps while four others make the last chunk's O, then the new state (16 x 8
 //                        of its numbers a warp, which stay in its registers as float32), all on the tensor cores with operands
 //                        in two terms.
+// W and B are zero above the diagonal, and zero times what is not finite is not zero: a sum that comes out not finite is made again from
+// its own terms, the tokens up to its own, so that a token reaches later ones only.
 // Chunks are counted through the step's portions of at least ``min_tokens`` tokens in order; a portion's last chunk is filled up
 // with tokens of beta 0, key 0 and decay 1.
 //
@@ -250,6 +252,18 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
       load_rows(a + 8 * k, 8 * TP, 4, ah, al);
       y.step(ah, al, split(b[8 * k * CP]), split(b[(8 * k + 4) * CP]));
     }
+    float total[4];
+    y.totals(total);
+    if (!all_finite(total)) {
+#pragma unroll 1
+      for (int e = 0; e < 4; ++e) {
+        const int i = i0 + 8 * (e >> 1);
+        float sum = 0.f;
+#pragma unroll 1
+        for (int j = 0; j <= i; ++j) sum = fmaf(ring[i * TP + j], u_of(c)[j * CP + oc + 2 * tg + (e & 1)], sum);
+        if (!is_finite(pick(total, e))) place(total, e, sum);
+      }
+    }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const int t = t0 + c * CHUNK + i0 + 8 * r, col = col0 + oc + 2 * tg;
@@ -262,7 +276,7 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
       }
       const float ci = ring[CHUNK * TP + i0 + 8 * r];
       if (t < t1 && col < vdim)
-        *reinterpret_cast<float2*>(o + ((size_t)t * H + h) * vdim + col) = make_float2(fmaf(ci, v.x, y.total(2 * r)), fmaf(ci, v.y, y.total(2 * r + 1)));
+        *reinterpret_cast<float2*>(o + ((size_t)t * H + h) * vdim + col) = make_float2(fmaf(ci, v.x, total[2 * r]), fmaf(ci, v.y, total[2 * r + 1]));
     }
   };
 
@@ -322,12 +336,28 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
         }
         u.step(ah, al, x[0], x[1]);
       }
+      float total[4];
+      u.totals(total);
+      if (!all_finite(total)) {
+#pragma unroll 1
+        for (int e = 0; e < 4; ++e) {
+          const int i = i0 + 8 * (e >> 1), col = uc + 2 * tg + (e & 1);
+          float sum = 0.f;
+#pragma unroll 1
+          for (int j = 0; j <= i; ++j) {
+            const float* q = part_of(c) + j * CP + col;
+            const float y = (q[0] + q[2 * CHUNK * CP]) + (q[4 * CHUNK * CP] + q[6 * CHUNK * CP]);
+            sum = fmaf(buf[Sh::SW_AT + i * TP + j], fmaf(-ring[CHUNK * TP + j], y, buf[Sh::V_AT + j * CP + col]), sum);
+          }
+          if (!is_finite(pick(total, e))) place(total, e, sum);
+        }
+      }
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int i = i0 + 8 * r, col = uc + 2 * tg;
         const float ri = ring[CHUNK * TP + CHUNK + i];
-        *reinterpret_cast<float2*>(u_of(c) + i * CP + col) = make_float2(u.total(2 * r), u.total(2 * r + 1));
-        store_split(uu + (i * SP + col) * 2, u.total(2 * r) * ri, u.total(2 * r + 1) * ri);
+        *reinterpret_cast<float2*>(u_of(c) + i * CP + col) = make_float2(total[2 * r], total[2 * r + 1]);
+        store_split(uu + (i * SP + col) * 2, total[2 * r] * ri, total[2 * r + 1] * ri);
       }
     } else if (warp < 8) {
       if (c > 0) read_out(c - 1);

@@ -57,8 +57,21 @@ struct Sums {
       for (int c = 0; c < n; ++c) s[c] += s[c + n];
     return s[0] + (small[0][e] + small[1][e]);
   }
+  __device__ __forceinline__ void totals(float (&out)[4]) const {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) out[e] = total(e);
+  }
 };
 using Sum = Sums<1>;
+
+__device__ __forceinline__ bool is_finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+__device__ __forceinline__ bool all_finite(const float (&x)[4]) { return is_finite(x[0]) && is_finite(x[1]) && is_finite(x[2]) && is_finite(x[3]); }
+// entry e of an array that stays in registers
+__device__ __forceinline__ float pick(const float (&x)[4], int e) { return e < 2 ? (e ? x[1] : x[0]) : (e == 3 ? x[3] : x[2]); }
+__device__ __forceinline__ void place(float (&x)[4], int e, float v) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) x[k] = k == e ? v : x[k];
+}
 // a fragment of the left operand: this lane's number, ``down`` for the row eight further, ``along`` for the place four further
 __device__ __forceinline__ void load_rows(const float* a, int down, int along, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
 #pragma unroll

@@ -78,3 +78,42 @@ def test_long_portions(dtype, groups, heads, dim, vdim, taps):
             at += n
         assert torch.allclose(state.double(), exact, atol=2e-5), (turn, (state.double() - exact).abs().max())
         starts = [s + n for s, n in zip(starts, lengths)]
+
+
+@pytest.mark.parametrize("what", ["value", "key", "query", "beta", "decay"])
+def test_a_token_that_is_not_finite_reaches_later_tokens_only(what):
+    """As in the recurrence itself: earlier tokens of its chunk, other requests and (through a value) other heads stay as they are."""
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import library
+    groups, heads, dim, vdim, taps, bad = 2, 4, 128, 64, 4, 45
+    g = torch.Generator(device="cuda").manual_seed(4)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    c, lengths = 2 * groups * dim + heads * vdim, [100, 40]
+    ctx, t = step(lengths, [3, 0]), sum(lengths)
+    conv, gain, a_log, dt_bias = 0.6 * rnd(c, taps), 1 + 0.1 * rnd(vdim), rnd(heads) - 1, rnd(heads) - 1
+    proj, ba, held = rnd(t, c + heads * vdim).bfloat16(), rnd(t, 2 * heads), 0.3 * rnd(2, (taps - 1) * c + heads * dim * vdim)
+
+    def run(proj, ba):
+        state = held.clone()
+        before = library.launch_counts.copy()
+        out = ops.delta_rule(proj, ba, conv, a_log, dt_bias, gain, state, ctx, groups=groups, heads=heads, dim=dim, vdim=vdim, eps=1e-5)
+        taken = library.launch_counts - before
+        assert taken["delta_chunks"] == 1 and taken["delta_rule"] == 1   # (the context does not say that no portion is short)
+        return out.double().view(t, heads, vdim), state[1, (taps - 1) * c:].view(heads, dim, vdim)   # (the first request's slot)
+
+    clean, _ = run(proj, ba)
+    proj, ba, nan = proj.clone(), ba.clone(), float("nan")
+    if what == "value":
+        proj[bad, 2 * groups * dim + 3] = float("inf")      # a number of the first head
+    elif what in ("key", "query"):
+        proj[bad, 5 + (groups * dim if what == "key" else 0)] = nan   # the first group: heads 0 and 1
+    else:
+        ba[bad, heads if what == "decay" else 0] = nan      # the first head
+    out, state = run(proj, ba)
+    hit = 2 if what in ("key", "query") else 1
+    # bfloat16 results: sums made again in another order may round to the neighbour
+    near = lambda a, b: ((a - b).abs() <= 2.0 ** -7 * b.abs() + 1e-4).all()
+    assert torch.isfinite(out[:bad]).all() and near(out[:bad], clean[:bad]) and near(out[100:], clean[100:]) and near(out[:, hit:], clean[:, hit:])
+    assert not torch.isfinite(out[bad, :hit]).all(-1).any() and torch.isfinite(state[hit:]).all()
+    if what != "query":
+        assert not torch.isfinite(out[99, :hit]).all(-1).any() and not torch.isfinite(state[:hit].flatten(1)).all(1).any()

@@ -11,6 +11,8 @@
 // q_i alpha_(start of i's run) .. alpha_i and k_j alpha_(j+1) .. alpha_(end of j's run) with whole runs' decays between them, on the
 // diagonal with a running product a column (four columns a warp, four channels a lane).
 // Products of float32 numbers enter the tensor cores in two terms (tf32_terms.cuh), the values, which are bfloat16, as they are.
+// P is zero above the diagonal, and zero times a value that is not finite is not zero: a result that comes out not finite is made
+// again from the tokens up to its own.
 // Running products of decays carry what their roundings lose: with that the error against float64 is that of the token-by-token
 // kernels (read-outs 1.3e-7 of their size as before, states 0.8e-7 instead of 0.9e-7); a float32 projection's values would need two
 // terms too and come out at 1.5e-7 instead of 1.4e-7, so those stay with the other kernels.
@@ -341,8 +343,25 @@ linear_read_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const f
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const int col = c0 + 8 * c + 2 * tg;
-      if (col < vdim)
-        *reinterpret_cast<float2*>(o + ((size_t)(t0 + i) * H + h) * vdim + col) = make_float2(y[c].total(2 * r) * scale, y[c].total(2 * r + 1) * scale);
+      if (col >= vdim) continue;
+      float v[2] = {y[c].total(2 * r), y[c].total(2 * r + 1)};
+      if (!is_finite(v[0]) || !is_finite(v[1])) {
+        float again[2] = {0.f, 0.f};
+#pragma unroll 1
+        for (int d = 0; d < dim; ++d) {
+          const float q = qs[i * KP + d] * fs[m * RP + d];
+          again[0] = fmaf(q, ss[d * VP + col], again[0]);
+          again[1] = fmaf(q, ss[d * VP + col + 1], again[1]);
+        }
+#pragma unroll 1
+        for (int j = 0; j <= i; ++j) {
+          again[0] = fmaf(ps[i * PP + j], vs[j * VP + col], again[0]);
+          again[1] = fmaf(ps[i * PP + j], vs[j * VP + col + 1], again[1]);
+        }
+        if (!is_finite(v[0])) v[0] = again[0];
+        if (!is_finite(v[1])) v[1] = again[1];
+      }
+      *reinterpret_cast<float2*>(o + ((size_t)(t0 + i) * H + h) * vdim + col) = make_float2(v[0] * scale, v[1] * scale);
     }
   }
 }

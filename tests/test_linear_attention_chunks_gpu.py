@@ -52,3 +52,45 @@ def test_long_portions(dtype, heads, dim, vdim):
             assert err <= 2e-5 * max(1.0, float(torch.stack(o).abs().max())), (turn, i, err)
         assert torch.allclose(state.double(), exact, rtol=1e-5, atol=2e-5), (turn, (state.double() - exact).abs().max())
         assert state.data_ptr() == held.data_ptr()
+
+
+@pytest.mark.parametrize("what", ["value", "key", "query", "decay"])
+def test_a_token_that_is_not_finite_reaches_later_tokens_only(what):
+    """As in the recurrence itself: earlier tokens of its chunk, other requests, other heads and (through a value) other columns stay as
+    they are."""
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import library
+    heads, dim, vdim, bad = 2, 128, 64, 74   # the eleventh token of a run
+    g = torch.Generator(device="cuda").manual_seed(4)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    dev = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    ctx = types.SimpleNamespace(item_start=dev([0, 130, 200]), slots=dev([0, 1]), num_items=2, max_new_tokens=130)
+    held, proj = rnd(2, heads * dim * vdim), rnd(200, heads * (2 * dim + vdim)).bfloat16()
+    alpha = torch.sigmoid(rnd(200, heads * dim)) ** (1 / 4)
+
+    def run(proj, alpha):
+        state = held.clone()
+        before = library.launch_counts.copy()
+        out = ops.linear_attention(proj, alpha, state, ctx, heads=heads, dim=dim, vdim=vdim)
+        assert (library.launch_counts - before)["linear_attention_chunks"] == 1
+        return out.double().view(200, heads, vdim), state.view(2, heads, dim, vdim)
+
+    clean, _ = run(proj, alpha)
+    proj, alpha = proj.clone(), alpha.clone()
+    if what == "value":
+        proj[bad, 2 * heads * dim + 3] = float("inf")
+    elif what == "decay":
+        alpha[bad, 5] = float("nan")
+    else:
+        proj[bad, 5 + (heads * dim if what == "key" else 0)] = float("nan")
+    out, state = run(proj, alpha)
+    near = lambda a, b: ((a - b).abs() <= 2e-5 * (1 + b.abs().max())).all()   # sums of some hundred products, made again in another order
+    assert torch.isfinite(out[:bad]).all() and near(out[:bad], clean[:bad]) and near(out[130:], clean[130:]) and near(out[:, 1:], clean[:, 1:])
+    assert torch.isfinite(state[:, 1:]).all() and torch.isfinite(state[1:]).all()
+    if what == "value":
+        rest = [i for i in range(vdim) if i != 3]
+        assert near(out[:, 0, rest], clean[:, 0, rest]) and not torch.isfinite(out[bad:130, 0, 3]).any()
+    else:
+        assert not torch.isfinite(out[bad, 0]).any()
+        if what != "query":
+            assert not torch.isfinite(out[129, 0]).any() and not torch.isfinite(state[0, 0, 5]).any()

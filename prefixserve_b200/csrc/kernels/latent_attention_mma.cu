@@ -216,6 +216,18 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const __nv_bfloat16
         on[j] = live.x != 0;
         on[j + 1] = live.y != 0;
       }
+      // An infinity of the row times a term that is 0 is NaN, and so is a query beyond bfloat16's range: such a score is made again
+      // from the numbers themselves, and -inf drops out as it should.  (A value that is infinite may still come out as NaN.)
+#pragma unroll
+      for (int j = 0; j < SPT; ++j) {
+        if (!on[j] || s[j] == s[j]) continue;
+        const float* query = q_lat + ((size_t)t * heads + h0 + head) * D;
+        const __nv_bfloat16* row = reinterpret_cast<const __nv_bfloat16*>(latent_smem + (i % Sh::STAGES) * Sh::TILE_BYTES) + (key_at + j) * PITCH;
+        float sum = 0.f;
+#pragma unroll 1
+        for (int d = 0; d < D; ++d) sum = fmaf(query[d], __bfloat162float(row[d]), sum);
+        s[j] = sum;
+      }
       float m_new = m_run;
 #pragma unroll
       for (int e = 0; e < SPT; ++e) {

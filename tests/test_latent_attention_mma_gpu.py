@@ -79,3 +79,26 @@ def test_other_sizes_and_types_keep_their_kernels():
     from prefixserve_b200.ops import kernels
     lib = kernels.lib()
     assert [lib.psb_latent_attention_mma_heads(*s) for s in ((512, 64, 8), (512, 64, 20), (256, 64, 32), (512, 32, 16), (512, 64, 96))] == [0, 0, 0, 0, 32]
+
+
+@pytest.mark.parametrize("heads", [16, 32])
+def test_a_row_that_scores_minus_infinity_drops_out(heads):
+    """A cached row with an infinite rotated number, against queries whose number there is one bfloat16 term (the others are 0); a row
+    that scores +inf, against other heads, makes their result NaN and nobody else's."""
+    from prefixserve_b200 import ops
+    lengths, page = [70, 200], 16
+    q, cache, table, rows, positions, items = case(lengths, heads, page, 1)
+    q[:, :, RANK + 3] = 1.0
+    q[1, 0, RANK + 3] = -1.0
+    for i, key in ((0, 5), (0, 69), (1, 150)):
+        cache[table[i, key // page], 0, 0, key % page, RANK + 3] = rows[i][key, RANK + 3] = float("-inf")
+    for hint in (0, 60000):
+        out = ops.latent_attention(q.cuda(), cache.cuda(), table.cuda(), positions.cuda(), torch.arange(2, dtype=torch.int32).cuda(), None, rank=RANK,
+                                   page_size=page, window=None, scale=0.07, out_dtype=torch.bfloat16, items=items, key_hint=hint).cpu().double()
+        for i, n in enumerate(lengths):
+            want = expected(q, rows, i, n, None, 0.07, None, page, ())
+            for h in range(heads):
+                if (i, h) == (1, 0):
+                    assert not torch.isfinite(out[i, h]).any()
+                else:   # as in test_single_tokens
+                    assert ((out[i, h] - want[h]).abs() <= 2.0 ** -8 * want[h].abs() + 1e-4).all(), (hint, i, h)

@@ -976,6 +976,51 @@ ROWS_DECODE_KEYS_PER_SPLIT = 128
 ROWS_DECODE_BLOCK_SHARE = 128
 
 
+# Beside portions of the tcgen05 kernel, single tokens and shorter portions go token by token through the kernels of a decode step, a
+# launch for every run of them (neighbours in the step) up to so many runs, else through the kernel on mma.sync, which has them walk
+# their keys a tile at a time.  A portion of 16 tokens and a decoded one behind 1,500 keys, 16 heads with capped scores: 55 us, with
+# mma.sync behind tcgen05 131 (113 on mma.sync alone); 1,500 tokens beside 16 decoded ones of 32 heads 98 us for 211 (254).
+ROWS_SHORT_RUNS = 3
+
+
+def _short_runs(ctx, most: int) -> list[tuple[int, int]]:
+    """[first, behind the last) token of every run of neighbouring portions of up to ``most`` tokens; none where the host does not hold the requests."""
+    runs, at = [], 0
+    for n in _portion_lengths(ctx) or []:
+        if n <= most:
+            if runs and runs[-1][1] == at:
+                runs[-1] = (runs[-1][0], at + n)
+            else:
+                runs.append((at, at + n))
+        at += n
+    return runs
+
+
+def _rows_single_tokens(q, positions, token_item, out, tail, *, kv, table, bias, sink, num_heads, num_kv_heads, dim, vdim, page_size, masks, keys):
+    """Attention over rows token by token, bfloat16 on the tensor cores; every token sees up to ``keys`` keys."""
+    t = q.shape[0]
+    if (ROWS_DECODE and t * num_kv_heads * keys >= ROWS_DECODE_LEAST
+            and bool(lib().psb_attention_rows_decode_supported(num_heads, num_kv_heads, dim, vdim, page_size))):
+        from .tensorcore import _sms
+        splits = _rows_splits(t * num_kv_heads, keys, lib().psb_attention_rows_decode_blocks() * _sms(q.device), 16,
+                              ROWS_DECODE_KEYS_PER_SPLIT, ROWS_DECODE_BLOCK_SHARE)
+        partial = torch.empty((t, num_heads, splits, vdim + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
+        check(lib().psb_attention_rows_decode(q.data_ptr(), kv.data_ptr(), kv.shape[0], table.data_ptr(), table.shape[1],
+                                              positions.data_ptr(), token_item.data_ptr(), _ptr(bias), _ptr(sink), out.data_ptr(), t,
+                                              num_heads, num_kv_heads, dim, vdim, page_size, *masks, _ptr(partial), splits, *tail, _stream()),
+              "attention_rows_single")
+        if splits > 1:
+            check(lib().psb_attention_rows_merge(partial.data_ptr(), _ptr(sink), out.data_ptr(), t, num_heads, vdim, splits, *tail[:4],
+                                                 _stream()), "attention_rows_merge")
+        return
+    blocks = t * num_kv_heads * -(-(num_heads // num_kv_heads) // 16)
+    splits = max(1, min(16, -(-ROWS_BLOCKS_WANTED // max(blocks, 1)), keys // 128))
+    partial = torch.empty((t, num_heads, splits, vdim + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
+    check(lib().psb_attention_rows_single(q.data_ptr(), kv.data_ptr(), table.data_ptr(), table.shape[1], positions.data_ptr(),
+                                          token_item.data_ptr(), _ptr(bias), _ptr(sink), out.data_ptr(), t, num_heads, num_kv_heads,
+                                          dim, vdim, page_size, *masks, _ptr(partial), splits, *tail, _stream()), "attention_rows_single")
+
+
 def biased_attention(qkv: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, ctx, *, num_heads: int, num_kv_heads: int,
                      dim: int, vdim: int, page_size: int, scale: float, window: int | None = None, chunk: int | None = None,
                      bias: torch.Tensor | None = None, sink: torch.Tensor | None = None) -> torch.Tensor:
@@ -1036,42 +1081,29 @@ def attention_over_rows(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, 
         ldg = max(int(gate.stride(0)), num_heads * vdim)
     tail = (_ptr(gate), ldg, ldo, float(out_scale), float(softcap or 0.0))
     win, chk = int(window or 0), int(chunk or 0)
-    # Portions of a bfloat16 step go tile by tile; what is left (single tokens, short portions) walks its keys.  Which
-    # kernel a token gets depends on the length of its portion only (decided on the device from the item offsets, so
-    # the launches have the same shape whatever the step holds).
+    # Portions of a bfloat16 step go tile by tile; what is left (single tokens, short portions) walks its keys.  Which kernel a
+    # token gets, and the launches' grids, follow from the step's number of tokens, its longest portion and, where the host holds
+    # the requests, all their lengths: what a captured step is keyed by.
     item_start = _i32(ctx.item_start, "item offsets")
     both16 = q.dtype == torch.bfloat16 and kv.dtype == torch.bfloat16
-    if BIASED_SPLIT_DECODE and ctx.max_new_tokens == 1:
-        extras = getattr(ctx, "extras", None) or {}
-        keys = int(extras.get("static_kv_len") or ctx.max_kv_len)  # a captured step is sized for its class of lengths
-        if win:
-            keys = min(keys, win + keep_first)
-        if chk:
-            keys = min(keys, chk)
-        if (both16 and ROWS_SINGLE and kv.data_ptr() % 16 == 0 and q.data_ptr() % 4 == 0
+
+    def keys_seen(beside: int = 0) -> int:  # by a token, at most, or by neighbours, ``beside`` of them
+        held = int((getattr(ctx, "extras", None) or {}).get("static_kv_len") or ctx.max_kv_len)  # a captured step is sized for its class of lengths
+        return min(held, win + keep_first + beside if win else held, chk + beside if chk else held)
+
+    def one_by_one(q, positions, token_item, out, tail) -> bool:  # the step's tokens, or a run of them; False: not for these operands
+        if not (both16 and ROWS_SINGLE and kv.data_ptr() % 16 == 0 and q.data_ptr() % 4 == 0
                 and bool(lib().psb_attention_rows_single_supported(num_heads, num_kv_heads, dim, vdim))):
-            if (ROWS_DECODE and t * num_kv_heads * keys >= ROWS_DECODE_LEAST
-                    and bool(lib().psb_attention_rows_decode_supported(num_heads, num_kv_heads, dim, vdim, page_size))):
-                from .tensorcore import _sms
-                splits = _rows_splits(t * num_kv_heads, keys, lib().psb_attention_rows_decode_blocks() * _sms(q.device), 16,
-                                      ROWS_DECODE_KEYS_PER_SPLIT, ROWS_DECODE_BLOCK_SHARE)
-                partial = torch.empty((t, num_heads, splits, vdim + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
-                check(lib().psb_attention_rows_decode(q.data_ptr(), kv.data_ptr(), kv.shape[0], table.data_ptr(), table.shape[1],
-                                                      positions.data_ptr(), token_item.data_ptr(), _ptr(bias), _ptr(sink), out.data_ptr(), t,
-                                                      num_heads, num_kv_heads, dim, vdim, page_size, win, chk, reach, float(scale), keep_first,
-                                                      _ptr(partial), splits, *tail, _stream()), "attention_rows_single")
-                if splits > 1:
-                    check(lib().psb_attention_rows_merge(partial.data_ptr(), _ptr(sink), out.data_ptr(), t, num_heads, vdim, splits, *tail[:4],
-                                                         _stream()), "attention_rows_merge")
-                return out
-            blocks = t * num_kv_heads * -(-(num_heads // num_kv_heads) // 16)
-            splits = max(1, min(16, -(-ROWS_BLOCKS_WANTED // max(blocks, 1)), keys // 128))
-            partial = torch.empty((t, num_heads, splits, vdim + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
-            check(lib().psb_attention_rows_single(q.data_ptr(), kv.data_ptr(), table.data_ptr(), table.shape[1], positions.data_ptr(),
-                                                  token_item.data_ptr(), _ptr(bias), _ptr(sink), out.data_ptr(), t, num_heads, num_kv_heads,
-                                                  dim, vdim, page_size, win, chk, reach, float(scale), keep_first, _ptr(partial), splits,
-                                                  *tail, _stream()), "attention_rows_single")
+            return False
+        _rows_single_tokens(q, positions, token_item, out, tail, kv=kv, table=table, bias=bias, sink=sink, num_heads=num_heads,
+                            num_kv_heads=num_kv_heads, dim=dim, vdim=vdim, page_size=page_size, masks=(win, chk, reach, float(scale), keep_first),
+                            keys=keys_seen())
+        return True
+
+    if BIASED_SPLIT_DECODE and ctx.max_new_tokens == 1:
+        if one_by_one(q, positions, token_item, out, tail):
             return out
+        keys = keys_seen()
         splits = max(1, min(16, -(-BIASED_BLOCKS_WANTED // max(t * num_heads, 1)), keys // 128))
         partial = torch.empty((t, num_heads, splits, vdim + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
         check(lib().psb_attention_biased(q.data_ptr(), _code(q, "queries"), kv.data_ptr(), _code(kv, "cache entry"),
@@ -1098,8 +1130,7 @@ def attention_over_rows(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, 
                                                                     0 if bias is None else 1))):
             most = ROWS_TCGEN05_MIN_TOKENS - 1
             tiles, others = _portion_tiles(ctx, t, most + 1, 128), _has_portions_below(ctx, most + 1)
-            keys = int((getattr(ctx, "extras", None) or {}).get("static_kv_len") or ctx.max_kv_len)
-            span = min(keys, win + keep_first + 128 if win else keys, chk + 128 if chk else keys)
+            span = keys_seen(128)
             together = lib().psb_attention_rows_tcgen05_heads(num_heads, num_kv_heads)
             units = tiles * (num_heads // together)
             whole, ranges = _rows_ranges(units, -(-span // 64), q.device)
@@ -1115,6 +1146,11 @@ def attention_over_rows(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, 
                   "attention_rows_tcgen05")
         else:
             others = True
+        if most < 0x7fffffff and others:
+            runs = _short_runs(ctx, most)
+            others = not 0 < len(runs) <= ROWS_SHORT_RUNS or not all(
+                one_by_one(q[a:b], positions[a:b], token_item[a:b], out[a:b], (None if gate is None else gate[a:b].data_ptr(), *tail[1:]))
+                for a, b in runs)
         if others:
             check(lib().psb_attention_biased_mma(q.data_ptr(), kv.data_ptr(), table.data_ptr(), table.shape[1], positions.data_ptr(),
                                                  item_start.data_ptr(), ctx.num_items, t, least, most, _ptr(bias), _ptr(sink), out.data_ptr(),
@@ -1136,6 +1172,7 @@ DELTA_LONG_LANES = 16   # measured: 32 lanes (a column a warp) took 807 us for a
 # groups of 128: one portion of 8 tokens 25 us in chunks and 37 token by token, of 32 tokens 28 and 44; three of 24 and fewer 37 and 63.
 # (Portions on both sides of the line pay for both: 8, 6 and 5 tokens 58 us instead of 41.)
 DELTA_CHUNKED = 8
+
 
 
 def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
@@ -1347,6 +1384,7 @@ def low_rank(a: torch.Tensor, w: torch.Tensor, function: str, *, bias: torch.Ten
 # LINEAR_ATTENTION_CHUNK cuts the portions into chunks that go token by token side by side.
 LINEAR_CHUNKED, LINEAR_SHORT = 96, 32
 LINEAR_ATTENTION_CHUNK = 64
+
 
 
 def linear_attention(proj: torch.Tensor, alpha: torch.Tensor, state: torch.Tensor, ctx, *, heads: int, dim: int, vdim: int) -> torch.Tensor:

@@ -188,3 +188,69 @@ def test_gates_far_out(ranges, monkeypatch):
     want = 2.0 ** 100 * torch.sigmoid(gate.double())
     # the result in bfloat16; a factor below the smallest normal number (2^-126) keeps at least 20 bits
     assert (gate.double() > -88.8).all() and ((out.double() / want - 1).abs() <= 2.0 ** -8 + 2.0 ** -16).all()
+
+
+def views(lengths, starts):
+    """The requests of a step as the engine's contexts hold them."""
+    return [types.SimpleNamespace(start=s, end=s + n) for n, s in zip(lengths, starts)]
+
+
+@pytest.mark.parametrize("lengths, starts, softcap", [([1500, 1200], [0, 40], 30.0), ([300, 2000, 16], [700, 0, 90], None)])
+def test_more_units_than_the_gpu_holds(lengths, starts, softcap, monkeypatch):
+    """Whole units and units cut into ranges of keys in one launch, tiles counted from the requests, nothing left to the kernel on mma.sync."""
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import kernels, library
+    seen, ranges = [], kernels._rows_ranges
+    monkeypatch.setattr(kernels, "_rows_ranges", lambda units, *a: seen.append((units,) + ranges(units, *a)) or seen[-1][1:])
+    hq, hkv = 16, 4
+    ctx, q, kv, table = own_rows(lengths, starts, hq, hkv)
+    ctx.items = views(lengths, starts)
+    before = library.launch_counts.copy()
+    out = ops.attention_over_rows(q, kv, table, ctx, num_heads=hq, num_kv_heads=hkv, dim=D, vdim=D, page_size=16, scale=0.1, softcap=softcap)
+    taken = library.launch_counts - before
+    assert taken["attention_rows_tcgen05"] == 1 and taken["attention_biased_mma"] == 0
+    (units, whole, cut), = seen
+    assert units == 8 * sum(-(-n // 128) for n in lengths) and 0 < whole < units and cut > 1
+    want = exact_rows(q, kv, table, lengths, starts, hq, hkv, 0.1, softcap)
+    # as in test_portions
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 3e-4).all()
+    assert library.tcgen05_status() == 0
+
+
+@pytest.mark.parametrize("lengths, runs", [([64, 1, 300, 7, 1], 2), ([1, 1, 15, 16], 1), ([1, 20, 1, 20, 1], 3), ([1, 20, 1, 20, 1, 20, 2], 0)])
+@pytest.mark.parametrize("options", [dict(), dict(window=200, softcap=3.0, gate=True, out_scale=-0.5), dict(window=90, keep_first=70, sink=True),
+                                     dict(chunk=256, bias=256, sink=True)])
+@pytest.mark.parametrize("least", [0, 1 << 30])
+def test_single_tokens_and_short_portions_beside_others(lengths, runs, options, least, monkeypatch):
+    """They go through the kernels of a decode step, a launch for each of up to three runs of neighbours; by themselves, where the host
+    does not hold the requests or there are more runs, through the kernel on mma.sync."""
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import kernels, library
+    monkeypatch.setattr(kernels, "ROWS_DECODE_LEAST", least)   # the kernel fed by the TMA unit, and the other one
+    starts = [(331 * i + 40) % 700 for i in range(len(lengths))]
+    hq, hkv, t = 4, 2, sum(lengths)
+    ctx, q, kv, table = own_rows(lengths, starts, hq, hkv)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    more = {k: v for k, v in options.items() if k not in ("gate", "sink", "bias")}
+    if "gate" in options:
+        more["gate"] = torch.randn(t, hq * D + 16, generator=g, device="cuda").bfloat16()[:, 8: 8 + hq * D]
+    if "sink" in options:
+        more["sink"] = torch.randn(hq, generator=g, device="cuda")
+    if "bias" in options:
+        more["bias"] = torch.randn(hq, options["bias"], generator=g, device="cuda")
+
+    def run():
+        before = library.launch_counts.copy()
+        wide = torch.full((t, hq * D + 16), 7.0, dtype=torch.bfloat16, device="cuda")
+        out = ops.attention_over_rows(q, kv, table, ctx, num_heads=hq, num_kv_heads=hkv, dim=D, vdim=D, page_size=16, scale=0.1, out=wide[:, 8: 8 + hq * D], **more)
+        assert bool((wide[:, :8] == 7.0).all()) and bool((wide[:, 8 + hq * D:] == 7.0).all())
+        return out.double(), library.launch_counts - before
+
+    want, taken = run()
+    assert taken["attention_biased_mma"] == 1 and taken["attention_rows_single"] == 0
+    ctx.items = views(lengths, starts)
+    got, taken = run()
+    assert taken["attention_rows_tcgen05"] == 1 and taken["attention_rows_single"] == runs and taken["attention_biased_mma"] == (runs == 0)
+    # two results within test_portions' bound of the exact one
+    assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 6e-4).all()
+    assert library.tcgen05_status() == 0

@@ -996,8 +996,21 @@ def _short_runs(ctx, most: int) -> list[tuple[int, int]]:
     return runs
 
 
-def _rows_single_tokens(q, positions, token_item, out, tail, *, kv, table, bias, sink, num_heads, num_kv_heads, dim, vdim, page_size, masks, keys):
+def _keys_seen(ctx, window: int, chunk: int, keep_first: int, beside: int = 0) -> int:
+    """Keys a token sees, at most, or ``beside`` neighbours together."""
+    held = int((getattr(ctx, "extras", None) or {}).get("static_kv_len") or ctx.max_kv_len)  # a captured step is sized for its class of lengths
+    return min(held, window + keep_first + beside if window else held, chunk + beside if chunk else held)
+
+
+def _rows_one_by_one(q, kv, sizes) -> bool:
+    """Whether the tensor-core kernels for single tokens take the operands."""
+    return (ROWS_SINGLE and q.dtype == torch.bfloat16 and kv.dtype == torch.bfloat16 and kv.data_ptr() % 16 == 0 and q.data_ptr() % 4 == 0
+            and bool(lib().psb_attention_rows_single_supported(*sizes[:4])))
+
+
+def _rows_single_tokens(q, positions, token_item, out, tail, kv, table, bias, sink, sizes, masks, keys) -> None:
     """Attention over rows token by token, bfloat16 on the tensor cores; every token sees up to ``keys`` keys."""
+    num_heads, num_kv_heads, dim, vdim, page_size = sizes
     t = q.shape[0]
     if (ROWS_DECODE and t * num_kv_heads * keys >= ROWS_DECODE_LEAST
             and bool(lib().psb_attention_rows_decode_supported(num_heads, num_kv_heads, dim, vdim, page_size))):
@@ -1018,7 +1031,8 @@ def _rows_single_tokens(q, positions, token_item, out, tail, *, kv, table, bias,
     partial = torch.empty((t, num_heads, splits, vdim + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
     check(lib().psb_attention_rows_single(q.data_ptr(), kv.data_ptr(), table.data_ptr(), table.shape[1], positions.data_ptr(),
                                           token_item.data_ptr(), _ptr(bias), _ptr(sink), out.data_ptr(), t, num_heads, num_kv_heads,
-                                          dim, vdim, page_size, *masks, _ptr(partial), splits, *tail, _stream()), "attention_rows_single")
+                                          dim, vdim, page_size, *masks, _ptr(partial), splits, *tail, _stream()),
+          "attention_rows_single")
 
 
 def biased_attention(qkv: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, ctx, *, num_heads: int, num_kv_heads: int,
@@ -1086,24 +1100,12 @@ def attention_over_rows(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, 
     # the requests, all their lengths: what a captured step is keyed by.
     item_start = _i32(ctx.item_start, "item offsets")
     both16 = q.dtype == torch.bfloat16 and kv.dtype == torch.bfloat16
-
-    def keys_seen(beside: int = 0) -> int:  # by a token, at most, or by neighbours, ``beside`` of them
-        held = int((getattr(ctx, "extras", None) or {}).get("static_kv_len") or ctx.max_kv_len)  # a captured step is sized for its class of lengths
-        return min(held, win + keep_first + beside if win else held, chk + beside if chk else held)
-
-    def one_by_one(q, positions, token_item, out, tail) -> bool:  # the step's tokens, or a run of them; False: not for these operands
-        if not (both16 and ROWS_SINGLE and kv.data_ptr() % 16 == 0 and q.data_ptr() % 4 == 0
-                and bool(lib().psb_attention_rows_single_supported(num_heads, num_kv_heads, dim, vdim))):
-            return False
-        _rows_single_tokens(q, positions, token_item, out, tail, kv=kv, table=table, bias=bias, sink=sink, num_heads=num_heads,
-                            num_kv_heads=num_kv_heads, dim=dim, vdim=vdim, page_size=page_size, masks=(win, chk, reach, float(scale), keep_first),
-                            keys=keys_seen())
-        return True
-
+    sizes, masks = (num_heads, num_kv_heads, dim, vdim, page_size), (win, chk, reach, float(scale), keep_first)
     if BIASED_SPLIT_DECODE and ctx.max_new_tokens == 1:
-        if one_by_one(q, positions, token_item, out, tail):
+        keys = _keys_seen(ctx, win, chk, keep_first)
+        if _rows_one_by_one(q, kv, sizes):
+            _rows_single_tokens(q, positions, token_item, out, tail, kv, table, bias, sink, sizes, masks, keys)
             return out
-        keys = keys_seen()
         splits = max(1, min(16, -(-BIASED_BLOCKS_WANTED // max(t * num_heads, 1)), keys // 128))
         partial = torch.empty((t, num_heads, splits, vdim + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
         check(lib().psb_attention_biased(q.data_ptr(), _code(q, "queries"), kv.data_ptr(), _code(kv, "cache entry"),
@@ -1130,7 +1132,7 @@ def attention_over_rows(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, 
                                                                     0 if bias is None else 1))):
             most = ROWS_TCGEN05_MIN_TOKENS - 1
             tiles, others = _portion_tiles(ctx, t, most + 1, 128), _has_portions_below(ctx, most + 1)
-            span = keys_seen(128)
+            span = _keys_seen(ctx, win, chk, keep_first, 128)
             together = lib().psb_attention_rows_tcgen05_heads(num_heads, num_kv_heads)
             units = tiles * (num_heads // together)
             whole, ranges = _rows_ranges(units, -(-span // 64), q.device)
@@ -1148,9 +1150,10 @@ def attention_over_rows(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, 
             others = True
         if most < 0x7fffffff and others:
             runs = _short_runs(ctx, most)
-            others = not 0 < len(runs) <= ROWS_SHORT_RUNS or not all(
-                one_by_one(q[a:b], positions[a:b], token_item[a:b], out[a:b], (None if gate is None else gate[a:b].data_ptr(), *tail[1:]))
-                for a, b in runs)
+            others = not 0 < len(runs) <= ROWS_SHORT_RUNS or not _rows_one_by_one(q, kv, sizes)
+            for a, b in [] if others else runs:
+                _rows_single_tokens(q[a:b], positions[a:b], token_item[a:b], out[a:b], (None if gate is None else gate[a:b].data_ptr(), *tail[1:]),
+                                    kv, table, bias, sink, sizes, masks, _keys_seen(ctx, win, chk, keep_first))
         if others:
             check(lib().psb_attention_biased_mma(q.data_ptr(), kv.data_ptr(), table.data_ptr(), table.shape[1], positions.data_ptr(),
                                                  item_start.data_ptr(), ctx.num_items, t, least, most, _ptr(bias), _ptr(sink), out.data_ptr(),

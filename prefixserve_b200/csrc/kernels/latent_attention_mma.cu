@@ -9,8 +9,11 @@
 //   O += P V    every warp takes 64 of the 512 value columns.
 // S of the next tile is computed together with P V of this one, so that the tensor cores wait for the softmax only.
 // Queries and weights are float32 and stay so: each goes in as three bfloat16 terms whose sum is the number to its last bit
-// (8 + 8 + 8 bits), against rows that are bfloat16 to begin with, so every product is exact and sums are float32.  A block
-// that shares a token's keys with others leaves maximum, sum and unscaled result for the merge kernel.
+// (8 + 8 + 8 bits), against rows that are bfloat16 to begin with, so every product is exact.  The instruction cuts its sums off
+// instead of rounding them, so its accumulators hold 32 numbers' (or keys') terms at a time, the smallest terms first, and what
+// comes out is added up in float32: 1.5e-7 from float64 over 3,500 keys (1.4e-6 with a chain of instructions over a block's
+// keys; 1.6e-7 on the CUDA cores).  A block that shares a token's keys with others leaves maximum, sum and unscaled result for
+// the merge kernel.
 //
 // What bounds it: the tensor cores' legacy path (three terms: 108 + 96 instructions a warp and tile, 1,024 multiply-adds a
 // clock and SM; busy 48 % of the time).  The kernel on the CUDA cores beside it (latent_attention_rows_kernel, still used for
@@ -49,6 +52,12 @@ __device__ __forceinline__ void latent_mma(float (&c)[4], const uint32_t (&a)[4]
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// c = a b, from nothing
+__device__ __forceinline__ void latent_mma_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 __device__ __forceinline__ void latent_ldmatrix(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
@@ -171,15 +180,28 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const __nv_bfloat16
       for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
     const uint32_t at = tile + ((key0 + (lane & 7) + 8 * (lane >> 4)) * PITCH + quarter * STEPS * 16 + 8 * ((lane >> 3) & 1)) * 2;
 #pragma unroll
-    for (int k = 0; k < STEPS; ++k) {
+    for (int k = 0; k < STEPS; k += 2) {
+      constexpr int LAST = STEPS - 1;
+      const int steps = k < LAST ? 2 : 1;
 #pragma unroll
       for (int n = 0; n < NT; n += 2) {
-        uint32_t b[4];
-        latent_ldmatrix(b, at + (n * 8 * PITCH + k * 16) * 2);
+        uint32_t b[2][4];
+        float d0[4], d1[4];
 #pragma unroll
-        for (int e = 2; e >= 0; --e) {
-          latent_mma(s[n], q[k][e], b[0], b[1]);
-          latent_mma(s[n + 1], q[k][e], b[2], b[3]);
+        for (int x = 0; x < steps; ++x) latent_ldmatrix(b[x], at + (n * 8 * PITCH + (k + x) * 16) * 2);
+        latent_mma_first(d0, q[k][2], b[0][0], b[0][1]);
+        latent_mma_first(d1, q[k][2], b[0][2], b[0][3]);
+#pragma unroll
+        for (int e = 2; e >= 0; --e)
+#pragma unroll
+          for (int x = e == 2 ? 1 : 0; x < steps; ++x) {
+            latent_mma(d0, q[k + x][e], b[x][0], b[x][1]);
+            latent_mma(d1, q[k + x][e], b[x][2], b[x][3]);
+          }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          s[n][x] += d0[x];
+          s[n + 1][x] += d1[x];
         }
       }
     }
@@ -258,35 +280,37 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const __nv_bfloat16
     if (i + 1 < ntiles) products(i + 1);
     {
       const uint32_t tile = tiles_at + (i % Sh::STAGES) * Sh::TILE_BYTES;
-#pragma unroll
-      for (int m = 0; m < MG; ++m) {
-        const float f0 = factors[16 * m + gr], f1 = factors[16 * m + gr + 8];
-#pragma unroll
-        for (int n = 0; n < 8; ++n) {
-          o[m][n][0] *= f0; o[m][n][1] *= f0;
-          o[m][n][2] *= f1; o[m][n][3] *= f1;
-        }
-      }
+      static_assert(KT == 32, "two steps of keys");
       const uint32_t at = tile + ((lane & 15) * PITCH + 64 * warp + 8 * (lane >> 4)) * 2;
       const uint32_t wat = weights_at + ((lane & 15) * Sh::P_PITCH + 8 * (lane >> 4)) * 2;
 #pragma unroll
-      for (int k = 0; k < KT / 16; ++k) {
-        uint32_t a[MG][3][4];
+      for (int m = 0; m < MG; ++m) {
+        const float f0 = factors[16 * m + gr], f1 = factors[16 * m + gr + 8];
+        uint32_t a[2][3][4];
 #pragma unroll
-        for (int m = 0; m < MG; ++m)
+        for (int k = 0; k < 2; ++k)
 #pragma unroll
-          for (int e = 0; e < 3; ++e) latent_ldmatrix(a[m][e], wat + ((e * HEADS + 16 * m) * Sh::P_PITCH + k * 16) * 2);
+          for (int e = 0; e < 3; ++e) latent_ldmatrix(a[k][e], wat + ((e * HEADS + 16 * m) * Sh::P_PITCH + k * 16) * 2);
 #pragma unroll
         for (int n = 0; n < 8; n += 2) {
-          uint32_t b[4];
-          latent_ldmatrix_trans(b, at + (k * 16 * PITCH + n * 8) * 2);
+          uint32_t b[2][4];
+          float d0[4], d1[4];
+#pragma unroll
+          for (int k = 0; k < 2; ++k) latent_ldmatrix_trans(b[k], at + (k * 16 * PITCH + n * 8) * 2);
+          latent_mma_first(d0, a[0][2], b[0][0], b[0][1]);
+          latent_mma_first(d1, a[0][2], b[0][2], b[0][3]);
 #pragma unroll
           for (int e = 2; e >= 0; --e)
 #pragma unroll
-            for (int m = 0; m < MG; ++m) {
-              latent_mma(o[m][n], a[m][e], b[0], b[1]);
-              latent_mma(o[m][n + 1], a[m][e], b[2], b[3]);
+            for (int k = e == 2 ? 1 : 0; k < 2; ++k) {
+              latent_mma(d0, a[k][e], b[k][0], b[k][1]);
+              latent_mma(d1, a[k][e], b[k][2], b[k][3]);
             }
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            o[m][n][x] = fmaf(o[m][n][x], x < 2 ? f0 : f1, d0[x]);
+            o[m][n + 1][x] = fmaf(o[m][n + 1][x], x < 2 ? f0 : f1, d1[x]);
+          }
         }
       }
     }

@@ -102,3 +102,24 @@ def test_a_row_that_scores_minus_infinity_drops_out(heads):
                     assert not torch.isfinite(out[i, h]).any()
                 else:   # as in test_single_tokens
                     assert ((out[i, h] - want[h]).abs() <= 2.0 ** -8 * want[h].abs() + 1e-4).all(), (hint, i, h)
+
+
+def test_sums_are_rounded_not_cut_off():
+    """Positive numbers, where what an accumulator cuts off at every step would add up to a bias: the shares that the blocks leave,
+    before they are joined and rounded to bfloat16."""
+    from prefixserve_b200.ops import kernels
+    heads, n, page, splits = 32, 3000, 16, 2
+    q, cache, table, rows, positions, _ = case([n], heads, page, 3)
+    q, cache, rows = q.abs() * 0.3, cache.abs(), [r.abs() for r in rows]
+    dev = [x.cuda() for x in (q, cache, table, positions, torch.zeros(1, dtype=torch.int32))]
+    out = torch.empty(1, heads, RANK, dtype=torch.bfloat16, device="cuda")
+    partial = torch.zeros(1, heads, splits, RANK + 2, device="cuda")
+    ptr = [x.data_ptr() for x in dev]
+    kernels.check(kernels.lib().psb_latent_attention_mma(ptr[0], ptr[1], ptr[2], table.shape[1], ptr[3], ptr[4], None, out.data_ptr(), 1, heads, RANK, ROT,
+                                                         page, cache.shape[0], 0, 0.07, splits, partial.data_ptr(), None, kernels._stream()), "latent_attention")
+    share = partial[0].cpu().double()
+    w = torch.exp(share[..., 0] - share[..., 0].amax(1, keepdim=True))
+    got = (share[..., 2:] * w[..., None]).sum(1) / (share[..., 1] * w).sum(1)[:, None]
+    off = got / expected(q, rows, 0, n, None, 0.07, None, page, ()) - 1
+    # an instruction cuts less than 2^-23 of what it holds off, and holds 32 keys' terms at a time; the rest is rounded both ways
+    assert off.mean().abs() <= 2.0 ** -23 and off.abs().max() <= 2.0 ** -20, (off.mean(), off.abs().max())

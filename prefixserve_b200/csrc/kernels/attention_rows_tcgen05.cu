@@ -146,11 +146,23 @@ __device__ __forceinline__ uint64_t capped_pair(uint64_t x, uint64_t rate, uint6
 }
 __device__ __forceinline__ float capped_far(float x, float rate2, float cap) { return fmaf(-2.f * cap, __fdividef(1.f, exp2f(x * rate2) + 1.f), cap); }
 
-// the output gate's factors of two neighbouring columns, with expf and a true division (as in attention_biased.cu): the quick forms
-// lose bits, and give 0 where 1 + exp(-g) is beyond 2^126
-__device__ __forceinline__ float2 gates_of(uint32_t pair) {
-  return make_float2(1.f / (1.f + expf(-__uint_as_float(pair << 16))), 1.f / (1.f + expf(-__uint_as_float(pair & 0xffff0000u))));
+// The output gate's factor 1 / (1 + exp(-g)).  expf and a reciprocal improved by a Newton step to the last place, as good as the
+// division in attention_biased.cu: the quick exponential and division lose bits, and give 0 where the sum is beyond 2^126.  (The sum
+// is taken 2^-8 of, so that its reciprocal is a normal number; the division proper cost 6 us of rows of 2,700 tokens' 77.)
+__device__ __forceinline__ float gate_of(float g) {
+  const float x = (1.f + expf(-g)) * 0x1p-8f;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  r = fmaf(r, fmaf(-x, r, 1.f), r);
+  return x > 0x1p120f ? 0.f : r * 0x1p-8f;  // (only an infinite sum is that large)
 }
+__device__ __forceinline__ float2 gates_of(uint32_t pair) {
+  return make_float2(gate_of(__uint_as_float(pair << 16)), gate_of(__uint_as_float(pair & 0xffff0000u)));
+}
+
+// bits ``at`` and up, and bits up to ``at``, of 32; ``at`` may lie outside
+__device__ __forceinline__ uint32_t bits_from(int at) { return at <= 0 ? ~0u : at > 31 ? 0u : ~0u << at; }
+__device__ __forceinline__ uint32_t bits_upto(int at) { return at < 0 ? 0u : at > 30 ? ~0u : (2u << at) - 1u; }
 
 // status codes: 1 producer, 2 MMA, 3 softmax
 template <int MODE>
@@ -393,25 +405,33 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
         const int key0 = base_of(i);
         const uint32_t s_addr = lane_addr + (seq_of(i) % NB) * KB;
         const bool need_mask = kept ? key0 + KB > args.keep_first : (key0 + KB - 1 > p_first || key0 < low_last);
-        // (without kept blocks of their own the kept keys lie inside the ordinary blocks)
-        const int first = kept ? 0 : low, last = kept ? args.keep_first - 1 : pr, also = kept || kept_blocks ? 0 : args.keep_first;
-        auto masked = [&](int key) { return key > last || (key < first && key >= also); };
+        uint32_t counts[2];  // the row's keys that count, a bit each (only where need_mask)
+        if (need_mask) {
+          // (without kept blocks of their own the kept keys lie inside the ordinary blocks)
+          const int first = kept ? 0 : low, last = kept ? args.keep_first - 1 : pr, also = kept || kept_blocks ? 0 : args.keep_first;
+#pragma unroll
+          for (int cc = 0; cc < 2; ++cc) {
+            const int at = key0 + cc * 32;
+            counts[cc] = bits_upto(last - at) & (bits_from(first - at) | bits_upto(also - 1 - at));
+          }
+        }
         tmem_ld_wait();
         if constexpr (MODE == CAPPED) {
           // Only scores that count have a say in the form: those of masked keys (later ones, rows of a page that nobody has written)
           // and of rows behind the portion (another request's queries) do not, or a result would depend on them.
-          if (need_mask || !valid) {
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc)
-#pragma unroll
-              for (int k = 0; k < 32; ++k)
-                if (!valid || masked(key0 + cc * 32 + k)) sv[cc][k] = 0.f;
-          }
           float top = 0.f;
 #pragma unroll
-          for (int cc = 0; cc < 2; ++cc)
+          for (int cc = 0; cc < 2; ++cc) {
+            if (need_mask) {
 #pragma unroll
-            for (int k = 0; k < 32; k += 2) top = max3(top, fabsf(sv[cc][k]), fabsf(sv[cc][k + 1]));
+              for (int k = 0; k < 32; k += 2)
+                top = max3(top, counts[cc] & (1u << k) ? fabsf(sv[cc][k]) : 0.f, counts[cc] & (2u << k) ? fabsf(sv[cc][k + 1]) : 0.f);
+            } else {
+#pragma unroll
+              for (int k = 0; k < 32; k += 2) top = max3(top, fabsf(sv[cc][k]), fabsf(sv[cc][k + 1]));
+            }
+          }
+          if (!valid) top = 0.f;
           if (__all_sync(0xffffffffu, top * rate <= CAP_SMALL)) {
             const uint64_t rate2 = pair_of(rate, rate), slope = pair_of(factor, factor);
 #pragma unroll
@@ -451,7 +471,7 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
           if (need_mask) {
 #pragma unroll
             for (int k = 0; k < 32; ++k)
-              if (masked(key0 + cc * 32 + k)) x[k] = -INFINITY;
+              if (!(counts[cc] & (1u << k))) x[k] = -INFINITY;
           }
 #pragma unroll
           for (int k = 0; k < 32; k += 8) {

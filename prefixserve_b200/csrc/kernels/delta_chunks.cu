@@ -30,6 +30,7 @@
 // token-by-token kernel (delta_rule.cu) waits for a butterfly every two tokens (611 us).  Eight warps a block and two blocks an
 // SM took as long.
 #include "delta_common.cuh"
+#include "portions.cuh"
 #include "tf32_terms.cuh"
 
 namespace {
@@ -44,21 +45,6 @@ constexpr int CHAIN_THREADS = 512, CHUNK_THREADS = 128;
 
 // a chunk's record of a head: W, B [32][32], c, r [32]
 constexpr int W_AT = 0, B_AT = CHUNK * CHUNK, C_AT = 2 * CHUNK * CHUNK, R_AT = C_AT + CHUNK, RECORD = R_AT + CHUNK;
-
-__device__ __forceinline__ bool find_chunk(const int32_t* __restrict__ item_start, int items, int min_tokens, int at, int& t0, int& n) {
-  for (int i = 0; i < items; ++i) {
-    const int a = item_start[i], b = item_start[i + 1];
-    if (b - a < min_tokens) continue;
-    const int c = (b - a + CHUNK - 1) / CHUNK;
-    if (at < c) {
-      t0 = a + at * CHUNK;
-      n = min(CHUNK, b - t0);
-      return true;
-    }
-    at -= c;
-  }
-  return false;
-}
 
 __device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
 __device__ __forceinline__ float both(uint64_t v) {  // the sum of a pair
@@ -85,7 +71,7 @@ delta_chunk_kernel(const float* __restrict__ qkv, const float* __restrict__ bd, 
   static_assert(WARPS * CHUNK * TP <= 2 * CHUNK * KP, "room for every warp's A");
   pdl_wait();
   int t0, n;
-  if (!find_chunk(item_start, items, min_tokens, blockIdx.x, t0, n)) return;
+  if (!portions::find_chunk<CHUNK>(item_start, items, min_tokens, blockIdx.x, t0, n)) return;
   const int g = blockIdx.y, C = 2 * G * dim + H * vdim;
   for (int i = threadIdx.x; i < CHUNK * RP / 4; i += CHUNK_THREADS) {
     const int t = i / (RP / 4), d = (i - t * (RP / 4)) * 4;
@@ -188,24 +174,21 @@ __device__ __forceinline__ Split load_split(const float* at) {
 __global__ void __launch_bounds__(CHAIN_THREADS, 1)
 delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ records, const __nv_bfloat16* __restrict__ proj, long long P,
                    float* __restrict__ state, const int32_t* __restrict__ item_start, const int32_t* __restrict__ slots,
-                   float* __restrict__ o, int min_tokens, int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats) {
+                   float* __restrict__ o, int items, int all_chunks, int min_tokens, int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats) {
   using Sh = ChainShape;
   extern __shared__ __align__(16) float chain[];
   float *st = chain + Sh::S_AT, *uu = chain + Sh::UU_AT;
   const int C = 2 * G * dim + H * vdim;
-  const int h = blockIdx.y, item = blockIdx.z, g = h / (H / G);
+  const int h = blockIdx.y, g = h / (H / G);
   const int col0 = blockIdx.x * COLS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gr = lane >> 2, tg = lane & 3;  // the lane's row (or column) and place in a fragment
   pdl_wait();
+  int item, first;  // (a block per portion: blocks for requests that have none would only be in the way, one fills an SM)
+  if (!portions::find_portion<CHUNK>(item_start, items, min_tokens, blockIdx.z, item, first)) return;
   const int t0 = item_start[item], t1 = item_start[item + 1];
-  if (t1 - t0 < min_tokens) return;
-  int first = 0;
-  for (int i = 0; i < item; ++i) {
-    const int ni = item_start[i + 1] - item_start[i];
-    if (ni >= min_tokens) first += (ni + CHUNK - 1) / CHUNK;
-  }
   const int chunks = (t1 - t0 + CHUNK - 1) / CHUNK;
+  if (first + chunks > all_chunks) return;  // (the caller counted fewer than there are: no records for them)
   int slot = slots[item];
   slot = slot < 0 ? 0 : (slot >= num_slots ? num_slots - 1 : slot);
   float* base = state + (size_t)slot * slot_floats;
@@ -403,19 +386,20 @@ PSB_API int psb_delta_chunk_record(int dim, int vdim) {
 PSB_API int psb_delta_chunk_tokens() { return CHUNK; }
 
 // The rule over every portion of at least ``min_tokens`` tokens, from what psb_delta_prepare left; other tokens, and the slots of
-// other portions, are left untouched.  records [chunks, H, RECORD] float32, chunks at least the number of these portions' chunks.
-// (qkv, bd, proj bfloat16, ld, state, item_start, slots, records, o_out, items, chunks, min_tokens, G, H, dim, vdim, K, num_slots,
-//  slot_floats, stream)
+// other portions, are left untouched.  records [chunks, H, RECORD] float32, portions and chunks at least the number of these portions
+// and of their chunks.
+// (qkv, bd, proj bfloat16, ld, state, item_start, slots, records, o_out, items, portions, chunks, min_tokens, G, H, dim, vdim, K,
+//  num_slots, slot_floats, stream)
 PSB_API int psb_delta_chunks(const void* qkv, const void* bd, const void* proj, long long ld, void* state, const void* item_start,
-                             const void* slots, void* records, void* o, int items, int chunks, int min_tokens, int G, int H, int dim, int vdim,
-                             int K, int num_slots, long long slot_floats, cudaStream_t stream) {
+                             const void* slots, void* records, void* o, int items, int portions, int chunks, int min_tokens, int G, int H,
+                             int dim, int vdim, int K, int num_slots, long long slot_floats, cudaStream_t stream) {
   if (items < 0 || G < 1 || H < 1 || H % G || !psb_delta_chunk_record(dim, vdim)) PSB_REFUSE("delta_chunks: bad sizes G=%d H=%d dim=%d vdim=%d", G, H, dim, vdim);
   if (K < 1 || K > MAX_TAPS || min_tokens < 1 || num_slots < 1) PSB_REFUSE("delta_chunks: %d taps are outside [1, %d], or no tokens or slots", K, MAX_TAPS);
   const long long C = 2LL * G * dim + (long long)H * vdim;
   if (ld < C || slot_floats != (K - 1) * C + (long long)H * dim * vdim) PSB_REFUSE("delta_chunks: the slot or the rows do not fit the sizes");
-  if (H > 65535 || items > 65535 || chunks < 0) PSB_REFUSE("delta_chunks: too many heads or requests for one launch");
+  if (H > 65535 || portions > 65535 || chunks < 0) PSB_REFUSE("delta_chunks: too many heads or requests for one launch");
   if (((uintptr_t)qkv | (uintptr_t)records) & 15) PSB_REFUSE("delta_chunks: operands must be 16-byte aligned");
-  if (items == 0 || chunks == 0) return 0;
+  if (items == 0 || portions < 1 || chunks == 0) return 0;
   constexpr int bytes = ChainShape::FLOATS * (int)sizeof(float);
   static PsbPerDevice configured;
   if (!configured.get()) {
@@ -426,9 +410,9 @@ PSB_API int psb_delta_chunks(const void* qkv, const void* bd, const void* proj, 
   psb_launch(delta_chunk_kernel, dim3(chunks, G), dim3(CHUNK_THREADS), 0, stream, (const float*)qkv, (const float*)bd, (const int32_t*)item_start,
              (float*)records, items, min_tokens, G, H, dim, vdim);
   PSB_LAUNCH_CHECK("delta_chunk");
-  psb_launch(delta_chain_kernel, dim3((vdim + COLS - 1) / COLS, H, items), dim3(CHAIN_THREADS), (size_t)bytes, stream, (const float*)qkv,
+  psb_launch(delta_chain_kernel, dim3((vdim + COLS - 1) / COLS, H, portions), dim3(CHAIN_THREADS), (size_t)bytes, stream, (const float*)qkv,
              (const float*)records, (const __nv_bfloat16*)proj, ld, (float*)state, (const int32_t*)item_start, (const int32_t*)slots, (float*)o,
-             min_tokens, G, H, dim, vdim, K, num_slots, slot_floats);
+             items, chunks, min_tokens, G, H, dim, vdim, K, num_slots, slot_floats);
   PSB_LAUNCH_CHECK("delta_chain");
   return 0;
 }

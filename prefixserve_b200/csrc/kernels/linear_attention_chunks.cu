@@ -22,28 +22,13 @@
 // 73, 13 and 114.  Eight warps a block took 112 us for the read-out.
 #include <type_traits>
 
+#include "portions.cuh"
 #include "tf32_terms.cuh"
 
 namespace {
 using namespace terms;
 
 constexpr int CHUNK = 64, RUN = 16, RUNS = CHUNK / RUN, RP = 128, KP = RP + 8, VP = RP + 4, PP = CHUNK + 8, THREADS = 512;
-
-// The chunk ``at`` of the portions of at least ``min_tokens`` tokens.
-__device__ __forceinline__ bool find_chunk(const int32_t* __restrict__ item_start, int items, int min_tokens, int at, int& t0, int& n) {
-  for (int i = 0; i < items; ++i) {
-    const int a = item_start[i], b = item_start[i + 1];
-    if (b - a < min_tokens) continue;
-    const int c = (b - a + CHUNK - 1) / CHUNK;
-    if (at < c) {
-      t0 = a + at * CHUNK;
-      n = min(CHUNK, b - t0);
-      return true;
-    }
-    at -= c;
-  }
-  return false;
-}
 
 // Products over k take the places 2 tg and 2 tg + 1 of every eight (instead of tg and tg + 4) of both operands: rows give them as one
 // 8-byte load.  Pitches are such that such loads (KP, PP), and loads down a column (VP), meet every bank once.
@@ -93,7 +78,7 @@ linear_local_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const 
   pdl_trigger();
   pdl_wait();
   int t0, n;
-  if (!find_chunk(item_start, items, min_tokens, blockIdx.y, t0, n)) return;
+  if (!portions::find_chunk<CHUNK>(item_start, items, min_tokens, blockIdx.y, t0, n)) return;
   const int h = blockIdx.x;
   bring<__nv_bfloat16, KP>(kr, proj + (size_t)t0 * ld + (size_t)H * dim + (size_t)h * dim, ld, n, dim);
   bring<__nv_bfloat16, KP>(vs, proj + (size_t)t0 * ld + 2 * (size_t)H * dim + (size_t)h * vdim, ld, n, vdim);
@@ -147,8 +132,8 @@ linear_local_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const 
 // A thread per four numbers of a portion's state: B of every chunk becomes the state the chunk starts from, the slot gets the last one.
 __global__ void __launch_bounds__(128)
 linear_starts_kernel(float* __restrict__ state, long long slot_floats, const int32_t* __restrict__ item_start,
-                     const int32_t* __restrict__ slots, float* __restrict__ local_b, const float* __restrict__ local_a, int min_tokens,
-                     int H, int dim, int vdim, int num_slots) {
+                     const int32_t* __restrict__ slots, float* __restrict__ local_b, const float* __restrict__ local_a, int chunks,
+                     int min_tokens, int H, int dim, int vdim, int num_slots) {
   pdl_trigger();
   pdl_wait();
   const int item = blockIdx.y, tokens = item_start[item + 1] - item_start[item];
@@ -159,6 +144,7 @@ linear_starts_kernel(float* __restrict__ state, long long slot_floats, const int
     if (ni >= min_tokens) first += (ni + CHUNK - 1) / CHUNK;
   }
   const int n = (tokens + CHUNK - 1) / CHUNK;
+  if (first + n > chunks) return;  // (the caller counted fewer than there are: no room for them)
   const long long per_chunk = (long long)H * dim * vdim, at = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (at >= per_chunk) return;
   int slot = slots[item];
@@ -205,7 +191,7 @@ linear_read_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const f
   pdl_trigger();
   pdl_wait();
   int t0, n;
-  if (!find_chunk(item_start, items, min_tokens, blockIdx.y, t0, n)) return;
+  if (!portions::find_chunk<CHUNK>(item_start, items, min_tokens, blockIdx.y, t0, n)) return;
   const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, tg = lane & 3;
   const __nv_bfloat16* rows = proj + (size_t)t0 * ld;
   bring<__nv_bfloat16, KP>(qs, rows + (size_t)h * dim, ld, n, dim);
@@ -401,7 +387,8 @@ PSB_API int psb_linear_chunks(const void* proj, long long ld, const void* alpha,
   PSB_LAUNCH_CHECK("linear_local");
   const long long fours = (long long)H * dim * vdim / 4;
   psb_launch(linear_starts_kernel, dim3((unsigned)((fours + 127) / 128), items), dim3(128), 0, stream, (float*)state, slot_floats,
-             (const int32_t*)item_start, (const int32_t*)slots, (float*)local_b, (const float*)local_a, min_tokens, H, dim, vdim, num_slots);
+             (const int32_t*)item_start, (const int32_t*)slots, (float*)local_b, (const float*)local_a, chunks, min_tokens, H, dim, vdim,
+             num_slots);
   PSB_LAUNCH_CHECK("linear_starts");
   psb_launch(linear_read_kernel, dim3(H, chunks), dim3(THREADS), (size_t)read_bytes, stream, (const __nv_bfloat16*)proj, ld, (const float*)alpha,
              (const int32_t*)item_start, (const float*)local_b, (float*)o, items, min_tokens, H, dim, vdim, scale);

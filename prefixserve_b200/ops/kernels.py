@@ -945,6 +945,12 @@ def _portion_tiles(ctx, t: int, tokens: int, tile: int) -> int:
     return t // tile + ctx.num_items if lengths is None else sum(-(-n // tile) for n in lengths if n >= tokens)
 
 
+def _portions_from(ctx, tokens: int) -> int:
+    """Portions of at least ``tokens`` tokens, at least."""
+    lengths = _portion_lengths(ctx)
+    return ctx.num_items if lengths is None else sum(n >= tokens for n in lengths)
+
+
 def _rows_ranges(units: int, blocks: int, device) -> tuple[int, int]:
     """(units that are one CTA's, ranges of keys each of the others is cut into) for units of about so many blocks."""
     from .tensorcore import _sms
@@ -1173,8 +1179,16 @@ DELTA_LONG_LANES = 16   # measured: 32 lanes (a column a warp) took 807 us for a
 
 # Portions of this many tokens in bfloat16 take the form that works 32 tokens at a time (keys of up to 128 numbers).  All four kernels, 16 heads over 8
 # groups of 128: one portion of 8 tokens 25 us in chunks and 37 token by token, of 32 tokens 28 and 44; three of 24 and fewer 37 and 63.
-# (Portions on both sides of the line pay for both: 8, 6 and 5 tokens 58 us instead of 41.)
 DELTA_CHUNKED = 8
+
+
+def _delta_one_by_one(lengths: list[int] | None) -> bool:
+    """Whether a step with portions on both sides of DELTA_CHUNKED is over sooner token by token: it pays for both forms, one after
+    the other, and the chunks' share has to be worth that.  The more so the longer and the more the short ones are (16 heads, both forms
+    and token by token: 16 tokens beside one 55 and 55 us, 24 beside eight 61 and 61; 24 beside 32 86 and 74, and 32, where that
+    kernel shares a column among more lanes, 86 and 104; 16, 12 and 7 tokens 73 and 61)."""
+    short = [n for n in lengths or [] if n < DELTA_CHUNKED]
+    return bool(short) and max(lengths) < min(DELTA_LONG_PORTION, 13 + 3 * max(short) + len(short) * 5 // 8)
 
 
 
@@ -1197,9 +1211,9 @@ def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: 
         if x.dtype != torch.float32 or x.numel() != n or not x.is_cuda or not x.is_contiguous():
             raise KernelError(f"delta rule: {what} must be float32 with {n} numbers on the device")
     dev = proj.device
-    # Long portions go in chunks; what is left, if anything can be, token by token.  Which of the two a portion takes depends on
-    # its own length only.
-    record = int(lib().psb_delta_chunk_record(dim, vdim)) if proj.dtype == torch.bfloat16 and ctx.max_new_tokens >= DELTA_CHUNKED else 0
+    # Long portions go in chunks; what is left, if anything can be, token by token.
+    chunked = proj.dtype == torch.bfloat16 and ctx.max_new_tokens >= DELTA_CHUNKED and not _delta_one_by_one(_portion_lengths(ctx))
+    record = int(lib().psb_delta_chunk_record(dim, vdim)) if chunked else 0
     short = not record or _has_portions_below(ctx, DELTA_CHUNKED)
     qkv = torch.empty((t, c), dtype=torch.float32, device=dev)
     bd = torch.empty((t, 5 * heads), dtype=torch.float32, device=dev)   # beta, decay and three state-free dot products per head
@@ -1213,11 +1227,11 @@ def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: 
     most = 0x7fffffff  # tokens of the longest portion left to the kernel that goes token by token
     if record:
         most = DELTA_CHUNKED - 1
-        chunks = t // lib().psb_delta_chunk_tokens() + ctx.num_items
+        portions, chunks = _portions_from(ctx, DELTA_CHUNKED), _portion_tiles(ctx, t, DELTA_CHUNKED, lib().psb_delta_chunk_tokens())
         records = torch.empty((chunks, heads, record), dtype=torch.float32, device=dev)
         check(lib().psb_delta_chunks(qkv.data_ptr(), bd.data_ptr(), proj.data_ptr(), proj.shape[1],
                                      state.data_ptr(), item_start.data_ptr(), slots.data_ptr(), records.data_ptr(), o.data_ptr(),
-                                     ctx.num_items, chunks, DELTA_CHUNKED, groups, heads, dim, vdim, k, state.shape[0], slot_floats,
+                                     ctx.num_items, portions, chunks, DELTA_CHUNKED, groups, heads, dim, vdim, k, state.shape[0], slot_floats,
                                      _stream()), "delta_chunks")
     if short:
         lanes = DELTA_LONG_LANES if min(ctx.max_new_tokens, most) >= DELTA_LONG_PORTION and dim >= DELTA_LONG_LANES else 4
@@ -1389,6 +1403,13 @@ LINEAR_CHUNKED, LINEAR_SHORT = 96, 32
 LINEAR_ATTENTION_CHUNK = 64
 
 
+def _linear_one_by_one(lengths: list[int] | None) -> bool:
+    """Whether a step that could go either way whole has so much in short portions, which the two forms take one after the other, that all
+    of it is over sooner token by token (16 heads, 100 tokens beside 8 single ones 49 us in chunks and 51, beside 32 78 and 59; 8 heads,
+    100 tokens beside 20 65 and 49)."""
+    short = [n for n in lengths or [] if n < LINEAR_SHORT]
+    return bool(short) and max(lengths) <= 2 * LINEAR_ATTENTION_CHUNK and (len(short) > 16 or max(short) > 8)
+
 
 def linear_attention(proj: torch.Tensor, alpha: torch.Tensor, state: torch.Tensor, ctx, *, heads: int, dim: int, vdim: int) -> torch.Tensor:
     """S <- diag(alpha_t) S + k_t v_t^T, o_t = S^T q_t * dim^-1/2 over every portion of the step.  proj [T, q | k | v | ...]
@@ -1407,9 +1428,9 @@ def linear_attention(proj: torch.Tensor, alpha: torch.Tensor, state: torch.Tenso
     most = 0x7fffffff  # tokens of the longest portion left to the kernels that go token by token
     if (ctx.max_new_tokens >= LINEAR_CHUNKED and proj.dtype == torch.bfloat16 and ld % 4 == 0 and stride % 4 == 0
             and proj.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0 and alpha.data_ptr() % 16 == 0
-            and bool(lib().psb_linear_chunks_supported(dim, vdim))):
+            and bool(lib().psb_linear_chunks_supported(dim, vdim)) and not _linear_one_by_one(_portion_lengths(ctx))):
         most = LINEAR_SHORT - 1
-        chunks = t // lib().psb_linear_chunk_tokens() + ctx.num_items
+        chunks = _portion_tiles(ctx, t, LINEAR_SHORT, lib().psb_linear_chunk_tokens())
         local_b = torch.empty((chunks, heads, dim, vdim), dtype=torch.float32, device=dev)
         local_a = torch.empty((chunks, heads, dim), dtype=torch.float32, device=dev)
         check(lib().psb_linear_chunks(proj.data_ptr(), ld, alpha.data_ptr(), state.data_ptr(), stride,

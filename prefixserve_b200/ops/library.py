@@ -215,9 +215,9 @@ _SIGNATURES: dict[str, list] = {
     # (dim, vdim) -> float32 numbers of a chunk's record of a head, 0: not built for the sizes; () -> tokens of a chunk
     "psb_delta_chunk_record": [I, I],
     "psb_delta_chunk_tokens": [],
-    # (qkv, bd, proj, ld, state, item_start, slots, records, o_out, items, chunks, min_tokens, G, H, dim, vdim, K, num_slots,
+    # (qkv, bd, proj, ld, state, item_start, slots, records, o_out, items, portions, chunks, min_tokens, G, H, dim, vdim, K, num_slots,
     #  slot_floats, stream)
-    "psb_delta_chunks": [P, P, P, L, P, P, P, P, P, I, I, I, I, I, I, I, I, I, L, P],
+    "psb_delta_chunks": [P, P, P, L, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, L, P],
     # (dim, vdim) -> float32 numbers of a chunk's record, 0 if the chunked form does not take the sizes
     "psb_channel_delta_record": [I, I],
     # (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, records, o_out, items, chunks, G, H, dim, vdim, K, num_slots,

@@ -117,3 +117,37 @@ def test_a_token_that_is_not_finite_reaches_later_tokens_only(what):
     assert not torch.isfinite(out[bad, :hit]).all(-1).any() and torch.isfinite(state[hit:]).all()
     if what != "query":
         assert not torch.isfinite(out[99, :hit]).all(-1).any() and not torch.isfinite(state[:hit].flatten(1)).all(1).any()
+
+
+def poisoned(monkeypatch):
+    """Scratch that nobody has written is NaN."""
+    empty = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: (lambda x: x.fill_(float("nan")) if x.is_floating_point() else x)(empty(*a, **k)))
+
+
+@pytest.mark.parametrize("lengths, short", [([64, 8, 97], False), ([64, 8, 97, 7], True), ([1, 33], True)])
+def test_steps_whose_requests_the_host_holds(lengths, short, monkeypatch):
+    """As the engine's contexts: without a short portion neither the token-by-token kernel nor what only it reads is made."""
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import library
+    groups, heads, dim, vdim, taps = 2, 4, 128, 64, 4
+    g = torch.Generator(device="cuda").manual_seed(len(lengths))
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    c, starts = 2 * groups * dim + heads * vdim, [5 * i for i in range(len(lengths))]
+    ctx, t = step(lengths, starts), sum(lengths)
+    conv, gain, a_log, dt_bias = 0.6 * rnd(c, taps), 1 + 0.1 * rnd(vdim), rnd(heads) - 1, rnd(heads) - 1
+    proj, ba, held = rnd(t, c + heads * vdim).bfloat16(), rnd(t, 2 * heads), 0.3 * rnd(len(lengths), (taps - 1) * c + heads * dim * vdim)
+
+    def run():
+        state = held.clone()
+        before = library.launch_counts.copy()
+        out = ops.delta_rule(proj, ba, conv, a_log, dt_bias, gain, state, ctx, groups=groups, heads=heads, dim=dim, vdim=vdim, eps=1e-5)
+        return out, state, library.launch_counts - before
+
+    out, state, taken = run()
+    assert taken["delta_rule"] == 1   # the host does not hold the requests
+    ctx.items = [types.SimpleNamespace(start=s, end=s + n) for n, s in zip(lengths, starts)]
+    poisoned(monkeypatch)
+    again, state_again, taken = run()
+    assert taken["delta_chunks"] == 1 and taken["delta_rule"] == short
+    assert torch.equal(out, again) and torch.equal(state, state_again)

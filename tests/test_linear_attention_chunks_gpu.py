@@ -94,3 +94,34 @@ def test_a_token_that_is_not_finite_reaches_later_tokens_only(what):
         assert not torch.isfinite(out[bad, 0]).any()
         if what != "query":
             assert not torch.isfinite(out[129, 0]).any() and not torch.isfinite(state[0, 0, 5]).any()
+
+
+@pytest.mark.parametrize("lengths, short", [([130, 32, 97], False), ([130, 32, 97, 31], True), ([1, 96], True)])
+def test_steps_whose_requests_the_host_holds(lengths, short, monkeypatch):
+    """As the engine's contexts: without a short portion the token-by-token kernels are not launched.  Scratch that nobody has written is NaN."""
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import library
+    heads, dim, vdim = 2, 64, 96
+    g = torch.Generator(device="cuda").manual_seed(len(lengths))
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    dev = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    t, offsets = sum(lengths), [0]
+    for n in lengths:
+        offsets.append(offsets[-1] + n)
+    ctx = types.SimpleNamespace(item_start=dev(offsets), slots=dev(list(range(len(lengths)))), num_items=len(lengths), max_new_tokens=max(lengths))
+    held, proj, alpha = rnd(len(lengths), heads * dim * vdim), rnd(t, heads * (2 * dim + vdim)).bfloat16(), torch.sigmoid(rnd(t, heads * dim)) ** (1 / 4)
+
+    def run():
+        state = held.clone()
+        before = library.launch_counts.copy()
+        out = ops.linear_attention(proj, alpha, state, ctx, heads=heads, dim=dim, vdim=vdim)
+        return out, state, library.launch_counts - before
+
+    out, state, taken = run()
+    assert taken["linear_attention"] == 1   # the host does not hold the requests
+    ctx.items = [types.SimpleNamespace(start=0, end=n) for n in lengths]
+    empty = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: (lambda x: x.fill_(float("nan")) if x.is_floating_point() else x)(empty(*a, **k)))
+    again, state_again, taken = run()
+    assert taken["linear_attention_chunks"] == 1 and taken["linear_attention"] == short
+    assert torch.equal(out, again) and torch.equal(state, state_again)

@@ -26,3 +26,19 @@ def test_portions(lengths, items):
         assert kernels._has_portions_below(ctx, 16) == below and kernels._portion_tiles(ctx, t, 16, 128) == tiles
     else:   # never too few tiles, and never none below where there are some
         assert kernels._has_portions_below(ctx, 16) >= below and kernels._portion_tiles(ctx, t, 16, 128) >= tiles
+
+
+@pytest.mark.parametrize("lengths, alone", [([2000], False), ([8, 9], False), ([8, 6, 5], True), ([15, 1], True), ([24, 1], False), ([24] + [1] * 32, True),
+                                            ([32] + [1] * 200, False), ([30, 25, 6], True), ([40, 7], False), ([1, 1], True)])
+def test_delta_steps_that_go_token_by_token(lengths, alone):
+    assert kernels._delta_one_by_one(lengths) == alone and not kernels._delta_one_by_one(None)
+
+
+@pytest.mark.parametrize("lengths, alone", [([128], False), ([100] + [1] * 16, False), ([100] + [1] * 17, True), ([129] + [1] * 200, False), ([96] + [32] * 20, False),
+                                            ([96, 8], False), ([96, 9], True), ([129, 31], False)])
+def test_linear_attention_steps_that_go_token_by_token(lengths, alone):
+    assert kernels._linear_one_by_one(lengths) == alone and not kernels._linear_one_by_one(None)
+
+
+def test_portions_counted():
+    assert kernels._portions_from(context([8, 7, 33], "held"), 8) == 2 and kernels._portions_from(context([8, 7, 33], "empty"), 8) == 3

@@ -1,7 +1,10 @@
 // The gated delta rule over long portions of bfloat16 projections, 32 tokens at a time, float32 throughout.
 //
-// Read-outs come out at 2.0e-7 of their size from float64 and states as from the token-by-token kernel, whose read-outs lie at 1.7e-7:
-// nothing beside the rounding to bfloat16 that follows, but float32 projections stay with that kernel.
+// Distances from float64 for the same inputs, token by token and here: read-outs, before they are rounded to bfloat16, 1.10e-7 to
+// 1.30e-7 and 1.08e-7 to 1.24e-7 (9, 31, 64, 700 and 2,000 tokens); states 0.9e-7 to 1.5e-7 and 0.7e-7 to 1.1e-7.  That takes products
+// of U, of B U and of the new state to their last bit (tf32_terms.cuh), and K K^T and Q K^T added up in pairs; with two terms throughout
+// and a chain over the numbers it was 1.8e-7 and 1.5e-7, 182 us for 2,000 tokens instead of 220.  Float32 projections stay with the
+// token-by-token kernel.
 //
 // Within a chunk, with g_l the decays, c_i = g_1 .. g_i (from the chunk's start up to token i), r_j = g_(j+1) .. g_32 and S the
 // state before the chunk, the writes u_i of its tokens are the rows of
@@ -18,7 +21,7 @@
 //                        comes in with cp.async one chunk ahead.  [K; Q] S (16 rows and a quarter of the keys' numbers a warp),
 //                        V - .. and W (..) by four warps while four others make the last chunk's O, then the new state (16 x 8
 //                        of its numbers a warp, which stay in its registers as float32), all on the tensor cores with operands
-//                        in two terms.
+//                        in terms.
 // W and B are zero above the diagonal, and zero times what is not finite is not zero: a sum that comes out not finite is made again from
 // its own terms, the tokens up to its own, so that a token reaches later ones only.
 // Chunks are counted through the step's portions of at least ``min_tokens`` tokens in order; a portion's last chunk is filled up
@@ -26,7 +29,7 @@
 //
 // What bounds it: the chain, by what its warps issue (53 % of the slots busy; splitting operands is the largest share) and the
 // barriers between its three phases, on as many SMs as there are heads and runs of 16 columns.  2,000 tokens of 16 heads:
-// chain 168 us, chunks 17.  The same chain on the CUDA cores was bound by what shared memory hands to registers (238 us); the
+// 220 us, all but about 20 of them the chain.  The same chain on the CUDA cores was bound by what shared memory hands to registers (238 us); the
 // token-by-token kernel (delta_rule.cu) waits for a butterfly every two tokens (611 us).  Eight warps a block and two blocks an
 // SM took as long.
 #include "delta_common.cuh"
@@ -88,27 +91,53 @@ delta_chunk_kernel(const float* __restrict__ qkv, const float* __restrict__ bd, 
     const bool query = threadIdx.x >= 64;
     const float* left = (query ? qs : ks) + ti * KP;
     const float* right = ks + tj * KP;
-    uint64_t acc[4][4] = {};
-#pragma unroll 4
-    for (int d = 0; d < RP; d += 4) {
-      Pairs a[4], b[4];
+    // 16 numbers at a time, then in pairs: a single chain over the 128 was what lost most of a read-out
+    auto block = [&](int d0, float (&out)[4][4]) {
+      uint64_t acc[4][4] = {};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        a[e] = load4(left + e * 8 * KP + d);
-        b[e] = load4(right + e * 8 * KP + d);
+      for (int d = d0; d < d0 + 16; d += 4) {
+        Pairs a[4], b[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          a[e] = load4(left + e * 8 * KP + d);
+          b[e] = load4(right + e * 8 * KP + d);
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+          for (int y = 0; y < 4; ++y) {
+            fma2(acc[x][y], a[x].lo, b[y].lo);
+            fma2(acc[x][y], a[x].hi, b[y].hi);
+          }
       }
 #pragma unroll
       for (int x = 0; x < 4; ++x)
 #pragma unroll
-        for (int y = 0; y < 4; ++y) {
-          fma2(acc[x][y], a[x].lo, b[y].lo);
-          fma2(acc[x][y], a[x].hi, b[y].hi);
-        }
+        for (int y = 0; y < 4; ++y) out[x][y] = both(acc[x][y]);
+    };
+    auto add = [](float (&to)[4][4], const float (&what)[4][4]) {
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) to[x][y] += what[x][y];
+    };
+    float total[4][4] = {};
+#pragma unroll 1
+    for (int d = 0; d < RP; d += 64) {
+      float p[4][4], r[4][4], u[4][4];
+      block(d, p);
+      block(d + 16, r);
+      add(p, r);
+      block(d + 32, r);
+      block(d + 48, u);
+      add(r, u);
+      add(p, r);
+      add(total, p);
     }
 #pragma unroll
     for (int x = 0; x < 4; ++x)
 #pragma unroll
-      for (int y = 0; y < 4; ++y) (query ? qk : kk)[ti + 8 * x][tj + 8 * y] = both(acc[x][y]);
+      for (int y = 0; y < 4; ++y) (query ? qk : kk)[ti + 8 * x][tj + 8 * y] = total[x][y];
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per = H / G;
@@ -153,7 +182,7 @@ delta_chunk_kernel(const float* __restrict__ qkv, const float* __restrict__ bd, 
   pdl_trigger();  // at the end: the chain's blocks are few and long (see delta_prepare_kernel)
 }
 
-// ---- the chain, on the tensor cores, operands in two terms (tf32_terms.cuh) ---------------------------------------------
+// ---- the chain, on the tensor cores, operands in terms (tf32_terms.cuh) --------------------------------------------------
 struct ChainShape {
   static constexpr int K_AT = 0, Q_AT = K_AT + CHUNK * KP, SW_AT = Q_AT + CHUNK * KP, V_AT = SW_AT + CHUNK * TP;
   static constexpr int STAGE = V_AT + CHUNK * CP;                          // floats of a stage
@@ -233,7 +262,7 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
       if (k >= 2 && i0 < 16) break;  // B is triangular
       uint32_t ah[4], al[4];
       load_rows(a + 8 * k, 8 * TP, 4, ah, al);
-      y.step(ah, al, split(b[8 * k * CP]), split(b[(8 * k + 4) * CP]));
+      y.step<6>(ah, al, split(b[8 * k * CP]), split(b[(8 * k + 4) * CP]));
     }
     float total[4];
     y.totals(total);
@@ -291,7 +320,7 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
         uint32_t ah[4], al[4];
         load_rows(a + 8 * k, 8 * KP, 4, ah, al);
 #pragma unroll
-        for (int n = 0; n < 2; ++n) y[n].step(ah, al, load_split(b + (8 * k * SP + 8 * n) * 2), load_split(b + ((8 * k + 4) * SP + 8 * n) * 2));
+        for (int n = 0; n < 2; ++n) y[n].step<4>(ah, al, load_split(b + (8 * k * SP + 8 * n) * 2), load_split(b + ((8 * k + 4) * SP + 8 * n) * 2));
       }
       float* part = part_of(c) + (quarter * 2 * CHUNK + mt * 16 + gr) * CP + 2 * tg;
 #pragma unroll
@@ -317,7 +346,7 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
           const float y = (part[i] + part[2 * CHUNK * CP + i]) + (part[4 * CHUNK * CP + i] + part[6 * CHUNK * CP + i]);
           x[e] = split(fmaf(-ring[CHUNK * TP + 8 * k + 4 * e + tg], y, v[i]));
         }
-        u.step(ah, al, x[0], x[1]);
+        u.step<6>(ah, al, x[0], x[1]);
       }
       float total[4];
       u.totals(total);
@@ -356,7 +385,7 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
       for (int k = 0; k < CHUNK / 8; ++k) {
         uint32_t ah[4], al[4];
         load_rows(a + 8 * k * KP, 8, 4 * KP, ah, al);
-        d.step(ah, al, load_split(b + 8 * k * SP * 2), load_split(b + (8 * k + 4) * SP * 2));
+        d.step<6>(ah, al, load_split(b + 8 * k * SP * 2), load_split(b + (8 * k + 4) * SP * 2));
       }
       const float all = ring[CHUNK * TP + CHUNK - 1];
 #pragma unroll

@@ -10,15 +10,17 @@
 // Decays are only ever multiplied, never divided by, so P is made in blocks of 16 x 16 tokens: off the diagonal as products of
 // q_i alpha_(start of i's run) .. alpha_i and k_j alpha_(j+1) .. alpha_(end of j's run) with whole runs' decays between them, on the
 // diagonal with a running product a column (four columns a warp, four channels a lane).
-// Products of float32 numbers enter the tensor cores in two terms (tf32_terms.cuh), the values, which are bfloat16, as they are.
+// Products of float32 numbers enter the tensor cores in terms (tf32_terms.cuh: all of them for P, those of lo lo too for (Q c) S, P to
+// its last bit for P V), the values, which are bfloat16, as they are.
 // P is zero above the diagonal, and zero times a value that is not finite is not zero: a result that comes out not finite is made
 // again from the tokens up to its own.
-// Running products of decays carry what their roundings lose: with that the error against float64 is that of the token-by-token
-// kernels (read-outs 1.3e-7 of their size as before, states 0.8e-7 instead of 0.9e-7); a float32 projection's values would need two
-// terms too and come out at 1.5e-7 instead of 1.4e-7, so those stay with the other kernels.
+// Running products of decays carry what their roundings lose.  With that read-outs lie at 1.15e-7 to 1.18e-7 from float64, token by
+// token at 1.21e-7 to 1.25e-7 (100, 300 and 1,811 tokens), states at 0.80e-7 and 0.95e-7; with two terms throughout read-outs came out
+// at 1.28e-7 to 1.30e-7, 1,811 tokens in 119 us instead of 129.  A float32 projection's values would need terms too; those stay with the
+// other kernels.
 //
 // What bounds it: the read-out, by what its warps issue and by its five phases one after the other, one block of 16 warps an SM
-// (190 KB of shared memory).  1,811 tokens of 16 heads of 128: local 31 us, starts 11, read-out 77; the token-by-token kernels took
+// (190 KB of shared memory).  1,811 tokens of 16 heads of 128: local 31 us, starts 11, read-out 87; the token-by-token kernels took
 // 73, 13 and 114.  Eight warps a block took 112 us for the read-out.
 #include <type_traits>
 
@@ -36,7 +38,7 @@ __device__ __forceinline__ void load_row_pairs(const float* a, int down, float2 
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     const float2 x = *reinterpret_cast<const float2*>(a + e * down);
-    const Split u = split_centred(x.x, factor.x), v = split_centred(x.y, factor.y);
+    const Split u = split_product(x.x, factor.x), v = split_product(x.y, factor.y);
     hi[e] = u.hi;
     lo[e] = u.lo;
     hi[2 + e] = v.hi;
@@ -117,7 +119,7 @@ linear_local_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const 
       load_rows(kr + (8 * k + tg) * KP + d0, 8, 4 * KP, ah, al);
       const float* b = vs + (8 * k + tg) * KP + c0 + gr;
 #pragma unroll
-      for (int m = 0; m < 2; ++m) y[m].step(ah, al, b[8 * m], b[4 * KP + 8 * m]);
+      for (int m = 0; m < 2; ++m) y[m].step<false>(ah, al, b[8 * m], b[4 * KP + 8 * m]);
     }
 #pragma unroll
     for (int m = 0; m < 2; ++m)
@@ -294,7 +296,7 @@ linear_read_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const f
       uint32_t ah[4], al[4];
       queries(m, f, k, ah, al);
       const float2 b = *reinterpret_cast<const float2*>(ks + (j * RUN + c0 + gr) * KP + 8 * k + 2 * tg);
-      y.step(ah, al, split_centred(b.x), split_centred(b.y), k & 1);
+      y.step<6>(ah, al, split(b.x), split(b.y), k & 1);
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r)
@@ -312,7 +314,7 @@ linear_read_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const f
     queries(m, fs + m * RP, k, ah, al);
     const float* b = ss + (8 * k + 2 * tg) * VP + c0 + gr;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) y[c].step(ah, al, split_centred(b[8 * c]), split_centred(b[VP + 8 * c]), k & 1);
+    for (int c = 0; c < 4; ++c) y[c].step<4>(ah, al, split(b[8 * c]), split(b[VP + 8 * c]), k & 1);
   }
 #pragma unroll 2
   for (int k = 0; k < 2 * (m + 1); ++k) {
@@ -320,7 +322,7 @@ linear_read_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const f
     load_row_pairs(ps + (m * RUN + gr) * PP + 8 * k + 2 * tg, 8 * PP, make_float2(1.f, 1.f), ah, al);
     const float* b = vs + (8 * k + 2 * tg) * VP + c0 + gr;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) y[c].step(ah, al, b[8 * c], b[VP + 8 * c], k & 1);
+    for (int c = 0; c < 4; ++c) y[c].step<true>(ah, al, b[8 * c], b[VP + 8 * c], k & 1);
   }
 #pragma unroll
   for (int r = 0; r < 2; ++r) {

@@ -1,8 +1,9 @@
 // Products of float32 numbers on the tensor cores.
 //
-// mma.sync m16n8k8 multiplies numbers of 11 bits.  A float32 number enters as hi (rounded to nearest) + lo (22 bits), and a product as
-// hi hi + hi lo + lo hi.  The sums of the hi hi products leave the tensor cores after every eight terms and are added up in float32
-// with rounding to nearest, since the instruction cuts its sums off instead of rounding them.
+// mma.sync m16n8k8 multiplies numbers of 11 bits.  A float32 number enters as hi (rounded to nearest) + lo, what is left: the instruction
+// takes 11 bits of that (22 in all), and what it does not look at, the rest, enters as a third term where sums have to come out as
+// float32's own would.  The sums of the hi hi products leave the tensor cores after every eight terms and are added up in float32 with
+// rounding to nearest, since the instruction cuts its sums off instead of rounding them.
 #pragma once
 #include "common.cuh"
 
@@ -15,33 +16,47 @@ __device__ __forceinline__ Split split(float x) {
   const uint32_t hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
   return {hi, __float_as_uint(x - __uint_as_float(hi))};  // (the instruction does not look at lo's last 13 bits)
 }
-// ... with half of lo's last place added, so that what the instruction cuts off is centred; of a product, without rounding it first
-__device__ __forceinline__ Split split_centred(float x, float factor = 1.f) {
+__device__ __forceinline__ uint32_t rest(uint32_t lo) { return __float_as_uint(__uint_as_float(lo) - __uint_as_float(lo & 0xffffe000u)); }
+__device__ __forceinline__ Split split_product(float x, float factor) {  // of a product, without rounding it first
   const uint32_t hi = (__float_as_uint(x * factor) + 0x1000u) & 0xffffe000u;
-  return {hi, __float_as_uint(fmaf(x, factor, -__uint_as_float(hi)) * (1.f + 0x1.6p-12f))};
+  return {hi, __float_as_uint(fmaf(x, factor, -__uint_as_float(hi)))};
 }
 __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const float (&c)[4]) {
   asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
                : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
 }
-// One step of eight terms: sum += hi hi (rounded to nearest), small += hi lo + lo hi.  Long sums go in several chains, which lose less.
+// One step of eight terms: sum += hi hi (rounded to nearest), small += hi lo + lo hi; with PRODUCTS 4 also lo lo, with 6 also hi rest +
+// rest hi: operands to their last bit.  Long sums go in several chains, which lose less.
 template <int CHAINS>
 struct Sums {
   float sum[CHAINS][4] = {}, small[2][4] = {};
+  template <int PRODUCTS>
   __device__ __forceinline__ void step(const uint32_t (&ah)[4], const uint32_t (&al)[4], Split b0, Split b1, int chain = 0) {
+    static_assert(PRODUCTS == 4 || PRODUCTS == 6, "lo lo, or all");
     const float zero[4] = {};
     float d[4];
+    if constexpr (PRODUCTS == 6) {
+      const uint32_t ar[4] = {rest(al[0]), rest(al[1]), rest(al[2]), rest(al[3])};
+      mma_tf32(small[0], ah, rest(b0.lo), rest(b1.lo), small[0]);
+      mma_tf32(small[1], ar, b0.hi, b1.hi, small[1]);
+    }
+    mma_tf32(small[1], al, b0.lo, b1.lo, small[1]);
     mma_tf32(d, ah, b0.hi, b1.hi, zero);
     mma_tf32(small[0], ah, b0.lo, b1.lo, small[0]);
     mma_tf32(small[1], al, b0.hi, b1.hi, small[1]);
 #pragma unroll
     for (int e = 0; e < 4; ++e) sum[chain][e] += d[e];
   }
-  // the right operand's numbers are of eleven bits or fewer themselves (bfloat16)
+  // the right operand's numbers are of eleven bits or fewer themselves (bfloat16); WHOLE: the left one's to their last bit
+  template <bool WHOLE>
   __device__ __forceinline__ void step(const uint32_t (&ah)[4], const uint32_t (&al)[4], float b0, float b1, int chain = 0) {
     const float zero[4] = {};
     float d[4];
+    if constexpr (WHOLE) {
+      const uint32_t ar[4] = {rest(al[0]), rest(al[1]), rest(al[2]), rest(al[3])};
+      mma_tf32(small[0], ar, __float_as_uint(b0), __float_as_uint(b1), small[0]);
+    }
     mma_tf32(d, ah, __float_as_uint(b0), __float_as_uint(b1), zero);
     mma_tf32(small[1], al, __float_as_uint(b0), __float_as_uint(b1), small[1]);
 #pragma unroll

@@ -11,7 +11,7 @@
 //
 // What bounds it: the cached rows (512 bytes a key and head).  32 tokens that read 255 MB of rows together: 56 us and the merge 6, 4.6
 // TB/s (the kernel it stands in for 119 us: it copied every row with a lane's own cp.async and spent two products on the weights).
-// A token by itself at 1,900 keys: 6 us and 5.
+// Calls that read few rows stay with that one (ROWS_DECODE_LEAST in ops/kernels.py).
 //
 // Every wait on an mbarrier is bounded (tcgen05.cuh).
 #include <cfloat>

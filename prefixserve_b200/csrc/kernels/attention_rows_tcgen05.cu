@@ -22,7 +22,8 @@
 // A launch takes as many rounds over the SMs as it has CTAs for, and a last round that is nearly empty costs as much as a full
 // one.  The units (128 tokens, two heads) of such a round are therefore cut into ranges of keys, a CTA each, which leave
 // unnormalised results for attention_rows_merge_kernel; so are those of a step that is small to begin with (two portions of
-// 1,500 and 1,200 tokens, 176 units for 148 SMs: 91 -> 76 us; 256 tokens behind 2,000: 49 -> 24).
+// 1,500 and 1,200 tokens, 176 units for 148 SMs: 91 -> 76 us, 80 since masked scores have no say in the form of the cap and the
+// gate is exact; 256 tokens behind 2,000: 49 -> 24).
 //
 // Every wait on an mbarrier is bounded (tcgen05.cuh).
 #include "tcgen05.cuh"

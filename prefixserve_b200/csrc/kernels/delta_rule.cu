@@ -22,8 +22,8 @@
 // per request also brings the slot's convolution inputs up to date (the last K-1 rows of the projection, or what
 // was there before, moved up, when the portion is shorter).
 //
-// Portions of a few dozen tokens and more of the usual sizes go through the kernels of delta_chunks.cu instead, which need
-// neither the single steps nor:
+// Portions of eight tokens and more of bfloat16 projections (keys of up to 128 numbers in fours) go through the kernels of
+// delta_chunks.cu instead, which need neither the single steps nor:
 //
 // delta_cross_kernel (a warp per token and head): q.k, and k.k' and q.k' with the key of the token before.
 //

@@ -17,8 +17,8 @@
 //
 // What bounds it: the tensor cores' legacy path (three terms: 108 + 96 instructions a warp and tile, 1,024 multiply-adds a
 // clock and SM; busy 48 % of the time).  The kernel on the CUDA cores beside it (latent_attention_rows_kernel, still used for
-// other sizes) reads every row once for each pair of heads: 16 tokens of 32 heads over up to 3,500 keys took it 401 us, this
-// one 47; 8 tokens of 16 heads over a window of 1,024 take 9.
+// other sizes) reads every row once for each pair of heads: 16 tokens of 32 heads over up to 3,500 keys took it 402 us a call, this
+// one and its merge 61 (54 with a chain of instructions over a block's keys).
 #include "common.cuh"
 
 #include <cfloat>

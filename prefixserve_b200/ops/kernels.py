@@ -1178,7 +1178,7 @@ DELTA_LONG_LANES = 16   # measured: 32 lanes (a column a warp) took 807 us for a
 
 
 # Portions of this many tokens in bfloat16 take the form that works 32 tokens at a time (keys of up to 128 numbers).  All four kernels, 16 heads over 8
-# groups of 128: one portion of 8 tokens 25 us in chunks and 37 token by token, of 32 tokens 28 and 44; three of 24 and fewer 37 and 63.
+# groups of 128, nothing in L2: one portion of 8 tokens 35 us in chunks and 47 token by token, of 32 tokens 37 and 55, of 128 53 and 86.
 DELTA_CHUNKED = 8
 
 
@@ -1396,9 +1396,9 @@ def low_rank(a: torch.Tensor, w: torch.Tensor, function: str, *, bias: torch.Ten
 
 
 # Steps with a portion of LINEAR_CHUNKED tokens take the kernels that work 64 tokens at a time on the tensor cores, where the sizes are
-# theirs, for portions of LINEAR_SHORT tokens and more; shorter ones go token by token beside them (30 us for one chunk against 29 for 64
-# tokens one by one and 44 for 100, 16 heads of 128; and up to 14 us for what stays).  In other steps a longest portion of more than two
-# LINEAR_ATTENTION_CHUNK cuts the portions into chunks that go token by token side by side.
+# theirs, for portions of LINEAR_SHORT tokens and more; shorter ones go token by token behind them (100 tokens 34 us against 48 one by one,
+# 8 heads of 128; and some 14 us for what stays).  In other steps a longest portion of more than two LINEAR_ATTENTION_CHUNK cuts the
+# portions into chunks that go token by token side by side.
 LINEAR_CHUNKED, LINEAR_SHORT = 96, 32
 LINEAR_ATTENTION_CHUNK = 64
 

@@ -206,11 +206,11 @@ _SIGNATURES: dict[str, list] = {
     "psb_attention_rows_merge": [P, P, P, I, I, I, I, P, L, L, F, P],
     "psb_delta_max_taps": [],
     # (proj, dtype, ld, beta_at, ba, decay, taps, a_log, dt_bias, state, positions, token_item, item_start, slots, qkv_out, bd_out, T,
-    #  G, H, dim, vdim, K, num_slots, slot_floats, stream)
+    #  G, H, dim, vdim, K, num_slots, slot_floats, cross, stream)
     "psb_delta_prepare": [P, I, L, I, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, L, I, P],
     # (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, o_out, items, G, H, dim, vdim, K, num_slots, slot_floats, lanes, stream)
     "psb_channel_delta_rule": [P, P, P, P, I, L, P, P, P, P, I, I, I, I, I, I, I, L, I, P],
-    # (qkv, bd, proj, dtype, state, item_start, slots, o_out, items, G, H, dim, vdim, K, num_slots, slot_floats, lanes, stream)
+    # (qkv, bd, proj, dtype, state, item_start, slots, o_out, items, G, H, dim, vdim, K, num_slots, slot_floats, lanes, max_tokens, stream)
     "psb_delta_rule": [P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, L, I, I, P],
     # (dim, vdim) -> float32 numbers of a chunk's record of a head, 0: not built for the sizes; () -> tokens of a chunk
     "psb_delta_chunk_record": [I, I],

@@ -126,7 +126,8 @@ class Part:
 
     # True when forward() launches the same device work for the same tensor shapes, reading everything that varies
     # from device memory (then a decode step can be captured once and replayed).  A part that loops over
-    # ``ctx.items`` on the host must leave this False.
+    # ``ctx.items`` on the host must leave this False.  (The items' lengths may choose among kernels and size their
+    # grids: a captured step is keyed by every item's length, in order.)
     graph_safe = False
 
     # A mixer or feed-forward whose result is one matrix product of rows it has made may offer those rows instead: how many

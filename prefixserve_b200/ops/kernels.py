@@ -1191,7 +1191,6 @@ def _delta_one_by_one(lengths: list[int] | None) -> bool:
     return bool(short) and max(lengths) < min(DELTA_LONG_PORTION, 13 + 3 * max(short) + len(short) * 5 // 8)
 
 
-
 def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
                gain: torch.Tensor, state: torch.Tensor, ctx, *, groups: int, heads: int, dim: int, vdim: int, eps: float) -> torch.Tensor:
     """The gated delta rule over every portion of the step.  proj [T, 2*groups*dim + 2*heads*vdim] (queries, keys,

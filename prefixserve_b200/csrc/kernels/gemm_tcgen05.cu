@@ -1,6 +1,6 @@
 // C[M,N] = A[M,K] * W[N,K]^T in bfloat16 on the 5th-generation tensor cores, for many rows (prefill).
 //
-// Persistent, warp-specialised CTAs (one per SM), 192 threads, output tiles of 128 rows by BN columns (256, 192 or
+// Persistent, warp-specialised CTAs (one per SM), 320 threads, output tiles of 128 rows by BN columns (256, 192 or
 // 128: the widest that still gives every SM a tile; a few hundred rows against a narrow matrix take the narrow ones):
 //   warp 0      producer: one lane issues TMA loads (cp.async.bulk.tensor.2d) of a 128x64 tile of A and two
 //               (BN/2)x64 tiles of W per stage into 128-byte-swizzled shared memory; completion by mbarrier
@@ -9,7 +9,8 @@
 //               with shared-memory matrix descriptors; accumulators are float32 in tensor memory (two buffers 256
 //               columns apart, so the epilogue of one tile overlaps the main loop of the next); tcgen05.commit hands
 //               stages back to the producer and finished accumulators to the epilogue;
-//   warps 2..5  epilogue: tcgen05.ld (32 lanes x 32 columns per instruction) -> registers -> bfloat16 -> global.
+//   warps 2..9  epilogue: tcgen05.ld (32 lanes x 32 columns per instruction) -> registers -> bfloat16 -> global.
+// Products of many tiles go two CTAs to a tile of 256 rows (gemm_tcgen05_pair_kernel below).
 // The two W tiles of a stage are rows [n0, n0+BN/2) and [n1, n1+BN/2): for a plain product n1 = n0 + BN/2; for the
 // gated feed-forward n0 indexes the gate rows and n1 the matching up rows, and the epilogue writes
 // silu(gate) * up, so the [T, 2I] intermediate never exists (prefixserve/model/llama.py:120-121 of PrefixServe;
@@ -30,7 +31,11 @@ namespace {
 
 constexpr int BM = 128, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;        // 16 KB
-constexpr int THREADS = 192;
+// Warps that store a tile: two on each quarter of its rows, half the columns each; four where a row's angles fill the registers.  With four, and a
+// division and a choice of the activation a number, the epilogue was what bounded products with short contractions: 8,148 rows of 32 experts, K 2,048
+// gated and 1,024 plain, 208 us with four and 129 with eight (two CTAs a tile both).
+constexpr int store_warps(int hb) { return hb > 0 ? 4 : 8; }
+constexpr int threads(int hb) { return 32 * (2 + store_warps(hb)); }
 constexpr int TMEM_COLS = 512;              // two accumulator buffers, 256 float32 columns apart
 constexpr int ACC_STRIDE = 256;
 constexpr int MAX_STAGES = 6;
@@ -74,7 +79,6 @@ enum : int { MODE_PLAIN = 0, MODE_GATED = 1, MODE_ROPE = 2, MODE_GATED_GELU = 3,
 // u = clamp(up, -limit, limit), the three numbers in a GluClip (common.cuh).
 using GluArgs = GluClip;
 __device__ __forceinline__ bool mode_is_gated(int mode) { return mode == MODE_GATED || mode == MODE_GATED_GELU || mode == MODE_GATED_CLIPPED || mode == MODE_GATED_SCALED; }
-__device__ __forceinline__ float clipped_gate(float g, float u, const GluArgs& a) { return clipped_gate_value(g, u, a); }
 // MODE_RELU2: columns as in 0, the epilogue stores max(sum, 0)^2.  MODE_SILU, MODE_GELU: the same with SiLU or the tanh form of
 // GELU of the sum.
 //
@@ -163,9 +167,121 @@ __device__ __forceinline__ void rope_store_row(uint32_t taddr, int row, int M, i
   }
 }
 
+// One thread's row of a tile of sums: what the epilogue does, in two parts around the wait for the sums.
+template <int BN, int HB>
+struct Epilogue {
+  static constexpr int BN_HALF = BN / 2, PARTS = store_warps(HB) / 4;
+  int pos = 0, page = -1;
+  float cs[HB > 0 ? HB : 1][8], sn[HB > 0 ? HB : 1][8];  // HB > 0: the angles of this row's position, all of a head's pairs
+
+  __device__ __forceinline__ void before(int row, int M, int mode, const RopeArgs& rope) {
+    if (mode == MODE_ROPE && row < M) {  // this row's token: where it stands and which page takes it (inputs of the step)
+      pos = rope.positions[row];
+      page = rope.table[(size_t)rope.token_item[row] * rope.table_width + (pos >> rope.page_shift)];
+      if (HB > 0 && rope.cos_t) {
+        const int safe = pos < 0 ? 0 : (pos >= rope.max_positions ? rope.max_positions - 1 : pos);
+        const float4* cp = reinterpret_cast<const float4*>(rope.cos_t + (size_t)safe * (rope.D >> 1));
+        const float4* sp = reinterpret_cast<const float4*>(rope.sin_t + (size_t)safe * (rope.D >> 1));
+#pragma unroll
+        for (int b = 0; b < (HB > 0 ? HB : 1); ++b) {
+          const float4 c0 = __ldg(cp + 2 * b), c1 = __ldg(cp + 2 * b + 1), s0 = __ldg(sp + 2 * b), s1 = __ldg(sp + 2 * b + 1);
+          cs[b][0] = c0.x; cs[b][1] = c0.y; cs[b][2] = c0.z; cs[b][3] = c0.w; cs[b][4] = c1.x; cs[b][5] = c1.y; cs[b][6] = c1.z; cs[b][7] = c1.w;
+          sn[b][0] = s0.x; sn[b][1] = s0.y; sn[b][2] = s0.z; sn[b][3] = s0.w; sn[b][4] = s1.x; sn[b][5] = s1.y; sn[b][6] = s1.z; sn[b][7] = s1.w;
+        }
+      }
+    }
+  }
+  template <typename Value>
+  __device__ __forceinline__ static void gated_columns(uint32_t taddr, int row, int M, int n0, __nv_bfloat16* crow, int N_out, int ldc, int part, Value value) {
+#pragma unroll 1
+    for (int c = part * (BN_HALF / PARTS); c < (part + 1) * (BN_HALF / PARTS); c += 32) {
+      uint32_t g[32], u[32];
+      tmem_ld32(taddr + c, g);
+      tmem_ld32(taddr + BN_HALF + c, u);
+      tmem_ld_wait();
+      if (row >= M) continue;
+#pragma unroll
+      for (int j = 0; j < 32; j += 8) {
+        const int col = n0 + c + j;
+        uint32_t packed[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          // the reference rounds both projections to bfloat16 before the activation
+          const uint32_t gb = pack2(__uint_as_float(g[j + 2 * q]), __uint_as_float(g[j + 2 * q + 1]));
+          const uint32_t ub = pack2(__uint_as_float(u[j + 2 * q]), __uint_as_float(u[j + 2 * q + 1]));
+          packed[q] = pack2(value(__uint_as_float(gb << 16), __uint_as_float(ub << 16)),
+                            value(__uint_as_float(gb & 0xffff0000u), __uint_as_float(ub & 0xffff0000u)));
+        }
+        if (col + 8 <= N_out && (ldc & 7) == 0) {
+          *reinterpret_cast<uint4*>(crow + col) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        } else {
+          const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(packed);
+          for (int q = 0; q < 8; ++q)
+            if (col + q < N_out) crow[col + q] = e[q];
+        }
+      }
+    }
+  }
+  // (M: rows there are; the tile's columns start at n0; part: which half of the columns, where two warps share the rows)
+  __device__ __forceinline__ void store(uint32_t taddr, int row, int M, int n0, __nv_bfloat16* __restrict__ C, int N_out, int ldc, int mode, bool gated,
+                                        const RopeArgs& rope, const GluArgs& glu, const float* __restrict__ row_scale, int part) const {
+    __nv_bfloat16* crow = C + (size_t)row * ldc;
+    if (mode == MODE_ROPE) {
+      rope_store_row<BN, HB>(taddr, row, M, n0, N_out, rope, pos, page, cs, sn);
+    } else if (gated) {
+      // the activation is chosen once a tile, not once a number
+      const float rs = mode == MODE_GATED_SCALED && row < M ? row_scale[row] : 1.f;
+      auto gate = [&](auto value) { gated_columns(taddr, row, M, n0, crow, N_out, ldc, part, value); };
+      // (__fdividef is within two units of the last place of float32; the result is rounded to bfloat16)
+      if (mode == MODE_GATED) gate([](float g, float u) { return __fdividef(g, 1.f + __expf(-g)) * u; });
+      else if (mode == MODE_GATED_SCALED) gate([rs](float g, float u) { return __fdividef(rs * g, 1.f + __expf(-rs * g)) * (rs * u); });
+      else if (mode == MODE_GATED_CLIPPED) gate([&](float g, float u) {
+        g = fminf(g, glu.limit), u = fminf(fmaxf(u, -glu.limit), glu.limit);
+        return __fdividef(g, 1.f + expf(-glu.alpha * g)) * (u + glu.offset);
+      });
+      else gate([](float g, float u) { return gate_act(g, PSB_ACT_GELU_TANH) * u; });
+    } else {
+      constexpr int SPAN = (BN / PARTS + 31) / 32 * 32;
+#pragma unroll 1
+      for (int c = part * SPAN; c < BN && c < (part + 1) * SPAN; c += 32) {
+        uint32_t v[32];
+        tmem_ld32(taddr + c, v);  // (a tile of 240 columns: the last load reads 16 columns beyond it, which nobody stores)
+        tmem_ld_wait();
+        if (row < M) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 8) {
+            if (BN % 32 != 0 && c + j >= BN) break;
+            const int col = n0 + c + j;
+            uint32_t packed[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              float v0 = __uint_as_float(v[j + 2 * q]), v1 = __uint_as_float(v[j + 2 * q + 1]);
+              if (mode == MODE_RELU2) {
+                v0 = fmaxf(v0, 0.f), v1 = fmaxf(v1, 0.f);
+                v0 *= v0, v1 *= v1;
+              } else if (mode == MODE_SILU || mode == MODE_GELU) {
+                const int act = mode == MODE_SILU ? PSB_ACT_SILU : PSB_ACT_GELU_TANH;
+                v0 = quick_act(v0, act), v1 = quick_act(v1, act);
+              }
+              packed[q] = pack2(v0, v1);
+            }
+            if (col + 8 <= N_out && (ldc & 7) == 0) {
+              *reinterpret_cast<uint4*>(crow + col) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            } else {
+              const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(packed);
+              for (int q = 0; q < 8; ++q)
+                if (col + q < N_out) crow[col + q] = e[q];
+            }
+          }
+        }
+      }
+    }
+  }
+};
+
 // BN: see Tile.  HB: see rope_store_row (0 unless mode is MODE_ROPE and the head size is 16 * HB).
 template <int BN, int HB>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(threads(HB), 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     __nv_bfloat16* __restrict__ C, int M, int N_out, int K, int ldc, int up_offset, int mode,
                     const RopeArgs rope, const int32_t* __restrict__ tile_expert, const GluArgs glu,
@@ -194,7 +310,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars->acc_full[b], 1);
-      mbar_init(&bars->acc_empty[b], 4);  // one arrival per epilogue warp
+      mbar_init(&bars->acc_empty[b], store_warps(HB));  // one arrival per epilogue warp
     }
     bars->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -280,100 +396,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int m0 = (tile % m_blocks) * BM;
       const int n0 = (tile / m_blocks) * n_span;
       const int row = m0 + quarter * 32 + lane;
-      int pos = 0, page = -1;
-      float cs[HB > 0 ? HB : 1][8], sn[HB > 0 ? HB : 1][8];  // HB > 0: the angles of this row's position, all of a head's pairs
-      if (mode == MODE_ROPE && row < M) {  // this row's token: where it stands and which page takes it (inputs of the step)
-        pos = rope.positions[row];
-        page = rope.table[(size_t)rope.token_item[row] * rope.table_width + (pos >> rope.page_shift)];
-        if (HB > 0 && rope.cos_t) {
-          const int safe = pos < 0 ? 0 : (pos >= rope.max_positions ? rope.max_positions - 1 : pos);
-          const float4* cp = reinterpret_cast<const float4*>(rope.cos_t + (size_t)safe * (rope.D >> 1));
-          const float4* sp = reinterpret_cast<const float4*>(rope.sin_t + (size_t)safe * (rope.D >> 1));
-#pragma unroll
-          for (int b = 0; b < (HB > 0 ? HB : 1); ++b) {
-            const float4 c0 = __ldg(cp + 2 * b), c1 = __ldg(cp + 2 * b + 1), s0 = __ldg(sp + 2 * b), s1 = __ldg(sp + 2 * b + 1);
-            cs[b][0] = c0.x; cs[b][1] = c0.y; cs[b][2] = c0.z; cs[b][3] = c0.w; cs[b][4] = c1.x; cs[b][5] = c1.y; cs[b][6] = c1.z; cs[b][7] = c1.w;
-            sn[b][0] = s0.x; sn[b][1] = s0.y; sn[b][2] = s0.z; sn[b][3] = s0.w; sn[b][4] = s1.x; sn[b][5] = s1.y; sn[b][6] = s1.z; sn[b][7] = s1.w;
-          }
-        }
-      }
+      Epilogue<BN, HB> epilogue;
+      epilogue.before(row, M, mode, rope);
       ok = mbar_wait(&bars->acc_full[buf], use & 1, abort, 3);
       if (!ok) break;
       fence_after();
       const uint32_t taddr = tmem_base + buf * ACC_STRIDE + ((uint32_t)(quarter * 32) << 16);
-      __nv_bfloat16* crow = C + (size_t)row * ldc;
-      if (mode == MODE_ROPE) {
-        rope_store_row<BN, HB>(taddr, row, M, n0, N_out, rope, pos, page, cs, sn);
-      } else if (gated) {
-        const float rs = mode == MODE_GATED_SCALED && row < M ? row_scale[row] : 1.f;
-#pragma unroll 1
-        for (int c = 0; c < BN_HALF; c += 32) {
-          uint32_t g[32], u[32];
-          tmem_ld32(taddr + c, g);
-          tmem_ld32(taddr + BN_HALF + c, u);
-          tmem_ld_wait();
-          if (row < M) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              const int col = n0 + c + j;
-              uint32_t packed[4];
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                // the reference rounds both projections to bfloat16 before the activation
-                const float g0 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(g[j + 2 * q])));
-                const float g1 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(g[j + 2 * q + 1])));
-                const float u0 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(u[j + 2 * q])));
-                const float u1 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(u[j + 2 * q + 1])));
-                packed[q] = mode == MODE_GATED ? pack2(g0 / (1.f + __expf(-g0)) * u0, g1 / (1.f + __expf(-g1)) * u1)
-                            : mode == MODE_GATED_SCALED ? pack2(rs * g0 / (1.f + __expf(-rs * g0)) * (rs * u0), rs * g1 / (1.f + __expf(-rs * g1)) * (rs * u1))
-                            : mode == MODE_GATED_CLIPPED ? pack2(clipped_gate(g0, u0, glu), clipped_gate(g1, u1, glu))
-                                               : pack2(gate_act(g0, PSB_ACT_GELU_TANH) * u0, gate_act(g1, PSB_ACT_GELU_TANH) * u1);
-              }
-              if (col + 8 <= N_out && (ldc & 7) == 0) {
-                *reinterpret_cast<uint4*>(crow + col) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-              } else {
-                const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(packed);
-                for (int q = 0; q < 8; ++q)
-                  if (col + q < N_out) crow[col + q] = e[q];
-              }
-            }
-          }
-        }
-      } else {
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t v[32];
-          tmem_ld32(taddr + c, v);  // (a tile of 240 columns: the last load reads 16 columns beyond it, which nobody stores)
-          tmem_ld_wait();
-          if (row < M) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (BN % 32 != 0 && c + j >= BN) break;
-              const int col = n0 + c + j;
-              uint32_t packed[4];
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                float v0 = __uint_as_float(v[j + 2 * q]), v1 = __uint_as_float(v[j + 2 * q + 1]);
-                if (mode == MODE_RELU2) {
-                  v0 = fmaxf(v0, 0.f), v1 = fmaxf(v1, 0.f);
-                  v0 *= v0, v1 *= v1;
-                } else if (mode == MODE_SILU || mode == MODE_GELU) {
-                  const int act = mode == MODE_SILU ? PSB_ACT_SILU : PSB_ACT_GELU_TANH;
-                  v0 = quick_act(v0, act), v1 = quick_act(v1, act);
-                }
-                packed[q] = pack2(v0, v1);
-              }
-              if (col + 8 <= N_out && (ldc & 7) == 0) {
-                *reinterpret_cast<uint4*>(crow + col) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-              } else {
-                const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(packed);
-                for (int q = 0; q < 8; ++q)
-                  if (col + q < N_out) crow[col + q] = e[q];
-              }
-            }
-          }
-        }
-      }
+      epilogue.store(taddr, row, M, n0, C, N_out, ldc, mode, gated, rope, glu, row_scale, (warp - 2) >> 2);
       fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->acc_empty[buf]);  // this warp has read its part of the buffer
@@ -389,6 +418,196 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   if (warp == 2) {
     fence_after();
     tmem_free(tmem_base, TMEM_COLS);
+  }
+}
+
+// ---- two CTAs on a tile of 256 rows by 256 columns ---------------------------------------------------------------------
+//
+// The same roles, in clusters of two CTAs (tcgen05 cta_group::2): each CTA brings its 128 rows of A and half of the tile's rows of W (the
+// gate's and the up rows, for the gated forms), the first one's MMA warp multiplies for both (M=256, N=256, K=16), and each CTA's
+// epilogue stores its own rows.  A stage is 32 KB instead of 48 for the same work, an operand of W crosses from L2 once for 256 rows, and six
+// stages are in flight.  The first CTA's full barriers count the bytes of both; commits arrive at both CTAs' barriers.
+//
+// Grouped products: a tile is a row tile of 128 and the next one if that is the same expert's (an expert's odd last one is a tile by itself whose other
+// half is computed against the wrong matrix and not stored); the CTAs list the tiles that hold rows first, so that every pair gets as many (dealt out
+// by the grid's stride with the empty ones among them, some CTAs had six and others two: 160 and 55 us for the products above, one CTA a tile).
+//
+// 1,979 tokens, K 4,096, 14,336 gated columns: 305 us on a cool GPU and 312 with one CTA a tile; in a loop, where power is the limit, both products of
+// the feed-forward take 557 us instead of 580.
+constexpr int PAIR_STAGES = 6, PAIR_STAGE = A_BYTES + 128 * BK * 2, MAX_UNITS = 2048;
+constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE + 1024 + 256 + MAX_UNITS * 2;
+constexpr int ALONE = 1 << 15;  // the unit's second row tile is another expert's
+static_assert(PAIR_STAGES <= MAX_STAGES && PAIR_SMEM <= 227 * 1024, "beyond a CTA's shared memory");
+
+template <int HB>
+__global__ void __launch_bounds__(threads(HB), 1)
+gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
+                         __nv_bfloat16* __restrict__ C, int M, int N_out, int K, int ldc, int up_offset, int mode,
+                         const RopeArgs rope, const int32_t* __restrict__ tile_expert, const GluArgs glu,
+                         const float* __restrict__ row_scale) {
+  constexpr int BN = 256, BN_HALF = BN / 2, STAGES = PAIR_STAGES;
+  constexpr uint32_t INSTR_DESC = instr_desc(2 * BM, BN, false);
+  const bool gated = mode_is_gated(mode);
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  Barriers* bars = reinterpret_cast<Barriers*>(tiles + STAGES * PAIR_STAGE);
+  uint16_t* units = reinterpret_cast<uint16_t*>(tiles + STAGES * PAIR_STAGE + 256);
+  volatile uint32_t* abort = &bars->abort;
+  __shared__ int listed;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+
+  const int n_span = gated ? BN_HALF : BN;
+  const int m_tiles = (M + BM - 1) / BM;
+  const int n_blocks = (N_out + n_span - 1) / n_span;
+  const int k_blocks = (K + BK - 1) / BK;
+
+  pdl_trigger();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&bars->full[s], 1);
+      mbar_init(&bars->empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&bars->acc_full[b], 1);
+      mbar_init(&bars->acc_empty[b], 2 * store_warps(HB));  // one arrival per epilogue warp of either CTA
+    }
+    bars->abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) tmem_alloc_pair(&bars->tmem_base, TMEM_COLS);
+  fence_before();
+  pdl_wait();  // A and the tiles' experts are the preceding kernels' output
+  if (tile_expert && warp == 0) {
+    int count = 0, run = 0, last = -1;  // units listed; row tiles of ``last`` so far
+    for (int t0 = 0; t0 < m_tiles; t0 += 32) {
+      const int t = t0 + lane;
+      const int expert = t < m_tiles ? tile_expert[t] : -1, next = t + 1 < m_tiles ? tile_expert[t + 1] : -1;
+      int before = __shfl_up_sync(0xffffffffu, expert, 1);
+      if (lane == 0) before = last;
+      const uint32_t starts = __ballot_sync(0xffffffffu, expert != before), upto = starts & (0xffffffffu >> (31 - lane));
+      const int place = upto ? lane - (31 - __clz(upto)) : run + lane;  // of its expert's row tiles
+      const bool opens = expert >= 0 && !(place & 1);
+      const uint32_t opening = __ballot_sync(0xffffffffu, opens);
+      const int at = count + __popc(opening & ((1u << lane) - 1));
+      if (opens && at < MAX_UNITS) units[at] = (uint16_t)(t | (next == expert ? 0 : ALONE));
+      count += __popc(opening);
+      last = __shfl_sync(0xffffffffu, expert, 31);
+      run = __shfl_sync(0xffffffffu, place, 31) + 1;
+    }
+    if (lane == 0) listed = count < MAX_UNITS ? count : MAX_UNITS;
+  }
+  __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers are there
+  fence_after();
+  const uint32_t tmem_base = bars->tmem_base;
+  const int m_units = tile_expert ? listed : (m_tiles + 1) / 2;
+  const int tiles_total = m_units * n_blocks;
+  // Tile -> row tile (its first), column tile, expert, and whether the second row tile counts.  Ungrouped, neighbours in time share a run of W and all of A
+  // is in use; grouped, they share an expert's rows, and its matrix is read from one end to the other.
+  struct Where {
+    int m0, n0, expert;
+    bool both;
+  };
+  auto where = [&](int tile) {
+    Where w;
+    if (tile_expert) {
+      const int u = units[tile / n_blocks];
+      w.n0 = tile % n_blocks * n_span;
+      w.both = !(u & ALONE);
+      w.m0 = (u & (ALONE - 1)) * BM;
+      w.expert = tile_expert[u & (ALONE - 1)];
+    } else {
+      w.m0 = tile % m_units * 2 * BM;
+      w.n0 = tile / m_units * n_span;
+      w.both = true;
+      w.expert = 0;
+    }
+    return w;
+  };
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ producer
+    if (elect_one()) {
+      uint32_t stage = 0, phase = 0;
+      bool ok = true;
+      for (int tile = pair; ok && tile < tiles_total; tile += pairs) {
+        const Where w = where(tile);
+        const int m0 = w.m0 + rank * BM;
+        int n0 = w.n0 + w.expert * (gated ? 2 * N_out : N_out);  // a gated expert holds its gate rows, then its up rows
+        if (rank) n0 += gated ? up_offset : BN_HALF;
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          ok = mbar_wait(&bars->empty[stage], phase ^ 1, abort, 1);
+          if (!ok) break;
+          unsigned char* a_dst = tiles + stage * PAIR_STAGE;
+          if (rank == 0) mbar_expect_tx(&bars->full[stage], 2 * PAIR_STAGE);
+          const uint32_t full = cluster_address(&bars->full[stage], 0);
+          tma_load_2d_pair(a_dst, &map_a, kb * BK, m0, full);
+          tma_load_2d_pair(a_dst + A_BYTES, &map_w, kb * BK, n0, full);
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ----------------------------------------------------------------------- MMA
+    if (rank == 0) {
+      uint32_t stage = 0, phase = 0, local = 0;
+      bool ok = true;
+      for (int tile = pair; ok && tile < tiles_total; tile += pairs) {
+        const uint32_t buf = local & 1, use = local >> 1;
+        ++local;
+        ok = mbar_wait(&bars->acc_empty[buf], (use & 1) ^ 1, abort, 4);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        fence_after();
+        const uint32_t acc = tmem_base + buf * ACC_STRIDE;
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          ok = mbar_wait(&bars->full[stage], phase, abort, 2);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          const uint64_t da = smem_desc(smem_u32(tiles + stage * PAIR_STAGE));
+          const uint64_t db = smem_desc(smem_u32(tiles + stage * PAIR_STAGE + A_BYTES));
+          const uint32_t hi = (uint32_t)(da >> 32), a_lo = (uint32_t)da, b_lo = (uint32_t)db;
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            if (elect_one()) mma_f16_split_pair(acc, a_lo + 2 * k, hi, b_lo + 2 * k, hi, INSTR_DESC, (kb | k) != 0);
+          if (elect_one()) mma_commit_pair(&bars->empty[stage]);
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+        if (ok && elect_one()) mma_commit_pair(&bars->acc_full[buf]);
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue
+    const int quarter = warp & 3;
+    uint32_t local = 0;
+    bool ok = true;
+    for (int tile = pair; ok && tile < tiles_total; tile += pairs) {
+      const uint32_t buf = local & 1, use = local >> 1;
+      ++local;
+      const Where w = where(tile);
+      const int row = w.m0 + rank * BM + quarter * 32 + lane, rows = rank && !w.both ? 0 : M;
+      Epilogue<BN, HB> epilogue;
+      epilogue.before(row, rows, mode, rope);
+      ok = mbar_wait(&bars->acc_full[buf], use & 1, abort, 3);
+      if (!ok) break;
+      fence_after();
+      epilogue.store(tmem_base + buf * ACC_STRIDE + ((uint32_t)(quarter * 32) << 16), row, rows, w.n0, C, N_out, ldc, mode, gated, rope, glu, row_scale, (warp - 2) >> 2);
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(cluster_address(&bars->acc_empty[buf], 0));
+    }
+  }
+  __syncwarp();
+  if (*abort) {
+    for (int i = 0; i < 200; ++i) __nanosleep(1000);  // copies in flight, as above
+  }
+  fence_before();
+  __syncthreads();
+  cluster_sync_all();  // the first CTA's instructions read the other's shared memory, and both arrive at each other's barriers
+  if (warp == 2) {
+    fence_after();
+    tmem_free_pair(tmem_base, TMEM_COLS);
   }
 }
 
@@ -413,7 +632,7 @@ int choose_width(int M, int N_out, bool gated, bool rope, int D, int sms) {
   for (int bn : {256, 240, 192, 128}) {
     if (bn == 192 && (gated || (rope && D == 128))) continue;
     if (bn == 240 && (gated || rope)) continue;  // whole heads and even halves want a power of two or 192
-    if (g_forced_width && bn != g_forced_width) continue;
+    if (g_forced_width && g_forced_width != 512 && bn != g_forced_width) continue;
     const int span = gated ? bn / 2 : bn;
     const long tiles = (long)m_blocks * ((N_out + span - 1) / span);
     const long cost = ((tiles + sms - 1) / sms) * (bn + 24);
@@ -424,6 +643,63 @@ int choose_width(int M, int N_out, bool gated, bool rope, int D, int sms) {
     }
   }
   return best;
+}
+
+// Whether two CTAs a tile get the product done sooner, by rounds: theirs of 256 x 256 takes about six sevenths of a single CTA's of 128 x 256 (the same work
+// an SM), the narrower tiles' as in choose_width.  Columns by K, rows, two CTAs against the best single width in us: 4,096 by 14,336, 1,979 rows 152 and
+// 176, 1,024 82 and 96, 700 (one round of 192 columns) 81 and 77; 2,048 by 8,192, 1,979 rows 53 and 61; 6,144 by 4,096, 1,979 rows 74 and 83;
+// 3,072 by 2,048, 1,979 rows (two rounds of 192) 35 and 30; gated 14,336 by 4,096, 1,024 rows 158 and 174.  Grouped products always: their rounds
+// depend on the routing, and pairs read an expert's matrix fewer times.
+bool pairs_pay(int M, int N_out, bool gated, int D, int bn, bool grouped, int sms) {
+  if (g_forced_width) return g_forced_width == 512;
+  if (sms < 2 || (M + BM - 1) / BM > MAX_UNITS) return false;
+  if (grouped) return true;
+  const long m_blocks = (M + BM - 1) / BM, span = gated ? bn / 2 : bn, span2 = gated ? 128 : 256;
+  const long rounds = (m_blocks * ((N_out + span - 1) / span) + sms - 1) / sms, rounds2 = ((m_blocks + 1) / 2 * ((N_out + span2 - 1) / span2) + sms / 2 - 1) / (sms / 2);
+  return rounds2 * (256 + 24) * 6 <= rounds * (bn + 24) * 7;
+}
+
+// ``tiles``: at most so many.  As many pairs as the device holds at once (asked once per device), no more than sms / 2.
+template <int HB>
+int launch_pairs(int tiles, int sms, cudaStream_t stream, const CUtensorMap& map_a, const CUtensorMap& map_w, void* c, int M, int N_out, int K, int ldc,
+                 int up_offset, int mode, const RopeArgs& rope, const int32_t* tile_expert, const GluArgs& glu, const float* row_scale) {
+  static PsbPerDevice configured;
+  static int resident[PsbPerDevice::kMaxDevices] = {};
+  auto kernel = gemm_tcgen05_pair_kernel<HB>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * (sms / 2));
+  cfg.blockDim = dim3(threads(HB));
+  cfg.dynamicSmemBytes = PAIR_SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const int dev = PsbPerDevice::current();
+  if (!configured.get()) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
+    if (e != cudaSuccess) PSB_REFUSE("gemm_tcgen05: cannot reserve %d bytes of shared memory: %s", PAIR_SMEM, cudaGetErrorString(e));
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = sms / 2;
+    }
+    if (dev >= 0) resident[dev] = n;
+    configured.set();
+  }
+  int pairs = dev >= 0 && resident[dev] > 0 && resident[dev] < sms / 2 ? resident[dev] : sms / 2;
+  if (tiles < pairs) pairs = tiles;
+  cfg.gridDim = dim3(2 * pairs);
+  if (psb_pdl_enabled) {
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
+  }
+  cudaLaunchKernelEx(&cfg, kernel, map_a, map_w, (__nv_bfloat16*)c, M, N_out, K, ldc, up_offset, mode, rope, tile_expert, glu, row_scale);
+  PSB_LAUNCH_CHECK("gemm_tcgen05");
+  return 0;
 }
 
 int launch(const void* a, const void* w, void* c, int M, int w_rows, int N_out, int K, int up_offset, int mode, int sms,
@@ -438,6 +714,13 @@ int launch(const void* a, const void* w, void* c, int M, int w_rows, int N_out, 
   const int bn = choose_width(M, N_out, gated, mode == MODE_ROPE, rope.D, sms);
   CUtensorMap map_a, map_w;
   if (int rc = make_map(&map_a, a, M, K, BM)) return rc;
+  if (pairs_pay(M, N_out, gated, mode == MODE_ROPE ? rope.D : 0, bn, tile_expert != nullptr, sms)) {
+    if (int rc = make_map(&map_w, w, w_rows, K, 128)) return rc;
+    const int span = gated ? 128 : 256, most = (tile_expert ? m_blocks : (m_blocks + 1) / 2) * ((N_out + span - 1) / span);
+    if (mode == MODE_ROPE && rope.D == 128) return launch_pairs<8>(most, sms, stream, map_a, map_w, c, M, N_out, K, ldc, up_offset, mode, rope, tile_expert, glu, row_scale);
+    if (mode == MODE_ROPE && rope.D == 64) return launch_pairs<4>(most, sms, stream, map_a, map_w, c, M, N_out, K, ldc, up_offset, mode, rope, tile_expert, glu, row_scale);
+    return launch_pairs<0>(most, sms, stream, map_a, map_w, c, M, N_out, K, ldc, up_offset, mode, rope, tile_expert, glu, row_scale);
+  }
   if (int rc = make_map(&map_w, w, w_rows, K, bn / 2)) return rc;
   const int n_span = gated ? bn / 2 : bn;
   const int tiles = m_blocks * ((N_out + n_span - 1) / n_span);
@@ -451,7 +734,7 @@ int launch(const void* a, const void* w, void* c, int M, int w_rows, int N_out, 
       if (e != cudaSuccess) PSB_REFUSE("gemm_tcgen05: cannot reserve %d bytes of shared memory: %s", Tile<BN>::SMEM_BYTES, cudaGetErrorString(e)); \
       configured.set();                                                                                              \
     }                                                                                                                \
-    psb_launch(gemm_tcgen05_kernel<BN, HB>, dim3(grid), dim3(THREADS), (size_t)Tile<BN>::SMEM_BYTES, stream, map_a,   \
+    psb_launch(gemm_tcgen05_kernel<BN, HB>, dim3(grid), dim3(threads(HB)), (size_t)Tile<BN>::SMEM_BYTES, stream, map_a,   \
                map_w, (__nv_bfloat16*)c, M, N_out, K, ldc, up_offset, mode, rope, tile_expert, glu, row_scale);      \
   } while (0)
   // the usual head sizes keep a row's angles in registers; every other multiple of 16 fetches them block by block
@@ -549,10 +832,10 @@ PSB_API int psb_gemm_tcgen05_rope(const void* a, const void* w, int M, int K, in
   return launch(a, w, q_out, M, N, N, K, 0, MODE_ROPE, sms, stream, rope);
 }
 
-// For tests: 128, 192, 240 or 256 makes every later product use that tile width where the shape allows it, 0 gives the
-// choice back.
+// For tests: 128, 192, 240 or 256 makes every later product use that tile width where the shape allows it, 512 two CTAs a tile of 256 x 256, 0 gives
+// the choice back.
 PSB_API int psb_gemm_tcgen05_tile_width(int width) {
-  if (width != 0 && width != 128 && width != 192 && width != 240 && width != 256) PSB_REFUSE("gemm_tcgen05: tile widths are 128, 192, 240 and 256, not %d", width);
+  if (width != 0 && width != 128 && width != 192 && width != 240 && width != 256 && width != 512) PSB_REFUSE("gemm_tcgen05: tile widths are 128, 192, 240, 256 and 512, not %d", width);
   g_forced_width = width;
   return 0;
 }

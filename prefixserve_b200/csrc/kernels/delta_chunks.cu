@@ -1,153 +1,209 @@
-// The gated delta rule over long portions of bfloat16 projections, 32 tokens at a time, float32 throughout.
+// The delta rules over portions, 32 tokens at a time, float32 throughout: the gated one (a decay per head; bfloat16 projections) and
+// the one with a decay per head and key channel.
 //
-// Distances from float64 for the same inputs, token by token and here: read-outs, before they are rounded to bfloat16, 1.10e-7 to
-// 1.30e-7 and 1.08e-7 to 1.24e-7 (9, 31, 64, 700 and 2,000 tokens); states 0.9e-7 to 1.5e-7 and 0.7e-7 to 1.1e-7.  That takes products
-// of U, of B U and of the new state to their last bit (tf32_terms.cuh), and K K^T and Q K^T added up in pairs; with two terms throughout
-// and a chain over the numbers it was 1.8e-7 and 1.5e-7, 182 us for 2,000 tokens instead of 220.  Float32 projections stay with the
-// token-by-token kernel.
+// Within a chunk, with g_l the decays (a vector over the key channels; the gated rule's are all alike), c_i = g_1 .. g_i (from the
+// chunk's start up to token i), r_j = g_(j+1) .. g_32 and S the state before the chunk, the writes u_i of its tokens are the rows of
 //
-// Within a chunk, with g_l the decays, c_i = g_1 .. g_i (from the chunk's start up to token i), r_j = g_(j+1) .. g_32 and S the
-// state before the chunk, the writes u_i of its tokens are the rows of
+//     U = W V - M S,         W = (I + diag(beta) A)^-1 diag(beta),  M = W (K c),   A_ij = sum_d k_i k_j g_(j+1) .. g_i   (j < i),
+//     O = (Q c) S + B U,     B_ij = sum_d q_i k_j g_(j+1) .. g_i   (j <= i),
+//     S <- c_32 S + (K r)^T U.
 //
-//     U = W (V - diag(c) K S),   W = (I + diag(beta) A)^-1 diag(beta),   A_ij = (k_i . k_j) g_(j+1) .. g_i   (j < i),
-//     O = diag(c) Q S + B U,     B_ij = (q_i . k_j) g_(j+1) .. g_i   (j <= i),
-//     S <- c_32 S + K^T diag(r) U.
-//
-// (Decays are only ever multiplied, never divided by.)  W and B do not depend on the state:
-//   delta_chunk_kernel   a block per chunk and query/key group, all chunks of the step side by side: K K^T and Q K^T of the group
-//                        once, then a warp per head its decays, B and W (forward substitution, a column a lane).  Leaves W, B, c
-//                        and r, 8.4 KB a chunk and head;
-//   delta_chain_kernel   a block of 16 warps per 16 columns of a head's state and request walks the chunks; what a chunk brings
-//                        comes in with cp.async one chunk ahead.  [K; Q] S (16 rows and a quarter of the keys' numbers a warp),
-//                        V - .. and W (..) by four warps while four others make the last chunk's O, then the new state (16 x 8
-//                        of its numbers a warp, which stay in its registers as float32), all on the tensor cores with operands
-//                        in terms.
-// W and B are zero above the diagonal, and zero times what is not finite is not zero: a sum that comes out not finite is made again from
-// its own terms, the tokens up to its own, so that a token reaches later ones only.
+// (Decays are only ever multiplied, never divided by, and their running products carry what the roundings lose.)  All but the products
+// with S and U is made beforehand:
+//   delta_chunk_kernel, channel_delta_chunk_kernel   a block per chunk and head, all chunks of the step side by side: A, B and W (forward
+//                        substitution, a column a lane), then M, Q c, K r, B, c_32 and W V, 98 KB a chunk and head;
+//   delta_chain_kernel   a block per 16 or 32 columns of a head's state and request walks the chunks, on the tensor cores.  Eight warps hold
+//                        16 key channels of S each, in registers, as the left operand of the first product and the sums of the second;
+//                        what a chunk brings each asks for a chunk ahead, straight into registers.  [M; Q c] S comes out in eight shares that go through shared
+//                        memory; four more warps make U of M's while the eight multiply Q c, and the read-outs while those bring S up to date.
+// Operands of the tensor cores are three bfloat16 terms a float32 number, to its last bit: the sums of the six products of terms that count are as
+// accurate as float32's own (the products of first terms are added up in float32 with rounding to nearest, sixteen tokens or channels
+// at a time, since the instruction cuts its sums off; the rest is smaller by 2^8).  M, Q, K and B are taken apart once, where they are made.
+// W and B are zero above the diagonal, and zero times what is not finite is not zero: M and W V are summed over the tokens up to their own, and
+// a read-out that comes out not finite is made again from those, so that a token reaches later ones only.
 // Chunks are counted through the step's portions of at least ``min_tokens`` tokens in order; a portion's last chunk is filled up
 // with tokens of beta 0, key 0 and decay 1.
 //
-// What bounds it: the chain, by what its warps issue (53 % of the slots busy; splitting operands is the largest share) and the
-// barriers between its three phases, on as many SMs as there are heads and runs of 16 columns.  2,000 tokens of 16 heads:
-// 220 us, all but about 20 of them the chain.  The same chain on the CUDA cores was bound by what shared memory hands to registers (238 us); the
-// token-by-token kernel (delta_rule.cu) waits for a butterfly every two tokens (611 us).  Eight warps a block and two blocks an
-// SM took as long.
-#include "delta_common.cuh"
-#include "portions.cuh"
-#include "tf32_terms.cuh"
+// Distances from float64 for the same unit vectors, strengths and decays, the gated rule token by token and here (9, 31, 64, 700 and 2,000 tokens of 16
+// heads): read-outs before they are rounded to bfloat16 0.95, 1.12, 0.93, 1.74 and 1.73e-7 and 0.82, 0.99, 1.02, 1.13 and 1.11e-7; states 0.92, 1.33, 0.90, 2.05
+// and 2.04e-7 and 0.64, 0.80, 0.98, 0.96 and 0.99e-7.  The rule with a decay per channel over 1,200 tokens, whole: read-outs 1.6e-7, states 1.4e-7;
+// sixteen tokens at a time on the CUDA cores, as it was, 2.1e-7 and 1.9e-7.
+//
+// What bounds it: the chain, by the latency of its steps one after the other (a share of [M; Q c] S 1,000 clocks, U 700 beside the other half, the new state
+// 1,000, and two barriers, of which the tensor cores are busy 1,280), and by how soon a chunk's record comes from L2.  2,000 tokens of 16 heads: chunk
+// kernel 44 us, chain 135; products of up to six TF32 terms whose operands every block split for itself 18 and 201.  Two portions of 1,200
+// and 960 tokens with decays per channel: 66 and 125 us; sixteen tokens at a time on the CUDA cores 87 and 211.  Register tiles of fma.rn.f32x2 for
+// the chain: 193 us, bound by what shared memory hands to the registers; two chunks ahead through shared memory: no faster.
+#include "chunk_products.cuh"
 
 namespace {
 using namespace delta;
-using namespace terms;
+using namespace chunks;
 
-constexpr int CHUNK = 32, COLS = 16;
-constexpr int RP = 128;                  // keys are filled up to so many numbers
-// pitches in shared memory, such that fragments of the products meet every bank once; SP: of rows of (hi, lo) pairs
-constexpr int KP = RP + 8, TP = CHUNK + 4, CP = COLS + 8, SP = COLS + 4;
-constexpr int CHAIN_THREADS = 512, CHUNK_THREADS = 128;
+// A chunk's record of a head, 32-bit words.  What the tensor cores take lies as their right operands' fragments, a lane's four words of a term
+// together (16 channels or tokens by 8, see mma_bf16), 128 words a term, three terms one after the other:
+//   M and Q c   per 16 channels w, per two eights of tokens (0, 1: M; 2, 3: Q c): both fragments of either eight;
+//   K r         per 16 channels, per eight of them: both fragments of tokens 0 .. 15, then of 16 .. 31;
+//   B           per eight of its rows: the same;
+// then c_32 [128], and W V [columns in runs of 16][32] as float32.
+constexpr int MQ_AT = 0, K_AT = MQ_AT + (RP / 16) * 4 * UNIT, B_AT = K_AT + (RP / 16) * 2 * UNIT, G_AT = B_AT + (CHUNK / 8) * UNIT, V_AT = G_AT + RP;
+constexpr int RUN = 16;
+__host__ __device__ constexpr int record_floats(int vdim) { return V_AT + (vdim + RUN - 1) / RUN * RUN * CHUNK; }
 
-// a chunk's record of a head: W, B [32][32], c, r [32]
-constexpr int W_AT = 0, B_AT = CHUNK * CHUNK, C_AT = 2 * CHUNK * CHUNK, R_AT = C_AT + CHUNK, RECORD = R_AT + CHUNK;
-
-__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
-__device__ __forceinline__ float both(uint64_t v) {  // the sum of a pair
-  float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-  return a + b;
+// W in A's place (the whole warp, a column a lane): row i of A is used up when W's is known.  ``beta``: of the lane's token.
+__device__ __forceinline__ void solve(float (*as)[TP], float beta, int lane) {
+  float w[CHUNK];
+#pragma unroll
+  for (int i = 0; i < CHUNK; ++i) {
+    float acc[4] = {};
+#pragma unroll
+    for (int l = 0; l < i; l += 4) {
+      const float4 a = *reinterpret_cast<const float4*>(&as[i][l]);  // zeros from the diagonal on
+      acc[0] = fmaf(a.x, w[l], acc[0]);
+      if (l + 1 < i) acc[1] = fmaf(a.y, w[l + 1], acc[1]);
+      if (l + 2 < i) acc[2] = fmaf(a.z, w[l + 2], acc[2]);
+      if (l + 3 < i) acc[3] = fmaf(a.w, w[l + 3], acc[3]);
+    }
+    const float b = __shfl_sync(0xffffffffu, beta, i);
+    w[i] = b * ((i == lane ? 1.f : 0.f) - ((acc[0] + acc[1]) + (acc[2] + acc[3])));
+    __syncwarp();
+    as[i][lane] = w[i];
+  }
+  __syncwarp();
 }
-struct Pairs {
-  uint64_t lo, hi;
+// 16 columns of X as a thread's share of right operands: [tokens 16 k + 8 r + 2 tg + 0, 1][columns 8 n + gr]
+struct Columns {
+  float v[2][2][2][2];  // [k][n][r][token]
+  template <typename X>
+  __device__ __forceinline__ void fetch(X x, int gr, int tg) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int t = 0; t < 2; ++t) v[k][n][r][t] = x(16 * k + 8 * r + 2 * tg + t, 8 * n + gr);
+  }
 };
-__device__ __forceinline__ Pairs load4(const float* p) {
-  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
-  return {v.x, v.y};
+// W X: rows gr and gr + 8 of either half, columns 2 tg and 2 tg + 1 of either eight, in out[half][eight][4].  W is zero above the diagonal, and a row that
+// comes out not finite is made again from the tokens up to its own, ``x(l, column)``.
+template <typename X>
+__device__ __forceinline__ void times_w(const float (*ws)[TP], const Left (&w)[3], const Columns& have, X x, float (&out)[2][2][4], int gr, int tg) {
+  float sum[2][2][4] = {}, small[2][2][4] = {};
+  Right b[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) b[n].put(r, split3(have.v[k][n][r][0], have.v[k][n][r][1]));
+    if (k == 0) step<2>(sum[0], small[0], w[0], b);
+    step<2>(sum[1], small[1], w[1 + k], b);
+  }
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) out[m][n][e] = sum[m][n][e] + small[m][n][e];
+  bool fine = true;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) fine = fine && is_finite(out[i >> 3][(i >> 2) & 1][i & 3]);
+  if (!fine) {
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i) {
+      const int row = 16 * (i >> 3) + gr + 8 * ((i >> 1) & 1), col = 8 * ((i >> 2) & 1) + 2 * tg + (i & 1);
+      float again = 0.f;
+#pragma unroll 1
+      for (int l = 0; l <= row; ++l) again = fmaf(ws[row][l], x(l, col), again);
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (j == i && !is_finite(out[j >> 3][(j >> 2) & 1][j & 3])) out[j >> 3][(j >> 2) & 1][j & 3] = again;
+    }
+  }
 }
+// M and W V of a head, 16 channels or columns a warp at a time.  K c is ``kc(l, d)``; ``ahead``: this warp's first columns of V (16 warp ..).
+template <int WARPS, typename KC, typename V>
+__device__ __forceinline__ void put_m_and_values(const float (*ws)[TP], KC kc, V v, Columns& ahead, int vdim, float* __restrict__ out, int warp, int lane) {
+  const int gr = lane >> 2, tg = lane & 3;
+  const Left w[3] = {left_rows(&ws[0][0], TP, gr, tg), left_rows(&ws[16][0], TP, gr, tg), left_rows(&ws[16][16], TP, gr, tg)};
+  float y[2][2][4];
+#pragma unroll 1
+  for (int u = warp; u < RP / 16; u += WARPS) {
+    auto x = [&](int l, int d) { return kc(l, 16 * u + d); };
+    Columns have;
+    have.fetch(x, gr, tg);
+    times_w(ws, w, have, x, y, gr, tg);
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const Terms t[4] = {split3(y[m][0][0], y[m][0][1]), split3(y[m][1][0], y[m][1][1]), split3(y[m][0][2], y[m][0][3]), split3(y[m][1][2], y[m][1][3])};
+      put_terms(out + MQ_AT + (u * 4 + m) * UNIT + 4 * lane, t);
+    }
+  }
+#pragma unroll 1
+  for (int col0 = 16 * warp; col0 < vdim; col0 += 16 * WARPS) {
+    const Columns have = ahead;
+    if (col0 + 16 * WARPS < vdim) ahead.fetch([&](int l, int c) { return v(l, col0 + 16 * WARPS + c); }, gr, tg);
+    times_w(ws, w, have, [&](int l, int c) { return v(l, col0 + c); }, y, gr, tg);
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) out[V_AT + (col0 + 8 * c + 2 * tg + (e & 1)) * CHUNK + 16 * m + gr + 8 * (e >> 1)] = y[m][c][e];
+  }
+}
+struct ChunkShape {
+  static constexpr int Q = CHUNK * KP, AS = 2 * CHUNK * KP, BS = AS + CHUNK * TP, CR = BS + CHUNK * TP, FLOATS = CR + 2 * CHUNK;
+};
 
-__global__ void __launch_bounds__(CHUNK_THREADS)
+// (The heads of a group each make K K^T and Q K^T again: a block per group had too few warps, and too few blocks, to hide one step's latency behind
+// another's.)
+__global__ void __launch_bounds__(CHUNK_THREADS, 4)
 delta_chunk_kernel(const float* __restrict__ qkv, const float* __restrict__ bd, const int32_t* __restrict__ item_start,
                    float* __restrict__ records, int items, int min_tokens, int G, int H, int dim, int vdim) {
-  constexpr int WARPS = CHUNK_THREADS / 32;
-  __shared__ __align__(16) float rows[2 * CHUNK * KP];
-  __shared__ float kk[CHUNK][CHUNK + 1], qk[CHUNK][CHUNK + 1];
-  float *ks = rows, *qs = rows + CHUNK * KP;
-  float(*as)[CHUNK][TP] = reinterpret_cast<float(*)[CHUNK][TP]>(rows);  // A of a warp's head, where the keys and queries were
-  static_assert(WARPS * CHUNK * TP <= 2 * CHUNK * KP, "room for every warp's A");
+  using Sh = ChunkShape;
+  extern __shared__ __align__(16) float chunk_smem[];
+  float *ks = chunk_smem, *qs = chunk_smem + Sh::Q;
+  float(*as)[TP] = reinterpret_cast<float(*)[TP]>(chunk_smem + Sh::AS);
+  float(*bs)[TP] = reinterpret_cast<float(*)[TP]>(chunk_smem + Sh::BS);
+  float *cs = chunk_smem + Sh::CR, *rs = cs + CHUNK;  // c and r of every token
+  const int h = blockIdx.x % H, chunk = (int)(gridDim.x / H) - 1 - (int)(blockIdx.x / H);  // the first chunks last: the chain starts with them
   pdl_wait();
   int t0, n;
-  if (!portions::find_chunk<CHUNK>(item_start, items, min_tokens, blockIdx.x, t0, n)) return;
-  const int g = blockIdx.y, C = 2 * G * dim + H * vdim;
-  for (int i = threadIdx.x; i < CHUNK * RP / 4; i += CHUNK_THREADS) {
-    const int t = i / (RP / 4), d = (i - t * (RP / 4)) * 4;
-    const bool there = t < n && d < dim;
-    const float* src = qkv + (size_t)(t0 + (there ? t : 0)) * C + (size_t)g * dim + (there ? d : 0);
-    copy_async16_or_zero(qs + t * KP + d, src, there);
-    copy_async16_or_zero(ks + t * KP + d, src + (size_t)G * dim, there);
-  }
+  if (!portions::find_chunk<CHUNK>(item_start, items, min_tokens, chunk, t0, n)) return;
+  const int g = h / (H / G), C = 2 * G * dim + H * vdim;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, tg = lane & 3;
+  float* out = records + ((size_t)chunk * H + h) * record_floats(vdim);
+  bring_rows(qs, qkv + (size_t)t0 * C + (size_t)g * dim, C, n, dim, true);
+  bring_rows(ks, qkv + (size_t)t0 * C + (size_t)(G + g) * dim, C, n, dim, true);
+  const float* mine = bd + (size_t)(t0 + min(lane, n - 1)) * BD * H + h;
+  const float beta = lane < n ? mine[0] : 0.f, decay = lane < n ? mine[H] : 1.f;
   copy_async_wait();
   __syncthreads();
-  {
-    // a thread: rows ti + 8a of K (or Q) against rows tj + 8b of K (rows eight apart, so that neighbours meet other banks)
-    const int ti = (threadIdx.x & 63) >> 3, tj = threadIdx.x & 7;
-    const bool query = threadIdx.x >= 64;
-    const float* left = (query ? qs : ks) + ti * KP;
-    const float* right = ks + tj * KP;
-    // 16 numbers at a time, then in pairs: a single chain over the 128 was what lost most of a read-out
-    auto block = [&](int d0, float (&out)[4][4]) {
-      uint64_t acc[4][4] = {};
-#pragma unroll
-      for (int d = d0; d < d0 + 16; d += 4) {
-        Pairs a[4], b[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          a[e] = load4(left + e * 8 * KP + d);
-          b[e] = load4(right + e * 8 * KP + d);
-        }
-#pragma unroll
-        for (int x = 0; x < 4; ++x)
-#pragma unroll
-          for (int y = 0; y < 4; ++y) {
-            fma2(acc[x][y], a[x].lo, b[y].lo);
-            fma2(acc[x][y], a[x].hi, b[y].hi);
-          }
-      }
-#pragma unroll
-      for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) out[x][y] = both(acc[x][y]);
-    };
-    auto add = [](float (&to)[4][4], const float (&what)[4][4]) {
-#pragma unroll
-      for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) to[x][y] += what[x][y];
-    };
-    float total[4][4] = {};
+  {  // K K^T and Q K^T, 16 rows a warp
+    static_assert(CHUNK_THREADS == 128, "four warps");
+    const float* rows = (warp < 2 ? ks : qs) + 16 * (warp & 1) * KP;
+    float sum[4][4] = {}, small[4][4] = {};
 #pragma unroll 1
-    for (int d = 0; d < RP; d += 64) {
-      float p[4][4], r[4][4], u[4][4];
-      block(d, p);
-      block(d + 16, r);
-      add(p, r);
-      block(d + 32, r);
-      block(d + 48, u);
-      add(r, u);
-      add(p, r);
-      add(total, p);
+    for (int k = 0; k < RP; k += 16) {
+      Right b[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) b[m] = right_rows(ks + 8 * m * KP + k, KP, gr, tg);
+      step<4>(sum, small, left_rows(rows + k, KP, gr, tg), b);
     }
+    float* to = (warp < 2 ? as : bs)[16 * (warp & 1) + gr] + 2 * tg;
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
+    for (int m = 0; m < 4; ++m)
 #pragma unroll
-      for (int y = 0; y < 4; ++y) (query ? qk : kk)[ti + 8 * x][tj + 8 * y] = total[x][y];
+      for (int e = 0; e < 4; ++e) to[8 * (e >> 1) * TP + 8 * m + (e & 1)] = sum[m][e] + small[m][e];
   }
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per = H / G;
-  for (int hh = warp; hh < per; hh += WARPS) {
-    const int h = g * per + hh;
-    float* out = records + ((size_t)blockIdx.x * H + h) * RECORD;
-    const float* mine = bd + (size_t)(t0 + min(lane, n - 1)) * BD * H + h;
-    const float beta = lane < n ? mine[0] : 0.f, decay = lane < n ? mine[H] : 1.f;
+  if (warp < 2) {  // (either warp of A and B, both with all the products)
+    float(*at)[TP] = warp ? bs : as;
     Product run, before, behind;  // lane j: products over the tokens between j and i, up to j, behind j
-#pragma unroll
+#pragma unroll 4
     for (int i = 0; i < CHUNK; ++i) {
       const float d = __shfl_sync(0xffffffffu, decay, i);
       if (i <= lane) before.times(d);
@@ -155,63 +211,143 @@ delta_chunk_kernel(const float* __restrict__ qkv, const float* __restrict__ bd, 
         run.times(d);
         behind.times(d);
       }
-      as[warp][i][lane] = i > lane ? run.value() * kk[i][lane] : 0.f;
-      out[B_AT + i * CHUNK + lane] = i >= lane ? run.value() * qk[i][lane] : 0.f;
+      at[i][lane] = i + warp > lane ? run.value() * at[i][lane] : 0.f;
     }
-    out[C_AT + lane] = before.value();
-    out[R_AT + lane] = behind.value();
-    __syncwarp();
-    float w[CHUNK];  // lane j: column j of W
-#pragma unroll
-    for (int i = 0; i < CHUNK; ++i) {
-      float acc[4] = {};
-#pragma unroll
-      for (int l = 0; l < i; l += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(&as[warp][i][l]);  // zeros from the diagonal on
-        acc[0] = fmaf(a.x, w[l], acc[0]);
-        if (l + 1 < i) acc[1] = fmaf(a.y, w[l + 1], acc[1]);
-        if (l + 2 < i) acc[2] = fmaf(a.z, w[l + 2], acc[2]);
-        if (l + 3 < i) acc[3] = fmaf(a.w, w[l + 3], acc[3]);
-      }
-      const float b = __shfl_sync(0xffffffffu, beta, i);
-      w[i] = b * ((i == lane ? 1.f : 0.f) - ((acc[0] + acc[1]) + (acc[2] + acc[3])));
-      out[W_AT + i * CHUNK + lane] = w[i];
+    if (warp) {
+      cs[lane] = before.value();
+      rs[lane] = behind.value();
     }
-    __syncwarp();
   }
+  __syncthreads();
+  const float* values = qkv + (size_t)t0 * C + 2 * (size_t)G * dim + (size_t)h * vdim;
+  auto v = [&](int l, int c) { return l < n && c < vdim ? values[(size_t)l * C + c] : 0.f; };
+  Columns ahead;
+  ahead.fetch([&](int l, int c) { return v(l, 16 * warp + c); }, gr, tg);
+  if (warp == 0) {
+    solve(as, beta, lane);
+  } else {  // what does not wait for W
+    put_rows(qs, out + MQ_AT + 2 * UNIT, 4, threadIdx.x - 32, CHUNK_THREADS - 32, [&](int t) { return cs[t]; });
+    put_keys(ks, out + K_AT, threadIdx.x - 32, CHUNK_THREADS - 32, [&](int t) { return rs[t]; });
+    put_b(bs, out + B_AT, threadIdx.x - 32, CHUNK_THREADS - 32);
+    for (int d = threadIdx.x - 32; d < RP; d += CHUNK_THREADS - 32) out[G_AT + d] = cs[CHUNK - 1];
+  }
+  __syncthreads();
+  put_m_and_values<CHUNK_THREADS / 32>(as, [&](int l, int d) { return ks[l * KP + d] * cs[l]; }, v, ahead, vdim, out, warp, lane);
   pdl_trigger();  // at the end: the chain's blocks are few and long (see delta_prepare_kernel)
 }
 
-// ---- the chain, on the tensor cores, operands in terms (tf32_terms.cuh) --------------------------------------------------
-struct ChainShape {
-  static constexpr int K_AT = 0, Q_AT = K_AT + CHUNK * KP, SW_AT = Q_AT + CHUNK * KP, V_AT = SW_AT + CHUNK * TP;
-  static constexpr int STAGE = V_AT + CHUNK * CP;                          // floats of a stage
-  static constexpr int B_SIZE = CHUNK * TP + 2 * CHUNK;                    // B, then c and r: read one chunk longer than the rest
-  static constexpr int RING_AT = 2 * STAGE, S_AT = RING_AT + 3 * B_SIZE;   // the state in (hi, lo) pairs
-  static constexpr int UU_AT = S_AT + RP * 2 * SP, U_AT = UU_AT + CHUNK * 2 * SP;  // U times r in (hi, lo) pairs; U of two chunks
-  static constexpr int PART_AT = U_AT + 2 * CHUNK * CP, FLOATS = PART_AT + 2 * 4 * 2 * CHUNK * CP;  // quarters of [K; Q] S, of two chunks
+// ---- a decay per channel -------------------------------------------------------------------------------------------------
+struct ChannelShape {
+  static constexpr int Q = CHUNK * KP, G = 2 * CHUNK * KP, AS = 3 * CHUNK * KP, BS = AS + CHUNK * TP, FLOATS = BS + CHUNK * TP;
 };
 
-__device__ __forceinline__ void store_split(float* at, float x, float y) {  // two neighbours of a row of pairs
-  const Split a = split(x), b = split(y);
-  *reinterpret_cast<uint4*>(at) = make_uint4(a.hi, a.lo, b.hi, b.lo);
-}
-__device__ __forceinline__ Split load_split(const float* at) {
-  const uint2 v = *reinterpret_cast<const uint2*>(at);
-  return {v.x, v.y};
-}
-__global__ void __launch_bounds__(CHAIN_THREADS, 1)
-delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ records, const __nv_bfloat16* __restrict__ proj, long long P,
-                   float* __restrict__ state, const int32_t* __restrict__ item_start, const int32_t* __restrict__ slots,
-                   float* __restrict__ o, int items, int all_chunks, int min_tokens, int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats) {
-  using Sh = ChainShape;
-  extern __shared__ __align__(16) float chain[];
-  float *st = chain + Sh::S_AT, *uu = chain + Sh::UU_AT;
-  const int C = 2 * G * dim + H * vdim;
-  const int h = blockIdx.y, g = h / (H / G);
-  const int col0 = blockIdx.x * COLS;
+// A and B in halves of 16 tokens: on the diagonal a running product a column, behind it as products of q_i (k_i) times the decays from the
+// half's start and k_j times those to its half's end.
+__global__ void __launch_bounds__(CHUNK_THREADS, 3)
+channel_delta_chunk_kernel(const float* __restrict__ qkv, const float* __restrict__ bd, const float* __restrict__ decay,
+                           const int32_t* __restrict__ item_start, float* __restrict__ records, int items, int min_tokens, int G, int H,
+                           int dim, int vdim, bool wide, bool wide_decay) {
+  using Sh = ChannelShape;
+  extern __shared__ __align__(16) float chunk_smem[];
+  float *ks = chunk_smem, *qs = chunk_smem + Sh::Q, *gs = chunk_smem + Sh::G;
+  float(*as)[TP] = reinterpret_cast<float(*)[TP]>(chunk_smem + Sh::AS);
+  float(*bs)[TP] = reinterpret_cast<float(*)[TP]>(chunk_smem + Sh::BS);
+  const int h = blockIdx.x % H, chunk = (int)(gridDim.x / H) - 1 - (int)(blockIdx.x / H);  // the first chunks last: the chain starts with them
+  pdl_wait();
+  int t0, n;
+  if (!portions::find_chunk<CHUNK>(item_start, items, min_tokens, chunk, t0, n)) return;
+  const int g = h / (H / G), C = 2 * G * dim + H * vdim;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int gr = lane >> 2, tg = lane & 3;  // the lane's row (or column) and place in a fragment
+  float* out = records + ((size_t)chunk * H + h) * record_floats(vdim);
+  bring_rows(qs, qkv + (size_t)t0 * C + (size_t)g * dim, C, n, dim, wide);
+  bring_rows(ks, qkv + (size_t)t0 * C + (size_t)(G + g) * dim, C, n, dim, wide);
+  bring_rows(gs, decay + ((size_t)t0 * H + h) * dim, (long long)H * dim, n, dim, wide_decay);  // (0 where there is none: the key is 0 too)
+  const float beta = lane < n ? bd[(size_t)(t0 + lane) * BD * H + h] : 0.f;
+  copy_async_wait();
+  __syncthreads();
+  products_on_diagonal<true, false>(ks, qs, gs, as, bs, warp, lane);
+  __syncthreads();
+  // a channel a thread: the running products
+  const int d = threadIdx.x;
+  float kc[CHUNK], qc[CHUNK];  // K c, Q c
+  {
+    Product c, front, tail, upto;
+    float f[CHUNK];
+#pragma unroll
+    for (int i = 0; i < CHUNK; ++i) f[i] = i < n && d < dim ? gs[i * KP + d] : 1.f;
+#pragma unroll
+    for (int i = 0; i < CHUNK; ++i) {
+      const float q = qs[i * KP + d], k = ks[i * KP + d];
+      c.times(f[i]);
+      kc[i] = k * c.value();
+      qc[i] = q * c.value();
+      if (i >= HALF) {
+        front.times(f[i]);
+        qs[i * KP + d] = q * front.value();
+        qs[(i - HALF) * KP + d] = k * front.value();   // (the first half's queries are done with)
+      }
+    }
+    out[G_AT + d] = c.value();
+#pragma unroll
+    for (int i = CHUNK - 1; i >= 0; --i) {
+      const float k = ks[i * KP + d];
+      if (i < HALF) {
+        gs[i * KP + d] = k * upto.value();  // to the end of the first half
+        upto.times(f[i]);
+      }
+      ks[i * KP + d] = k * tail.value();
+      tail.times(f[i]);
+    }
+  }
+  __syncthreads();
+  products_behind<true>(qs, gs, as, bs);  // (rows 0 .. 15 of the queries' place are the second half's keys now, 16 .. 31 its queries)
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < CHUNK; ++i) {
+    qs[i * KP + d] = qc[i];
+    gs[i * KP + d] = kc[i];
+  }
+  __syncthreads();
+  const float* values = qkv + (size_t)t0 * C + 2 * (size_t)G * dim + (size_t)h * vdim;
+  auto v = [&](int l, int c) { return l < n && c < vdim ? values[(size_t)l * C + c] : 0.f; };
+  Columns ahead;
+  ahead.fetch([&](int l, int c) { return v(l, 16 * warp + c); }, lane >> 2, lane & 3);
+  if (warp == 0) {
+    solve(as, beta, lane);
+  } else {
+    auto one = [](int) { return 1.f; };
+    put_rows(qs, out + MQ_AT + 2 * UNIT, 4, threadIdx.x - 32, CHUNK_THREADS - 32, one);
+    put_keys(ks, out + K_AT, threadIdx.x - 32, CHUNK_THREADS - 32, one);
+    put_b(bs, out + B_AT, threadIdx.x - 32, CHUNK_THREADS - 32);
+  }
+  __syncthreads();
+  put_m_and_values<CHUNK_THREADS / 32>(as, [&](int l, int c) { return gs[l * KP + c]; }, v, ahead, vdim, out, warp, lane);
+  pdl_trigger();  // at the end, as in delta_chunk_kernel
+}
+
+// ---- the chain -----------------------------------------------------------------------------------------------------------
+constexpr int PP = 2 * CHUNK + 8;   // of the shares: columns first
+template <int TILES>
+struct Chain {
+  static constexpr int COLS = 16 * TILES;
+  static constexpr int U_AT = WORKERS / 32 * COLS * PP, FLOATS = U_AT + TILES * 2 * UNIT;  // U per 16 columns and 16 tokens: fragments, as in a record
+  static_assert(FLOATS * 4 <= 227 * 1024, "beyond a block's shared memory");
+};
+
+
+template <int TILES, typename T>
+__global__ void __launch_bounds__(CHAIN_THREADS, 1)
+delta_chain_kernel(const float* __restrict__ records, const T* __restrict__ proj, long long P, float* __restrict__ state,
+                   const int32_t* __restrict__ item_start, const int32_t* __restrict__ slots, float* __restrict__ o, int items,
+                   int all_chunks, int min_tokens, int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats) {
+  using Sh = Chain<TILES>;
+  constexpr int COLS = Sh::COLS, SHARES = WORKERS / 32;
+  extern __shared__ __align__(16) float chain[];
+  float* parts = chain;                                               // [SHARES][COLS][PP]: M S of the chunk's tokens, then Q c S
+  uint32_t* us = reinterpret_cast<uint32_t*>(chain + Sh::U_AT);       // [TILES][2][3][32 lanes][4]
+  const int C = 2 * G * dim + H * vdim;
+  const int h = blockIdx.y, col0 = blockIdx.x * COLS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, tg = lane & 3;
   pdl_wait();
   int item, first;  // (a block per portion: blocks for requests that have none would only be in the way, one fills an SM)
   if (!portions::find_portion<CHUNK>(item_start, items, min_tokens, blockIdx.z, item, first)) return;
@@ -222,201 +358,258 @@ delta_chain_kernel(const float* __restrict__ qkv, const float* __restrict__ reco
   slot = slot < 0 ? 0 : (slot >= num_slots ? num_slots - 1 : slot);
   float* base = state + (size_t)slot * slot_floats;
   float* S = base + (size_t)(K - 1) * C + (size_t)h * dim * vdim;
-
-  auto stage = [&](int c, int thread, int threads) {
-    float *buf = chain + (c & 1) * Sh::STAGE, *ring = chain + Sh::RING_AT + c % 3 * Sh::B_SIZE;
-    const int ts = t0 + c * CHUNK, n = min(CHUNK, t1 - ts);
-    const float* rows = qkv + (size_t)ts * C;
-    const float* record = records + ((size_t)(first + c) * H + h) * RECORD;
-    for (int i = thread; i < CHUNK * RP / 4; i += threads) {
-      const int t = i / (RP / 4), d = (i % (RP / 4)) * 4;
-      const bool there = t < n && d < dim;
-      const float* src = rows + (there ? (size_t)t * C + d : 0) + (size_t)g * dim;
-      copy_async16_or_zero(buf + Sh::K_AT + t * KP + d, src + (size_t)G * dim, there);
-      copy_async16_or_zero(buf + Sh::Q_AT + t * KP + d, src, there);
+  const size_t size = record_floats(vdim);
+  auto record_of = [&](int c) { return records + ((size_t)(first + c) * H + h) * size; };
+  auto left_of = [&](int at) {  // 16 columns of U, 16 tokens
+    Left u;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      const uint4 x = *reinterpret_cast<const uint4*>(us + at * UNIT + p * TERM + 4 * lane);
+      u.v[p][0] = x.x, u.v[p][1] = x.y, u.v[p][2] = x.z, u.v[p][3] = x.w;
     }
-    for (int i = thread; i < CHUNK * CHUNK / 4; i += threads) {
-      const int row = i / (CHUNK / 4), piece = (i % (CHUNK / 4)) * 4;
-      copy_async16(buf + Sh::SW_AT + row * TP + piece, record + W_AT + row * CHUNK + piece);
-      copy_async16(ring + row * TP + piece, record + B_AT + row * CHUNK + piece);
-    }
-    for (int i = thread; i < CHUNK * COLS / 4; i += threads) {
-      const int t = i / (COLS / 4), v = (i % (COLS / 4)) * 4;
-      const bool there = t < n && col0 + v < vdim;
-      copy_async16_or_zero(buf + Sh::V_AT + t * CP + v, rows + (there ? (size_t)t * C + 2 * (size_t)G * dim + (size_t)h * vdim + col0 + v : 0), there);
-    }
-    for (int i = thread; i < 2 * CHUNK / 4; i += threads)  // c and r
-      copy_async16(ring + CHUNK * TP + 4 * i, record + C_AT + 4 * i);
+    return u;
   };
-  auto part_of = [&](int c) { return chain + Sh::PART_AT + (c & 1) * 4 * 2 * CHUNK * CP; };
-  auto u_of = [&](int c) { return chain + Sh::U_AT + (c & 1) * CHUNK * CP; };
-
-  // the read-out of chunk c, 16 rows and 8 columns a warp: while the next chunk's U is made
-  auto read_out = [&](int c) {
-    const int i0 = 16 * ((warp >> 1) & 1) + gr, oc = 8 * (warp & 1);
-    const float *ring = chain + Sh::RING_AT + c % 3 * Sh::B_SIZE, *part = part_of(c) + (CHUNK + i0) * CP + oc + 2 * tg;
-    const float *a = ring + i0 * TP + tg, *b = u_of(c) + tg * CP + oc + gr;
-    Sum y;
+  auto unit = [&](const float* at, uint4 (&to)[3]) {
 #pragma unroll
-    for (int k = 0; k < CHUNK / 8; ++k) {
-      if (k >= 2 && i0 < 16) break;  // B is triangular
-      uint32_t ah[4], al[4];
-      load_rows(a + 8 * k, 8 * TP, 4, ah, al);
-      y.step<6>(ah, al, split(b[8 * k * CP]), split(b[(8 * k + 4) * CP]));
-    }
-    float total[4];
-    y.totals(total);
-    if (!all_finite(total)) {
-#pragma unroll 1
-      for (int e = 0; e < 4; ++e) {
-        const int i = i0 + 8 * (e >> 1);
-        float sum = 0.f;
-#pragma unroll 1
-        for (int j = 0; j <= i; ++j) sum = fmaf(ring[i * TP + j], u_of(c)[j * CP + oc + 2 * tg + (e & 1)], sum);
-        if (!is_finite(pick(total, e))) place(total, e, sum);
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const int t = t0 + c * CHUNK + i0 + 8 * r, col = col0 + oc + 2 * tg;
-      float2 v = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float2 p = *reinterpret_cast<const float2*>(part + (q * 2 * CHUNK + 8 * r) * CP);
-        v.x += p.x;
-        v.y += p.y;
-      }
-      const float ci = ring[CHUNK * TP + i0 + 8 * r];
-      if (t < t1 && col < vdim)
-        *reinterpret_cast<float2*>(o + ((size_t)t * H + h) * vdim + col) = make_float2(fmaf(ci, v.x, total[2 * r]), fmaf(ci, v.y, total[2 * r + 1]));
-    }
+    for (int p = 0; p < 3; ++p)  // (volatile: where they are asked for, not where they are used)
+      asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(to[p].x), "=r"(to[p].y), "=r"(to[p].z), "=r"(to[p].w) : "l"(at + p * TERM + 4 * lane));
   };
 
-  stage(0, threadIdx.x, CHAIN_THREADS);
-  // the state: rows 16 (warp / 2) + gr and + 8, columns 8 (warp % 2) + 2 tg and + 1 are this thread's
-  float s[4];
-  const int d0 = 16 * (warp >> 1) + gr, sc = 8 * (warp & 1) + 2 * tg;
+  if (threadIdx.x < WORKERS) {
+    uint4 mq[4][3], kr[2][3];  // asked for a chunk ahead, each as soon as the last one's is used up
+    float2 g[2];
+    const float* r = record_of(0);
+    const size_t stride = (size_t)H * size;
+    auto fetch_mq = [&](int first) {
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int d = d0 + 8 * (e >> 1), col = col0 + sc + (e & 1);
-    s[e] = (d < dim && col < vdim) ? S[(size_t)d * vdim + col] : 0.f;
-  }
-  store_split(st + (d0 * SP + sc) * 2, s[0], s[1]);
-  store_split(st + ((d0 + 8) * SP + sc) * 2, s[2], s[3]);
-  // [K; Q] S: 16 rows (of K: mt 0 and 1, of Q: 2 and 3) over a quarter of the keys' numbers
-  const int mt = warp >> 2, quarter = warp & 3;
-
-  for (int c = 0; c < chunks; ++c) {
-    copy_async_wait();
-    __syncthreads();  // this chunk and the state have landed, and everybody has left the other buffer
-    const float* buf = chain + (c & 1) * Sh::STAGE;
-    const float* ring = chain + Sh::RING_AT + c % 3 * Sh::B_SIZE;
-    {
-      Sum y[2];
-      const float* a = buf + (mt < 2 ? Sh::K_AT : Sh::Q_AT) + ((mt & 1) * 16 + gr) * KP + quarter * (RP / 4) + tg;
-      const float* b = st + ((quarter * (RP / 4) + tg) * SP + gr) * 2;
+      for (int p = 0; p < 2; ++p) unit(r + MQ_AT + (warp * 4 + first + p) * UNIT, mq[first + p]);
+    };
+    auto fetch_rest = [&] {
 #pragma unroll
-      for (int k = 0; k < RP / 32; ++k) {
-        uint32_t ah[4], al[4];
-        load_rows(a + 8 * k, 8 * KP, 4, ah, al);
-#pragma unroll
-        for (int n = 0; n < 2; ++n) y[n].step<4>(ah, al, load_split(b + (8 * k * SP + 8 * n) * 2), load_split(b + ((8 * k + 4) * SP + 8 * n) * 2));
+      for (int m = 0; m < 2; ++m) {
+        unit(r + K_AT + (warp * 2 + m) * UNIT, kr[m]);
+        g[m] = __ldg(reinterpret_cast<const float2*>(r + G_AT + 16 * warp + 8 * m + 2 * tg));
       }
-      float* part = part_of(c) + (quarter * 2 * CHUNK + mt * 16 + gr) * CP + 2 * tg;
+    };
+    fetch_mq(0);
+    fetch_mq(2);
+    fetch_rest();
+    // S, columns first: columns gr and gr + 8 of every 16, channels 16 warp + 8 m + 2 tg and + 1
+    float s[TILES][2][4];
+    Left a[TILES];
+    auto at = [&](int tile, int m, int e) -> float* {
+      const int d = 16 * warp + 8 * m + 2 * tg + (e & 1), col = col0 + 16 * tile + gr + 8 * (e >> 1);
+      return d < dim && col < vdim ? S + (size_t)d * vdim + col : nullptr;
+    };
+    auto take_apart = [&](int tile) {  // the sums of the second product lie as the left operand of the first
 #pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        *reinterpret_cast<float2*>(part + 8 * n) = make_float2(y[n].total(0), y[n].total(1));
-        *reinterpret_cast<float2*>(part + 8 * CP + 8 * n) = make_float2(y[n].total(2), y[n].total(3));
-      }
-    }
-    __syncthreads();
-    if (warp < 4) {  // U = W (V - ..): 16 rows and 8 columns a warp, which puts the right side together itself
-      const int i0 = 16 * (warp >> 1) + gr, uc = 8 * (warp & 1);
-      const float *a = buf + Sh::SW_AT + i0 * TP + tg, *v = buf + Sh::V_AT + tg * CP + uc + gr, *part = part_of(c) + tg * CP + uc + gr;
-      Sum u;
+      for (int r = 0; r < 4; ++r) a[tile].put(r, split3(s[tile][r >> 1][2 * (r & 1)], s[tile][r >> 1][2 * (r & 1) + 1]));
+    };
 #pragma unroll
-      for (int k = 0; k < CHUNK / 8; ++k) {
-        if (k >= 2 && i0 < 16) break;  // W is triangular
-        uint32_t ah[4], al[4];
-        load_rows(a + 8 * k, 8 * TP, 4, ah, al);
-        Split x[2];
+    for (int tile = 0; tile < TILES; ++tile) {
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i = (8 * k + 4 * e) * CP;
-          const float y = (part[i] + part[2 * CHUNK * CP + i]) + (part[4 * CHUNK * CP + i] + part[6 * CHUNK * CP + i]);
-          x[e] = split(fmaf(-ring[CHUNK * TP + 8 * k + 4 * e + tg], y, v[i]));
-        }
-        u.step<6>(ah, al, x[0], x[1]);
-      }
-      float total[4];
-      u.totals(total);
-      if (!all_finite(total)) {
-#pragma unroll 1
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int i = i0 + 8 * (e >> 1), col = uc + 2 * tg + (e & 1);
-          float sum = 0.f;
-#pragma unroll 1
-          for (int j = 0; j <= i; ++j) {
-            const float* q = part_of(c) + j * CP + col;
-            const float y = (q[0] + q[2 * CHUNK * CP]) + (q[4 * CHUNK * CP] + q[6 * CHUNK * CP]);
-            sum = fmaf(buf[Sh::SW_AT + i * TP + j], fmaf(-ring[CHUNK * TP + j], y, buf[Sh::V_AT + j * CP + col]), sum);
-          }
-          if (!is_finite(pick(total, e))) place(total, e, sum);
+          const float* p = at(tile, m, e);
+          s[tile][m][e] = p ? *p : 0.f;
+        }
+      take_apart(tile);
+    }
+    auto share = [&](int half) {  // this warp's share of M S, or of Q c S
+      Right b[4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          const uint4 v = mq[2 * half + (n >> 1)][p];
+          b[n].v[p][0] = n & 1 ? v.z : v.x;
+          b[n].v[p][1] = n & 1 ? v.w : v.y;
+        }
+#pragma unroll
+      for (int tile = 0; tile < TILES; ++tile) {
+        float sum[4][4] = {}, small[4][4] = {};
+        step<4>(sum, small, a[tile], b);
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+          float* to = parts + (warp * COLS + 16 * tile + gr) * PP + 8 * (4 * half + n) + 2 * tg;
+          *reinterpret_cast<float2*>(to) = make_float2(sum[n][0] + small[n][0], sum[n][1] + small[n][1]);
+          *reinterpret_cast<float2*>(to + 8 * PP) = make_float2(sum[n][2] + small[n][2], sum[n][3] + small[n][3]);
         }
       }
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const int i = i0 + 8 * r, col = uc + 2 * tg;
-        const float ri = ring[CHUNK * TP + CHUNK + i];
-        *reinterpret_cast<float2*>(u_of(c) + i * CP + col) = make_float2(total[2 * r], total[2 * r + 1]);
-        store_split(uu + (i * SP + col) * 2, total[2 * r] * ri, total[2 * r + 1] * ri);
+    };
+    for (int c = 0; c < chunks; ++c) {
+      share(0);
+      if (c + 1 < chunks) {
+        r += stride;
+        fetch_mq(0);
       }
-    } else if (warp < 8) {
-      if (c > 0) read_out(c - 1);
-    } else if (c + 1 < chunks) {
-      stage(c + 1, threadIdx.x - 256, CHAIN_THREADS - 256);
-    }
-    __syncthreads();
-    {
-      Sum d;
-      const float* a = buf + Sh::K_AT + tg * KP + d0;
-      const float* b = uu + (tg * SP + 8 * (warp & 1) + gr) * 2;
+      __syncthreads();  // the others make U of it
+      share(1);
+      if (c + 1 < chunks) fetch_mq(2);
+      __syncthreads();
 #pragma unroll
-      for (int k = 0; k < CHUNK / 8; ++k) {
-        uint32_t ah[4], al[4];
-        load_rows(a + 8 * k * KP, 8, 4 * KP, ah, al);
-        d.step<6>(ah, al, load_split(b + 8 * k * SP * 2), load_split(b + (8 * k + 4) * SP * 2));
+      for (int tile = 0; tile < TILES; ++tile) {
+        float sum[2][2][4], small[2][2][4] = {};  // of either half of the tokens
+        const Left u[2] = {left_of(2 * tile), left_of(2 * tile + 1)};
+        Right b[2][2];
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int p = 0; p < 3; ++p) {
+            b[0][m].v[p][0] = kr[m][p].x, b[0][m].v[p][1] = kr[m][p].y;
+            b[1][m].v[p][0] = kr[m][p].z, b[1][m].v[p][1] = kr[m][p].w;
+          }
+        step_halves(sum, small, u, b);
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            s[tile][m][e] = fmaf(e & 1 ? g[m].y : g[m].x, s[tile][m][e], (sum[0][m][e] + sum[1][m][e]) + (small[0][m][e] + small[1][m][e]));
+        take_apart(tile);
       }
-      const float all = ring[CHUNK * TP + CHUNK - 1];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) s[e] = fmaf(all, s[e], d.total(e));
-      store_split(st + (d0 * SP + sc) * 2, s[0], s[1]);
-      store_split(st + ((d0 + 8) * SP + sc) * 2, s[2], s[3]);
+      if (c + 1 < chunks) fetch_rest();
     }
-  }
-  if (warp >= 4 && warp < 8 && chunks > 0) read_out(chunks - 1);
-  pdl_trigger();  // at the end, as in delta_chunk_kernel
+    pdl_trigger();  // at the end, as in delta_chunk_kernel
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int d = d0 + 8 * (e >> 1), col = col0 + sc + (e & 1);
-    if (d < dim && col < vdim) S[(size_t)d * vdim + col] = s[e];
+    for (int tile = 0; tile < TILES; ++tile)
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (float* p = at(tile, m, e)) *p = s[tile][m][e];
+  } else {
+    const int eight = warp - WORKERS / 32;  // of the read-outs: tokens 8 eight .. + 7 of every chunk; of U: columns 4 eight .. + 3 of every 16
+    uint4 b[3];
+    float2 wv[TILES][2];
+    const int vp = lane & 15;  // this thread's pair of tokens of U
+    auto column = [&](int m) { return 4 * eight + 2 * m + (lane >> 4); };
+    auto fetch = [&](int c) {
+      unit(record_of(c) + B_AT + eight * UNIT, b);
+#pragma unroll
+      for (int tile = 0; tile < TILES; ++tile)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const int col = col0 + 16 * tile + column(m);
+          wv[tile][m] = col < (vdim + RUN - 1) / RUN * RUN ? __ldg(reinterpret_cast<const float2*>(record_of(c) + V_AT + (size_t)col * CHUNK) + vp) : make_float2(0.f, 0.f);
+        }
+    };
+    auto sum_of_shares = [&](int col, int token) {
+      float2 v[SHARES];
+#pragma unroll
+      for (int q = 0; q < SHARES; ++q) v[q] = *reinterpret_cast<const float2*>(parts + (q * COLS + col) * PP + token);
+#pragma unroll
+      for (int m = SHARES / 2; m > 0; m >>= 1)
+#pragma unroll
+        for (int q = 0; q < m; ++q) v[q].x += v[q + m].x, v[q].y += v[q + m].y;
+      return v[0];
+    };
+    fetch(0);
+    for (int c = 0; c < chunks; ++c) {
+      __syncthreads();
+      const int n = t1 - (t0 + c * CHUNK);  // tokens left
+#pragma unroll
+      for (int tile = 0; tile < TILES; ++tile)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {  // U = W V - M S
+          const int col = column(m);
+          const float2 y = sum_of_shares(16 * tile + col, 2 * vp);
+          const Terms t = split3(2 * vp < n ? wv[tile][m].x - y.x : 0.f, 2 * vp + 1 < n ? wv[tile][m].y - y.y : 0.f);
+          uint32_t* to = us + (tile * 2 + (vp >> 3)) * UNIT + ((col & 7) * 4 + (vp & 3)) * 4 + (col >> 3) + 2 * ((vp >> 2) & 1);
+#pragma unroll
+          for (int p = 0; p < 3; ++p) to[p * TERM] = t.v[p];
+        }
+      __syncthreads();
+#pragma unroll
+      for (int tile = 0; tile < TILES; ++tile) {
+        float sum[2][1][4] = {}, small[2][1][4] = {};
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          if (k && eight < 2) break;  // B is triangular
+          Right x[1];
+#pragma unroll
+          for (int p = 0; p < 3; ++p) {
+            x[0].v[p][0] = k ? b[p].z : b[p].x;
+            x[0].v[p][1] = k ? b[p].w : b[p].y;
+          }
+          step<1>(sum[k], small[k], left_of(tile * 2 + k), x);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float2 read = sum_of_shares(16 * tile + gr + 8 * r, CHUNK + 8 * eight + 2 * tg);  // Q c S
+#pragma unroll
+          for (int e = 2 * r; e < 2 * r + 2; ++e) {
+            const int in = gr + 8 * r, i = 8 * eight + 2 * tg + (e & 1), t = t0 + c * CHUNK + i, col = col0 + 16 * tile + in;
+            const float of_state = e & 1 ? read.y : read.x;
+            float v = of_state + ((sum[0][0][e] + sum[1][0][e]) + (small[0][0][e] + small[1][0][e]));
+            if (!is_finite(v)) {
+              float again = 0.f;
+              const uint32_t* rec = reinterpret_cast<const uint32_t*>(record_of(c)) + B_AT + eight * UNIT;
+#pragma unroll 1
+              for (int j = 0; j <= i; ++j) {
+                const int q = (j & 7) >> 1, k = j >> 4, h8 = (j >> 3) & 1;
+                float x = 0.f, y = 0.f;
+                for (int p = 2; p >= 0; --p) {
+                  x += term(rec[p * TERM + ((i & 7) * 4 + q) * 4 + 2 * k + h8], j & 1);
+                  y += term(us[(tile * 2 + k) * UNIT + p * TERM + ((in & 7) * 4 + q) * 4 + (in >> 3) + 2 * h8], j & 1);
+                }
+                again = fmaf(x, y, again);
+              }
+              v = of_state + again;
+            }
+            if (t < t1 && col < vdim) o[((size_t)t * H + h) * vdim + col] = v;
+          }
+        }
+      }
+      if (c + 1 < chunks) fetch(c + 1);
+    }
+    pdl_trigger();
   }
-  if (blockIdx.x == 0 && h == 0) keep_conv_inputs<__nv_bfloat16>(proj, P, base, t0, t1, C, K);
+  if (blockIdx.x == 0 && h == 0) keep_conv_inputs<T>(proj, P, base, t0, t1, C, K);
+}
+
+template <int TILES, typename T>
+int launch_chain(const float* records, const T* proj, long long ld, float* state, const int32_t* item_start, const int32_t* slots, float* o,
+                 int items, int portions, int chunks, int min_tokens, int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats,
+                 cudaStream_t stream) {
+  constexpr int COLS = 16 * TILES, bytes = Chain<TILES>::FLOATS * (int)sizeof(float);
+  auto kernel = delta_chain_kernel<TILES, T>;
+  static PsbPerDevice configured;
+  if (!configured.get()) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) PSB_REFUSE("delta_chain: cannot raise the shared-memory limit");
+    configured.set();
+  }
+  psb_launch(kernel, dim3((vdim + COLS - 1) / COLS, H, portions), dim3(CHAIN_THREADS), (size_t)bytes, stream, records, proj, ld, state, item_start, slots, o,
+             items, chunks, min_tokens, G, H, dim, vdim, K, num_slots, slot_floats);
+  PSB_LAUNCH_CHECK("delta_chain");
+  return 0;
+}
+
+// Runs of columns a block takes.  One block fills an SM, so by rounds over the SMs: a chunk takes a block of one run 2.15 us and one of two 3.3 (the gated
+// rule over 2,000 tokens of 16 heads, 128 blocks, and the other over 1,200 and 960 tokens, 128 blocks).
+template <typename T>
+int chain_of(const void* records, const void* proj, long long ld, void* state, const void* item_start, const void* slots, void* o, int items,
+             int portions, int chunks, int min_tokens, int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats, cudaStream_t stream) {
+  const long long heads = (long long)H * portions, sms = current_sms();
+  const long long rounds16 = (heads * ((vdim + 15) / 16) + sms - 1) / sms, rounds32 = (heads * ((vdim + 31) / 32) + sms - 1) / sms;
+  auto launch = rounds32 * 31 < rounds16 * 20 ? launch_chain<2, T> : launch_chain<1, T>;
+  return launch((const float*)records, (const T*)proj, ld, (float*)state, (const int32_t*)item_start, (const int32_t*)slots, (float*)o, items, portions, chunks,
+                min_tokens, G, H, dim, vdim, K, num_slots, slot_floats, stream);
 }
 
 }  // namespace
 
 // (dim, vdim) -> float32 numbers of a chunk's record of a head, 0 if the kernels are not built for the sizes
 PSB_API int psb_delta_chunk_record(int dim, int vdim) {
-  return dim >= 4 && dim <= RP && dim % 4 == 0 && vdim >= 4 && vdim % 4 == 0 ? RECORD : 0;
+  return dim >= 4 && dim <= RP && dim % 4 == 0 && vdim >= 4 && vdim % 4 == 0 && vdim <= (1 << 20) ? record_floats(vdim) : 0;
 }
 
 // () -> tokens of a chunk
 PSB_API int psb_delta_chunk_tokens() { return CHUNK; }
 
 // The rule over every portion of at least ``min_tokens`` tokens, from what psb_delta_prepare left; other tokens, and the slots of
-// other portions, are left untouched.  records [chunks, H, RECORD] float32, portions and chunks at least the number of these portions
-// and of their chunks.
+// other portions, are left untouched.  records [chunks, H, psb_delta_chunk_record] float32, portions and chunks at least the number of these
+// portions and of their chunks.
 // (qkv, bd, proj bfloat16, ld, state, item_start, slots, records, o_out, items, portions, chunks, min_tokens, G, H, dim, vdim, K,
 //  num_slots, slot_floats, stream)
 PSB_API int psb_delta_chunks(const void* qkv, const void* bd, const void* proj, long long ld, void* state, const void* item_start,
@@ -426,22 +619,50 @@ PSB_API int psb_delta_chunks(const void* qkv, const void* bd, const void* proj, 
   if (K < 1 || K > MAX_TAPS || min_tokens < 1 || num_slots < 1) PSB_REFUSE("delta_chunks: %d taps are outside [1, %d], or no tokens or slots", K, MAX_TAPS);
   const long long C = 2LL * G * dim + (long long)H * vdim;
   if (ld < C || slot_floats != (K - 1) * C + (long long)H * dim * vdim) PSB_REFUSE("delta_chunks: the slot or the rows do not fit the sizes");
-  if (H > 65535 || portions > 65535 || chunks < 0) PSB_REFUSE("delta_chunks: too many heads or requests for one launch");
-  if (((uintptr_t)qkv | (uintptr_t)records) & 15) PSB_REFUSE("delta_chunks: operands must be 16-byte aligned");
+  if (H > 65535 || portions > 65535 || chunks < 0 || (long long)chunks * H > 0x7fffffffLL) PSB_REFUSE("delta_chunks: too many heads or requests for one launch");
+  if (((uintptr_t)qkv | (uintptr_t)records | (uintptr_t)o) & 15) PSB_REFUSE("delta_chunks: operands must be 16-byte aligned");
   if (items == 0 || portions < 1 || chunks == 0) return 0;
-  constexpr int bytes = ChainShape::FLOATS * (int)sizeof(float);
+  constexpr int bytes = ChunkShape::FLOATS * (int)sizeof(float);
   static PsbPerDevice configured;
   if (!configured.get()) {
-    if (cudaFuncSetAttribute(delta_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
-      PSB_REFUSE("delta_chunks: cannot raise the shared-memory limit");
+    if (cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) PSB_REFUSE("delta_chunks: cannot raise the shared-memory limit");
     configured.set();
   }
-  psb_launch(delta_chunk_kernel, dim3(chunks, G), dim3(CHUNK_THREADS), 0, stream, (const float*)qkv, (const float*)bd, (const int32_t*)item_start,
+  psb_launch(delta_chunk_kernel, dim3((unsigned)chunks * H), dim3(CHUNK_THREADS), (size_t)bytes, stream, (const float*)qkv, (const float*)bd, (const int32_t*)item_start,
              (float*)records, items, min_tokens, G, H, dim, vdim);
   PSB_LAUNCH_CHECK("delta_chunk");
-  psb_launch(delta_chain_kernel, dim3((vdim + COLS - 1) / COLS, H, portions), dim3(CHAIN_THREADS), (size_t)bytes, stream, (const float*)qkv,
-             (const float*)records, (const __nv_bfloat16*)proj, ld, (float*)state, (const int32_t*)item_start, (const int32_t*)slots, (float*)o,
-             items, chunks, min_tokens, G, H, dim, vdim, K, num_slots, slot_floats);
-  PSB_LAUNCH_CHECK("delta_chain");
+  return chain_of<__nv_bfloat16>(records, proj, ld, state, item_start, slots, o, items, portions, chunks, min_tokens, G, H, dim, vdim, K, num_slots, slot_floats, stream);
+}
+
+// (dim, vdim) -> float32 numbers of a chunk's record of a head for the rule with a decay per channel, 0 if the kernels are not built for the sizes
+PSB_API int psb_channel_delta_chunk_record(int dim, int vdim) { return dim >= 1 && dim <= RP && vdim >= 1 && vdim <= 4096 ? record_floats(vdim) : 0; }
+
+// The rule with a decay per channel: as above, with decay float32 [T, H, dim] and a projection of either type.
+// (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, records, o_out, items, portions, chunks, min_tokens, G, H, dim, vdim, K,
+//  num_slots, slot_floats, stream)
+PSB_API int psb_channel_delta_chunks32(const void* qkv, const void* bd, const void* decay, const void* proj, int dtype, long long ld, void* state,
+                                       const void* item_start, const void* slots, void* records, void* o, int items, int portions, int chunks, int min_tokens,
+                                       int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats, cudaStream_t stream) {
+  if (items < 0 || G < 1 || H < 1 || H % G || !psb_channel_delta_chunk_record(dim, vdim)) PSB_REFUSE("channel_delta_chunks: bad sizes G=%d H=%d dim=%d vdim=%d", G, H, dim, vdim);
+  if (K < 1 || K > MAX_TAPS || min_tokens < 1 || num_slots < 1) PSB_REFUSE("channel_delta_chunks: %d taps are outside [1, %d], or no tokens or slots", K, MAX_TAPS);
+  const long long C = 2LL * G * dim + (long long)H * vdim;
+  if (ld < C || slot_floats != (K - 1) * C + (long long)H * dim * vdim) PSB_REFUSE("channel_delta_chunks: the slot or the rows do not fit the sizes");
+  if (H > 65535 || portions > 65535 || chunks < 0 || (long long)chunks * H > 0x7fffffffLL) PSB_REFUSE("channel_delta_chunks: too many heads or requests for one launch");
+  if (((uintptr_t)records | (uintptr_t)o) & 15) PSB_REFUSE("channel_delta_chunks: records and read-out must be 16-byte aligned");
+  if (items == 0 || portions < 1 || chunks == 0) return 0;
+  constexpr int bytes = ChannelShape::FLOATS * (int)sizeof(float);
+  static PsbPerDevice configured;
+  if (!configured.get()) {
+    if (cudaFuncSetAttribute(channel_delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+      PSB_REFUSE("channel_delta_chunks: cannot raise the shared-memory limit");
+    configured.set();
+  }
+  const bool wide_decay = dim % 4 == 0 && ((uintptr_t)decay & 15) == 0, wide = dim % 4 == 0 && C % 4 == 0 && ((uintptr_t)qkv & 15) == 0;
+  psb_launch(channel_delta_chunk_kernel, dim3((unsigned)chunks * H), dim3(CHUNK_THREADS), (size_t)bytes, stream, (const float*)qkv, (const float*)bd, (const float*)decay,
+             (const int32_t*)item_start, (float*)records, items, min_tokens, G, H, dim, vdim, wide, wide_decay);
+  PSB_LAUNCH_CHECK("channel_delta_chunk");
+  PSB_DISPATCH_DTYPE(dtype, T_, {
+    return chain_of<T_>(records, proj, ld, state, item_start, slots, o, items, portions, chunks, min_tokens, G, H, dim, vdim, K, num_slots, slot_floats, stream);
+  });
   return 0;
 }

@@ -44,6 +44,9 @@ using namespace delta;
 __device__ __forceinline__ float softplusf_(float x) { return log1pf(expf(-fabsf(x))) + fmaxf(x, 0.f); }
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + expf(-x)); }
 __device__ __forceinline__ float siluf_(float x) { return x / (1.f + expf(-x)); }
+// what makes a vector with this sum of squares a unit vector, over sqrt(dim) for queries (keys: 1).  (rsqrtf(dim) is off by up to two units of the last place,
+// in every query alike.)
+__device__ __forceinline__ float unit_factor(float squares, int dim) { return 1.f / sqrtf((float)dim) / sqrtf(squares + 1e-6f); }
 
 // A block per (token, unit); a unit is one query group, one key group (dim channels each) or one value head (vdim).
 template <typename T>
@@ -96,7 +99,7 @@ delta_prepare_kernel(const T* __restrict__ proj, const float* __restrict__ ba, c
     if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
     __syncthreads();
     const float total = scratch[0] + scratch[1] + scratch[2] + scratch[3];
-    factor = (unit < G ? rsqrtf((float)dim) : 1.f) / sqrtf(total + 1e-6f);
+    factor = unit_factor(total, unit < G ? dim : 1);
   }
   float* out = qkv + (size_t)t * C + c0;
   for (int i = threadIdx.x; i < len; i += blockDim.x) out[i] = row[i] * factor;  // a thread reads back what it wrote
@@ -197,7 +200,7 @@ delta_prepare_run_kernel(const T* __restrict__ proj, const float* __restrict__ b
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < RUN_TOKENS; ++i)
-      factor[i] = (unit < G ? rsqrtf((float)dim) : 1.f) / sqrtf(scratch[i][0] + scratch[i][1] + scratch[i][2] + scratch[i][3] + 1e-6f);
+      factor[i] = unit_factor(scratch[i][0] + scratch[i][1] + scratch[i][2] + scratch[i][3], unit < G ? dim : 1);
   }
 #pragma unroll
   for (int u = 0; u < CH; ++u) {
@@ -325,7 +328,7 @@ delta_prepare_wide_kernel(const T* __restrict__ proj, const float* __restrict__ 
       float ss = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; ++j) ss = fmaf(y[i][j], y[i][j], ss);
-      const float factor = (unit < G ? rsqrtf((float)dim) : 1.f) / sqrtf(warp_sum(ss) + 1e-6f);
+      const float factor = unit_factor(warp_sum(ss), unit < G ? dim : 1);
 #pragma unroll
       for (int j = 0; j < 4; ++j) y[i][j] *= factor;
     }
@@ -587,7 +590,7 @@ __global__ void __launch_bounds__(RULE_WARPS * 32)
 channel_delta_rule_kernel(const float* __restrict__ qkv, const float* __restrict__ bd, const float* __restrict__ decay,
                           const T* __restrict__ proj, long long P, float* __restrict__ state, const int32_t* __restrict__ item_start,
                           const int32_t* __restrict__ slots, float* __restrict__ o, int G, int H, int dim, int vdim, int K,
-                          int num_slots, long long slot_floats, int stage_tokens) {
+                          int num_slots, long long slot_floats, int stage_tokens, int max_tokens) {
   extern __shared__ __align__(16) float staged[];  // [2][stage_tokens][W]: q, k, g (RP each, zeros beyond dim), values, bd
   constexpr int COLS = 32 / R, RP = R * PER, BC = RULE_WARPS * COLS, W = (3 * RP + BC + BD + 3) / 4 * 4;
   static_assert(RP % 4 == 0, "a token's vectors start on 16 bytes");
@@ -602,6 +605,7 @@ channel_delta_rule_kernel(const float* __restrict__ qkv, const float* __restrict
   const bool wide = dim % 4 == 0 && C % 4 == 0 && (((uintptr_t)qkv | (uintptr_t)decay) & 15) == 0;
   pdl_wait();
   const int t0 = item_start[item], t1 = item_start[item + 1];
+  if (t1 - t0 > max_tokens) return;  // a portion of the kernels that work in chunks
   int slot = slots[item];
   slot = slot < 0 ? 0 : (slot >= num_slots ? num_slots - 1 : slot);
   float* base = state + (size_t)slot * slot_floats;
@@ -733,7 +737,7 @@ channel_delta_rule_kernel(const float* __restrict__ qkv, const float* __restrict
   if (blockIdx.x == 0 && h == 0) keep_conv_inputs<T>(proj, P, base, t0, t1, C, K);
 }
 
-// The same rule for long portions, sixteen tokens at a time.  Within a chunk, with c_i = g_1 ... g_i (the decays from the
+// The same rule for long portions and keys of 129 to 256 numbers, sixteen tokens at a time (shorter keys: delta_chunks.cu).  Within a chunk, with c_i = g_1 ... g_i (the decays from the
 // chunk's start up to token i, each a product of numbers of at most one, nothing is ever divided by a decay) and S the state
 // before the chunk,
 //
@@ -1221,11 +1225,11 @@ PSB_API int psb_delta_rule(const void* qkv, const void* bd, const void* proj, in
   return 0;
 }
 
-// (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, o_out, items, G, H, dim, vdim, K, num_slots, slot_floats, lanes, stream)
-// ``lanes`` as for psb_delta_rule (4, 8, 16 or 32).
+// (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, o_out, items, G, H, dim, vdim, K, num_slots, slot_floats, lanes, max_tokens,
+//  stream)  ``lanes`` (4, 8, 16 or 32) and ``max_tokens`` as for psb_delta_rule.
 PSB_API int psb_channel_delta_rule(const void* qkv, const void* bd, const void* decay, const void* proj, int dtype, long long ld,
                                    void* state, const void* item_start, const void* slots, void* o, int items, int G, int H, int dim,
-                                   int vdim, int K, int num_slots, long long slot_floats, int lanes, cudaStream_t stream) {
+                                   int vdim, int K, int num_slots, long long slot_floats, int lanes, int max_tokens, cudaStream_t stream) {
   if (items < 0 || G < 1 || H < 1 || H % G || dim < 1 || vdim < 1) PSB_REFUSE("channel_delta_rule: bad sizes G=%d H=%d dim=%d vdim=%d", G, H, dim, vdim);
   if (K < 1 || K > MAX_TAPS) PSB_REFUSE("channel_delta_rule: %d taps are outside [1, %d]", K, MAX_TAPS);
   if (lanes != 4 && lanes != 8 && lanes != 16 && lanes != 32) PSB_REFUSE("channel_delta_rule: %d lanes a column is not built (4, 8, 16 or 32)", lanes);
@@ -1253,7 +1257,7 @@ PSB_API int psb_channel_delta_rule(const void* qkv, const void* bd, const void* 
     }                                                                                                                              \
     psb_launch(kernel, grid, dim3(RULE_WARPS * 32), (size_t)smem, stream, (const float*)qkv, (const float*)bd, (const float*)decay, \
                (const T_*)proj, ld, (float*)state, (const int32_t*)item_start, (const int32_t*)slots, (float*)o, G, H, dim, vdim, K, \
-               num_slots, slot_floats, stage_tokens);                                                                              \
+               num_slots, slot_floats, stage_tokens, max_tokens);                                                                  \
   } while (0)
   PSB_DISPATCH_DTYPE(dtype, T_, {
     if (lanes == 4) {
@@ -1272,10 +1276,11 @@ PSB_API int psb_channel_delta_rule(const void* qkv, const void* bd, const void* 
   return 0;
 }
 
-// (dim, vdim) -> float32 numbers of a chunk's record, 0 if the chunked form does not take the sizes
+// (dim, vdim) -> float32 numbers of a chunk's record, 0 if the chunked form does not take the sizes (keys of up to 128 numbers go through
+// the kernels of delta_chunks.cu)
 PSB_API int psb_channel_delta_record(int dim, int vdim) {
-  if (dim < 1 || vdim < 1 || dim > 256 || vdim > 4096) return 0;
-  return ChunkRecord{dim <= 128 ? 128 : 256, (vdim + CHAIN_COLS - 1) / CHAIN_COLS * CHAIN_COLS}.floats();
+  if (dim <= 128 || vdim < 1 || dim > 256 || vdim > 4096) return 0;
+  return ChunkRecord{256, (vdim + CHAIN_COLS - 1) / CHAIN_COLS * CHAIN_COLS}.floats();
 }
 
 // The chunked form: (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, records, o_out, items, chunks, G, H, dim, vdim, K,
@@ -1292,33 +1297,27 @@ PSB_API int psb_channel_delta_chunks(const void* qkv, const void* bd, const void
   if (((uintptr_t)records | (uintptr_t)o) & 15) PSB_REFUSE("channel_delta_chunks: records and read-out must be 16-byte aligned");
   if (items == 0) return 0;
   const int vpad = (vdim + CHAIN_COLS - 1) / CHAIN_COLS * CHAIN_COLS;
-#define PSB_CHAIN(LR_)                                                                                                            \
-  do {                                                                                                                            \
-    constexpr int RP = 32 * LR_;                                                                                                  \
-    constexpr int chunk_bytes = 3 * CH * RP * (int)sizeof(float);                                                                 \
-    constexpr int chain_bytes = 2 * ((3 * CH + 1) * RP + CH * B_PITCH + CH * CHAIN_COLS) * (int)sizeof(float);                    \
-    auto chunk = channel_delta_chunk_kernel<LR_>;                                                                                 \
-    auto chain = channel_delta_chain_kernel<T_, LR_>;                                                                             \
-    static PsbPerDevice configured;                                                                                               \
-    if (!configured.get()) {                                                                                                      \
-      if (cudaFuncSetAttribute(chunk, cudaFuncAttributeMaxDynamicSharedMemorySize, chunk_bytes) != cudaSuccess ||                 \
-          cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize, chain_bytes) != cudaSuccess)                   \
-        PSB_REFUSE("channel_delta_chunks: cannot raise the shared-memory limit");                                                 \
-      configured.set();                                                                                                           \
-    }                                                                                                                             \
-    psb_launch(chunk, dim3(chunks, H), dim3(128), (size_t)chunk_bytes, stream, (const float*)qkv, (const float*)bd,               \
-               (const float*)decay, (const int32_t*)item_start, (float*)records, items, G, H, dim, vdim, vpad);                   \
-    PSB_LAUNCH_CHECK("channel_delta_chunk");                                                                                      \
-    psb_launch(chain, dim3(vpad / CHAIN_COLS, H, items), dim3(RULE_WARPS * 32), (size_t)chain_bytes, stream, (const float*)records, \
-               (const T_*)proj, ld, (float*)state, (const int32_t*)item_start, (const int32_t*)slots, (float*)o, G, H, dim, vdim, \
-               vpad, K, num_slots, slot_floats);                                                                                  \
-    PSB_LAUNCH_CHECK("channel_delta_chain");                                                                                      \
-  } while (0)
+constexpr int LR = 8, RP = 32 * LR;
+  constexpr int chunk_bytes = 3 * CH * RP * (int)sizeof(float);
+  constexpr int chain_bytes = 2 * ((3 * CH + 1) * RP + CH * B_PITCH + CH * CHAIN_COLS) * (int)sizeof(float);
   PSB_DISPATCH_DTYPE(dtype, T_, {
-    if (dim <= 128) PSB_CHAIN(4);
-    else PSB_CHAIN(8);
+    auto chunk = channel_delta_chunk_kernel<LR>;
+    auto chain = channel_delta_chain_kernel<T_, LR>;
+    static PsbPerDevice configured;
+    if (!configured.get()) {
+      if (cudaFuncSetAttribute(chunk, cudaFuncAttributeMaxDynamicSharedMemorySize, chunk_bytes) != cudaSuccess ||
+          cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize, chain_bytes) != cudaSuccess)
+        PSB_REFUSE("channel_delta_chunks: cannot raise the shared-memory limit");
+      configured.set();
+    }
+    psb_launch(chunk, dim3(chunks, H), dim3(128), (size_t)chunk_bytes, stream, (const float*)qkv, (const float*)bd,
+               (const float*)decay, (const int32_t*)item_start, (float*)records, items, G, H, dim, vdim, vpad);
+    PSB_LAUNCH_CHECK("channel_delta_chunk");
+    psb_launch(chain, dim3(vpad / CHAIN_COLS, H, items), dim3(RULE_WARPS * 32), (size_t)chain_bytes, stream, (const float*)records,
+               (const T_*)proj, ld, (float*)state, (const int32_t*)item_start, (const int32_t*)slots, (float*)o, G, H, dim, vdim,
+               vpad, K, num_slots, slot_floats);
+    PSB_LAUNCH_CHECK("channel_delta_chain");
   });
-#undef PSB_CHAIN
   return 0;
 }
 

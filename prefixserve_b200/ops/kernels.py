@@ -1178,17 +1178,17 @@ DELTA_LONG_LANES = 16   # measured: 32 lanes (a column a warp) took 807 us for a
 
 
 # Portions of this many tokens in bfloat16 take the form that works 32 tokens at a time (keys of up to 128 numbers).  All four kernels, 16 heads over 8
-# groups of 128, nothing in L2: one portion of 8 tokens 35 us in chunks and 47 token by token, of 32 tokens 37 and 55, of 128 53 and 86.
+# groups of 128, nothing in L2: one portion of 8 tokens 38 us in chunks and 48 token by token, of 32 tokens 40 and 56, of 128 52 and 89.
 DELTA_CHUNKED = 8
 
 
 def _delta_one_by_one(lengths: list[int] | None) -> bool:
     """Whether a step with portions on both sides of DELTA_CHUNKED is over sooner token by token: it pays for both forms, one after
     the other, and the chunks' share has to be worth that.  The more so the longer and the more the short ones are (16 heads, both forms
-    and token by token: 16 tokens beside one 55 and 55 us, 24 beside eight 61 and 61; 24 beside 32 86 and 74, and 32, where that
-    kernel shares a column among more lanes, 86 and 104; 16, 12 and 7 tokens 73 and 61)."""
+    and token by token: 16 tokens beside one 55 and 52 us, 24 beside eight 64 and 64; 24 beside 32 86 and 71, and 32, where that
+    kernel shares a column among more lanes, 86 and 103; 16, 12 and 7 tokens 76 and 59)."""
     short = [n for n in lengths or [] if n < DELTA_CHUNKED]
-    return bool(short) and max(lengths) < min(DELTA_LONG_PORTION, 13 + 3 * max(short) + len(short) * 5 // 8)
+    return bool(short) and max(lengths) < min(DELTA_LONG_PORTION, 14 + 3 * max(short) + len(short) * 5 // 8)
 
 
 def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
@@ -1524,8 +1524,21 @@ def matrix_memory(proj: torch.Tensor, bias_i: torch.Tensor, bias_f: torch.Tensor
     return out
 
 
-CHANNEL_DELTA_CHUNKED = 24     # steps whose longest portion has this many tokens take the form that works 16 tokens at a time
+# Steps whose longest portion has this many tokens take the form that works 32 tokens at a time (keys of up to 128 numbers; 16 heads over 8 groups of 128,
+# nothing in L2: 8 tokens 40 us in chunks and 44 token by token, 24 tokens 42 and 52, 128 tokens 67 and 103).  Where many portions are shorter, those go
+# token by token.
+CHANNEL_DELTA_LEAST = 8
+CHANNEL_DELTA_CHUNKED = 24     # ... with longer keys the form that works 16 tokens at a time
 CHANNEL_DELTA_LONG_LANES = 16  # ... or, with keys of more than 256 numbers, this many lanes a column instead of 4
+
+
+def _channel_delta_apart(ctx, blocks: int) -> bool:
+    """Whether portions below CHANNEL_DELTA_LEAST tokens go token by token beside longer ones in chunks: each of them would be ``blocks``
+    blocks of the chain that fill an SM and have next to nothing to do.  Single tokens beside 64 and beside 512 tokens, us apart and together
+    (64 blocks each): 4 of them 72 and 50, 109 and 104; 8 74 and 63, 115 and 120; 16 90 and 106, 121 and 136; 64 121 and 253, 156 and 280."""
+    lengths = _portion_lengths(ctx)
+    count = ctx.num_items - 1 if lengths is None else sum(n < CHANNEL_DELTA_LEAST for n in lengths)
+    return count * blocks > 5 * 148
 
 
 def channel_delta_rule(proj: torch.Tensor, beta_at: int, decay: torch.Tensor, taps: torch.Tensor, state: torch.Tensor, ctx, *,
@@ -1548,28 +1561,42 @@ def channel_delta_rule(proj: torch.Tensor, beta_at: int, decay: torch.Tensor, ta
     bd = torch.empty((t, 5 * heads), dtype=torch.float32, device=dev)
     item_start, slots = _i32(ctx.item_start, "item offsets"), _i32(ctx.slots, "slots")
     code, ld = _code(proj, "projection output"), proj.shape[1]
-    long = ctx.max_new_tokens >= CHANNEL_DELTA_CHUNKED
-    record = int(lib().psb_channel_delta_record(dim, vdim)) if long else 0
-    check(lib().psb_delta_prepare(proj.data_ptr(), code, ld, beta_at, None, None if record else decay.data_ptr(), taps.data_ptr(), None, None,
+    record = tokens = least = 0   # of a chunk: numbers, tokens; portions of at least ``least`` tokens go in chunks
+    narrow = dim <= 128
+    if ctx.max_new_tokens >= (CHANNEL_DELTA_LEAST if narrow else CHANNEL_DELTA_CHUNKED):
+        record = int((lib().psb_channel_delta_chunk_record if narrow else lib().psb_channel_delta_record)(dim, vdim))
+        tokens = lib().psb_delta_chunk_tokens() if narrow else 16
+        least = CHANNEL_DELTA_LEAST if narrow and _channel_delta_apart(ctx, heads * -(-vdim // 32)) else 1
+    short = not record or (least > 1 and _has_portions_below(ctx, least))
+    check(lib().psb_delta_prepare(proj.data_ptr(), code, ld, beta_at, None, decay.data_ptr() if short else None, taps.data_ptr(), None, None,
                                   state.data_ptr(), _i32(ctx.positions, "positions").data_ptr(),
                                   _i32(ctx.token_item, "token-to-item map").data_ptr(), item_start.data_ptr(), slots.data_ptr(),
                                   qkv.data_ptr(), bd.data_ptr(), t, groups, heads, dim, vdim, k, state.shape[0], slot_floats, 1, _stream()),
           "delta_prepare")
     o = torch.empty((t, heads, vdim), dtype=torch.float32, device=dev)
-    if record:
-        chunks = t // 16 + ctx.num_items
+    most = 0x7fffffff  # tokens of the longest portion left to the kernel that goes token by token
+    if record and dim <= 128:
+        most = least - 1
+        portions, chunks = _portions_from(ctx, least), _portion_tiles(ctx, t, least, tokens)
+        records = torch.empty((chunks, heads, record), dtype=torch.float32, device=dev)
+        check(lib().psb_channel_delta_chunks32(qkv.data_ptr(), bd.data_ptr(), decay.data_ptr(), proj.data_ptr(), code, ld, state.data_ptr(),
+                                               item_start.data_ptr(), slots.data_ptr(), records.data_ptr(), o.data_ptr(), ctx.num_items, portions,
+                                               chunks, least, groups, heads, dim, vdim, k, state.shape[0], slot_floats, _stream()),
+              "channel_delta_chunks")
+    elif record:
+        chunks = t // tokens + ctx.num_items
         records = torch.empty((chunks, heads, record), dtype=torch.float32, device=dev)
         check(lib().psb_channel_delta_chunks(qkv.data_ptr(), bd.data_ptr(), decay.data_ptr(), proj.data_ptr(), code, ld, state.data_ptr(),
                                              item_start.data_ptr(), slots.data_ptr(), records.data_ptr(), o.data_ptr(), ctx.num_items,
                                              chunks, groups, heads, dim, vdim, k, state.shape[0], slot_floats, _stream()),
               "channel_delta_chunks")
-        return o
-    lanes = CHANNEL_DELTA_LONG_LANES if long and dim >= CHANNEL_DELTA_LONG_LANES else 4
-    while dim > 32 * lanes and lanes < 32:
-        lanes *= 2
-    check(lib().psb_channel_delta_rule(qkv.data_ptr(), bd.data_ptr(), decay.data_ptr(), proj.data_ptr(), code, ld, state.data_ptr(),
-                                       item_start.data_ptr(), slots.data_ptr(), o.data_ptr(), ctx.num_items, groups, heads, dim, vdim, k,
-                                       state.shape[0], slot_floats, lanes, _stream()), "channel_delta_rule")
+    if short:
+        lanes = CHANNEL_DELTA_LONG_LANES if min(ctx.max_new_tokens, most) >= CHANNEL_DELTA_CHUNKED and dim >= CHANNEL_DELTA_LONG_LANES else 4
+        while dim > 32 * lanes and lanes < 32:
+            lanes *= 2
+        check(lib().psb_channel_delta_rule(qkv.data_ptr(), bd.data_ptr(), decay.data_ptr(), proj.data_ptr(), code, ld, state.data_ptr(),
+                                           item_start.data_ptr(), slots.data_ptr(), o.data_ptr(), ctx.num_items, groups, heads, dim, vdim, k,
+                                           state.shape[0], slot_floats, lanes, most, _stream()), "channel_delta_rule")
     return o
 
 

@@ -208,8 +208,8 @@ _SIGNATURES: dict[str, list] = {
     # (proj, dtype, ld, beta_at, ba, decay, taps, a_log, dt_bias, state, positions, token_item, item_start, slots, qkv_out, bd_out, T,
     #  G, H, dim, vdim, K, num_slots, slot_floats, cross, stream)
     "psb_delta_prepare": [P, I, L, I, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, L, I, P],
-    # (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, o_out, items, G, H, dim, vdim, K, num_slots, slot_floats, lanes, stream)
-    "psb_channel_delta_rule": [P, P, P, P, I, L, P, P, P, P, I, I, I, I, I, I, I, L, I, P],
+    # (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, o_out, items, G, H, dim, vdim, K, num_slots, slot_floats, lanes, max_tokens, stream)
+    "psb_channel_delta_rule": [P, P, P, P, I, L, P, P, P, P, I, I, I, I, I, I, I, L, I, I, P],
     # (qkv, bd, proj, dtype, state, item_start, slots, o_out, items, G, H, dim, vdim, K, num_slots, slot_floats, lanes, max_tokens, stream)
     "psb_delta_rule": [P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, L, I, I, P],
     # (dim, vdim) -> float32 numbers of a chunk's record of a head, 0: not built for the sizes; () -> tokens of a chunk
@@ -222,6 +222,11 @@ _SIGNATURES: dict[str, list] = {
     "psb_channel_delta_record": [I, I],
     # (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, records, o_out, items, chunks, G, H, dim, vdim, K, num_slots,
     #  slot_floats, stream)
+    # (dim, vdim) -> float32 numbers of a 32-token chunk's record, 0: not built
+    "psb_channel_delta_chunk_record": [I, I],
+    # (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, records, o, items, portions, chunks, min_tokens, G, H, dim, vdim, K,
+    #  num_slots, slot_floats, stream)
+    "psb_channel_delta_chunks32": [P, P, P, P, I, L, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, L, P],
     "psb_channel_delta_chunks": [P, P, P, P, I, L, P, P, P, P, P, I, I, I, I, I, I, I, I, L, P],
     # (o, proj, dtype, gain, out, T, G, H, dim, vdim, eps, stream)
     "psb_delta_finish": [P, P, I, P, P, I, I, I, I, I, F, P],

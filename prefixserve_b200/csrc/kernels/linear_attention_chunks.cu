@@ -1,399 +1,415 @@
-// Gated linear attention (linear_attention.cu) over long portions of bfloat16 projections, 64 tokens at a time on the tensor cores,
+// Gated linear attention (linear_attention.cu) over long portions of bfloat16 projections, 32 tokens at a time on the tensor cores,
 // float32 throughout:
 //
 //     S <- diag(alpha_t) S + k_t v_t^T,    o_t = S^T q_t * scale.
 //
-// With c_i = alpha_1 .. alpha_i from a chunk's start and r_j = alpha_(j+1) .. alpha_64, per key channel,
-//   linear_local_kernel    every chunk from a zero state: B = sum_j (k_j r_j) v_j^T, and A = c_64;
-//   linear_starts_kernel   per portion, chunk by chunk: the state every chunk starts from (over B), and the slot's new state;
-//   linear_read_kernel     O = (Q c) S + P V,  P_ij = sum_d q_i k_j alpha_(j+1) .. alpha_i  (j <= i).
-// Decays are only ever multiplied, never divided by, so P is made in blocks of 16 x 16 tokens: off the diagonal as products of
-// q_i alpha_(start of i's run) .. alpha_i and k_j alpha_(j+1) .. alpha_(end of j's run) with whole runs' decays between them, on the
-// diagonal with a running product a column (four columns a warp, four channels a lane).
-// Products of float32 numbers enter the tensor cores in terms (tf32_terms.cuh: all of them for P, those of lo lo too for (Q c) S, P to
-// its last bit for P V), the values, which are bfloat16, as they are.
+// With c_i = alpha_1 .. alpha_i from a chunk's start, r_j = alpha_(j+1) .. alpha_32, per key channel, and S the state before the chunk,
+//     O = (Q c) S + P V,  P_ij = sum_d q_i k_j alpha_(j+1) .. alpha_i  (j <= i),    S <- diag(c_32) S + (K r)^T V.
+//   linear_chunk_kernel   a block per chunk and head, all chunks of the step side by side: P, Q c, K r, c_32 and V as the chain takes them, 64 KB;
+//   linear_chain_kernel   a block per 16 or 32 columns of a head's state and portion walks the chunks: eight warps hold 16 key channels of S
+//                         each, in registers, multiply Q c by it (eight shares, through shared memory) and bring it up to date, four more
+//                         add the shares and P V up behind them.  What a chunk brings goes straight into the registers of those who use it, a chunk ahead.
+// Decays are only ever multiplied, never divided by, and the running ones of a chunk carry what the roundings lose.  float32 numbers enter the tensor cores in three
+// terms (chunk_products.cuh), the values, which are bfloat16, as they are.
 // P is zero above the diagonal, and zero times a value that is not finite is not zero: a result that comes out not finite is made
 // again from the tokens up to its own.
-// Running products of decays carry what their roundings lose.  With that read-outs lie at 1.15e-7 to 1.18e-7 from float64, token by
-// token at 1.21e-7 to 1.25e-7 (100, 300 and 1,811 tokens), states at 0.80e-7 and 0.95e-7; with two terms throughout read-outs came out
-// at 1.28e-7 to 1.30e-7, 1,811 tokens in 119 us instead of 129.  A float32 projection's values would need terms too; those stay with the
-// other kernels.
+// A float32 projection's values would need terms too; those stay with the other kernels.
 //
-// What bounds it: the read-out, by what its warps issue and by its five phases one after the other, one block of 16 warps an SM
-// (190 KB of shared memory).  1,811 tokens of 16 heads of 128: local 31 us, starts 11, read-out 87; the token-by-token kernels took
-// 73, 13 and 114.  Eight warps a block took 112 us for the read-out.
-#include <type_traits>
-
-#include "portions.cuh"
-#include "tf32_terms.cuh"
+// Distances from float64, token by token and here (150 and 700 tokens): read-outs 1.2e-7 and 1.03e-7, states 0.95e-7 and 0.59e-7.
+//
+// What bounds it: the chain, by what a chunk brings from L2 (64 KB an SM and chunk, 1.1 us) and the latency of its steps.  1,811 tokens of 16 heads of 128:
+// chunk kernel 42 us, chain 63; chunks of 64 tokens all side by side, the states they start from in a pass between two kernels, took 31, 11 and 87 us
+// and were bound by the read-out's phases, one block an SM, in four rounds.  Two chunks ahead through shared memory: no faster.
+#include "chunk_products.cuh"
 
 namespace {
-using namespace terms;
+using namespace chunks;
 
-constexpr int CHUNK = 64, RUN = 16, RUNS = CHUNK / RUN, RP = 128, KP = RP + 8, VP = RP + 4, PP = CHUNK + 8, THREADS = 512;
+// A chunk's record of a head, 32-bit words: Q c (per 16 channels, per two eights of tokens, both fragments of either), K r (per 16 channels, per eight
+// of them, the fragments of either half of the tokens), P (per eight of its rows, the same), c_32 [128], and V per 16 columns and half of the tokens as
+// left operands' fragments.
+constexpr int Q_AT = 0, K_AT = Q_AT + (RP / 16) * 2 * UNIT, P_AT = K_AT + (RP / 16) * 2 * UNIT, G_AT = P_AT + (CHUNK / 8) * UNIT, V_AT = G_AT + RP;
+__host__ __device__ constexpr int record_floats(int vdim) { return V_AT + (vdim + 15) / 16 * 2 * TERM; }
 
-// Products over k take the places 2 tg and 2 tg + 1 of every eight (instead of tg and tg + 4) of both operands: rows give them as one
-// 8-byte load.  Pitches are such that such loads (KP, PP), and loads down a column (VP), meet every bank once.
-__device__ __forceinline__ void load_row_pairs(const float* a, int down, float2 factor, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
-#pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    const float2 x = *reinterpret_cast<const float2*>(a + e * down);
-    const Split u = split_product(x.x, factor.x), v = split_product(x.y, factor.y);
-    hi[e] = u.hi;
-    lo[e] = u.lo;
-    hi[2 + e] = v.hi;
-    lo[2 + e] = v.lo;
-  }
-}
-
-// 64 rows of ``src`` (row pitch ld, ``width`` numbers, zeros beyond them and beyond n rows) as float32
-template <typename T, int PITCH>
-__device__ __forceinline__ void bring(float* dst, const T* __restrict__ src, long long ld, int n, int width) {
-  constexpr int EACH = CHUNK * RP / 4 / THREADS;
-  using Raw = typename std::conditional<sizeof(T) == 2, uint2, float4>::type;
-  Raw raw[EACH];
+// 32 rows of bfloat16 (row pitch ld, ``dim`` numbers in fours, zeros beyond them and beyond n rows) as float32 [32][KP]
+__device__ __forceinline__ void widen_rows(float* dst, const __nv_bfloat16* __restrict__ src, long long ld, int n, int dim) {
+  constexpr int EACH = CHUNK * RP / 4 / CHUNK_THREADS;
+  uint2 raw[EACH];
 #pragma unroll
   for (int e = 0; e < EACH; ++e) {  // asked for together
-    const int i = threadIdx.x + e * THREADS, t = i / (RP / 4), d = (i % (RP / 4)) * 4;
-    raw[e] = Raw{};
-    if (t < n && d < width) raw[e] = *reinterpret_cast<const Raw*>(src + (size_t)t * ld + d);
+    const int i = threadIdx.x + e * CHUNK_THREADS, t = i / (RP / 4), d = (i % (RP / 4)) * 4;
+    raw[e] = make_uint2(0, 0);
+    if (t < n && d < dim) raw[e] = *reinterpret_cast<const uint2*>(src + (size_t)t * ld + d);
   }
 #pragma unroll
   for (int e = 0; e < EACH; ++e) {
-    const int i = threadIdx.x + e * THREADS, t = i / (RP / 4), d = (i % (RP / 4)) * 4;
-    float4 v;
-    if constexpr (sizeof(T) == 2) {
-      const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[e].x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[e].y));
-      v = make_float4(a.x, a.y, b.x, b.y);
-    } else {
-      v = raw[e];
-    }
-    *reinterpret_cast<float4*>(dst + t * PITCH + d) = v;
+    const int i = threadIdx.x + e * CHUNK_THREADS, t = i / (RP / 4), d = (i % (RP / 4)) * 4;
+    *reinterpret_cast<float4*>(dst + t * KP + d) = make_float4(__uint_as_float(raw[e].x << 16), __uint_as_float(raw[e].x & 0xffff0000u),
+                                                               __uint_as_float(raw[e].y << 16), __uint_as_float(raw[e].y & 0xffff0000u));
   }
 }
 
-__global__ void __launch_bounds__(THREADS, 2)
-linear_local_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const float* __restrict__ alpha, const int32_t* __restrict__ item_start,
-                    float* __restrict__ local_b, float* __restrict__ local_a, int items, int min_tokens, int H, int dim, int vdim) {
-  extern __shared__ __align__(16) float linear_smem[];
-  float *kr = linear_smem, *vs = kr + CHUNK * KP, *whole = vs + CHUNK * KP;  // [64][KP] each, [RUNS][RP]
-  pdl_trigger();
-  pdl_wait();
-  int t0, n;
-  if (!portions::find_chunk<CHUNK>(item_start, items, min_tokens, blockIdx.y, t0, n)) return;
-  const int h = blockIdx.x;
-  bring<__nv_bfloat16, KP>(kr, proj + (size_t)t0 * ld + (size_t)H * dim + (size_t)h * dim, ld, n, dim);
-  bring<__nv_bfloat16, KP>(vs, proj + (size_t)t0 * ld + 2 * (size_t)H * dim + (size_t)h * vdim, ld, n, vdim);
-  const int d = threadIdx.x & (RP - 1), at = threadIdx.x / RP;
-  float a[RUN];  // this thread's channel over a quarter of the tokens
-#pragma unroll
-  for (int i = 0; i < RUN; ++i) {
-    const int t = at * RUN + i;
-    a[i] = t < n && d < dim ? alpha[((size_t)(t0 + t) * H + h) * dim + d] : 1.f;
-  }
-  Product all;
-#pragma unroll
-  for (int i = 0; i < RUN; ++i) all.times(a[i]);
-  whole[at * RP + d] = all.value();
-  __syncthreads();
-  Product run;
-  for (int r = RUNS - 1; r > at; --r) run.times(whole[r * RP + d]);
-#pragma unroll
-  for (int i = RUN - 1; i >= 0; --i) {
-    kr[(at * RUN + i) * KP + d] *= run.value();
-    run.times(a[i]);
-  }
-  if (at == 0 && d < dim) local_a[((size_t)blockIdx.y * H + h) * dim + d] = run.value();
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, tg = lane & 3;
-  const int d0 = 16 * (warp & 7) + gr;
-  float* dst = local_b + ((size_t)blockIdx.y * H + h) * dim * vdim;
-#pragma unroll 1
-  for (int pass = 0; pass < 4; ++pass) {  // 16 rows and 16 columns a warp
-    const int c0 = (warp >> 3) * 64 + pass * 16;
-    if (c0 >= vdim || 16 * (warp & 7) >= dim) break;
-    Sum y[2];
-#pragma unroll
-    for (int k = 0; k < CHUNK / 8; ++k) {
-      uint32_t ah[4], al[4];
-      load_rows(kr + (8 * k + tg) * KP + d0, 8, 4 * KP, ah, al);
-      const float* b = vs + (8 * k + tg) * KP + c0 + gr;
-#pragma unroll
-      for (int m = 0; m < 2; ++m) y[m].step<false>(ah, al, b[8 * m], b[4 * KP + 8 * m]);
-    }
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const int col = c0 + 8 * m + 2 * tg;
-        if (d0 + 8 * r < dim && col < vdim) *reinterpret_cast<float2*>(dst + (size_t)(d0 + 8 * r) * vdim + col) = make_float2(y[m].total(2 * r), y[m].total(2 * r + 1));
-      }
-  }
-}
-
-// A thread per four numbers of a portion's state: B of every chunk becomes the state the chunk starts from, the slot gets the last one.
-__global__ void __launch_bounds__(128)
-linear_starts_kernel(float* __restrict__ state, long long slot_floats, const int32_t* __restrict__ item_start,
-                     const int32_t* __restrict__ slots, float* __restrict__ local_b, const float* __restrict__ local_a, int chunks,
-                     int min_tokens, int H, int dim, int vdim, int num_slots) {
-  pdl_trigger();
-  pdl_wait();
-  const int item = blockIdx.y, tokens = item_start[item + 1] - item_start[item];
-  if (tokens < min_tokens) return;
-  int first = 0;
-  for (int i = 0; i < item; ++i) {
-    const int ni = item_start[i + 1] - item_start[i];
-    if (ni >= min_tokens) first += (ni + CHUNK - 1) / CHUNK;
-  }
-  const int n = (tokens + CHUNK - 1) / CHUNK;
-  if (first + n > chunks) return;  // (the caller counted fewer than there are: no room for them)
-  const long long per_chunk = (long long)H * dim * vdim, at = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-  if (at >= per_chunk) return;
-  int slot = slots[item];
-  slot = slot < 0 ? 0 : (slot >= num_slots ? num_slots - 1 : slot);
-  float4 run = *reinterpret_cast<const float4*>(state + (size_t)slot * slot_floats + at);
-  const long long hd = at / vdim;
-  constexpr int AHEAD = 8;
-  for (int c0 = 0; c0 < n; c0 += AHEAD) {
-    float4 b[AHEAD];
-    float a[AHEAD];
-#pragma unroll
-    for (int j = 0; j < AHEAD; ++j) {  // asked for together
-      const int c = min(c0 + j, n - 1);
-      b[j] = *reinterpret_cast<const float4*>(local_b + (size_t)(first + c) * per_chunk + at);
-      a[j] = local_a[(size_t)(first + c) * H * dim + hd];
-    }
-#pragma unroll
-    for (int j = 0; j < AHEAD; ++j) {
-      if (c0 + j >= n) break;
-      *reinterpret_cast<float4*>(local_b + (size_t)(first + c0 + j) * per_chunk + at) = run;
-      run.x = fmaf(a[j], run.x, b[j].x);
-      run.y = fmaf(a[j], run.y, b[j].y);
-      run.z = fmaf(a[j], run.z, b[j].z);
-      run.w = fmaf(a[j], run.w, b[j].w);
-    }
-  }
-  *reinterpret_cast<float4*>(state + (size_t)slot * slot_floats + at) = run;
-}
-
-struct ReadShape {
-  static constexpr int Q_AT = 0, K_AT = Q_AT + CHUNK * KP, V_AT = K_AT + CHUNK * KP, S_AT = V_AT + CHUNK * VP;
-  static constexpr int P_AT = S_AT + RP * VP, W_AT = P_AT + CHUNK * PP;      // W: decays of whole runs
-  static constexpr int F_AT = W_AT + RUNS * RP, FLOATS = F_AT + 7 * RP;      // F: products of those
+struct ChunkShape {
+  static constexpr int Q = CHUNK * KP, G = 2 * CHUNK * KP, PS = 3 * CHUNK * KP, FLOATS = PS + CHUNK * TP;
 };
 
-__global__ void __launch_bounds__(THREADS, 1)
-linear_read_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const float* __restrict__ alpha, const int32_t* __restrict__ item_start,
-                   const float* __restrict__ starts, float* __restrict__ o, int items, int min_tokens, int H, int dim, int vdim, float scale) {
-  using Sh = ReadShape;
-  extern __shared__ __align__(16) float linear_smem[];
-  float *qs = linear_smem + Sh::Q_AT, *ks = linear_smem + Sh::K_AT, *vs = linear_smem + Sh::V_AT, *ss = linear_smem + Sh::S_AT;
-  float *ps = linear_smem + Sh::P_AT, *whole = linear_smem + Sh::W_AT, *fs = linear_smem + Sh::F_AT;
-  float* as = ss;  // the decays, [64][KP], until the state takes their place
-  pdl_trigger();
+__global__ void __launch_bounds__(CHUNK_THREADS, 3)
+linear_chunk_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const float* __restrict__ alpha, const int32_t* __restrict__ item_start,
+                    float* __restrict__ records, int items, int min_tokens, int H, int dim, int vdim) {
+  using Sh = ChunkShape;
+  extern __shared__ __align__(16) float chunk_smem[];
+  float *ks = chunk_smem, *qs = chunk_smem + Sh::Q, *gs = chunk_smem + Sh::G;
+  float(*ps)[TP] = reinterpret_cast<float(*)[TP]>(chunk_smem + Sh::PS);
   pdl_wait();
   int t0, n;
   if (!portions::find_chunk<CHUNK>(item_start, items, min_tokens, blockIdx.y, t0, n)) return;
   const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, tg = lane & 3;
+  float* out = records + ((size_t)blockIdx.y * H + h) * record_floats(vdim);
   const __nv_bfloat16* rows = proj + (size_t)t0 * ld;
-  bring<__nv_bfloat16, KP>(qs, rows + (size_t)h * dim, ld, n, dim);
-  bring<__nv_bfloat16, KP>(ks, rows + (size_t)H * dim + (size_t)h * dim, ld, n, dim);
-  bring<__nv_bfloat16, VP>(vs, rows + 2 * (size_t)H * dim + (size_t)h * vdim, ld, n, vdim);
-  bring<float, KP>(as, alpha + ((size_t)t0 * H + h) * dim, (long long)H * dim, n, dim);  // (channels and tokens that are not there: q and k are 0)
-  for (int i = threadIdx.x; i < CHUNK * PP; i += THREADS) ps[i] = 0.f;
+  bring_rows(gs, alpha + ((size_t)t0 * H + h) * dim, (long long)H * dim, n, dim, true);  // (0 where there is none: q and k are 0 too)
+  widen_rows(qs, rows + (size_t)h * dim, ld, n, dim);
+  widen_rows(ks, rows + (size_t)(H + h) * dim, ld, n, dim);
+  delta::copy_async_wait();
   __syncthreads();
-  // P on the diagonal: columns j0 .. j0 + 3 of a run, the lane's four channels, down the run's rows
-  static_assert(THREADS / 32 == RUNS * RUN / 4, "a warp per four columns");
+  products_on_diagonal<false, false>(ks, qs, gs, nullptr, ps, warp, lane);
+  // the values, columns first: nobody else waits for them
+  const uint16_t* values = reinterpret_cast<const uint16_t*>(rows + 2 * (size_t)H * dim + (size_t)h * vdim);
+#pragma unroll 2
+  for (int i = threadIdx.x; i < (vdim + 15) / 16 * 2 * 32; i += CHUNK_THREADS) {
+    const int col0 = (i >> 6) * 16, k = (i >> 5) & 1;  // (i & 31 is the lane)
+    uint32_t w[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int col = col0 + gr + 8 * (r & 1), t = 16 * k + 8 * (r >> 1) + 2 * tg;
+      const uint32_t a = t < n && col < vdim ? values[(size_t)t * ld + col] : 0, b = t + 1 < n && col < vdim ? values[(size_t)(t + 1) * ld + col] : 0;
+      w[r] = a | b << 16;
+    }
+    *reinterpret_cast<uint4*>(out + V_AT + (i >> 5) * TERM + 4 * lane) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  __syncthreads();
+  // a channel a thread: the running products
+  const int d = threadIdx.x;
+  float qc[CHUNK];  // Q c
   {
-    const int j0 = ((warp + (warp >> 2)) & 3) * 4, base = (warp >> 2) * RUN;
-    Product run[4][4];  // with what the roundings lose: up to fifteen decays a product
+    Product c, front, tail, upto;
+    float f[CHUNK];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float4 row = *reinterpret_cast<const float4*>(ks + (base + j0 + j) * KP + 4 * lane);
-      run[j][0].hi = row.x;
-      run[j][1].hi = row.y;
-      run[j][2].hi = row.z;
-      run[j][3].hi = row.w;
-    }
-#pragma unroll 2
-    for (int i = j0; i < RUN; ++i) {
-      const float4 q = *reinterpret_cast<const float4*>(qs + (base + i) * KP + 4 * lane), a = *reinterpret_cast<const float4*>(as + (base + i) * KP + 4 * lane);
-      float v[4];
+    for (int i = 0; i < CHUNK; ++i) f[i] = i < n && d < dim ? gs[i * KP + d] : 1.f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (i > j0 + j) {
-          run[j][0].times(a.x);
-          run[j][1].times(a.y);
-          run[j][2].times(a.z);
-          run[j][3].times(a.w);
-        }
-        v[j] = fmaf(q.x, run[j][0].value(), q.y * run[j][1].value()) + fmaf(q.z, run[j][2].value(), q.w * run[j][3].value());
+    for (int i = 0; i < CHUNK; ++i) {
+      const float q = qs[i * KP + d];
+      c.times(f[i]);
+      qc[i] = q * c.value();
+      if (i >= HALF) {
+        front.times(f[i]);
+        qs[i * KP + d] = q * front.value();
       }
-      // the four sums over the warp: lane's bits 3 and 4 choose which of them it ends up with
-      const bool up4 = lane & 16, up3 = lane & 8;
-      const float x0 = (up4 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, up4 ? v[0] : v[2], 16);
-      const float x1 = (up4 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, up4 ? v[1] : v[3], 16);
-      float y = (up3 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, up3 ? x0 : x1, 8);
-      y += __shfl_xor_sync(0xffffffffu, y, 4);
-      y += __shfl_xor_sync(0xffffffffu, y, 2);
-      y += __shfl_xor_sync(0xffffffffu, y, 1);
-      const int j = j0 + (up4 ? 2 : 0) + (up3 ? 1 : 0);
-      if ((lane & 7) == 0 && j <= i) ps[(base + i) * PP + base + j] = y;
+    }
+    out[G_AT + d] = c.value();
+#pragma unroll
+    for (int i = CHUNK - 1; i >= 0; --i) {
+      const float k = ks[i * KP + d];
+      if (i < HALF) {
+        gs[i * KP + d] = k * upto.value();  // to the end of the first half
+        upto.times(f[i]);
+      }
+      ks[i * KP + d] = k * tail.value();
+      tail.times(f[i]);
     }
   }
   __syncthreads();
-  {  // queries times the decays from their run's start, keys times those to their run's end
-    const int d = threadIdx.x & (RP - 1), base = threadIdx.x / RP * RUN;
-    float a[RUN];
-#pragma unroll
-    for (int i = 0; i < RUN; ++i) a[i] = base + i < n && d < dim ? as[(base + i) * KP + d] : 1.f;
-    Product front, behind;
-#pragma unroll
-    for (int i = 0; i < RUN; ++i) {
-      front.times(a[i]);
-      qs[(base + i) * KP + d] *= front.value();
-    }
-    whole[(base / RUN) * RP + d] = front.value();
-#pragma unroll
-    for (int i = RUN - 1; i >= 0; --i) {
-      ks[(base + i) * KP + d] *= behind.value();
-      behind.times(a[i]);
-    }
-  }
+  products_behind<false>(qs + HALF * KP, gs, nullptr, ps);
   __syncthreads();
-  {  // the state the chunk starts from, in the decays' place
-    const float* S = starts + ((size_t)blockIdx.y * H + h) * dim * vdim;
-    for (int i = threadIdx.x; i < RP * RP / 4; i += THREADS) {
-      const int d = i / (RP / 4), c = (i % (RP / 4)) * 4;
-      const bool there = d < dim && c < vdim;
-      const float* src = S + (there ? (size_t)d * vdim + c : 0);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(ss + d * VP + c)), "l"(src), "r"(there ? 16 : 0) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
-  if (threadIdx.x < RP) {
-    const int d = threadIdx.x;
-    const float w0 = whole[d], w1 = whole[RP + d], w2 = whole[2 * RP + d];
-    fs[d] = 1.f;                        // 0 .. 3: in front of run 0, 1, 2, 3
-    fs[RP + d] = w0;
-    fs[2 * RP + d] = w0 * w1;
-    fs[3 * RP + d] = w0 * w1 * w2;
-    fs[4 * RP + d] = w1;                // between runs 0 and 2
-    fs[5 * RP + d] = w2;                // ... 1 and 3
-    fs[6 * RP + d] = w1 * w2;           // ... 0 and 3
-  }
+#pragma unroll
+  for (int i = 0; i < CHUNK; ++i) qs[i * KP + d] = qc[i];
   __syncthreads();
-  // a fragment of the queries of run m times a vector of F
-  auto queries = [&](int m, const float* f, int k, uint32_t (&ah)[4], uint32_t (&al)[4]) {
-    load_row_pairs(qs + (m * RUN + gr) * KP + 8 * k + 2 * tg, 8 * KP, *reinterpret_cast<const float2*>(f + 8 * k + 2 * tg), ah, al);
+  auto one = [](int) { return 1.f; };
+  put_rows(qs, out + Q_AT, 2, threadIdx.x, CHUNK_THREADS, one);
+  put_keys(ks, out + K_AT, threadIdx.x, CHUNK_THREADS, one);
+  put_b(ps, out + P_AT, threadIdx.x, CHUNK_THREADS);
+  pdl_trigger();  // at the end: the chain's blocks are few and long
+}
+
+constexpr int PP = CHUNK + 8;  // of the shares: columns first
+template <int TILES>
+struct Chain {
+  static constexpr int COLS = 16 * TILES, SHARES = WORKERS / 32, FLOATS = 2 * SHARES * COLS * PP;  // of two chunks
+  static_assert(FLOATS * 4 <= 227 * 1024, "beyond a block's shared memory");
+};
+// One step of sixteen terms of N sums whose left operand is bfloat16 as it is (see step).
+template <int N>
+__device__ __forceinline__ void step_whole(float (&sum)[N][4], float (&small)[N][4], const uint32_t (&a)[4], const Right (&b)[N]) {
+  const float zero[4] = {};
+  float d[N][4];
+#pragma unroll
+  for (int n = 0; n < N; ++n) mma_bf16(small[n], a, b[n].v[2][0], b[n].v[2][1], small[n]);
+#pragma unroll
+  for (int n = 0; n < N; ++n) mma_bf16(d[n], a, b[n].v[0][0], b[n].v[0][1], zero);
+#pragma unroll
+  for (int n = 0; n < N; ++n) mma_bf16(small[n], a, b[n].v[1][0], b[n].v[1][1], small[n]);
+#pragma unroll
+  for (int n = 0; n < N; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sum[n][e] += d[n][e];
+}
+
+template <int TILES>
+__global__ void __launch_bounds__(CHAIN_THREADS, 1)
+linear_chain_kernel(const float* __restrict__ records, float* __restrict__ state, long long slot_floats, const int32_t* __restrict__ item_start,
+                    const int32_t* __restrict__ slots, float* __restrict__ o, int items, int all_chunks, int min_tokens, int H, int dim, int vdim,
+                    int num_slots, float scale) {
+  using Sh = Chain<TILES>;
+  constexpr int COLS = Sh::COLS, SHARES = Sh::SHARES;
+  extern __shared__ __align__(16) float chain[];  // [2][SHARES][COLS][PP]
+  const int h = blockIdx.y, col0 = blockIdx.x * COLS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, tg = lane & 3;
+  pdl_wait();
+  int item, first;
+  if (!portions::find_portion<CHUNK>(item_start, items, min_tokens, blockIdx.z, item, first)) return;
+  const int t0 = item_start[item], t1 = item_start[item + 1];
+  const int chunks = (t1 - t0 + CHUNK - 1) / CHUNK;
+  if (first + chunks > all_chunks) return;  // (the caller counted fewer than there are: no records for them)
+  int slot = slots[item];
+  slot = slot < 0 ? 0 : (slot >= num_slots ? num_slots - 1 : slot);
+  float* S = state + (size_t)slot * slot_floats + (size_t)h * dim * vdim;
+  const size_t size = record_floats(vdim), stride = (size_t)H * size;
+  const float* r = records + ((size_t)first * H + h) * size;
+  auto fetch4 = [&](const float* at) {  // (volatile: where it is asked for, not where it is used)
+    uint4 v;
+    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(at + 4 * lane));
+    return v;
   };
-  if (warp < 12) {  // P off the diagonal: runs (1,0) (2,0) (2,1) (3,0) (3,1) (3,2), eight columns a warp
-    const int pair = warp >> 1, m = pair < 1 ? 1 : pair < 3 ? 2 : 3, j = pair - m * (m - 1) / 2, c0 = 8 * (warp & 1);
-    const float* f = fs + (m - j == 1 ? 0 : m - j == 3 ? 6 : m == 2 ? 4 : 5) * RP;
-    Sums<2> y;
-#pragma unroll 4
-    for (int k = 0; k < RP / 8; ++k) {
-      uint32_t ah[4], al[4];
-      queries(m, f, k, ah, al);
-      const float2 b = *reinterpret_cast<const float2*>(ks + (j * RUN + c0 + gr) * KP + 8 * k + 2 * tg);
-      y.step<6>(ah, al, split(b.x), split(b.y), k & 1);
-    }
+  auto unit = [&](const float* at, uint4 (&to)[3]) {
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
-      *reinterpret_cast<float2*>(ps + (m * RUN + gr + 8 * r) * PP + j * RUN + c0 + 2 * tg) = make_float2(y.total(2 * r), y.total(2 * r + 1));
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();
-  // O: the 16 rows of run m, 32 columns a warp (the runs in turn, so that no scheduler gets all the long ones)
-  const int m = (warp + (warp >> 2)) & 3, c0 = (warp >> 2) * 32;
-  if (m * RUN >= n || c0 >= vdim) return;
-  Sums<2> y[4];
-#pragma unroll 4
-  for (int k = 0; k < RP / 8; ++k) {
-    uint32_t ah[4], al[4];
-    queries(m, fs + m * RP, k, ah, al);
-    const float* b = ss + (8 * k + 2 * tg) * VP + c0 + gr;
+    for (int p = 0; p < 3; ++p) to[p] = fetch4(at + p * TERM);
+  };
+  uint4 vt[TILES][2];  // V of the chunk: columns gr and gr + 8 of every 16
+  auto fetch_values = [&] {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) y[c].step<4>(ah, al, split(b[8 * c]), split(b[VP + 8 * c]), k & 1);
-  }
-#pragma unroll 2
-  for (int k = 0; k < 2 * (m + 1); ++k) {
-    uint32_t ah[4], al[4];
-    load_row_pairs(ps + (m * RUN + gr) * PP + 8 * k + 2 * tg, 8 * PP, make_float2(1.f, 1.f), ah, al);
-    const float* b = vs + (8 * k + 2 * tg) * VP + c0 + gr;
+    for (int tile = 0; tile < TILES; ++tile)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) y[c].step<true>(ah, al, b[8 * c], b[VP + 8 * c], k & 1);
-  }
+      for (int k = 0; k < 2; ++k)
+        vt[tile][k] = col0 + 16 * tile < vdim ? fetch4(r + V_AT + ((size_t)(col0 / 16 + tile) * 2 + k) * TERM) : make_uint4(0, 0, 0, 0);
+  };
+
+  if (threadIdx.x < WORKERS) {
+    uint4 qc[2][3], kr[2][3];
+    float2 g[2];
+    auto fetch_queries = [&] {
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const int i = m * RUN + gr + 8 * r;
-    if (i >= n) continue;
+      for (int p = 0; p < 2; ++p) unit(r + Q_AT + (warp * 2 + p) * UNIT, qc[p]);
+    };
+    auto fetch_keys = [&] {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int col = c0 + 8 * c + 2 * tg;
-      if (col >= vdim) continue;
-      float v[2] = {y[c].total(2 * r), y[c].total(2 * r + 1)};
-      if (!is_finite(v[0]) || !is_finite(v[1])) {
-        float again[2] = {0.f, 0.f};
-#pragma unroll 1
-        for (int d = 0; d < dim; ++d) {
-          const float q = qs[i * KP + d] * fs[m * RP + d];
-          again[0] = fmaf(q, ss[d * VP + col], again[0]);
-          again[1] = fmaf(q, ss[d * VP + col + 1], again[1]);
-        }
-#pragma unroll 1
-        for (int j = 0; j <= i; ++j) {
-          again[0] = fmaf(ps[i * PP + j], vs[j * VP + col], again[0]);
-          again[1] = fmaf(ps[i * PP + j], vs[j * VP + col + 1], again[1]);
-        }
-        if (!is_finite(v[0])) v[0] = again[0];
-        if (!is_finite(v[1])) v[1] = again[1];
+      for (int m = 0; m < 2; ++m) {
+        unit(r + K_AT + (warp * 2 + m) * UNIT, kr[m]);
+        g[m] = __ldg(reinterpret_cast<const float2*>(r + G_AT + 16 * warp + 8 * m + 2 * tg));
       }
-      *reinterpret_cast<float2*>(o + ((size_t)(t0 + i) * H + h) * vdim + col) = make_float2(v[0] * scale, v[1] * scale);
+    };
+    fetch_queries();
+    fetch_keys();
+    fetch_values();
+    // S, columns first: columns gr and gr + 8 of every 16, channels 16 warp + 8 m + 2 tg and + 1
+    float s[TILES][2][4];
+    auto at = [&](int tile, int m, int e) -> float* {
+      const int d = 16 * warp + 8 * m + 2 * tg + (e & 1), col = col0 + 16 * tile + gr + 8 * (e >> 1);
+      return d < dim && col < vdim ? S + (size_t)d * vdim + col : nullptr;
+    };
+#pragma unroll
+    for (int tile = 0; tile < TILES; ++tile)
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float* p = at(tile, m, e);
+          s[tile][m][e] = p ? *p : 0.f;
+        }
+    for (int c = 0; c < chunks; ++c) {
+      float* parts = chain + (c & 1) * SHARES * COLS * PP;
+      {  // this warp's share of Q c S
+        Right b[4];
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+          for (int p = 0; p < 3; ++p) {
+            const uint4 v = qc[n >> 1][p];
+            b[n].v[p][0] = n & 1 ? v.z : v.x;
+            b[n].v[p][1] = n & 1 ? v.w : v.y;
+          }
+#pragma unroll
+        for (int tile = 0; tile < TILES; ++tile) {
+          Left a;  // the state's sums lie as a left operand
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a.put(e, split3(s[tile][e >> 1][2 * (e & 1)], s[tile][e >> 1][2 * (e & 1) + 1]));
+          float sum[4][4] = {}, small[4][4] = {};
+          step<4>(sum, small, a, b);
+#pragma unroll
+          for (int n = 0; n < 4; ++n) {
+            float* to = parts + (warp * COLS + 16 * tile + gr) * PP + 8 * n + 2 * tg;
+            *reinterpret_cast<float2*>(to) = make_float2(sum[n][0] + small[n][0], sum[n][1] + small[n][1]);
+            *reinterpret_cast<float2*>(to + 8 * PP) = make_float2(sum[n][2] + small[n][2], sum[n][3] + small[n][3]);
+          }
+        }
+      }
+      const float* next = r + stride;
+      if (c + 1 < chunks) {
+        r = next;
+        fetch_queries();
+      }
+      __syncthreads();  // (the shares of the chunk before last have been added up)
+#pragma unroll
+      for (int tile = 0; tile < TILES; ++tile) {
+        float sum[2][2][4] = {}, small[2][2][4] = {};  // of either half of the tokens
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const uint32_t a[4] = {vt[tile][k].x, vt[tile][k].y, vt[tile][k].z, vt[tile][k].w};
+          Right b[2];
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+              b[m].v[p][0] = k ? kr[m][p].z : kr[m][p].x;
+              b[m].v[p][1] = k ? kr[m][p].w : kr[m][p].y;
+            }
+          step_whole<2>(sum[k], small[k], a, b);
+        }
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            s[tile][m][e] = fmaf(e & 1 ? g[m].y : g[m].x, s[tile][m][e], (sum[0][m][e] + sum[1][m][e]) + (small[0][m][e] + small[1][m][e]));
+      }
+      if (c + 1 < chunks) {
+        fetch_keys();
+        fetch_values();
+      }
     }
+    pdl_trigger();  // at the end, as in linear_chunk_kernel
+#pragma unroll
+    for (int tile = 0; tile < TILES; ++tile)
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (float* p = at(tile, m, e)) *p = s[tile][m][e];
+  } else {
+    const int eight = warp - WORKERS / 32;  // tokens 8 eight .. + 7 of every chunk
+    uint4 b[3];
+    unit(r + P_AT + eight * UNIT, b);
+    fetch_values();
+    for (int c = 0; c < chunks; ++c) {
+      const float* parts = chain + (c & 1) * SHARES * COLS * PP;
+      float of_values[TILES][4];  // P V: columns gr and gr + 8, tokens 2 tg and 2 tg + 1
+#pragma unroll
+      for (int tile = 0; tile < TILES; ++tile) {
+        float sum[2][1][4] = {}, small[2][1][4] = {};
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          if (k && eight < 2) break;  // P is triangular
+          const uint32_t a[4] = {vt[tile][k].x, vt[tile][k].y, vt[tile][k].z, vt[tile][k].w};
+          Right x[1];
+#pragma unroll
+          for (int p = 0; p < 3; ++p) {
+            x[0].v[p][0] = k ? b[p].z : b[p].x;
+            x[0].v[p][1] = k ? b[p].w : b[p].y;
+          }
+          step_whole<1>(sum[k], small[k], a, x);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) of_values[tile][e] = (sum[0][0][e] + sum[1][0][e]) + (small[0][0][e] + small[1][0][e]);
+      }
+      const uint32_t* record = reinterpret_cast<const uint32_t*>(r);
+      if (c + 1 < chunks) {
+        r += stride;
+        unit(r + P_AT + eight * UNIT, b);
+        fetch_values();
+      }
+      __syncthreads();
+#pragma unroll
+      for (int tile = 0; tile < TILES; ++tile)
+#pragma unroll
+        for (int e2 = 0; e2 < 2; ++e2) {
+          const int in = gr + 8 * e2, col = col0 + 16 * tile + in;
+          float2 v[SHARES];
+#pragma unroll
+          for (int q = 0; q < SHARES; ++q) v[q] = *reinterpret_cast<const float2*>(parts + (q * COLS + 16 * tile + in) * PP + 8 * eight + 2 * tg);
+#pragma unroll
+          for (int m = SHARES / 2; m > 0; m >>= 1)
+#pragma unroll
+            for (int q = 0; q < m; ++q) v[q].x += v[q + m].x, v[q].y += v[q + m].y;
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int i = 8 * eight + 2 * tg + e, t = t0 + c * CHUNK + i;
+            const float of_state = e ? v[0].y : v[0].x;
+            float y = of_state + of_values[tile][2 * e2 + e];
+            if (!is_finite(y) && col < vdim) {
+              float again = 0.f;
+#pragma unroll 1
+              for (int j = 0; j <= i; ++j) {
+                const int q = (j & 7) >> 1, k = j >> 4, h8 = (j >> 3) & 1;
+                float x = 0.f;
+                for (int p = 2; p >= 0; --p) x += term(record[P_AT + eight * UNIT + p * TERM + ((i & 7) * 4 + q) * 4 + 2 * k + h8], j & 1);
+                again = fmaf(x, term(record[V_AT + ((size_t)(col0 / 16 + tile) * 2 + k) * TERM + ((in & 7) * 4 + q) * 4 + (in >> 3) + 2 * h8], j & 1), again);
+              }
+              y = of_state + again;
+            }
+            if (t < t1 && col < vdim) o[((size_t)t * H + h) * vdim + col] = y * scale;
+          }
+        }
+    }
+    pdl_trigger();
   }
+}
+
+template <int TILES>
+int launch_chain(const float* records, float* state, long long slot_floats, const int32_t* item_start, const int32_t* slots, float* o, int items, int portions,
+                 int chunks, int min_tokens, int H, int dim, int vdim, int num_slots, float scale, cudaStream_t stream) {
+  constexpr int bytes = Chain<TILES>::FLOATS * (int)sizeof(float), COLS = Chain<TILES>::COLS;
+  static PsbPerDevice configured;
+  if (!configured.get()) {
+    if (cudaFuncSetAttribute(linear_chain_kernel<TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) PSB_REFUSE("linear_chunks: cannot raise the shared-memory limit");
+    configured.set();
+  }
+  psb_launch(linear_chain_kernel<TILES>, dim3((vdim + COLS - 1) / COLS, H, portions), dim3(CHAIN_THREADS), (size_t)bytes, stream, records, state, slot_floats,
+             item_start, slots, o, items, chunks, min_tokens, H, dim, vdim, num_slots, scale);
+  PSB_LAUNCH_CHECK("linear_chain");
+  return 0;
 }
 
 }  // namespace
 
-// (dim, vdim) -> 1 if these kernels take the sizes
-PSB_API int psb_linear_chunks_supported(int dim, int vdim) { return dim >= 4 && dim <= RP && dim % 4 == 0 && vdim >= 4 && vdim <= RP && vdim % 4 == 0 ? 1 : 0; }
+// (dim, vdim) -> float32 numbers of a chunk's record of a head, 0 if these kernels do not take the sizes
+PSB_API int psb_linear_chunk_record(int dim, int vdim) { return dim >= 4 && dim <= RP && dim % 4 == 0 && vdim >= 4 && vdim <= RP && vdim % 4 == 0 ? record_floats(vdim) : 0; }
 
 // () -> tokens of a chunk
 PSB_API int psb_linear_chunk_tokens() { return CHUNK; }
 
-// Every portion of at least ``min_tokens`` tokens, and its slot; other tokens and slots are left untouched.  local_b [chunks, H, dim,
-// vdim] and local_a [chunks, H, dim] float32 are scratch, chunks at least the number of these portions' chunks.
-// (proj bfloat16, ld, alpha, state, slot_floats, item_start, slots, local_b, local_a, o, items, chunks, min_tokens, H, dim, vdim, num_slots,
+// Every portion of at least ``min_tokens`` tokens, and its slot; other tokens and slots are left untouched.  records [chunks, H,
+// psb_linear_chunk_record] float32 is scratch, portions and chunks at least the number of these portions and of their chunks.
+// (proj bfloat16, ld, alpha, state, slot_floats, item_start, slots, records, o, items, portions, chunks, min_tokens, H, dim, vdim, num_slots,
 //  scale, stream)
 PSB_API int psb_linear_chunks(const void* proj, long long ld, const void* alpha, void* state, long long slot_floats,
-                              const void* item_start, const void* slots, void* local_b, void* local_a, void* o, int items, int chunks,
+                              const void* item_start, const void* slots, void* records, void* o, int items, int portions, int chunks,
                               int min_tokens, int H, int dim, int vdim, int num_slots, float scale, cudaStream_t stream) {
-  if (items < 0 || H < 1 || num_slots < 1 || min_tokens < 1 || !psb_linear_chunks_supported(dim, vdim)) PSB_REFUSE("linear_chunks: bad sizes H=%d dim=%d vdim=%d", H, dim, vdim);
+  if (items < 0 || H < 1 || num_slots < 1 || min_tokens < 1 || !psb_linear_chunk_record(dim, vdim)) PSB_REFUSE("linear_chunks: bad sizes H=%d dim=%d vdim=%d", H, dim, vdim);
   if (ld < 2LL * H * dim + (long long)H * vdim || ld % 4) PSB_REFUSE("linear_chunks: row stride %lld is shorter than the row or no multiple of 4", ld);
-  if (slot_floats < (long long)H * dim * vdim || slot_floats % 4) PSB_REFUSE("linear_chunks: a slot of %lld numbers does not hold the state, or is no multiple of 4", slot_floats);
-  if (((uintptr_t)proj & 7) || (((uintptr_t)alpha | (uintptr_t)state | (uintptr_t)local_b | (uintptr_t)o) & 15))
-    PSB_REFUSE("linear_chunks: operands are not aligned");
-  if (H > 65535 || chunks > 65535 || items > 65535) PSB_REFUSE("linear_chunks: too many heads, requests or chunks for one launch");
-  if (items == 0 || chunks < 1) return 0;
-  constexpr int local_bytes = (2 * CHUNK * KP + RUNS * RP) * (int)sizeof(float), read_bytes = ReadShape::FLOATS * (int)sizeof(float);
+  if (slot_floats < (long long)H * dim * vdim) PSB_REFUSE("linear_chunks: a slot of %lld numbers does not hold the state", slot_floats);
+  if (((uintptr_t)proj & 7) || (((uintptr_t)alpha | (uintptr_t)records) & 15)) PSB_REFUSE("linear_chunks: operands are not aligned");
+  if (H > 65535 || chunks > 65535 || portions > 65535) PSB_REFUSE("linear_chunks: too many heads, requests or chunks for one launch");
+  if (items == 0 || portions < 1 || chunks < 1) return 0;
+  constexpr int bytes = ChunkShape::FLOATS * (int)sizeof(float);
   static PsbPerDevice configured;
   if (!configured.get()) {
-    if (cudaFuncSetAttribute(linear_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, local_bytes) != cudaSuccess ||
-        cudaFuncSetAttribute(linear_read_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, read_bytes) != cudaSuccess)
-      PSB_REFUSE("linear_chunks: cannot raise the shared-memory limit");
+    if (cudaFuncSetAttribute(linear_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) PSB_REFUSE("linear_chunks: cannot raise the shared-memory limit");
     configured.set();
   }
-  psb_launch(linear_local_kernel, dim3(H, chunks), dim3(THREADS), (size_t)local_bytes, stream, (const __nv_bfloat16*)proj, ld, (const float*)alpha,
-             (const int32_t*)item_start, (float*)local_b, (float*)local_a, items, min_tokens, H, dim, vdim);
-  PSB_LAUNCH_CHECK("linear_local");
-  const long long fours = (long long)H * dim * vdim / 4;
-  psb_launch(linear_starts_kernel, dim3((unsigned)((fours + 127) / 128), items), dim3(128), 0, stream, (float*)state, slot_floats,
-             (const int32_t*)item_start, (const int32_t*)slots, (float*)local_b, (const float*)local_a, chunks, min_tokens, H, dim, vdim,
-             num_slots);
-  PSB_LAUNCH_CHECK("linear_starts");
-  psb_launch(linear_read_kernel, dim3(H, chunks), dim3(THREADS), (size_t)read_bytes, stream, (const __nv_bfloat16*)proj, ld, (const float*)alpha,
-             (const int32_t*)item_start, (const float*)local_b, (float*)o, items, min_tokens, H, dim, vdim, scale);
-  PSB_LAUNCH_CHECK("linear_read");
-  return 0;
+  psb_launch(linear_chunk_kernel, dim3(H, chunks), dim3(CHUNK_THREADS), (size_t)bytes, stream, (const __nv_bfloat16*)proj, ld, (const float*)alpha,
+             (const int32_t*)item_start, (float*)records, items, min_tokens, H, dim, vdim);
+  PSB_LAUNCH_CHECK("linear_chunk");
+  // runs of columns a block takes: as for the delta rules' chain (delta_chunks.cu)
+  const long long heads = (long long)H * portions, sms = current_sms();
+  const long long rounds16 = (heads * ((vdim + 15) / 16) + sms - 1) / sms, rounds32 = (heads * ((vdim + 31) / 32) + sms - 1) / sms;
+  auto launch = rounds32 * 31 < rounds16 * 20 ? launch_chain<2> : launch_chain<1>;
+  return launch((const float*)records, (float*)state, slot_floats, (const int32_t*)item_start, (const int32_t*)slots, (float*)o, items, portions, chunks,
+                min_tokens, H, dim, vdim, num_slots, scale, stream);
 }

@@ -1394,20 +1394,24 @@ def low_rank(a: torch.Tensor, w: torch.Tensor, function: str, *, bias: torch.Ten
     return out
 
 
-# Steps with a portion of LINEAR_CHUNKED tokens take the kernels that work 64 tokens at a time on the tensor cores, where the sizes are
-# theirs, for portions of LINEAR_SHORT tokens and more; shorter ones go token by token behind them (100 tokens 34 us against 48 one by one,
-# 8 heads of 128; and some 14 us for what stays).  In other steps a longest portion of more than two LINEAR_ATTENTION_CHUNK cuts the
+# Steps with a portion of LINEAR_CHUNKED tokens take the kernels that work 32 tokens at a time on the tensor cores, where the sizes are
+# theirs, for portions of LINEAR_SHORT tokens and more; shorter ones go token by token behind them (8 heads of 128: 32 tokens 21.5 us against 21.3 one
+# by one, 48 tokens 21.5 and 28, 128 tokens 24 and 59).  In other steps a longest portion of more than two LINEAR_ATTENTION_CHUNK cuts the
 # portions into chunks that go token by token side by side.
-LINEAR_CHUNKED, LINEAR_SHORT = 96, 32
+LINEAR_CHUNKED, LINEAR_SHORT = 48, 32
 LINEAR_ATTENTION_CHUNK = 64
+LINEAR_MIXED = 96
 
 
 def _linear_one_by_one(lengths: list[int] | None) -> bool:
     """Whether a step that could go either way whole has so much in short portions, which the two forms take one after the other, that all
-    of it is over sooner token by token (16 heads, 100 tokens beside 8 single ones 49 us in chunks and 51, beside 32 78 and 59; 8 heads,
-    100 tokens beside 20 65 and 49)."""
+    of it is over sooner token by token (16 heads, both forms and token by token: 48 tokens beside 32 single ones 48 and 39 us, 64 beside eight of
+    16 tokens 42 and 39, 64 beside one of 31 38 and 35, 64 beside a single one 28 and 34; 96 beside one of 31 40 and 47, 100 beside eight
+    single ones 34 and 51, beside 32 51 and 60)."""
     short = [n for n in lengths or [] if n < LINEAR_SHORT]
-    return bool(short) and max(lengths) <= 2 * LINEAR_ATTENTION_CHUNK and (len(short) > 16 or max(short) > 8)
+    if not short or max(lengths) > 2 * LINEAR_ATTENTION_CHUNK:
+        return False
+    return len(short) > 48 or (max(lengths) < LINEAR_MIXED and (len(short) > 8 or max(short) > 8))
 
 
 def linear_attention(proj: torch.Tensor, alpha: torch.Tensor, state: torch.Tensor, ctx, *, heads: int, dim: int, vdim: int) -> torch.Tensor:
@@ -1427,14 +1431,13 @@ def linear_attention(proj: torch.Tensor, alpha: torch.Tensor, state: torch.Tenso
     most = 0x7fffffff  # tokens of the longest portion left to the kernels that go token by token
     if (ctx.max_new_tokens >= LINEAR_CHUNKED and proj.dtype == torch.bfloat16 and ld % 4 == 0 and stride % 4 == 0
             and proj.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0 and alpha.data_ptr() % 16 == 0
-            and bool(lib().psb_linear_chunks_supported(dim, vdim)) and not _linear_one_by_one(_portion_lengths(ctx))):
+            and (record := int(lib().psb_linear_chunk_record(dim, vdim))) and not _linear_one_by_one(_portion_lengths(ctx))):
         most = LINEAR_SHORT - 1
-        chunks = _portion_tiles(ctx, t, LINEAR_SHORT, lib().psb_linear_chunk_tokens())
-        local_b = torch.empty((chunks, heads, dim, vdim), dtype=torch.float32, device=dev)
-        local_a = torch.empty((chunks, heads, dim), dtype=torch.float32, device=dev)
+        portions, chunks = _portions_from(ctx, LINEAR_SHORT), _portion_tiles(ctx, t, LINEAR_SHORT, lib().psb_linear_chunk_tokens())
+        records = torch.empty((chunks, heads, record), dtype=torch.float32, device=dev)
         check(lib().psb_linear_chunks(proj.data_ptr(), ld, alpha.data_ptr(), state.data_ptr(), stride,
-                                      _i32(ctx.item_start, "item offsets").data_ptr(), _i32(ctx.slots, "slots").data_ptr(), local_b.data_ptr(),
-                                      local_a.data_ptr(), o.data_ptr(), ctx.num_items, chunks, LINEAR_SHORT, heads, dim, vdim,
+                                      _i32(ctx.item_start, "item offsets").data_ptr(), _i32(ctx.slots, "slots").data_ptr(), records.data_ptr(),
+                                      o.data_ptr(), ctx.num_items, portions, chunks, LINEAR_SHORT, heads, dim, vdim,
                                       state.shape[0], dim ** -0.5, _stream()), "linear_attention_chunks")
         if not _has_portions_below(ctx, LINEAR_SHORT):
             return o

@@ -265,11 +265,12 @@ _SIGNATURES: dict[str, list] = {
     # (proj, dtype, ld, alpha, state, slot_floats, item_start, slots, local_b, local_a, o, items, chunks, H, dim, vdim, num_slots,
     #  chunk, max_tokens, scale, stream)
     "psb_linear_attention": [P, I, L, P, P, L, P, P, P, P, P, I, I, I, I, I, I, I, I, F, P],
-    "psb_linear_chunks_supported": [I, I],
+    # (dim, vdim) -> float32 numbers of a chunk's record of a head, 0: not built
+    "psb_linear_chunk_record": [I, I],
     "psb_linear_chunk_tokens": [],
-    # (proj, ld, alpha, state, slot_floats, item_start, slots, local_b, local_a, o, items, chunks, min_tokens, H, dim, vdim, num_slots,
+    # (proj, ld, alpha, state, slot_floats, item_start, slots, records, o, items, portions, chunks, min_tokens, H, dim, vdim, num_slots,
     #  scale, stream)
-    "psb_linear_chunks": [P, L, P, P, L, P, P, P, P, P, I, I, I, I, I, I, I, F, P],
+    "psb_linear_chunks": [P, L, P, P, L, P, P, P, P, I, I, I, I, I, I, I, I, F, P],
     # (o, gate, gate_dtype, ldg, gate_act, gain, head_gains, out, out_dtype, ldo, T, H, vdim, eps, stream)
     "psb_normed_readout": [P, P, I, L, I, P, I, P, I, L, I, I, I, F, P],
     # (h, pending, dtype, gain1, shift1, gain2, shift2, rows, x1, x2, n_rows, W, eps, update, stream)

@@ -96,6 +96,27 @@ def test_two_runs_of_columns_decay_per_head(heads, dim, vdim, lengths):
         assert (state[len(lengths) - 1 - i].double().view_as(m) - m).abs().max() < 2e-5 * m.abs().max()
 
 
+@pytest.mark.parametrize("heads, dim, vdim, lengths", [(20, 128, 64, [96, 33]), (24, 36, 44, [100, 32, 63])])
+def test_two_runs_of_columns_linear_attention(heads, dim, vdim, lengths):
+    from prefixserve_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    ctx, offsets = step(lengths)
+    t = sum(lengths)
+    proj, alpha, held = rnd(t, heads * (2 * dim + vdim)).bfloat16(), torch.sigmoid(rnd(t, heads * dim)) ** 0.25, rnd(len(lengths), heads * dim * vdim)
+    state = held.clone()
+    out = ops.linear_attention(proj, alpha, state, ctx, heads=heads, dim=dim, vdim=vdim).double()
+    p, a = proj.double(), alpha.double().view(t, heads, dim, 1)
+    q, k, v = p[:, : heads * dim].view(t, heads, dim), p[:, heads * dim: 2 * heads * dim].view(t, heads, dim), p[:, 2 * heads * dim:].view(t, heads, vdim)
+    for i, n in enumerate(lengths):
+        m = held[len(lengths) - 1 - i].double().view(heads, dim, vdim)
+        for j in range(offsets[i], offsets[i] + n):
+            m = a[j] * m + k[j, :, :, None] * v[j, :, None]
+            want = torch.einsum("hd,hdv->hv", q[j], m) * dim ** -0.5
+            assert (out[j] - want).abs().max() <= 2e-5 * max(1.0, float(want.abs().max())), j
+        assert (state[len(lengths) - 1 - i].double().view_as(m) - m).abs().max() < 2e-5 * m.abs().max()
+
+
 @pytest.mark.parametrize("short, apart", [([1] * 70, True), ([7, 3], False), ([1], False)])
 def test_short_portions_beside_long_ones(short, apart):
     """Many short portions go token by token, a few in chunks like the long ones."""

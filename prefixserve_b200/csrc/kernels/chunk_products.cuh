@@ -319,16 +319,4 @@ __device__ __forceinline__ void products_behind(const float* left, const float* 
 constexpr int WORKERS = 256, READERS = 128, CHAIN_THREADS = WORKERS + READERS;
 static_assert(WORKERS / 32 == RP / 16 && READERS / 32 == CHUNK / 8, "a worker warp per 16 channels, a reader warp per eight tokens");
 
-// SMs of the current device, asked for once a device
-inline int current_sms() {
-  static int known[PsbPerDevice::kMaxDevices] = {};
-  const int d = PsbPerDevice::current();
-  if (d >= 0 && known[d] > 0) return known[d];
-  int sms = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d < 0 ? 0 : d);
-  sms = std::max(sms, 1);
-  if (d >= 0) known[d] = sms;
-  return sms;
-}
-
 }  // namespace chunks

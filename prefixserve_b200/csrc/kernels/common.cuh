@@ -81,6 +81,18 @@ struct PsbPerDevice {
   }
 };
 
+// SMs of the current device, asked for once a device
+inline int psb_current_sms() {
+  static int known[PsbPerDevice::kMaxDevices] = {};
+  const int d = PsbPerDevice::current();
+  if (d >= 0 && known[d] > 0) return known[d];
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d < 0 ? 0 : d);
+  if (sms < 1) sms = 1;
+  if (d >= 0) known[d] = sms;
+  return sms;
+}
+
 // (x1, x2) turned by the angle whose cosine and sine are given.  Written with explicit roundings, so that every
 // kernel that rotates (the rotary kernels, the projection that rotates in its epilogue) rounds alike whatever the
 // compiler would make of the plain expression around it.

@@ -590,7 +590,7 @@ int launch_chain(const float* records, const T* proj, long long ld, float* state
 template <typename T>
 int chain_of(const void* records, const void* proj, long long ld, void* state, const void* item_start, const void* slots, void* o, int items,
              int portions, int chunks, int min_tokens, int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats, cudaStream_t stream) {
-  const long long heads = (long long)H * portions, sms = current_sms();
+  const long long heads = (long long)H * portions, sms = psb_current_sms();
   const long long rounds16 = (heads * ((vdim + 15) / 16) + sms - 1) / sms, rounds32 = (heads * ((vdim + 31) / 32) + sms - 1) / sms;
   auto launch = rounds32 * 31 < rounds16 * 20 ? launch_chain<2, T> : launch_chain<1, T>;
   return launch((const float*)records, (const T*)proj, ld, (float*)state, (const int32_t*)item_start, (const int32_t*)slots, (float*)o, items, portions, chunks,

@@ -18,7 +18,7 @@
 // What bounds it: the tensor cores' legacy path (three terms: 108 + 96 instructions a warp and tile, 1,024 multiply-adds a
 // clock and SM; busy 48 % of the time).  The kernel on the CUDA cores beside it (latent_attention_rows_kernel, still used for
 // other sizes) reads every row once for each pair of heads: 16 tokens of 32 heads over up to 3,500 keys took it 402 us a call, this
-// one and its merge 61 (54 with a chain of instructions over a block's keys).
+// one and its merge 50 (61 with the same number of blocks for every token).
 #include "common.cuh"
 
 #include <cfloat>
@@ -29,6 +29,7 @@ constexpr int RANK = 512, ROT = 64, D = RANK + ROT;
 constexpr int WARPS = 8, THREADS = 32 * WARPS;
 constexpr int QUARTERS = 4, STEPS = D / 16 / QUARTERS;   // steps of 16 numbers a group of warps takes of a row
 constexpr int PITCH = D + 8;                             // elements from row to row: an odd number of 16-byte pieces
+constexpr int KEYS = 32;                                 // of a tile
 constexpr int MAX_SPLITS = 32;
 static_assert(D % (16 * QUARTERS) == 0 && RANK == 64 * WARPS, "shares of the warps");
 
@@ -36,7 +37,7 @@ static_assert(D % (16 * QUARTERS) == 0 && RANK == 64 * WARPS, "shares of the war
 template <int HEADS>
 struct LatentShape {
   static constexpr int MG = HEADS / 16;
-  static constexpr int KT = 32, STAGES = 4;
+  static constexpr int KT = KEYS, STAGES = 4;
   static constexpr int SPT = HEADS * KT / THREADS;  // scores a thread has in the softmax
   static constexpr int S_PITCH = KT + 8, P_PITCH = KT + 8;
   static constexpr int TILE_BYTES = KT * PITCH * 2;
@@ -81,12 +82,74 @@ __device__ __forceinline__ void three_terms(float x, float y, uint32_t (&out)[3]
   }
 }
 
+// How the tokens' keys are shared out: every share is a run of at most ``per`` tiles of one token, with the smallest ``per`` for
+// which no more than ``shares`` are needed (and no more than MAX_SPLITS of a token).  Every warp finds it from the positions, so
+// that a captured step of other lengths is shared out anew.  With the same number of shares for every token, the blocks of the
+// shorter ones were done early: 16 tokens of 3,500 keys down to half, 55 us -> 45.  That is for a single round of blocks: the
+// search costs a block 0.7 us with 16 tokens and 1.5 with 90, and in several rounds the blocks that are done early make room for
+// others anyway (90 tokens of 3,400 keys down to half: 231 us so, 205 with equal numbers), so there every token gets ``each``, its shares
+// side by side (226 with the tokens side by side).
+struct LatentRun {
+  int token, position, item;
+  int first, count;  // the token's shares
+  int per;           // tiles of a share
+};
+__device__ __forceinline__ int latent_lowest(int p, int window) { return (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0; }
+// tiles of a token's keys; one that has none is given a share all the same
+__device__ __forceinline__ int latent_tiles(int p, int window) { return max(1, (p - latent_lowest(p, window) + KEYS) / KEYS); }
+
+// the run that share ``mine`` is of (token -1: nobody needs that share)
+__device__ __forceinline__ LatentRun latent_share(const int32_t* positions, const int32_t* token_item, int tokens, int window, int shares,
+                                                  int mine, int lane) {
+  int p = lane < tokens ? positions[lane] : 0, item = lane < tokens ? token_item[lane] : 0;  // of the first 32 tokens
+  const int n0 = lane < tokens ? latent_tiles(p, window) : 0;
+  int total = n0, most = n0;
+  for (int t = lane + 32; t < tokens; t += 32) {
+    const int n = latent_tiles(positions[t], window);
+    total += n;
+    most = max(most, n);
+  }
+  total = __reduce_add_sync(0xffffffffu, total);
+  most = __reduce_max_sync(0xffffffffu, most);
+  int lo = max((total + shares - 1) / shares, (most + MAX_SPLITS - 1) / MAX_SPLITS);
+  // enough: total / (shares - tokens) tiles each
+  int hi = max(lo, min(most, (total + shares - tokens - 1) / (shares - tokens)));
+  while (lo < hi) {
+    const int per = (lo + hi) >> 1;
+    int needed = (n0 + per - 1) / per;
+    for (int t = lane + 32; t < tokens; t += 32) needed += (latent_tiles(positions[t], window) + per - 1) / per;
+    if (__reduce_add_sync(0xffffffffu, needed) <= shares) hi = per;
+    else lo = per + 1;
+  }
+  int before = 0;
+  for (int t0 = 0; t0 < tokens; t0 += 32) {
+    if (t0 > 0 && t0 + lane < tokens) p = positions[t0 + lane], item = token_item[t0 + lane];
+    const int n = t0 + lane < tokens ? (latent_tiles(p, window) + lo - 1) / lo : 0;
+    int upto = n;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, upto, off);
+      if (lane >= off) upto += x;
+    }
+    const unsigned beyond = __ballot_sync(0xffffffffu, mine < before + upto);
+    if (beyond) {
+      const int who = __ffs(beyond) - 1;
+      const int count = __shfl_sync(0xffffffffu, n, who);
+      return {t0 + who, __shfl_sync(0xffffffffu, p, who), __shfl_sync(0xffffffffu, item, who),
+              before + __shfl_sync(0xffffffffu, upto, who) - count, count, lo};
+    }
+    before += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  return {-1, 0, 0, 0, 0, lo};
+}
+
 template <int HEADS>
 __global__ void __launch_bounds__(THREADS, 1)
 latent_attention_mma_kernel(const float* __restrict__ q_lat, const __nv_bfloat16* __restrict__ cache, const int32_t* __restrict__ table,
                             int table_width, const int32_t* __restrict__ positions, const int32_t* __restrict__ token_item,
-                            const float* __restrict__ gate, __nv_bfloat16* __restrict__ out, float* __restrict__ partial, int heads,
-                            int page_size, int num_pages, int window, float scale, const float* __restrict__ sink) {
+                            const float* __restrict__ gate, __nv_bfloat16* __restrict__ out, float* __restrict__ partial, int tokens,
+                            int shares, int each, int heads, int page_size, int num_pages, int window, float scale,
+                            const float* __restrict__ sink) {
   using Sh = LatentShape<HEADS>;
   constexpr int KT = Sh::KT, MG = Sh::MG;
   extern __shared__ __align__(16) unsigned char latent_smem[];
@@ -100,15 +163,22 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const __nv_bfloat16
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = heads / HEADS;
-  const int t = blockIdx.x / groups, h0 = (blockIdx.x - t * groups) * HEADS;
-  const int splits = gridDim.y, split = blockIdx.y;
-  const int p = positions[t];
-  const int32_t* pages = table + (size_t)token_item[t] * table_width;
-  const int lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
-  const int all = (p - lo + KT) / KT;                    // tiles of the token's keys, and this block's run of them
-  const int per = (all + splits - 1) / splits;
+  const int share = blockIdx.x / groups, h0 = (blockIdx.x - share * groups) * HEADS;
+  LatentRun run;
+  if (each > 0) {
+    const int t = share / each;
+    if (t >= tokens) return;  // what the tokens leave over
+    const int p = positions[t];
+    run = LatentRun{t, p, token_item[t], t * each, each, (latent_tiles(p, window) + each - 1) / each};
+  } else {
+    run = latent_share(positions, token_item, tokens, window, shares, share, lane);
+    if (run.token < 0) return;
+  }
+  const int t = run.token, split = share - run.first, splits = run.count, p = run.position, per = run.per;
+  const int32_t* pages = table + (size_t)run.item * table_width;
+  const int lo = latent_lowest(p, window);
   const int first = lo + split * per * KT;
-  const int end = min(p + 1, first + per * KT);
+  const int end = p + 1 - first > per * KT ? first + per * KT : p + 1;
   const int ntiles = max(0, (end - first + KT - 1) / KT);
 
   // A warp brings in four neighbouring rows of a tile; where they lie is looked up one tile earlier (lane r: row r), so that
@@ -317,8 +387,9 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const __nv_bfloat16
   }
 #pragma unroll
   for (int off = 1; off < PER_HEAD; off <<= 1) l_run += __shfl_xor_sync(0xffffffffu, l_run, off);
-  if (splits > 1) {
-    float* mine = partial + (((size_t)t * heads + h0) * splits + split) * (RANK + 2);
+  if (shares > tokens) {  // a token's shares together: [heads, splits, RANK + 2]; where they are stands in its rows of the result, if that's to be found
+    float* mine = partial + ((size_t)run.first * heads + (size_t)h0 * splits + split) * (RANK + 2);
+    if (each == 0 && split == 0 && threadIdx.x < HEADS) *reinterpret_cast<int2*>(out + ((size_t)t * heads + h0 + threadIdx.x) * RANK) = make_int2(run.first, splits);
     if (key_at == 0) *reinterpret_cast<float2*>(mine + (size_t)head * splits * (RANK + 2)) = make_float2(m_run, l_run);
 #pragma unroll
     for (int m = 0; m < MG; ++m)
@@ -352,16 +423,37 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const __nv_bfloat16
     }
 }
 
-// A block per (token, head): the shares of the blocks that split its keys, in split order.
-__global__ void __launch_bounds__(RANK / 4)
-latent_attention_mma_merge_kernel(const float* __restrict__ partial, const float* __restrict__ gate, __nv_bfloat16* __restrict__ out,
-                                  int splits, const float* __restrict__ sink, int heads) {
+// A block per (token, head): the shares of the blocks that split its keys, every other one a group of threads, asked for before
+// their weights are known (up to ten of them): 16 tokens of 32 heads, 9 shares each, 4.0 us; one group of threads and a share after
+// the other 5.3.
+constexpr int MERGE_AHEAD = 5, MERGE_COLS = RANK / 4;
+template <int GROUPS>
+__global__ void __launch_bounds__(GROUPS * MERGE_COLS)
+latent_attention_mma_merge_kernel(const float* __restrict__ partial, const float* __restrict__ gate, __nv_bfloat16* out, int each,
+                                  const float* __restrict__ sink, int heads) {
   __shared__ float by[MAX_SPLITS];
+  __shared__ float4 sums[GROUPS > 1 ? GROUPS - 1 : 1][MERGE_COLS];
   pdl_trigger();
   pdl_wait();
   const size_t unit = blockIdx.x;
-  const float* mine = partial + unit * splits * (RANK + 2);
-  const int lane = threadIdx.x & 31;
+  // first share and number of shares; what stands in the result is overwritten at the end
+  const int2 run = each > 0 ? make_int2((int)(unit / heads) * each, each) : *reinterpret_cast<const int2*>(out + unit * RANK);
+  const int splits = run.y;
+  const float* mine = partial + ((size_t)run.x * heads + unit % heads * splits) * (RANK + 2);
+  const int group = threadIdx.x / MERGE_COLS, column = threadIdx.x % MERGE_COLS, lane = threadIdx.x & 31;
+  const float* src = mine + 2 + 4 * column;  // rows start on 8 bytes
+  float2 a[MERGE_AHEAD], b[MERGE_AHEAD];
+  auto ask = [&](int s0) {
+#pragma unroll
+    for (int j = 0; j < MERGE_AHEAD; ++j) {
+      const int s = s0 + j * GROUPS;
+      a[j] = b[j] = make_float2(0.f, 0.f);
+      if (s >= splits) continue;
+      a[j] = *reinterpret_cast<const float2*>(src + (size_t)s * (RANK + 2));
+      b[j] = *reinterpret_cast<const float2*>(src + (size_t)s * (RANK + 2) + 2);
+    }
+  };
+  ask(group);
   if (threadIdx.x < 32) {
     const float2 ml = lane < splits ? *reinterpret_cast<const float2*>(mine + (size_t)lane * (RANK + 2)) : make_float2(-FLT_MAX, 0.f);
     const float sk = sink ? sink[unit % heads] : -FLT_MAX;
@@ -371,31 +463,44 @@ latent_attention_mma_merge_kernel(const float* __restrict__ partial, const float
     by[lane] = f * (gate ? gate[unit] : 1.f) / sum;
   }
   __syncthreads();
-  float v[4] = {0.f, 0.f, 0.f, 0.f};
-  const float* src = mine + 2 + 4 * threadIdx.x;  // rows start on 8 bytes
-#pragma unroll 4
-  for (int s = 0; s < splits; ++s) {
-    const float2 a = *reinterpret_cast<const float2*>(src + (size_t)s * (RANK + 2)), b = *reinterpret_cast<const float2*>(src + (size_t)s * (RANK + 2) + 2);
-    const float f = by[s];
-    v[0] = fmaf(a.x, f, v[0]); v[1] = fmaf(a.y, f, v[1]);
-    v[2] = fmaf(b.x, f, v[2]); v[3] = fmaf(b.y, f, v[3]);
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = group; s0 < splits; s0 += MERGE_AHEAD * GROUPS) {
+    if (s0 > group) ask(s0);
+#pragma unroll
+    for (int j = 0; j < MERGE_AHEAD; ++j) {
+      if (s0 + j * GROUPS >= splits) break;
+      const float f = by[s0 + j * GROUPS];
+      v.x = fmaf(a[j].x, f, v.x); v.y = fmaf(a[j].y, f, v.y);
+      v.z = fmaf(b[j].x, f, v.z); v.w = fmaf(b[j].y, f, v.w);
+    }
   }
-  __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
-  *reinterpret_cast<uint2*>(out + unit * RANK + 4 * threadIdx.x) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+  if constexpr (GROUPS > 1) {
+    if (group) sums[group - 1][column] = v;
+    __syncthreads();
+    if (group) return;
+#pragma unroll
+    for (int g = 0; g < GROUPS - 1; ++g) {
+      const float4 x = sums[g][column];
+      v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+    }
+  }
+  __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+  *reinterpret_cast<uint2*>(out + unit * RANK + 4 * column) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
 }
 
 template <int HEADS>
 int launch_latent_mma(const float* q, const __nv_bfloat16* cache, const int32_t* table, int width, const int32_t* positions,
                       const int32_t* token_item, const float* gate, __nv_bfloat16* out, float* partial, int T, int heads, int page_size,
-                      int num_pages, int window, float scale, int splits, const float* sink, cudaStream_t stream) {
+                      int num_pages, int window, float scale, int shares, int each, const float* sink, cudaStream_t stream) {
   static PsbPerDevice configured;
   if (!configured.get()) {
     if (cudaFuncSetAttribute(latent_attention_mma_kernel<HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, LatentShape<HEADS>::BYTES) != cudaSuccess)
       PSB_REFUSE("latent_attention_mma: cannot raise the shared-memory limit");
     configured.set();
   }
-  psb_launch(latent_attention_mma_kernel<HEADS>, dim3((unsigned)(T * (heads / HEADS)), splits), dim3(THREADS), (size_t)LatentShape<HEADS>::BYTES,
-             stream, q, cache, table, width, positions, token_item, gate, out, partial, heads, page_size, num_pages, window, scale, sink);
+  psb_launch(latent_attention_mma_kernel<HEADS>, dim3((unsigned)(shares * (heads / HEADS))), dim3(THREADS), (size_t)LatentShape<HEADS>::BYTES,
+             stream, q, cache, table, width, positions, token_item, gate, out, partial, T, shares, each, heads, page_size, num_pages, window,
+             scale, sink);
   PSB_LAUNCH_CHECK("latent_attention_mma");
   return 0;
 }
@@ -408,27 +513,30 @@ PSB_API int psb_latent_attention_mma_heads(int rank, int rot, int heads) {
   return heads % 32 == 0 ? 32 : heads % 16 == 0 ? 16 : 0;
 }
 
-// bfloat16 cache and output, float32 queries [T, heads, RANK + ROT]; ``splits`` (1..32) blocks share a token's keys, with
-// ``partial`` float32 [T, heads, splits, RANK + 2] as their meeting place.
+// bfloat16 cache and output, float32 queries [T, heads, RANK + ROT]; ``shares`` (T..32 T) blocks share out the tokens' keys, for
+// every group of heads, with ``partial`` float32 [shares, heads, RANK + 2] as their meeting place if they are more than the tokens.
 PSB_API int psb_latent_attention_mma(const void* q_lat, const void* cache, const void* table, int table_width, const void* positions,
                                      const void* token_item, const void* gate, void* out, int T, int heads, int rank, int rot, int page_size,
-                                     int num_pages, int window, float scale, int splits, void* partial, const void* sink, cudaStream_t stream) {
+                                     int num_pages, int window, float scale, int shares, void* partial, const void* sink, cudaStream_t stream) {
   const int per_block = psb_latent_attention_mma_heads(rank, rot, heads);
   if (!per_block || T < 0) PSB_REFUSE("latent_attention_mma: not built for T=%d heads=%d rank=%d rot=%d", T, heads, rank, rot);
   if (page_size < 1 || num_pages < 1 || table_width < 1) PSB_REFUSE("latent_attention_mma: bad paging (page_size=%d pages=%d width=%d)", page_size, num_pages, table_width);
   if (window < 0) PSB_REFUSE("latent_attention_mma: negative window");
-  if (splits < 1 || splits > MAX_SPLITS || (splits > 1 && !partial)) PSB_REFUSE("latent_attention_mma: 1 to %d splits (with their scratch), not %d", MAX_SPLITS, splits);
   if (((uintptr_t)cache | (uintptr_t)q_lat | (uintptr_t)out | (uintptr_t)partial) & 15) PSB_REFUSE("latent_attention_mma: queries, cache, scratch and output must be 16-byte aligned");
   if (T == 0) return 0;
-  if ((long long)T * heads > 0x7fffffffLL) PSB_REFUSE("latent_attention_mma: batch too large");
+  if (shares < T || shares > (long long)T * MAX_SPLITS || (shares > T && !partial))
+    PSB_REFUSE("latent_attention_mma: 1 to %d shares a token (with their scratch), not %d for %d", MAX_SPLITS, shares, T);
+  if ((long long)T * heads > 0x7fffffffLL || (long long)shares * (heads / per_block) > 0x7fffffffLL) PSB_REFUSE("latent_attention_mma: batch too large");
+  const int each = shares == T || (long long)shares * (heads / per_block) > psb_current_sms() ? shares / T : 0;
   auto launch = per_block == 32 ? launch_latent_mma<32> : launch_latent_mma<16>;
   const int status = launch((const float*)q_lat, (const __nv_bfloat16*)cache, (const int32_t*)table, table_width, (const int32_t*)positions,
                             (const int32_t*)token_item, (const float*)gate, (__nv_bfloat16*)out, (float*)partial, T, heads, page_size,
-                            num_pages, window, scale, splits, (const float*)sink, stream);
+                            num_pages, window, scale, shares, each, (const float*)sink, stream);
   if (status) return status;
-  if (splits > 1) {
-    psb_launch(latent_attention_mma_merge_kernel, dim3((unsigned)(T * heads)), dim3(RANK / 4), 0, stream, (const float*)partial,
-               (const float*)gate, (__nv_bfloat16*)out, splits, (const float*)sink, heads);
+  if (shares > T) {
+    const auto merge = each > 0 ? latent_attention_mma_merge_kernel<1> : latent_attention_mma_merge_kernel<2>;
+    psb_launch(merge, dim3((unsigned)(T * heads)), dim3((each > 0 ? 1 : 2) * MERGE_COLS), 0, stream, (const float*)partial, (const float*)gate,
+               (__nv_bfloat16*)out, each, (const float*)sink, heads);
     PSB_LAUNCH_CHECK("latent_attention_mma_merge");
   }
   return 0;

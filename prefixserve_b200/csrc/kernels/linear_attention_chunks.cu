@@ -407,7 +407,7 @@ PSB_API int psb_linear_chunks(const void* proj, long long ld, const void* alpha,
              (const int32_t*)item_start, (float*)records, items, min_tokens, H, dim, vdim);
   PSB_LAUNCH_CHECK("linear_chunk");
   // runs of columns a block takes: as for the delta rules' chain (delta_chunks.cu)
-  const long long heads = (long long)H * portions, sms = current_sms();
+  const long long heads = (long long)H * portions, sms = psb_current_sms();
   const long long rounds16 = (heads * ((vdim + 15) / 16) + sms - 1) / sms, rounds32 = (heads * ((vdim + 31) / 32) + sms - 1) / sms;
   auto launch = rounds32 * 31 < rounds16 * 20 ? launch_chain<2> : launch_chain<1>;
   return launch((const float*)records, (float*)state, slot_floats, (const int32_t*)item_start, (const int32_t*)slots, (float*)o, items, portions, chunks,

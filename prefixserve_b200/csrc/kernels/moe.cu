@@ -603,18 +603,6 @@ static_assert(MAX_EXPERTS == 1 << 9, "an expert is nine bits of a pass");
 
 PsbPerDevice fewrows_attr[2];
 
-// SMs of the current device, asked for once a device
-int current_sms() {
-  static int known[PsbPerDevice::kMaxDevices] = {};
-  const int d = PsbPerDevice::current();
-  if (d >= 0 && known[d] > 0) return known[d];
-  int sms = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d < 0 ? 0 : d);
-  sms = std::max(sms, 1);
-  if (d >= 0) known[d] = sms;
-  return sms;
-}
-
 template <typename TY, typename TS, typename TO>
 __global__ void moe_combine_kernel(const TY* __restrict__ Y, const int32_t* __restrict__ pair_row, const float* __restrict__ weight,
                                    const TS* __restrict__ shared, const float* __restrict__ gate, int ldg, TO* __restrict__ out,
@@ -779,7 +767,7 @@ PSB_API int psb_moe_gemm(const void* a, int a_dtype, const void* w, int w_dtype,
   const size_t few_smem = few_rows * few_row;
   if (a_dtype == PSB_BF16 && w_dtype == PSB_BF16 && K % 8 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0 &&
       pairs <= FEW_PAIRS * E && few_smem <= FEW_SMEM) {
-    const dim3 few_grid(2 * current_sms());
+    const dim3 few_grid(2 * psb_current_sms());
     PSB_DISPATCH_DTYPE(c_dtype, TC, {
       auto kernel = moe_fewrows_kernel<TC>;
       PsbPerDevice& done = fewrows_attr[c_dtype == PSB_F32 ? 0 : 1];

@@ -740,7 +740,8 @@ def latent_attention(q_lat: torch.Tensor, cache: torch.Tensor, table: torch.Tens
 ROWS_BLOCK_SHARE = 96      # what a block costs beyond its keys, in keys
 ROWS_KEYS_PER_SPLIT = 128  # no block of that kernel is given fewer keys than this by splitting
 # The tensor-core kernel (rows of 512 + 64 numbers, heads in groups of 16 or 32): a block's queries and its unscaled result
-# cost about what 64 keys do, and up to 32 blocks may share a token's keys.  Down to the shortest walks it is ahead of the
+# cost about what 64 keys do, and up to 32 blocks may share a token's keys; how many do is up to the token's length (the kernel shares
+# the blocks out), so that one round of blocks takes as many as there are places.  Down to the shortest walks it is ahead of the
 # kernel that reads rows side by side (32 tokens of 32 heads over up to 100 keys: 17 us).
 LATENT_MMA = True
 LATENT_MMA_BLOCK_SHARE = 64
@@ -770,14 +771,19 @@ def _latent_attention_walk(q_lat, cache, table, positions, token_item, gate, out
     if LATENT_MMA and cache.dtype == torch.bfloat16 and out.dtype == torch.bfloat16:
         per_block = lib().psb_latent_attention_mma_heads(rank, d - rank, heads)
     if per_block and q_lat.data_ptr() % 16 == 0 and cache.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0:
+        shares, groups = t, heads // per_block
         if key_hint >= 2 * LATENT_MMA_KEYS_PER_SPLIT:
             from .tensorcore import _sms
-            splits = _rows_splits(t * heads // per_block, key_hint, _sms(q_lat.device), 32, LATENT_MMA_KEYS_PER_SPLIT, LATENT_MMA_BLOCK_SHARE)
-        if splits > 1:
-            partial = torch.empty((t, heads, splits, rank + 2), dtype=torch.float32, device=q_lat.device)
+            slots, most = _sms(q_lat.device), min(32, key_hint // LATENT_MMA_KEYS_PER_SPLIT)
+            splits = _rows_splits(t * groups, key_hint, slots, most, LATENT_MMA_KEYS_PER_SPLIT, LATENT_MMA_BLOCK_SHARE)
+            shares = t * splits
+            if t < shares <= slots // groups:  # one round: all of it
+                shares = min(slots // groups, t * most)
+        if shares > t:
+            partial = torch.empty((shares, heads, rank + 2), dtype=torch.float32, device=q_lat.device)
         check(lib().psb_latent_attention_mma(q_lat.data_ptr(), cache.data_ptr(), table.data_ptr(), table.shape[1], positions.data_ptr(),
                                              token_item.data_ptr(), _ptr(gate), out.data_ptr(), t, heads, rank, d - rank, page_size,
-                                             cache.shape[0], int(window or 0), float(scale), splits, _ptr(partial), _ptr(sink), _stream()),
+                                             cache.shape[0], int(window or 0), float(scale), shares, _ptr(partial), _ptr(sink), _stream()),
               "latent_attention")
         return
     if lib().psb_latent_attention_rows_supported(_code(cache, "cache entry"), rank, d - rank):

@@ -150,7 +150,7 @@ _SIGNATURES: dict[str, list] = {
     # (rank, rot, heads) -> heads a block of the tensor-core kernel takes, 0 if it is not built for the sizes
     "psb_latent_attention_mma_heads": [I, I, I],
     # (q_lat, cache, table, table_width, positions, token_item, gate, out, T, heads, rank, rot, page_size, num_pages, window,
-    #  scale, splits, partial, sink, stream)
+    #  scale, shares, partial, sink, stream)
     "psb_latent_attention_mma": [P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, F, I, P, P, P],
     # (cache, dtype, table, table_width, positions, token_item, band, values2, t0, n, KP, D, rank, page_size, num_pages, window, stream)
     "psb_latent_band_gather": [P, I, P, I, P, P, P, P, I, I, I, I, I, I, I, I, P],

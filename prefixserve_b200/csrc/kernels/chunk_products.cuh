@@ -6,16 +6,24 @@
 // off); the rest is smaller by 2^8.  As many terms as float32's own accuracy takes in TF32 (six products of eleven bits) take twice as long, and
 // fma.rn.f32x2 as long as these, but for what shared memory has to hand to the registers (16 bytes a lane: four cycles a warp).
 #pragma once
-#include <algorithm>
-
 #include "delta_common.cuh"
 #include "portions.cuh"
-#include "tf32_terms.cuh"
 
 namespace chunks {
 using delta::copy_async16_or_zero;
-using terms::is_finite;
-using terms::Product;
+
+__device__ __forceinline__ bool is_finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+
+// A running product of decays with what its roundings lose carried along, rounded once where it is read.
+struct Product {
+  float hi = 1.f, lo = 0.f;
+  __device__ __forceinline__ void times(float a) {
+    const float p = hi * a;
+    lo = fmaf(lo, a, fmaf(hi, a, -p));
+    hi = p;
+  }
+  __device__ __forceinline__ float value() const { return hi + lo; }
+};
 
 constexpr int CHUNK = 32;
 constexpr int RP = 128;                            // keys are filled up to so many numbers

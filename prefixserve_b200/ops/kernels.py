@@ -1412,12 +1412,13 @@ LINEAR_MIXED = 96
 def _linear_one_by_one(lengths: list[int] | None) -> bool:
     """Whether a step that could go either way whole has so much in short portions, which the two forms take one after the other, that all
     of it is over sooner token by token (16 heads, both forms and token by token: 48 tokens beside 32 single ones 48 and 39 us, 64 beside eight of
-    16 tokens 42 and 39, 64 beside one of 31 38 and 35, 64 beside a single one 28 and 34; 96 beside one of 31 40 and 47, 100 beside eight
-    single ones 34 and 51, beside 32 51 and 60)."""
+    16 tokens 42 and 39, 64 beside one of 31 38 and 35, 64 beside a single one 28 and 34; 100 beside eight single ones 34 and 51.  From 96
+    tokens on the chunks are ahead a little beyond the line, 96 beside one of 31 40 and 47, 100 beside 32 51 and 60, which is kept where
+    longer chunks had it)."""
     short = [n for n in lengths or [] if n < LINEAR_SHORT]
     if not short or max(lengths) > 2 * LINEAR_ATTENTION_CHUNK:
         return False
-    return len(short) > 48 or (max(lengths) < LINEAR_MIXED and (len(short) > 8 or max(short) > 8))
+    return len(short) > (8 if max(lengths) < LINEAR_MIXED else 16) or max(short) > 8
 
 
 def linear_attention(proj: torch.Tensor, alpha: torch.Tensor, state: torch.Tensor, ctx, *, heads: int, dim: int, vdim: int) -> torch.Tensor:

@@ -1015,20 +1015,6 @@ PSB_API int psb_attention_biased(const void* q, int dtype, const void* kv, int k
   return 0;
 }
 
-// Joins the shares that several blocks left of every (token, head): (partial [T * hq, splits, vdim + 2] float32, sink, out bfloat16,
-// T, hq, vdim, splits, gate, ldg, ldo, out_scale, stream)
-PSB_API int psb_attention_rows_merge(const void* partial, const void* sink, void* out, int T, int hq, int vdim, int splits, const void* gate,
-                                     long long ldg, long long ldo, float out_scale, cudaStream_t stream) {
-  if (T < 0 || hq < 1 || vdim < 1 || vdim > MAX_D || splits < 1 || splits > MAX_KEY_SPLITS || !partial) PSB_REFUSE("attention_rows_merge: bad sizes");
-  if (ldo < (long long)hq * vdim || (gate && ldg < (long long)hq * vdim)) PSB_REFUSE("attention_rows_merge: bad output or gate rows");
-  if (T == 0) return 0;
-  const RowsTail tail{gate, ldg, ldo, out_scale, 0.f};
-  psb_launch(attention_biased_merge_kernel<__nv_bfloat16>, dim3((unsigned)(T * hq)), dim3(32), 0, stream, (const float*)partial,
-             (const float*)sink, (__nv_bfloat16*)out, hq, vdim, splits, tail);
-  PSB_LAUNCH_CHECK("attention_rows_merge");
-  return 0;
-}
-
 // (hq, hkv, dim, vdim) -> 1 if the tensor-core kernel for single tokens takes the shape
 PSB_API int psb_attention_rows_single_supported(int hq, int hkv, int dim, int vdim) {
   return hq >= 1 && hkv >= 1 && hq % hkv == 0 && dim >= 8 && dim <= 128 && dim % 8 == 0 && vdim >= 8 && vdim <= 128 && vdim % 8 == 0 ? 1 : 0;

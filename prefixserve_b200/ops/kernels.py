@@ -979,7 +979,9 @@ BIASED_BLOCKS_WANTED = 2368
 ROWS_SINGLE = True
 ROWS_BLOCKS_WANTED = 592
 # ... and heads of 128, at most eight to a key/value head: the kernel fed by the TMA unit.  Its blocks cost, beside their keys, about
-# what ROWS_DECODE_BLOCK_SHARE keys do.
+# what ROWS_DECODE_BLOCK_SHARE keys do.  Where a round of them has a whole number of blocks for every (token, key/value head), so many are
+# issued, and their shares end where a token's keys do (16 tokens of 8 key/value heads, 384 blocks 34 us, 444 blocks 35); else as many as
+# the device holds share everything out evenly (32 tokens 61 -> 54 us, 64 tokens 105 -> 89, against whole numbers in several rounds).
 # Below so many (key/value head, key) pairs a step's rows are read in 12 us or less by either kernel, and the host takes longer to issue
 # one than that; the other kernel is issued with less (two tokens of 16 heads over 413 keys: 25 us a call instead of 36).
 ROWS_DECODE = True
@@ -1027,16 +1029,19 @@ def _rows_single_tokens(q, positions, token_item, out, tail, kv, table, bias, si
     if (ROWS_DECODE and t * num_kv_heads * keys >= ROWS_DECODE_LEAST
             and bool(lib().psb_attention_rows_decode_supported(num_heads, num_kv_heads, dim, vdim, page_size))):
         from .tensorcore import _sms
-        splits = _rows_splits(t * num_kv_heads, keys, lib().psb_attention_rows_decode_blocks() * _sms(q.device), 16,
-                              ROWS_DECODE_KEYS_PER_SPLIT, ROWS_DECODE_BLOCK_SHARE)
-        partial = torch.empty((t, num_heads, splits, vdim + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
+        blocks, scratch, least = 0, None, max(1, ROWS_DECODE_KEYS_PER_SPLIT // 16)
+        if keys >= 2 * ROWS_DECODE_KEYS_PER_SPLIT:
+            units, slots = t * num_kv_heads, lib().psb_attention_rows_decode_blocks() * _sms(q.device)
+            splits = _rows_splits(units, keys, slots, 16, ROWS_DECODE_KEYS_PER_SPLIT, ROWS_DECODE_BLOCK_SHARE)
+            blocks = units * splits if 1 < splits <= slots // units else min(slots, units * (keys // ROWS_DECODE_KEYS_PER_SPLIT))
+            scratch = torch.empty(4 * t * num_kv_heads + 2 * blocks * (num_heads // num_kv_heads) * (vdim + 2), dtype=torch.float32, device=q.device)
         check(lib().psb_attention_rows_decode(q.data_ptr(), kv.data_ptr(), kv.shape[0], table.data_ptr(), table.shape[1],
                                               positions.data_ptr(), token_item.data_ptr(), _ptr(bias), _ptr(sink), out.data_ptr(), t,
-                                              num_heads, num_kv_heads, dim, vdim, page_size, *masks, _ptr(partial), splits, *tail, _stream()),
+                                              num_heads, num_kv_heads, dim, vdim, page_size, *masks, _ptr(scratch), blocks, least, *tail, _stream()),
               "attention_rows_single")
-        if splits > 1:
-            check(lib().psb_attention_rows_merge(partial.data_ptr(), _ptr(sink), out.data_ptr(), t, num_heads, vdim, splits, *tail[:4],
-                                                 _stream()), "attention_rows_merge")
+        if blocks:
+            check(lib().psb_attention_rows_decode_merge(scratch.data_ptr(), _ptr(sink), out.data_ptr(), t, num_heads, num_kv_heads, *tail[:4],
+                                                        _stream()), "attention_rows_merge")
         return
     blocks = t * num_kv_heads * -(-(num_heads // num_kv_heads) // 16)
     splits = max(1, min(16, -(-ROWS_BLOCKS_WANTED // max(blocks, 1)), keys // 128))

@@ -199,11 +199,11 @@ _SIGNATURES: dict[str, list] = {
     "psb_attention_rows_decode_supported": [I, I, I, I, I],
     "psb_attention_rows_decode_blocks": [],
     # (q, kv, num_pages, table, table_width, positions, token_item, bias, sink, out, T, hq, hkv, dim, vdim, page_size, window, chunk, reach,
-    #  scale, keep_first, partial, splits, gate, ldg, ldo, out_scale, softcap, stream)
-    "psb_attention_rows_decode": [P, P, L, P, I, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P, I, P, L, L, F, F, P],
+    #  scale, keep_first, scratch, blocks, least_runs, gate, ldg, ldo, out_scale, softcap, stream)
+    "psb_attention_rows_decode": [P, P, L, P, I, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P, I, I, P, L, L, F, F, P],
     "psb_attention_rows_decode_status": [],
-    # (partial, sink, out, T, hq, vdim, splits, gate, ldg, ldo, out_scale, stream)
-    "psb_attention_rows_merge": [P, P, P, I, I, I, I, P, L, L, F, P],
+    # (scratch, sink, out, T, hq, hkv, gate, ldg, ldo, out_scale, stream)
+    "psb_attention_rows_decode_merge": [P, P, P, I, I, I, P, L, L, F, P],
     "psb_delta_max_taps": [],
     # (proj, dtype, ld, beta_at, ba, decay, taps, a_log, dt_bias, state, positions, token_item, item_start, slots, qkv_out, bd_out, T,
     #  G, H, dim, vdim, K, num_slots, slot_floats, cross, stream)

@@ -5,7 +5,7 @@ Mirrors what the reference's engine offers a driver
 (prefixserve/engine.py:10-29, prefixserve/llama_engine.py:46-150):
 ``num_blocks``, ``max_seq_len``, ``stop_token_ids`` and a blocking
 ``step(batch) -> {request id: token}``; the pool is sized from free memory
-after a worst-case trial step when ``num_blocks`` is not given
+after worst-case trial steps when ``num_blocks`` is not given
 (prefixserve/llama_engine.py:231-267).
 """
 
@@ -54,6 +54,27 @@ class PendingStep:
     host: torch.Tensor | None            # the same in pinned host memory once ``done`` has passed
     done: torch.cuda.Event | None
     logits: torch.Tensor | None = None   # with ``Engine.capture_logits``: float32 [len(sampling), vocab], a copy on the device
+
+
+def trial_steps(budget: int, requests: int, longest: int) -> list[list[int]]:
+    """New tokens of every request in the steps that the pool is sized by: ``budget`` tokens of prompts, no portion longer than ``longest``.
+
+    One long portion beside single tokens takes most of what grows with a step's tokens.  The recurrences that work 32 tokens at a time hold a
+    record for every chunk begun (97 KB a head), so they take most for as many portions as there may be: of eight tokens, from which on
+    the delta rules go in chunks, and a token beyond a chunk, for those that go in chunks from 32 on."""
+    steps = []
+    for least in (1, 8, 33):
+        many = 1 if least == 1 else min(requests, budget // least)
+        if many < 1 or least > longest:
+            continue
+        new, rest = [], budget
+        while len(new) < requests and rest > 0:  # as much as goes into the first, with ``least`` left for each of the others
+            new.append(min(longest, rest - least * max(0, many - 1 - len(new))))
+            rest -= new[-1]
+        new += [1] * (requests - len(new))  # single tokens do not count against the budget
+        if new not in steps:
+            steps.append(new)
+    return steps
 
 
 class Engine:
@@ -219,10 +240,11 @@ class Engine:
 
     # ---- pool sizing ----------------------------------------------------------
     def _size_pool(self) -> int:
-        """Pages that fit beside the weights and the activations of a worst-case step."""
+        """Pages that fit beside the weights and the activations of the worst-case steps."""
         cfg = self.cfg
         prefill = min(cfg.max_prefill_tokens, cfg.max_seq_len)
-        trial_pages = pages_for(prefill, cfg.page_size) + cfg.max_num_seqs
+        steps = trial_steps(cfg.max_prefill_tokens, cfg.max_num_seqs, cfg.max_seq_len)
+        trial_pages = max(sum(pages_for(n, cfg.page_size) for n in step) for step in steps) + 1
         torch.cuda.synchronize()
         gc.collect()
         torch.cuda.empty_cache()
@@ -231,14 +253,16 @@ class Engine:
         cache = self._make_cache(trial_pages)
         runner = ModelRunner(self.model, cache, device=self.device, use_graphs=False)
         held = torch.cuda.memory_allocated() - before
-        items = []
-        for i in range(cfg.max_num_seqs):
-            n = prefill if i == 0 else 1
-            slot = cache.open()
-            cache.reserve(slot, n)
-            items.append(StepItem(slot, 0, np.zeros(n, dtype=np.int32), (n - 1,)))
-        runner.step(items)
-        torch.cuda.synchronize()
+        for step in steps:
+            items = []
+            for n in step:
+                slot = cache.open()
+                cache.reserve(slot, n)
+                items.append(StepItem(slot, 0, np.zeros(n, dtype=np.int32), (n - 1,)))
+            runner.step(items)
+            torch.cuda.synchronize()
+            for it in items:
+                cache.close(it.slot)
         activations = torch.cuda.max_memory_allocated() - before - held
         cache.release_device_memory()  # the trial pages go back before the real pool is measured for
         del cache, runner
@@ -266,5 +290,5 @@ class Engine:
                     sizes[gi] = n
         elif usable < 0:
             raise EngineError(f"the windowed cache groups alone do not fit ({-usable / 1e9:.2f} GB short)")
-        log.info("trial step: activations %.0f MB, %.2f GB free -> pages per group %s", activations / 1e6, free / 1e9, sizes)
+        log.info("trial steps: activations %.0f MB, %.2f GB free -> pages per group %s", activations / 1e6, free / 1e9, sizes)
         return sizes if len(sizes) != 1 else next(iter(sizes.values()))

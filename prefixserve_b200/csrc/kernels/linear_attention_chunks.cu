@@ -71,7 +71,7 @@ linear_chunk_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const 
   widen_rows(ks, rows + (size_t)(H + h) * dim, ld, n, dim);
   delta::copy_async_wait();
   __syncthreads();
-  products_on_diagonal<false, false>(ks, qs, gs, nullptr, ps, warp, lane);
+  products_on_diagonal<false, true>(ks, qs, gs, nullptr, ps, warp, lane);
   // the values, columns first: nobody else waits for them
   const uint16_t* values = reinterpret_cast<const uint16_t*>(rows + 2 * (size_t)H * dim + (size_t)h * vdim);
 #pragma unroll 2

@@ -12,7 +12,7 @@
 // Decays are only ever multiplied, never divided by, and the running ones of a chunk carry what the roundings lose.  float32 numbers enter the tensor cores in three
 // terms (chunk_products.cuh), the values, which are bfloat16, as they are.
 // P is zero above the diagonal, and zero times a value that is not finite is not zero: a result that comes out not finite is made
-// again from the tokens up to its own.
+// again from the tokens up to its own, and from the state as it is, whose terms are no sum where it is infinite.
 // A float32 projection's values would need terms too; those stay with the other kernels.
 //
 // Distances from float64, token by token and here (150 and 700 tokens): read-outs 1.2e-7 and 1.03e-7, states 0.95e-7 and 0.59e-7.
@@ -131,9 +131,10 @@ linear_chunk_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const 
 }
 
 constexpr int PP = CHUNK + 8;  // of the shares: columns first
+constexpr int SP = RP + 8;     // of the state: columns first, as pairs of channels
 template <int TILES>
 struct Chain {
-  static constexpr int COLS = 16 * TILES, SHARES = WORKERS / 32, FLOATS = 2 * SHARES * COLS * PP;  // of two chunks
+  static constexpr int COLS = 16 * TILES, SHARES = WORKERS / 32, S_AT = 2 * SHARES * COLS * PP, FLOATS = S_AT + 2 * COLS * SP;  // of two chunks
   static_assert(FLOATS * 4 <= 227 * 1024, "beyond a block's shared memory");
 };
 // One step of sixteen terms of N sums whose left operand is bfloat16 as it is (see step).
@@ -153,6 +154,12 @@ __device__ __forceinline__ void step_whole(float (&sum)[N][4], float (&small)[N]
     for (int e = 0; e < 4; ++e) sum[n][e] += d[n][e];
 }
 
+// the number whose first term lies in this word of a record
+__device__ __forceinline__ float number(const uint32_t* word, int half) {
+  const float first = term(word[0], half);
+  return is_finite(first) ? first + (term(word[TERM], half) + term(word[2 * TERM], half)) : first;
+}
+
 template <int TILES>
 __global__ void __launch_bounds__(CHAIN_THREADS, 1)
 linear_chain_kernel(const float* __restrict__ records, float* __restrict__ state, long long slot_floats, const int32_t* __restrict__ item_start,
@@ -160,7 +167,7 @@ linear_chain_kernel(const float* __restrict__ records, float* __restrict__ state
                     int num_slots, float scale) {
   using Sh = Chain<TILES>;
   constexpr int COLS = Sh::COLS, SHARES = Sh::SHARES;
-  extern __shared__ __align__(16) float chain[];  // [2][SHARES][COLS][PP]
+  extern __shared__ __align__(16) float chain[];  // [2][SHARES][COLS][PP], and the state each chunk starts from, [2][COLS][SP]
   const int h = blockIdx.y, col0 = blockIdx.x * COLS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, tg = lane & 3;
   pdl_wait();
@@ -238,6 +245,11 @@ linear_chain_kernel(const float* __restrict__ records, float* __restrict__ state
           }
 #pragma unroll
         for (int tile = 0; tile < TILES; ++tile) {
+          float* held = chain + Sh::S_AT + ((c & 1) * COLS + 16 * tile + gr) * SP + 16 * warp + 2 * tg;  // for read-outs that are made again
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) *reinterpret_cast<float2*>(held + 8 * r * SP + 8 * m) = make_float2(s[tile][m][2 * r], s[tile][m][2 * r + 1]);
           Left a;  // the state's sums lie as a left operand
 #pragma unroll
           for (int e = 0; e < 4; ++e) a.put(e, split3(s[tile][e >> 1][2 * (e & 1)], s[tile][e >> 1][2 * (e & 1) + 1]));
@@ -340,16 +352,23 @@ linear_chain_kernel(const float* __restrict__ records, float* __restrict__ state
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int i = 8 * eight + 2 * tg + e, t = t0 + c * CHUNK + i;
-            const float of_state = e ? v[0].y : v[0].x;
+            float of_state = e ? v[0].y : v[0].x;
             float y = of_state + of_values[tile][2 * e2 + e];
             if (!is_finite(y) && col < vdim) {
+              if (!is_finite(of_state)) {  // an infinite number's lower terms are not zero: the state as it is, until it is not a number
+                const float* held = chain + Sh::S_AT + ((c & 1) * COLS + 16 * tile + in) * SP;
+                of_state = 0.f;
+#pragma unroll 1
+                for (int d = 0; d < RP && of_state == of_state; ++d)
+                  of_state = fmaf(number(record + Q_AT + ((d >> 4) * 2 + (i >> 4)) * UNIT + ((i & 7) * 4 + ((d & 7) >> 1)) * 4 + 2 * ((i >> 3) & 1) + ((d >> 3) & 1), d & 1),
+                                  held[d], of_state);
+              }
               float again = 0.f;
 #pragma unroll 1
               for (int j = 0; j <= i; ++j) {
                 const int q = (j & 7) >> 1, k = j >> 4, h8 = (j >> 3) & 1;
-                float x = 0.f;
-                for (int p = 2; p >= 0; --p) x += term(record[P_AT + eight * UNIT + p * TERM + ((i & 7) * 4 + q) * 4 + 2 * k + h8], j & 1);
-                again = fmaf(x, term(record[V_AT + ((size_t)(col0 / 16 + tile) * 2 + k) * TERM + ((in & 7) * 4 + q) * 4 + (in >> 3) + 2 * h8], j & 1), again);
+                again = fmaf(number(record + P_AT + eight * UNIT + ((i & 7) * 4 + q) * 4 + 2 * k + h8, j & 1),
+                             term(record[V_AT + ((size_t)(col0 / 16 + tile) * 2 + k) * TERM + ((in & 7) * 4 + q) * 4 + (in >> 3) + 2 * h8], j & 1), again);
               }
               y = of_state + again;
             }

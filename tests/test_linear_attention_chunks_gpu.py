@@ -151,3 +151,34 @@ def test_no_further_from_float64_than_token_by_token(tokens, monkeypatch):
         off[which] = [float((x.double() - e).norm() / e.norm()) for x, e in ((out, want), (state.view(heads, dim, vdim), m))]
     # (the distances are sums of millions of roundings and hold to a few hundredths; 0.94 and 0.84 of the other kernels')
     assert off["chunks"][0] <= off["tokens"][0] and off["chunks"][1] <= off["tokens"][1], off
+
+
+@pytest.mark.parametrize("heads", [1, 40])   # a run of columns a block, and two
+def test_read_outs_of_an_infinite_state(heads):
+    """As in the recurrence: a query reads infinity of that channel's sign from the column, and the other columns as they are."""
+    from prefixserve_b200 import ops
+    from prefixserve_b200.ops import library
+    n, dim, vdim = 100, 128, 64
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    dev = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    ctx = types.SimpleNamespace(item_start=dev([0, n]), slots=dev([0]), num_items=1, max_new_tokens=n)
+    held, proj, alpha = rnd(1, heads, dim, vdim), rnd(n, heads * (2 * dim + vdim)).bfloat16(), 0.5 + 0.5 * torch.sigmoid(rnd(n, heads * dim))
+
+    def run(held):
+        state = held.clone().view(1, -1)
+        before = library.launch_counts.copy()
+        out = ops.linear_attention(proj, alpha, state, ctx, heads=heads, dim=dim, vdim=vdim)
+        assert (library.launch_counts - before)["linear_attention_chunks"] == 1
+        return out.view(n, heads, vdim), state.view(heads, dim, vdim)
+
+    clean, state = run(held)
+    held[0, 0, 77, 21], held[0, 0, 3, 40] = float("inf"), float("-inf")
+    out, after = run(held)
+    query = proj[:, : heads * dim].float().view(n, heads, dim)
+    rest = [c for c in range(vdim) if c not in (21, 40)]
+    for channel, column, sign in ((77, 21, 1.0), (3, 40, -1.0)):
+        assert torch.equal(out[:, 0, column], sign * torch.sign(query[:, 0, channel]) * float("inf")) and after[0, channel, column] == sign * float("inf")
+    assert torch.equal(out[:, 0, rest], clean[:, 0, rest]) and torch.equal(out[:, 1:], clean[:, 1:])
+    finite = torch.isfinite(after)
+    assert int((~finite).sum()) == 2 and torch.equal(after[finite], state[finite])

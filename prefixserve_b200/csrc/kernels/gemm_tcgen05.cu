@@ -36,6 +36,8 @@ constexpr int A_BYTES = BM * BK * 2;        // 16 KB
 // gated and 1,024 plain, 208 us with four and 129 with eight (two CTAs a tile both).
 constexpr int store_warps(int hb) { return hb > 0 ? 4 : 8; }
 constexpr int threads(int hb) { return 32 * (2 + store_warps(hb)); }
+// Columns of a tile that are one warp's (as many as loads from tensor memory bring; the last warp's may be fewer).
+__host__ __device__ constexpr int part_columns(int bn, int parts) { return (bn / parts + 31) / 32 * 32; }
 constexpr int TMEM_COLS = 512;              // two accumulator buffers, 256 float32 columns apart
 constexpr int ACC_STRIDE = 256;
 constexpr int MAX_STAGES = 6;
@@ -95,19 +97,21 @@ __device__ __forceinline__ bool mode_is_gated(int mode) { return mode == MODE_GA
 // head (first-half elements, then the ones they are rotated with), so the job of the rotary kernel is done on the sums
 // while they are in registers.  Each value is first rounded to bfloat16, which is what a separate projection would have
 // stored for the rotary kernel to read.  HB > 0: a head is HB blocks of 16 columns and the caller holds the angles of
-// the row's position in registers (cs, sn); HB == 0: any head size, angles fetched block by block.
+// the row's position in registers (cs, sn); HB == 0: any head size, angles fetched block by block, and two warps share the
+// columns.
 template <int BN, int HB>
 __device__ __forceinline__ void rope_store_row(uint32_t taddr, int row, int M, int n0, int N_out, const RopeArgs& rope, int pos,
                                                int page, const float (&cs)[HB > 0 ? HB : 1][8],
-                                               const float (&sn)[HB > 0 ? HB : 1][8]) {
+                                               const float (&sn)[HB > 0 ? HB : 1][8], int part) {
   static_assert(HB % 2 == 0 && BN % (16 * (HB > 0 ? HB : 1)) == 0, "tiles must start at a head's first column");
   constexpr int SPAN = HB > 0 ? 16 * HB : 32;  // columns per round: one head, or one load from tensor memory
+  constexpr int MINE = part_columns(BN, store_warps(HB) / 4);
   const int D = rope.D, q_cols = rope.hq * D, k_cols = rope.hkv * D;
   const int safe = pos < 0 ? 0 : (pos >= rope.max_positions ? rope.max_positions - 1 : pos);
   const bool page_ok = page >= 0 && page < rope.num_pages;  // the host checks tables before launch; a bad id is skipped
   const size_t in_page = (size_t)(pos & ((1 << rope.page_shift) - 1)) * D;
 #pragma unroll 1
-  for (int c0 = 0; c0 < BN; c0 += SPAN) {
+  for (int c0 = part * MINE; c0 < BN && c0 < (part + 1) * MINE; c0 += SPAN) {
 #pragma unroll
     for (int cc = 0; cc < SPAN; cc += 32) {
       uint32_t v[32];
@@ -227,7 +231,7 @@ struct Epilogue {
                                         const RopeArgs& rope, const GluArgs& glu, const float* __restrict__ row_scale, int part) const {
     __nv_bfloat16* crow = C + (size_t)row * ldc;
     if (mode == MODE_ROPE) {
-      rope_store_row<BN, HB>(taddr, row, M, n0, N_out, rope, pos, page, cs, sn);
+      rope_store_row<BN, HB>(taddr, row, M, n0, N_out, rope, pos, page, cs, sn, part);
     } else if (gated) {
       // the activation is chosen once a tile, not once a number
       const float rs = mode == MODE_GATED_SCALED && row < M ? row_scale[row] : 1.f;
@@ -241,9 +245,9 @@ struct Epilogue {
       });
       else gate([](float g, float u) { return gate_act(g, PSB_ACT_GELU_TANH) * u; });
     } else {
-      constexpr int SPAN = (BN / PARTS + 31) / 32 * 32;
+      constexpr int MINE = part_columns(BN, PARTS);
 #pragma unroll 1
-      for (int c = part * SPAN; c < BN && c < (part + 1) * SPAN; c += 32) {
+      for (int c = part * MINE; c < BN && c < (part + 1) * MINE; c += 32) {
         uint32_t v[32];
         tmem_ld32(taddr + c, v);  // (a tile of 240 columns: the last load reads 16 columns beyond it, which nobody stores)
         tmem_ld_wait();

@@ -678,14 +678,27 @@ int choose_width(int M, int N_out, bool gated, bool rope, int D, int sms) {
 // Whether two CTAs a tile get the product done sooner, by rounds: theirs of 256 x 256 takes about six sevenths of a single CTA's of 128 x 256 (the same work
 // an SM), the narrower tiles' as in choose_width.  Columns by K, rows, two CTAs against the best single width in us: 4,096 by 14,336, 1,979 rows 152 and
 // 176, 1,024 82 and 96, 700 (one round of 192 columns) 81 and 77; 2,048 by 8,192, 1,979 rows 53 and 61; 6,144 by 4,096, 1,979 rows 74 and 83;
-// 3,072 by 2,048, 1,979 rows (two rounds of 192) 35 and 30; gated 14,336 by 4,096, 1,024 rows 158 and 174.  Grouped products always: their rounds
-// depend on the routing, and pairs read an expert's matrix fewer times.
-bool pairs_pay(int M, int N_out, bool gated, int D, int bn, bool grouped, int sms) {
-  if (g_forced_width) return g_forced_width == 512;
+// 3,072 by 2,048, 1,979 rows (two rounds of 192) 35 and 30; gated 14,336 by 4,096, 1,024 rows 158 and 174.
+//
+// Grouped products (``experts`` > 0; the rows hold up to 127 of nobody an expert): rounds depend on the routing, which is not known here, so for rows dealt out
+// evenly.  A pair's tile reads half of the matrix a single one's does, but an expert's only (or odd last) row tile keeps just one of its CTAs busy; what a
+// tile costs beside its K, in columns, was fitted to experts, width by columns of the first product (with 4 to 256 rows an expert on average), us in pairs
+// and single: 32 of 2,048 by 2,048, 8 rows 76 and 70, 48 rows 76 and 81, 256 rows 84 and 116, their second product (K 1,024) 47 and 43, 48 and 49, 55 and 66;
+// 8 of them, 32 rows 31 and 27; 64 of 1,536, 8 rows 104 and 102, 64 rows 104 and 113; 128 of 1,536, 4 rows 173 and 205; 32 of 4,096 by 4,096, 8 rows 215
+// and 217, 64 rows 215 and 245.  Short contractions are bounded by the stores of their tiles, of which a pair of CTAs does half as many at once: 64 experts of
+// 512 by 1,024, 8 rows 39 and 29, 256 rows 51 and 44.
+bool pairs_pay(int M, int N_out, int K, bool gated, int bn, int experts, int sms) {
   if (sms < 2 || (M + BM - 1) / BM > MAX_UNITS) return false;
-  if (grouped) return true;
-  const long m_blocks = (M + BM - 1) / BM, span = gated ? bn / 2 : bn, span2 = gated ? 128 : 256;
-  const long rounds = (m_blocks * ((N_out + span - 1) / span) + sms - 1) / sms, rounds2 = ((m_blocks + 1) / 2 * ((N_out + span2 - 1) / span2) + sms / 2 - 1) / (sms / 2);
+  if (g_forced_width) return g_forced_width == 512;
+  const long m_blocks = (M + BM - 1) / BM, span = gated ? bn / 2 : bn, span2 = gated ? 128 : 256, n_blocks = (N_out + span2 - 1) / span2;
+  const long rounds = (m_blocks * ((N_out + span - 1) / span) + sms - 1) / sms;
+  if (experts > 0) {
+    if (K < 768) return false;
+    const long rows = std::max(1L, (long)M - 127L * experts), units = std::min(rows, std::max((long)experts, (rows + 255) / 256 + experts / 2));
+    const long rounds2 = (units * n_blocks + sms / 2 - 1) / (sms / 2);
+    return (10 * rounds2 + 11) * (115 + 36000 / K) <= 10 * rounds * (bn + 24);
+  }
+  const long rounds2 = ((m_blocks + 1) / 2 * n_blocks + sms / 2 - 1) / (sms / 2);
   return rounds2 * (256 + 24) * 6 <= rounds * (bn + 24) * 7;
 }
 
@@ -740,11 +753,12 @@ int launch(const void* a, const void* w, void* c, int M, int w_rows, int N_out, 
   if (ldc < N_out) PSB_REFUSE("gemm_tcgen05: output rows %d numbers apart do not hold %d", ldc, N_out);
   if (M < 1 || N_out < 1 || K < 8 || K % 8) PSB_REFUSE("gemm_tcgen05: needs K a multiple of 8 (M=%d N=%d K=%d)", M, N_out, K);
   if (((uintptr_t)a | (uintptr_t)w | (uintptr_t)c) & 15) PSB_REFUSE("gemm_tcgen05: operands must be 16-byte aligned");
+  const int experts = tile_expert ? w_rows / (gated ? 2 * N_out : N_out) : 0;
   const int m_blocks = (M + BM - 1) / BM;
   const int bn = choose_width(M, N_out, gated, mode == MODE_ROPE, rope.D, sms);
   CUtensorMap map_a, map_w;
   if (int rc = make_map(&map_a, a, M, K, BM)) return rc;
-  if (pairs_pay(M, N_out, gated, mode == MODE_ROPE ? rope.D : 0, bn, tile_expert != nullptr, sms)) {
+  if (pairs_pay(M, N_out, K, gated, bn, experts, sms)) {
     if (int rc = make_map(&map_w, w, w_rows, K, 128)) return rc;
     const int span = gated ? 128 : 256, most = (tile_expert ? m_blocks : (m_blocks + 1) / 2) * ((N_out + span - 1) / span);
     if (mode == MODE_ROPE && rope.D == 128) return launch_pairs<8>(most, sms, stream, map_a, map_w, c, M, N_out, K, ldc, up_offset, mode, rope, tile_expert, glu, row_scale);
@@ -868,6 +882,12 @@ PSB_API int psb_gemm_tcgen05_tile_width(int width) {
   if (width != 0 && width != 128 && width != 192 && width != 240 && width != 256 && width != 512) PSB_REFUSE("gemm_tcgen05: tile widths are 128, 192, 240, 256 and 512, not %d", width);
   g_forced_width = width;
   return 0;
+}
+
+// (M, N, K, experts, gated, sms) -> 1 if the product goes two CTAs a tile (experts 0: not grouped; N: columns of the result; not for the rotating one)
+PSB_API int psb_gemm_tcgen05_pairs(int M, int N_out, int K, int experts, int gated, int sms) {
+  if (M < 1 || N_out < 1 || K < 8 || experts < 0 || sms < 1) return 0;
+  return pairs_pay(M, N_out, K, gated != 0, choose_width(M, N_out, gated != 0, false, 0, sms), experts, sms) ? 1 : 0;
 }
 
 // How many output tiles the kernel would cut a product into (kind: 0 plain [M, N], 1 gated [M, N] from 2N rows, 2 the

@@ -93,6 +93,8 @@ _SIGNATURES: dict[str, list] = {
     "psb_gemm_tcgen05_tile_width": [I],
     # (M, N_out, kind, D, sms) -> output tiles at the width the kernel would choose
     "psb_gemm_tcgen05_tiles": [I, I, I, I, I],
+    # (M, N, K, experts, gated, sms) -> 1 if the product goes two CTAs a tile (experts 0: not grouped)
+    "psb_gemm_tcgen05_pairs": [I, I, I, I, I, I],
     "psb_gemm_tcgen05_rope": [P, P, I, I, I, P, P, P, I, P, P, P, P, I, I, I, I, I, I, P],
     # () -> 0 while no bounded wait of the tcgen05 kernel has ever run out
     "psb_tcgen05_status": [],

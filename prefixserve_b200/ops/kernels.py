@@ -1547,13 +1547,14 @@ CHANNEL_DELTA_CHUNKED = 24     # ... with longer keys the form that works 16 tok
 CHANNEL_DELTA_LONG_LANES = 16  # ... or, with keys of more than 256 numbers, this many lanes a column instead of 4
 
 
-def _channel_delta_apart(ctx, blocks: int) -> bool:
+def _channel_delta_apart(ctx, blocks: int, sms: int) -> bool:
     """Whether portions below CHANNEL_DELTA_LEAST tokens go token by token beside longer ones in chunks: each of them would be ``blocks``
-    blocks of the chain that fill an SM and have next to nothing to do.  Single tokens beside 64 and beside 512 tokens, us apart and together
-    (64 blocks each): 4 of them 72 and 50, 109 and 104; 8 74 and 63, 115 and 120; 16 90 and 106, 121 and 136; 64 121 and 253, 156 and 280."""
+    blocks of the chain (of 32 columns of a head; where so many leave SMs empty it takes twice as many of 16) that fill an SM and have next to nothing to do.
+    Where the host does not hold the requests all but one are taken to be short.  Single tokens beside 64 and beside 512 tokens, us apart and together
+    (64 blocks each, 148 SMs): 4 of them 72 and 50, 109 and 104; 8 74 and 63, 115 and 120; 16 90 and 106, 121 and 136; 64 121 and 253, 156 and 280."""
     lengths = _portion_lengths(ctx)
     count = ctx.num_items - 1 if lengths is None else sum(n < CHANNEL_DELTA_LEAST for n in lengths)
-    return count * blocks > 5 * 148
+    return count * blocks > 5 * sms
 
 
 def channel_delta_rule(proj: torch.Tensor, beta_at: int, decay: torch.Tensor, taps: torch.Tensor, state: torch.Tensor, ctx, *,
@@ -1576,12 +1577,13 @@ def channel_delta_rule(proj: torch.Tensor, beta_at: int, decay: torch.Tensor, ta
     bd = torch.empty((t, 5 * heads), dtype=torch.float32, device=dev)
     item_start, slots = _i32(ctx.item_start, "item offsets"), _i32(ctx.slots, "slots")
     code, ld = _code(proj, "projection output"), proj.shape[1]
+    from .tensorcore import _sms
     record = tokens = least = 0   # of a chunk: numbers, tokens; portions of at least ``least`` tokens go in chunks
     narrow = dim <= 128
     if ctx.max_new_tokens >= (CHANNEL_DELTA_LEAST if narrow else CHANNEL_DELTA_CHUNKED):
         record = int((lib().psb_channel_delta_chunk_record if narrow else lib().psb_channel_delta_record)(dim, vdim))
         tokens = lib().psb_delta_chunk_tokens() if narrow else 16
-        least = CHANNEL_DELTA_LEAST if narrow and _channel_delta_apart(ctx, heads * -(-vdim // 32)) else 1
+        least = CHANNEL_DELTA_LEAST if narrow and _channel_delta_apart(ctx, heads * -(-vdim // 32), _sms(dev)) else 1
     short = not record or (least > 1 and _has_portions_below(ctx, least))
     check(lib().psb_delta_prepare(proj.data_ptr(), code, ld, beta_at, None, decay.data_ptr() if short else None, taps.data_ptr(), None, None,
                                   state.data_ptr(), _i32(ctx.positions, "positions").data_ptr(),

@@ -42,3 +42,10 @@ def test_linear_attention_steps_that_go_token_by_token(lengths, alone):
 
 def test_portions_counted():
     assert kernels._portions_from(context([8, 7, 33], "held"), 8) == 2 and kernels._portions_from(context([8, 7, 33], "empty"), 8) == 3
+
+
+@pytest.mark.parametrize("sms, short, apart", [(148, 11, False), (148, 12, True), (132, 10, False), (132, 11, True), (16, 1, False), (16, 2, True)])
+def test_short_portions_beside_chunks_of_the_channel_rule(sms, short, apart):
+    """By the SMs of the device that runs them (64 blocks a portion)."""
+    assert kernels._channel_delta_apart(context([64] + [1] * short, "held"), 64, sms) == apart
+    assert kernels._channel_delta_apart(context([64] + [1] * short, "none"), 64, sms) == apart

@@ -62,9 +62,10 @@ linear_chunk_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const 
   float(*ps)[TP] = reinterpret_cast<float(*)[TP]>(chunk_smem + Sh::PS);
   pdl_wait();
   int t0, n;
-  if (!portions::find_chunk<CHUNK>(item_start, items, min_tokens, blockIdx.y, t0, n)) return;
-  const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, tg = lane & 3;
-  float* out = records + ((size_t)blockIdx.y * H + h) * record_floats(vdim);
+  const int h = blockIdx.x % H, chunk = blockIdx.x / H;
+  if (!portions::find_chunk<CHUNK>(item_start, items, min_tokens, chunk, t0, n)) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, tg = lane & 3;
+  float* out = records + ((size_t)chunk * H + h) * record_floats(vdim);
   const __nv_bfloat16* rows = proj + (size_t)t0 * ld;
   bring_rows(gs, alpha + ((size_t)t0 * H + h) * dim, (long long)H * dim, n, dim, true);  // (0 where there is none: q and k are 0 too)
   widen_rows(qs, rows + (size_t)h * dim, ld, n, dim);
@@ -414,7 +415,7 @@ PSB_API int psb_linear_chunks(const void* proj, long long ld, const void* alpha,
   if (ld < 2LL * H * dim + (long long)H * vdim || ld % 4) PSB_REFUSE("linear_chunks: row stride %lld is shorter than the row or no multiple of 4", ld);
   if (slot_floats < (long long)H * dim * vdim) PSB_REFUSE("linear_chunks: a slot of %lld numbers does not hold the state", slot_floats);
   if (((uintptr_t)proj & 7) || (((uintptr_t)alpha | (uintptr_t)records) & 15)) PSB_REFUSE("linear_chunks: operands are not aligned");
-  if (H > 65535 || chunks > 65535 || portions > 65535) PSB_REFUSE("linear_chunks: too many heads, requests or chunks for one launch");
+  if (H > 65535 || portions > 65535 || (long long)chunks * H > 0x7fffffffLL) PSB_REFUSE("linear_chunks: too many heads, requests or chunks for one launch");
   if (items == 0 || portions < 1 || chunks < 1) return 0;
   constexpr int bytes = ChunkShape::FLOATS * (int)sizeof(float);
   static PsbPerDevice configured;
@@ -422,7 +423,7 @@ PSB_API int psb_linear_chunks(const void* proj, long long ld, const void* alpha,
     if (cudaFuncSetAttribute(linear_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) PSB_REFUSE("linear_chunks: cannot raise the shared-memory limit");
     configured.set();
   }
-  psb_launch(linear_chunk_kernel, dim3(H, chunks), dim3(CHUNK_THREADS), (size_t)bytes, stream, (const __nv_bfloat16*)proj, ld, (const float*)alpha,
+  psb_launch(linear_chunk_kernel, dim3((unsigned)chunks * H), dim3(CHUNK_THREADS), (size_t)bytes, stream, (const __nv_bfloat16*)proj, ld, (const float*)alpha,
              (const int32_t*)item_start, (float*)records, items, min_tokens, H, dim, vdim);
   PSB_LAUNCH_CHECK("linear_chunk");
   // runs of columns a block takes: as for the delta rules' chain (delta_chunks.cu)

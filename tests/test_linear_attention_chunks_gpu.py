@@ -182,3 +182,21 @@ def test_read_outs_of_an_infinite_state(heads):
     assert torch.equal(out[:, 0, rest], clean[:, 0, rest]) and torch.equal(out[:, 1:], clean[:, 1:])
     finite = torch.isfinite(after)
     assert int((~finite).sum()) == 2 and torch.equal(after[finite], state[finite])
+
+
+def test_more_chunks_than_a_grid_has_rows():
+    """A portion of more than 65,535 chunks, against the same tokens in two portions, one after the other."""
+    from prefixserve_b200 import ops
+    n, first, dim, vdim = 32 * 65536 + 1, 32 * 40000, 4, 4
+    g = torch.Generator(device="cuda").manual_seed(6)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    held, proj, alpha = rnd(1, dim * vdim), rnd(n, 2 * dim + vdim).bfloat16(), torch.sigmoid(rnd(n, dim)) ** 0.25
+
+    def run(state, a, b):
+        dev = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+        ctx = types.SimpleNamespace(item_start=dev([0, b - a]), slots=dev([0]), num_items=1, max_new_tokens=b - a, items=[types.SimpleNamespace(start=a, end=b)])
+        return ops.linear_attention(proj[a:b], alpha[a:b], state, ctx, heads=1, dim=dim, vdim=vdim)
+
+    whole, parts = held.clone(), held.clone()
+    out = run(whole, 0, n)
+    assert torch.equal(out, torch.cat([run(parts, 0, first), run(parts, first, n)])) and torch.equal(whole, parts)

@@ -149,3 +149,71 @@ def test_a_token_that_is_not_finite_reaches_later_tokens_only(what):
     assert not torch.isfinite(out[bad, :hit]).all(-1).any() and torch.isfinite(state[0]).all() and torch.isfinite(state[1, hit:]).all()
     if what != "query":
         assert not torch.isfinite(out[99, :hit]).all(-1).any() and not torch.isfinite(state[1, :hit].flatten(1)).all(1).any()
+
+
+# Two runs of columns a block (as above), and one.  Read-outs and states lie 0.6e-7 to 2.1e-7 from float64 (norm of the difference over norm), with what is in front
+# of the rule; numbers in two terms instead of three would be off by some 2^-18 = 4e-6.
+CLOSE = 4e-7
+
+
+def off(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("heads, vdim", [(20, 64), (4, 64)])
+def test_distance_from_float64_decay_per_channel(heads, vdim):
+    case = Channel([300, 33, 64], 2, heads, 128, vdim, torch.bfloat16, heads)
+    (out, state), (want, held) = case.run(), case.exact()
+    assert off(out, want) <= CLOSE and off(state, held) <= CLOSE
+
+
+@pytest.mark.parametrize("heads, vdim", [(20, 64), (4, 64)])
+def test_distance_from_float64_decay_per_head(heads, vdim):
+    """Read-outs as the chain leaves them, and states, from the same unit vectors, strengths and decays."""
+    from prefixserve_b200.ops import kernels
+    lib, groups, dim, lengths = kernels.lib(), 2, 128, [300, 33, 64]
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    (ctx, offsets), t, c = step(lengths), sum(lengths), 2 * groups * dim + heads * vdim
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)
+    qkv = torch.cat([unit(rnd(t, 2 * groups, dim)).flatten(1), rnd(t, heads * vdim)], 1)
+    bd = torch.cat([torch.rand(t, 2 * heads, generator=g, device="cuda"), rnd(t, 3 * heads)], 1)
+    bd[:, heads: 2 * heads] **= 0.1
+    proj, held, o = rnd(t, c).bfloat16(), 0.3 * rnd(3, heads * dim * vdim), torch.empty(t, heads, vdim, device="cuda")
+    state, chunks = held.clone(), sum(-(-n // 32) for n in lengths)
+    records = torch.empty(chunks, heads, lib.psb_delta_chunk_record(dim, vdim), device="cuda")
+    kernels.check(lib.psb_delta_chunks(qkv.data_ptr(), bd.data_ptr(), proj.data_ptr(), c, state.data_ptr(), ctx.item_start.data_ptr(), ctx.slots.data_ptr(),
+                                       records.data_ptr(), o.data_ptr(), 3, 3, chunks, 1, groups, heads, dim, vdim, 1, 3, held.shape[1], kernels._stream()), "delta_chunks")
+    q, k = (qkv[:, a: a + groups * dim].double().view(t, groups, dim).repeat_interleave(heads // groups, 1) for a in (0, groups * dim))
+    v, beta, decay = qkv[:, 2 * groups * dim:].double().view(t, heads, vdim), bd[:, :heads].double(), bd[:, heads: 2 * heads].double()
+    want, after = [], torch.empty_like(held, dtype=torch.float64)
+    for i, n in enumerate(lengths):
+        m = held[2 - i].double().view(heads, dim, vdim)
+        for j in range(offsets[i], offsets[i] + n):
+            m = m * decay[j, :, None, None]
+            m = m + k[j, :, :, None] * (beta[j, :, None] * (v[j] - torch.einsum("hd,hdv->hv", k[j], m)))[:, None]
+            want.append(torch.einsum("hd,hdv->hv", q[j], m))
+        after[2 - i] = m.reshape(-1)
+    assert off(o, torch.stack(want)) <= CLOSE and off(state, after) <= CLOSE
+
+
+@pytest.mark.parametrize("heads, vdim", [(20, 64), (4, 64)])
+def test_distance_from_float64_linear_attention(heads, vdim):
+    from prefixserve_b200 import ops
+    dim, lengths = 128, [300, 33, 64]
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    (ctx, offsets), t = step(lengths), sum(lengths)
+    proj, alpha, held = rnd(t, heads * (2 * dim + vdim)).bfloat16(), torch.sigmoid(rnd(t, heads * dim)) ** (1 / 16), rnd(3, heads * dim * vdim)
+    state = held.clone()
+    out = ops.linear_attention(proj, alpha, state, ctx, heads=heads, dim=dim, vdim=vdim).view(t, heads, vdim)
+    p, a = proj.double(), alpha.double().view(t, heads, dim, 1)
+    q, k, v = p[:, : heads * dim].view(t, heads, dim), p[:, heads * dim: 2 * heads * dim].view(t, heads, dim), p[:, 2 * heads * dim:].view(t, heads, vdim)
+    want, after = [], torch.empty_like(held, dtype=torch.float64)
+    for i, n in enumerate(lengths):
+        m = held[2 - i].double().view(heads, dim, vdim)
+        for j in range(offsets[i], offsets[i] + n):
+            m = a[j] * m + k[j, :, :, None] * v[j, :, None]
+            want.append(torch.einsum("hd,hdv->hv", q[j], m) * dim ** -0.5)
+        after[2 - i] = m.reshape(-1)
+    assert off(out, torch.stack(want)) <= CLOSE and off(state, after) <= CLOSE

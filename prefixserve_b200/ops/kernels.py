@@ -1411,19 +1411,19 @@ def low_rank(a: torch.Tensor, w: torch.Tensor, function: str, *, bias: torch.Ten
 # portions into chunks that go token by token side by side.
 LINEAR_CHUNKED, LINEAR_SHORT = 48, 32
 LINEAR_ATTENTION_CHUNK = 64
-LINEAR_MIXED = 96
 
 
-def _linear_one_by_one(lengths: list[int] | None) -> bool:
+def _linear_one_by_one(lengths: list[int] | None, heads: int = 16) -> bool:
     """Whether a step that could go either way whole has so much in short portions, which the two forms take one after the other, that all
-    of it is over sooner token by token (16 heads, both forms and token by token: 48 tokens beside 32 single ones 48 and 39 us, 64 beside eight of
-    16 tokens 42 and 39, 64 beside one of 31 38 and 35, 64 beside a single one 28 and 34; 100 beside eight single ones 34 and 51.  From 96
-    tokens on the chunks are ahead a little beyond the line, 96 beside one of 31 40 and 47, 100 beside 32 51 and 60, which is kept where
-    longer chunks had it)."""
+    of it is over sooner token by token: the more and the longer they are, and the shorter the longest one is, whose tokens that form takes one behind
+    the other.  Both forms and token by token, us, 16 heads: 48 tokens beside one of 16 34 and 29; 64 beside eight single ones 34 and 37, beside 32
+    52 and 45, beside eight of 16 tokens 42 and 39; 100 beside 32 50 and 59 (eight heads 38 and 53), 96 beside one of 31 40 and 47, beside 48 single ones
+    64 and 61, beside 20 of 31 75 and 64; 128 beside 20 of 16 58 and 72, beside 64 single ones 83 and 78 (eight heads: 54 and 70).  Over 276 such
+    steps of 8 and 16 heads the line loses 15 % at the most (64 tokens beside one of 31, 40 and 35) and 0.4 % in all."""
     short = [n for n in lengths or [] if n < LINEAR_SHORT]
     if not short or max(lengths) > 2 * LINEAR_ATTENTION_CHUNK:
         return False
-    return len(short) > (8 if max(lengths) < LINEAR_MIXED else 16) or max(short) > 8
+    return len(short) * (12 + max(short)) * heads > 160 * (max(lengths) - LINEAR_CHUNKED)
 
 
 def linear_attention(proj: torch.Tensor, alpha: torch.Tensor, state: torch.Tensor, ctx, *, heads: int, dim: int, vdim: int) -> torch.Tensor:
@@ -1443,7 +1443,7 @@ def linear_attention(proj: torch.Tensor, alpha: torch.Tensor, state: torch.Tenso
     most = 0x7fffffff  # tokens of the longest portion left to the kernels that go token by token
     if (ctx.max_new_tokens >= LINEAR_CHUNKED and proj.dtype == torch.bfloat16 and ld % 4 == 0 and stride % 4 == 0
             and proj.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0 and alpha.data_ptr() % 16 == 0
-            and (record := int(lib().psb_linear_chunk_record(dim, vdim))) and not _linear_one_by_one(_portion_lengths(ctx))):
+            and (record := int(lib().psb_linear_chunk_record(dim, vdim))) and not _linear_one_by_one(_portion_lengths(ctx), heads)):
         most = LINEAR_SHORT - 1
         portions, chunks = _portions_from(ctx, LINEAR_SHORT), _portion_tiles(ctx, t, LINEAR_SHORT, lib().psb_linear_chunk_tokens())
         records = torch.empty((chunks, heads, record), dtype=torch.float32, device=dev)

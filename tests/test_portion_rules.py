@@ -34,10 +34,17 @@ def test_delta_steps_that_go_token_by_token(lengths, alone):
     assert kernels._delta_one_by_one(lengths) == alone and not kernels._delta_one_by_one(None)
 
 
-@pytest.mark.parametrize("lengths, alone", [([128], False), ([100] + [1] * 16, False), ([100] + [1] * 17, True), ([129] + [1] * 200, False), ([96] + [32] * 20, False),
-                                            ([96, 8], False), ([96, 9], True), ([129, 31], False)])
+@pytest.mark.parametrize("lengths, alone", [([128], False), ([100] + [1] * 16, False), ([100] + [1] * 17, False), ([100] + [1] * 64, True), ([129] + [1] * 200, False), ([96] + [32] * 20, False),
+                                            ([96, 8], False), ([96, 9], False), ([96] + [31] * 12, True), ([64] + [1] * 8, False), ([64] + [1] * 32, True),
+                                            ([48, 16], True), ([129, 31], False)])
 def test_linear_attention_steps_that_go_token_by_token(lengths, alone):
+    """16 heads; us in chunks and token by token: [100] + [1] * 17 38 and 55, [96, 9] 32 and 47 (both were left token by token by chunks of 64 tokens, which
+    were slower there)."""
     assert kernels._linear_one_by_one(lengths) == alone and not kernels._linear_one_by_one(None)
+
+
+def test_linear_attention_steps_of_fewer_heads():
+    assert kernels._linear_one_by_one([100] + [1] * 64, 16) and not kernels._linear_one_by_one([100] + [1] * 64, 8)
 
 
 def test_portions_counted():

@@ -8,8 +8,8 @@
 //     O = (Q c) S + B U,     B_ij = sum_d q_i k_j g_(j+1) .. g_i   (j <= i),
 //     S <- c_32 S + (K r)^T U.
 //
-// (Decays are only ever multiplied, never divided by, and their running products carry what the roundings lose.)  All but the products
-// with S and U is made beforehand:
+// (Decays are only ever multiplied, never divided by, and their running products carry what the roundings lose, but for A and B within sixteen
+// tokens where the decays are per channel: plain float32, up to fifteen factors.)  All but the products with S and U is made beforehand:
 //   delta_chunk_kernel, channel_delta_chunk_kernel   a block per chunk and head, all chunks of the step side by side: A, B and W (forward
 //                        substitution, a column a lane), then M, Q c, K r, B, c_32 and W V, 98 KB a chunk and head;
 //   delta_chain_kernel   a block per 16 or 32 columns of a head's state and request walks the chunks, on the tensor cores.  Eight warps hold

@@ -737,9 +737,9 @@ channel_delta_rule_kernel(const float* __restrict__ qkv, const float* __restrict
   if (blockIdx.x == 0 && h == 0) keep_conv_inputs<T>(proj, P, base, t0, t1, C, K);
 }
 
-// The same rule for long portions and keys of 129 to 256 numbers, sixteen tokens at a time (shorter keys: delta_chunks.cu).  Within a chunk, with c_i = g_1 ... g_i (the decays from the
-// chunk's start up to token i, each a product of numbers of at most one, nothing is ever divided by a decay) and S the state
-// before the chunk,
+// The same rule for long portions and keys of 129 to 256 numbers, sixteen tokens at a time (shorter keys: delta_chunks.cu).
+// Within a chunk, with c_i = g_1 ... g_i (the decays from the chunk's start up to token i, each a product of numbers of at most
+// one, nothing is ever divided by a decay) and S the state before the chunk,
 //
 //     A_ij = sum_d k_i k_j g_(j+1) .. g_i   (j < i),      B_ij = the same with q_i   (j <= i),
 //     (I + diag(beta) A) U = diag(beta) (V - (k c) S),    O = (q c) S + B U,    S <- c_16 S + sum_j (k_j g_(j+1) .. g_16) u_j^T.
@@ -752,10 +752,10 @@ channel_delta_rule_kernel(const float* __restrict__ qkv, const float* __restrict
 // 32 products with S, then U, O and the new S.  A chain step costs sixteen tokens one such round instead of sixteen.
 // Chunks are counted through the step's items in order; a portion's last chunk is filled up with tokens of beta 0, key 0
 // and decay 1.
-constexpr int CH = 16, B_PITCH = 20, CHAIN_COLS = 16;
+constexpr int CH = 16, B_PITCH = 20, CHAIN_COLS = 16, LR = 8, RP = 32 * LR;  // LR rows of S a lane, RP of them in all
 
 struct ChunkRecord {
-  int RP, vpad;
+  int vpad;
   __host__ __device__ int b_at() const { return (3 * CH + 1) * RP; }
   __host__ __device__ int wv_at() const { return b_at() + CH * B_PITCH; }
   __host__ __device__ int floats() const { return wv_at() + CH * vpad; }
@@ -789,13 +789,10 @@ __device__ __forceinline__ float reduce32(float (&v)[32], int lane) {
   return v[0];
 }
 
-// LR rows of S a lane: RP = 32 * LR >= dim.
-template <int LR>
 __global__ void __launch_bounds__(128)
 channel_delta_chunk_kernel(const float* __restrict__ qkv, const float* __restrict__ bd, const float* __restrict__ decay,
                            const int32_t* __restrict__ item_start, float* __restrict__ records, int items, int G, int H, int dim,
                            int vdim, int vpad) {
-  constexpr int RP = 32 * LR;
   extern __shared__ __align__(16) float chunk_smem[];  // k, q, g: [CH][RP] each
   __shared__ float As[CH][CH + 1], Ws[CH][CH + 1], beta[CH];
   float *ks = chunk_smem, *qs = ks + CH * RP, *gs = qs + CH * RP;
@@ -804,7 +801,7 @@ channel_delta_chunk_kernel(const float* __restrict__ qkv, const float* __restric
   if (!find_delta_chunk(item_start, items, blockIdx.x, t0, n)) return;
   const int h = blockIdx.y, g = h / (H / G);
   const int C = 2 * G * dim + H * vdim;
-  const ChunkRecord rec{RP, vpad};
+  const ChunkRecord rec{vpad};
   float* out = records + ((size_t)blockIdx.x * H + h) * rec.floats();
   for (int i = threadIdx.x; i < CH * RP; i += blockDim.x) {
     const int t = i / RP, d = i - t * RP;
@@ -899,9 +896,8 @@ struct Four {
 
 // The four columns' sums of vectors BASE .. BASE + N - 1 (rows of RP numbers at ``rows``) with the lane's rows of S, brought
 // together over the warp so that the lane whose low bits are r holds vector BASE + r's.
-template <int LR, int N, int BASE>
+template <int N, int BASE>
 __device__ __forceinline__ Four chain_products(const float* __restrict__ rows, const float (&s)[4][LR], int lane) {
-  constexpr int RP = 32 * LR;
   Four out;
   if constexpr (N == 1) {
 #pragma unroll
@@ -914,7 +910,7 @@ __device__ __forceinline__ Four chain_products(const float* __restrict__ rows, c
         out.v[j] = fmaf(m.w, s[j][e + 3], fmaf(m.z, s[j][e + 2], fmaf(m.y, s[j][e + 1], fmaf(m.x, s[j][e], out.v[j]))));
     }
   } else {
-    const Four a = chain_products<LR, N / 2, BASE>(rows, s, lane), b = chain_products<LR, N / 2, BASE + N / 2>(rows, s, lane);
+    const Four a = chain_products<N / 2, BASE>(rows, s, lane), b = chain_products<N / 2, BASE + N / 2>(rows, s, lane);
     const bool up = lane & (N / 2);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -926,13 +922,12 @@ __device__ __forceinline__ Four chain_products(const float* __restrict__ rows, c
 }
 
 // A block: 16 columns of a request's and head's state, four a warp; lane's rows of S: e / 4 * 128 + lane * 4 + e % 4.
-template <typename T, int LR>
+template <typename T>
 __global__ void __launch_bounds__(RULE_WARPS * 32)
 channel_delta_chain_kernel(const float* __restrict__ records, const T* __restrict__ proj, long long P, float* __restrict__ state,
                            const int32_t* __restrict__ item_start, const int32_t* __restrict__ slots, float* __restrict__ o, int G,
                            int H, int dim, int vdim, int vpad, int K, int num_slots, long long slot_floats) {
-  constexpr int RP = 32 * LR;
-  const ChunkRecord rec{RP, vpad};
+  const ChunkRecord rec{vpad};
   constexpr int HEAD = (3 * CH + 1) * RP + CH * B_PITCH, BUF = HEAD + CH * CHAIN_COLS;  // floats: the record up to B, then W V's columns
   extern __shared__ __align__(16) float chain_smem[];  // [2][BUF]
   __shared__ __align__(16) float us[RULE_WARPS][CH][4];
@@ -972,7 +967,7 @@ channel_delta_chain_kernel(const float* __restrict__ records, const T* __restric
     __syncthreads();  // this chunk has landed for everybody, and everybody has left the other buffer
     if (c + 1 < chunks) stage(c + 1, chain_smem + ((c + 1) & 1) * BUF);
     const float* buf = chain_smem + (c & 1) * BUF;
-    const Four y = chain_products<LR, 32, 0>(buf, s, lane);
+    const Four y = chain_products<32, 0>(buf, s, lane);
     if (lane < CH) {
       const float4 wv = *reinterpret_cast<const float4*>(buf + HEAD + lane * CHAIN_COLS + warp * 4);
       *reinterpret_cast<float4*>(us[warp][lane]) = make_float4(wv.x - y.v[0], wv.y - y.v[1], wv.z - y.v[2], wv.w - y.v[3]);
@@ -1280,7 +1275,7 @@ PSB_API int psb_channel_delta_rule(const void* qkv, const void* bd, const void* 
 // the kernels of delta_chunks.cu)
 PSB_API int psb_channel_delta_record(int dim, int vdim) {
   if (dim <= 128 || vdim < 1 || dim > 256 || vdim > 4096) return 0;
-  return ChunkRecord{256, (vdim + CHAIN_COLS - 1) / CHAIN_COLS * CHAIN_COLS}.floats();
+  return ChunkRecord{(vdim + CHAIN_COLS - 1) / CHAIN_COLS * CHAIN_COLS}.floats();
 }
 
 // The chunked form: (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, records, o_out, items, chunks, G, H, dim, vdim, K,
@@ -1297,12 +1292,11 @@ PSB_API int psb_channel_delta_chunks(const void* qkv, const void* bd, const void
   if (((uintptr_t)records | (uintptr_t)o) & 15) PSB_REFUSE("channel_delta_chunks: records and read-out must be 16-byte aligned");
   if (items == 0) return 0;
   const int vpad = (vdim + CHAIN_COLS - 1) / CHAIN_COLS * CHAIN_COLS;
-constexpr int LR = 8, RP = 32 * LR;
   constexpr int chunk_bytes = 3 * CH * RP * (int)sizeof(float);
   constexpr int chain_bytes = 2 * ((3 * CH + 1) * RP + CH * B_PITCH + CH * CHAIN_COLS) * (int)sizeof(float);
   PSB_DISPATCH_DTYPE(dtype, T_, {
-    auto chunk = channel_delta_chunk_kernel<LR>;
-    auto chain = channel_delta_chain_kernel<T_, LR>;
+    auto chunk = channel_delta_chunk_kernel;
+    auto chain = channel_delta_chain_kernel<T_>;
     static PsbPerDevice configured;
     if (!configured.get()) {
       if (cudaFuncSetAttribute(chunk, cudaFuncAttributeMaxDynamicSharedMemorySize, chunk_bytes) != cudaSuccess ||

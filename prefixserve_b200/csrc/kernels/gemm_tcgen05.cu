@@ -19,7 +19,7 @@
 // prefixserve/model/attention.py:105-106 of PrefixServe), so the [T, (hq + 2 hkv) D] matrix never exists either.
 //
 // Rows of A past M, rows of W past N and columns past K are filled with zeros by the TMA unit (K only needs to be a
-// multiple of 8: a 16-byte row pitch).  No cluster, no multicast: every CTA loads its own tiles.
+// multiple of 8: a 16-byte row pitch).  No load is multicast: every CTA brings its own tiles, the two of a pair each its part.
 //
 // Every wait on an mbarrier is bounded.  If one runs out, the CTA raises a flag that all its warps poll, stops
 // issuing work, pauses long enough for copies in flight to land, frees its tensor memory and returns; the host finds
@@ -681,12 +681,12 @@ int choose_width(int M, int N_out, bool gated, bool rope, int D, int sms) {
 // 3,072 by 2,048, 1,979 rows (two rounds of 192) 35 and 30; gated 14,336 by 4,096, 1,024 rows 158 and 174.
 //
 // Grouped products (``experts`` > 0; the rows hold up to 127 of nobody an expert): rounds depend on the routing, which is not known here, so for rows dealt out
-// evenly.  A pair's tile reads half of the matrix a single one's does, but an expert's only (or odd last) row tile keeps just one of its CTAs busy; what a
-// tile costs beside its K, in columns, was fitted to experts, width by columns of the first product (with 4 to 256 rows an expert on average), us in pairs
-// and single: 32 of 2,048 by 2,048, 8 rows 76 and 70, 48 rows 76 and 81, 256 rows 84 and 116, their second product (K 1,024) 47 and 43, 48 and 49, 55 and 66;
-// 8 of them, 32 rows 31 and 27; 64 of 1,536, 8 rows 104 and 102, 64 rows 104 and 113; 128 of 1,536, 4 rows 173 and 205; 32 of 4,096 by 4,096, 8 rows 215
-// and 217, 64 rows 215 and 245.  Short contractions are bounded by the stores of their tiles, of which a pair of CTAs does half as many at once: 64 experts of
-// 512 by 1,024, 8 rows 39 and 29, 256 rows 51 and 44.
+// evenly, half of the experts with an odd last row tile.  A pair brings W in once for 256 rows, but an expert's only (or odd last) row tile keeps just one of
+// its CTAs busy.  What a tile costs beside its K, in columns, was fitted to experts of 4 to 256 rows on average, columns by K, us in pairs and single:
+// 32 of 2,048 by 2,048, 8 rows 76 and 70, 48 rows 76 and 81, 256 rows 84 and 116; 32 of 2,048 by 1,024 47 and 43, 48 and 49, 55 and 66; 8 of 2,048 by 2,048,
+// 32 rows 31 and 27; 64 of 1,536 by 2,048, 8 rows 104 and 102, 64 rows 104 and 113; 128 of them, 4 rows 173 and 205; 32 of 4,096 by 4,096, 8 rows 215 and 217,
+// 64 rows 215 and 245.  Short contractions are bounded by the stores of their tiles, of which pairs do half as many at once: 64 of 1,024 by 512, 8 rows
+// 39 and 29, 256 rows 51 and 44.
 bool pairs_pay(int M, int N_out, int K, bool gated, int bn, int experts, int sms) {
   if (sms < 2 || (M + BM - 1) / BM > MAX_UNITS) return false;
   if (g_forced_width) return g_forced_width == 512;

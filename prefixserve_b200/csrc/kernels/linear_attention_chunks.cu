@@ -15,10 +15,11 @@
 // again from the tokens up to its own, and from the state as it is, whose terms are no sum where it is infinite.
 // A float32 projection's values would need terms too; those stay with the other kernels.
 //
-// Distances from float64, token by token and here (150 and 700 tokens): read-outs 1.2e-7 and 1.03e-7, states 0.95e-7 and 0.59e-7.
+// Distances from float64, token by token and here (150 and 700 tokens): read-outs 1.2e-7 and 1.0e-7, states 0.95e-7 and 0.59e-7.  A decay product between two
+// tokens of the same sixteen is rounded once (in plain float32, 5 us less for the call below, it was up to 3.9 times as far off).
 //
 // What bounds it: the chain, by what a chunk brings from L2 (64 KB an SM and chunk, 1.1 us) and the latency of its steps.  1,811 tokens of 16 heads of 128:
-// chunk kernel 42 us, chain 63; chunks of 64 tokens all side by side, the states they start from in a pass between two kernels, took 31, 11 and 87 us
+// chunk kernel 47 us, chain 64; chunks of 64 tokens all side by side, the states they start from in a pass between two kernels, took 31, 11 and 87 us
 // and were bound by the read-out's phases, one block an SM, in four rounds.  Two chunks ahead through shared memory: no faster.
 #include "chunk_products.cuh"
 

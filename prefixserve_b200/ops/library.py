@@ -222,13 +222,13 @@ _SIGNATURES: dict[str, list] = {
     "psb_delta_chunks": [P, P, P, L, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, L, P],
     # (dim, vdim) -> float32 numbers of a chunk's record, 0 if the chunked form does not take the sizes
     "psb_channel_delta_record": [I, I],
-    # (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, records, o_out, items, chunks, G, H, dim, vdim, K, num_slots,
-    #  slot_floats, stream)
     # (dim, vdim) -> float32 numbers of a 32-token chunk's record, 0: not built
     "psb_channel_delta_chunk_record": [I, I],
     # (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, records, o, items, portions, chunks, min_tokens, G, H, dim, vdim, K,
     #  num_slots, slot_floats, stream)
     "psb_channel_delta_chunks32": [P, P, P, P, I, L, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, L, P],
+    # (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, records, o_out, items, chunks, G, H, dim, vdim, K, num_slots,
+    #  slot_floats, stream)
     "psb_channel_delta_chunks": [P, P, P, P, I, L, P, P, P, P, P, I, I, I, I, I, I, I, I, L, P],
     # (o, proj, dtype, gain, out, T, G, H, dim, vdim, eps, stream)
     "psb_delta_finish": [P, P, I, P, P, I, I, I, I, I, F, P],

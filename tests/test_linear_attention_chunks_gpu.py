@@ -1,4 +1,4 @@
-"""Gated linear attention over long portions, 64 tokens at a time, against the recurrence in float64: portions at and around multiples of
+"""Gated linear attention over long portions, 32 tokens at a time, against the recurrence in float64: portions at and around multiples of
 a chunk and of its runs of 16 tokens beside short ones and single tokens, one after the other from carried states, keys and values of
 fewer numbers than the kernels' tiles, channels that forget everything and channels that forget nothing, rows and slots that are runs of
 wider ones.  (Projections in float32 stay with the kernels that go token by token.)"""

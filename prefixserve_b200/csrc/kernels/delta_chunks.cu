@@ -15,7 +15,7 @@
 //   delta_chain_kernel   a block per 16 or 32 columns of a head's state and request walks the chunks, on the tensor cores.  Eight warps hold
 //                        16 key channels of S each, in registers, as the left operand of the first product and the sums of the second;
 //                        what a chunk brings each asks for a chunk ahead, straight into registers.  [M; Q c] S comes out in eight shares that go through shared
-//                        memory; four more warps make U of M's while the eight multiply Q c, and the read-outs while those bring S up to date.
+//                        memory; eight more warps make U of M's while the first multiply Q c, and the read-outs while those bring S up to date.
 // Operands of the tensor cores are three bfloat16 terms a float32 number, to its last bit: the sums of the six products of terms that count are as
 // accurate as float32's own (the products of first terms are added up in float32 with rounding to nearest, sixteen tokens or channels
 // at a time, since the instruction cuts its sums off; the rest is smaller by 2^8).  M, Q, K and B are taken apart once, where they are made.
@@ -29,11 +29,12 @@
 // and 2.04e-7 and 0.64, 0.80, 0.98, 0.96 and 0.99e-7.  The rule with a decay per channel over 1,200 tokens, whole: read-outs 1.6e-7, states 1.4e-7;
 // sixteen tokens at a time on the CUDA cores, as it was, 2.1e-7 and 1.9e-7.
 //
-// What bounds it: the chain, by the latency of its steps one after the other (a share of [M; Q c] S 1,000 clocks, U 700 beside the other half, the new state
-// 1,000, and two barriers, of which the tensor cores are busy 1,280), and by how soon a chunk's record comes from L2.  2,000 tokens of 16 heads: chunk
-// kernel 44 us, chain 135; products of up to six TF32 terms whose operands every block split for itself 18 and 201.  Two portions of 1,200
-// and 960 tokens with decays per channel: 66 and 125 us; sixteen tokens at a time on the CUDA cores 87 and 211.  Register tiles of fma.rn.f32x2 for
-// the chain: 193 us, bound by what shared memory hands to the registers; two chunks ahead through shared memory: no faster.
+// What bounds it: the chain, by the latency of its steps one after the other (in clocks, a block of 16 columns: a share of [M; Q c] S 900, U 500 beside the other
+// half, the new state 1,000, and two barriers; the tensor cores are busy 1,280 of 3,000).  2,000 tokens of 16 heads: chunk kernel 44 us, chain 110; two portions of
+// 1,200 and 960 tokens with decays per channel 66 and 112.  The chain was 135 and 125 with four warps beside the workers, who then waited for U and for the
+// read-outs (1,750), with W V asked for just before its use, and with records that came from DRAM no more than a chunk ahead; products of up to six TF32 terms
+// whose operands every block split for itself took 201 us, sixteen tokens at a time on the CUDA cores 211, register tiles of fma.rn.f32x2 193, bound by
+// what shared memory hands to the registers; two chunks ahead through shared memory: no faster.
 #include "chunk_products.cuh"
 
 namespace {
@@ -335,8 +336,18 @@ struct Chain {
 };
 
 
+// Eight warps beside the workers make U, two columns of every 16 each, and the read-outs, eight tokens of 16 columns each.  A block is launched with 128 registers
+// a thread; who gets how many of them, us for 2,000 tokens (16 columns a block) and for portions of 1,200 and 960 (32): workers 168 and makers 88 205 and 222, 152
+// and 104 197 and 206, 144 and 112 189 and 214, 136 and 120 196 and 215.
+constexpr int MAKERS = 256, DELTA_THREADS = WORKERS + MAKERS;
+template <int TILES>
+struct Registers {
+  static constexpr int WORKER = TILES == 1 ? 144 : 152, MAKER = 256 - WORKER;
+  static_assert(WORKERS == MAKERS, "what the workers get beyond 128 the makers give");
+};
+
 template <int TILES, typename T>
-__global__ void __launch_bounds__(CHAIN_THREADS, 1)
+__global__ void __launch_bounds__(DELTA_THREADS, 1)
 delta_chain_kernel(const float* __restrict__ records, const T* __restrict__ proj, long long P, float* __restrict__ state,
                    const int32_t* __restrict__ item_start, const int32_t* __restrict__ slots, float* __restrict__ o, int items,
                    int all_chunks, int min_tokens, int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats) {
@@ -376,6 +387,7 @@ delta_chain_kernel(const float* __restrict__ records, const T* __restrict__ proj
   };
 
   if (threadIdx.x < WORKERS) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Registers<TILES>::WORKER));
     uint4 mq[4][3], kr[2][3];  // asked for a chunk ahead, each as soon as the last one's is used up
     float2 g[2];
     const float* r = record_of(0);
@@ -479,20 +491,21 @@ delta_chain_kernel(const float* __restrict__ records, const T* __restrict__ proj
         for (int e = 0; e < 4; ++e)
           if (float* p = at(tile, m, e)) *p = s[tile][m][e];
   } else {
-    const int eight = warp - WORKERS / 32;  // of the read-outs: tokens 8 eight .. + 7 of every chunk; of U: columns 4 eight .. + 3 of every 16
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Registers<TILES>::MAKER));
+    const int mine = warp - WORKERS / 32;
+    const int tile = mine / (CHUNK / 8), eight = mine % (CHUNK / 8);  // of the read-outs: tokens 8 eight .. + 7 of every chunk, the tile's columns
+    const int column = 2 * mine + (lane >> 4), vp = lane & 15;        // of U: this thread's column of every 16 and its pair of tokens
     uint4 b[3];
-    float2 wv[TILES][2];
-    const int vp = lane & 15;  // this thread's pair of tokens of U
-    auto column = [&](int m) { return 4 * eight + 2 * m + (lane >> 4); };
-    auto fetch = [&](int c) {
-      unit(record_of(c) + B_AT + eight * UNIT, b);
+    float2 wv[TILES];
+    auto fetch_b = [&](int c) {
+      if (tile < TILES) unit(record_of(c) + B_AT + eight * UNIT, b);
+    };
+    auto fetch_values = [&](int c) {
 #pragma unroll
-      for (int tile = 0; tile < TILES; ++tile)
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-          const int col = col0 + 16 * tile + column(m);
-          wv[tile][m] = col < (vdim + RUN - 1) / RUN * RUN ? __ldg(reinterpret_cast<const float2*>(record_of(c) + V_AT + (size_t)col * CHUNK) + vp) : make_float2(0.f, 0.f);
-        }
+      for (int n = 0; n < TILES; ++n) {
+        const int col = col0 + 16 * n + column;
+        wv[n] = col < (vdim + RUN - 1) / RUN * RUN ? __ldg(reinterpret_cast<const float2*>(record_of(c) + V_AT + (size_t)col * CHUNK) + vp) : make_float2(0.f, 0.f);
+      }
     };
     auto sum_of_shares = [&](int col, int token) {
       float2 v[SHARES];
@@ -504,24 +517,31 @@ delta_chain_kernel(const float* __restrict__ records, const T* __restrict__ proj
         for (int q = 0; q < m; ++q) v[q].x += v[q + m].x, v[q].y += v[q + m].y;
       return v[0];
     };
-    fetch(0);
+    // A record's way from DRAM takes longer than a chunk: every block of a head asks for its share of the one after the next into L2.
+    const size_t bytes = size * sizeof(float), share_bytes = (bytes / gridDim.x + 15) & ~(size_t)15, share_at = share_bytes * blockIdx.x;
+    auto ask_for = [&](int c) {
+      if (threadIdx.x == WORKERS && c < chunks && share_at < bytes)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<const char*>(record_of(c)) + share_at),
+                     "r"((uint32_t)min(share_bytes, bytes - share_at)) : "memory");
+    };
+    fetch_b(0);
+    fetch_values(0);
+    ask_for(1);
     for (int c = 0; c < chunks; ++c) {
+      ask_for(c + 2);
       __syncthreads();
       const int n = t1 - (t0 + c * CHUNK);  // tokens left
 #pragma unroll
-      for (int tile = 0; tile < TILES; ++tile)
+      for (int m = 0; m < TILES; ++m) {  // U = W V - M S
+        const float2 y = sum_of_shares(16 * m + column, 2 * vp);
+        const Terms t = split3(2 * vp < n ? wv[m].x - y.x : 0.f, 2 * vp + 1 < n ? wv[m].y - y.y : 0.f);
+        uint32_t* to = us + (m * 2 + (vp >> 3)) * UNIT + ((column & 7) * 4 + (vp & 3)) * 4 + (column >> 3) + 2 * ((vp >> 2) & 1);
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {  // U = W V - M S
-          const int col = column(m);
-          const float2 y = sum_of_shares(16 * tile + col, 2 * vp);
-          const Terms t = split3(2 * vp < n ? wv[tile][m].x - y.x : 0.f, 2 * vp + 1 < n ? wv[tile][m].y - y.y : 0.f);
-          uint32_t* to = us + (tile * 2 + (vp >> 3)) * UNIT + ((col & 7) * 4 + (vp & 3)) * 4 + (col >> 3) + 2 * ((vp >> 2) & 1);
-#pragma unroll
-          for (int p = 0; p < 3; ++p) to[p * TERM] = t.v[p];
-        }
+        for (int p = 0; p < 3; ++p) to[p * TERM] = t.v[p];
+      }
       __syncthreads();
-#pragma unroll
-      for (int tile = 0; tile < TILES; ++tile) {
+      if (c + 1 < chunks) fetch_values(c + 1);  // as early as their registers are free: U is what all the others wait for
+      if (tile < TILES) {
         float sum[2][1][4] = {}, small[2][1][4] = {};
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
@@ -534,34 +554,45 @@ delta_chain_kernel(const float* __restrict__ records, const T* __restrict__ proj
           }
           step<1>(sum[k], small[k], left_of(tile * 2 + k), x);
         }
+        float v[4];
+        bool fine = true;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          v[e] = (sum[0][0][e] + sum[1][0][e]) + (small[0][0][e] + small[1][0][e]);
+          fine = fine && is_finite(v[e]);
+        }
+        if (!fine) {
+#pragma unroll 1
+          for (int e = 0; e < 4; ++e) {
+            const int in = gr + 8 * (e >> 1), i = 8 * eight + 2 * tg + (e & 1);
+            float again = 0.f;
+            const uint32_t* rec = reinterpret_cast<const uint32_t*>(record_of(c)) + B_AT + eight * UNIT;
+#pragma unroll 1
+            for (int j = 0; j <= i; ++j) {
+              const int q = (j & 7) >> 1, k = j >> 4, h8 = (j >> 3) & 1;
+              float x = 0.f, y = 0.f;
+              for (int p = 2; p >= 0; --p) {
+                x += term(rec[p * TERM + ((i & 7) * 4 + q) * 4 + 2 * k + h8], j & 1);
+                y += term(us[(tile * 2 + k) * UNIT + p * TERM + ((in & 7) * 4 + q) * 4 + (in >> 3) + 2 * h8], j & 1);
+              }
+              again = fmaf(x, y, again);
+            }
+#pragma unroll
+            for (int f = 0; f < 4; ++f)
+              if (f == e && !is_finite(v[f])) v[f] = again;
+          }
+        }
+        float* row = o + ((size_t)(t0 + c * CHUNK + 8 * eight + 2 * tg) * H + h) * vdim + col0 + 16 * tile + gr;
+        const int left = n - (8 * eight + 2 * tg);  // tokens from this thread's first on
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const float2 read = sum_of_shares(16 * tile + gr + 8 * r, CHUNK + 8 * eight + 2 * tg);  // Q c S
-#pragma unroll
-          for (int e = 2 * r; e < 2 * r + 2; ++e) {
-            const int in = gr + 8 * r, i = 8 * eight + 2 * tg + (e & 1), t = t0 + c * CHUNK + i, col = col0 + 16 * tile + in;
-            const float of_state = e & 1 ? read.y : read.x;
-            float v = of_state + ((sum[0][0][e] + sum[1][0][e]) + (small[0][0][e] + small[1][0][e]));
-            if (!is_finite(v)) {
-              float again = 0.f;
-              const uint32_t* rec = reinterpret_cast<const uint32_t*>(record_of(c)) + B_AT + eight * UNIT;
-#pragma unroll 1
-              for (int j = 0; j <= i; ++j) {
-                const int q = (j & 7) >> 1, k = j >> 4, h8 = (j >> 3) & 1;
-                float x = 0.f, y = 0.f;
-                for (int p = 2; p >= 0; --p) {
-                  x += term(rec[p * TERM + ((i & 7) * 4 + q) * 4 + 2 * k + h8], j & 1);
-                  y += term(us[(tile * 2 + k) * UNIT + p * TERM + ((in & 7) * 4 + q) * 4 + (in >> 3) + 2 * h8], j & 1);
-                }
-                again = fmaf(x, y, again);
-              }
-              v = of_state + again;
-            }
-            if (t < t1 && col < vdim) o[((size_t)t * H + h) * vdim + col] = v;
-          }
+          if (col0 + 16 * tile + gr + 8 * r >= vdim) continue;
+          if (left > 0) row[8 * r] = read.x + v[2 * r];
+          if (left > 1) row[(size_t)H * vdim + 8 * r] = read.y + v[2 * r + 1];
         }
       }
-      if (c + 1 < chunks) fetch(c + 1);
+      if (c + 1 < chunks) fetch_b(c + 1);
     }
     pdl_trigger();
   }
@@ -579,20 +610,20 @@ int launch_chain(const float* records, const T* proj, long long ld, float* state
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) PSB_REFUSE("delta_chain: cannot raise the shared-memory limit");
     configured.set();
   }
-  psb_launch(kernel, dim3((vdim + COLS - 1) / COLS, H, portions), dim3(CHAIN_THREADS), (size_t)bytes, stream, records, proj, ld, state, item_start, slots, o,
+  psb_launch(kernel, dim3((vdim + COLS - 1) / COLS, H, portions), dim3(DELTA_THREADS), (size_t)bytes, stream, records, proj, ld, state, item_start, slots, o,
              items, chunks, min_tokens, G, H, dim, vdim, K, num_slots, slot_floats);
   PSB_LAUNCH_CHECK("delta_chain");
   return 0;
 }
 
-// Runs of columns a block takes.  One block fills an SM, so by rounds over the SMs: a chunk takes a block of one run 2.15 us and one of two 3.3 (the gated
+// Runs of columns a block takes.  One block fills an SM, so by rounds over the SMs: a chunk takes a block of one run 1.75 us and one of two 2.95 (the gated
 // rule over 2,000 tokens of 16 heads, 128 blocks, and the other over 1,200 and 960 tokens, 128 blocks).
 template <typename T>
 int chain_of(const void* records, const void* proj, long long ld, void* state, const void* item_start, const void* slots, void* o, int items,
              int portions, int chunks, int min_tokens, int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats, cudaStream_t stream) {
   const long long heads = (long long)H * portions, sms = psb_current_sms();
   const long long rounds16 = (heads * ((vdim + 15) / 16) + sms - 1) / sms, rounds32 = (heads * ((vdim + 31) / 32) + sms - 1) / sms;
-  auto launch = rounds32 * 31 < rounds16 * 20 ? launch_chain<2, T> : launch_chain<1, T>;
+  auto launch = rounds32 * 59 < rounds16 * 35 ? launch_chain<2, T> : launch_chain<1, T>;
   return launch((const float*)records, (const T*)proj, ld, (float*)state, (const int32_t*)item_start, (const int32_t*)slots, (float*)o, items, portions, chunks,
                 min_tokens, G, H, dim, vdim, K, num_slots, slot_floats, stream);
 }

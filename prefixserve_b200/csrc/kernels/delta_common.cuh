@@ -9,6 +9,13 @@ constexpr int MAX_TAPS = 16;
 // not depend on the state: q.k of the token, and k.k' and q.k' with the key k' of the token before it in the portion.
 constexpr int BD = 5;
 
+__device__ __forceinline__ float softplusf_(float x) { return log1pf(expf(-fabsf(x))) + fmaxf(x, 0.f); }
+__device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + expf(-x)); }
+__device__ __forceinline__ float siluf_(float x) { return x / (1.f + expf(-x)); }
+// what makes a vector with this sum of squares a unit vector, over sqrt(dim) for queries (keys: 1).  (rsqrtf(dim) is off by up to two units of the last place,
+// in every query alike.)
+__device__ __forceinline__ float unit_factor(float squares, int dim) { return 1.f / sqrtf((float)dim) / sqrtf(squares + 1e-6f); }
+
 __device__ __forceinline__ void copy_async4(float* dst, const float* src) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");

@@ -41,13 +41,6 @@ namespace {
 
 using namespace delta;
 
-__device__ __forceinline__ float softplusf_(float x) { return log1pf(expf(-fabsf(x))) + fmaxf(x, 0.f); }
-__device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + expf(-x)); }
-__device__ __forceinline__ float siluf_(float x) { return x / (1.f + expf(-x)); }
-// what makes a vector with this sum of squares a unit vector, over sqrt(dim) for queries (keys: 1).  (rsqrtf(dim) is off by up to two units of the last place,
-// in every query alike.)
-__device__ __forceinline__ float unit_factor(float squares, int dim) { return 1.f / sqrtf((float)dim) / sqrtf(squares + 1e-6f); }
-
 // A block per (token, unit); a unit is one query group, one key group (dim channels each) or one value head (vdim).
 template <typename T>
 __global__ void __launch_bounds__(128)

@@ -1202,6 +1202,12 @@ def _delta_one_by_one(lengths: list[int] | None) -> bool:
     return bool(short) and max(lengths) < min(DELTA_LONG_PORTION, 14 + 3 * max(short) + len(short) * 5 // 8)
 
 
+def _delta_singles(ctx, state: torch.Tensor, groups: int, heads: int, dim: int, vdim: int, taps: int) -> bool:
+    """Whether the step is of single tokens, in sizes and on addresses that the kernel for those takes."""
+    return (ctx.max_new_tokens == 1 and state.shape[1] % 4 == 0 and state.data_ptr() % 16 == 0
+            and bool(lib().psb_delta_single_supported(groups, heads, dim, vdim, taps)))
+
+
 def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
                gain: torch.Tensor, state: torch.Tensor, ctx, *, groups: int, heads: int, dim: int, vdim: int, eps: float) -> torch.Tensor:
     """The gated delta rule over every portion of the step.  proj [T, 2*groups*dim + 2*heads*vdim] (queries, keys,
@@ -1221,6 +1227,14 @@ def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: 
         if x.dtype != torch.float32 or x.numel() != n or not x.is_cuda or not x.is_contiguous():
             raise KernelError(f"delta rule: {what} must be float32 with {n} numbers on the device")
     dev = proj.device
+    if _delta_singles(ctx, state, groups, heads, dim, vdim, k):
+        out = torch.empty((t, heads * vdim), dtype=proj.dtype, device=dev)
+        check(lib().psb_delta_single(proj.data_ptr(), _code(proj, "projection output"), proj.shape[1], 0, ba.data_ptr(), None, taps.data_ptr(),
+                                     a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), _i32(ctx.positions, "positions").data_ptr(),
+                                     _i32(ctx.item_start, "item offsets").data_ptr(), _i32(ctx.slots, "slots").data_ptr(), gain.data_ptr(),
+                                     out.data_ptr(), ctx.num_items, groups, heads, dim, vdim, k, state.shape[0], slot_floats, float(eps), _stream()),
+              "delta_single")
+        return out
     # Long portions go in chunks; what is left, if anything can be, token by token.
     chunked = proj.dtype == torch.bfloat16 and ctx.max_new_tokens >= DELTA_CHUNKED and not _delta_one_by_one(_portion_lengths(ctx))
     record = int(lib().psb_delta_chunk_record(dim, vdim)) if chunked else 0
@@ -1573,6 +1587,13 @@ def channel_delta_rule(proj: torch.Tensor, beta_at: int, decay: torch.Tensor, ta
         raise KernelError(f"channel delta rule: state must be float32 [slots, {slot_floats}], is {state.dtype} {tuple(state.shape)}")
     _f32_vector(taps, c * k, "taps")
     dev = proj.device
+    if _delta_singles(ctx, state, groups, heads, dim, vdim, k):
+        o = torch.empty((t, heads, vdim), dtype=torch.float32, device=dev)
+        check(lib().psb_delta_single(proj.data_ptr(), _code(proj, "projection output"), proj.shape[1], beta_at, None, decay.data_ptr(), taps.data_ptr(),
+                                     None, None, state.data_ptr(), _i32(ctx.positions, "positions").data_ptr(),
+                                     _i32(ctx.item_start, "item offsets").data_ptr(), _i32(ctx.slots, "slots").data_ptr(), None, o.data_ptr(),
+                                     ctx.num_items, groups, heads, dim, vdim, k, state.shape[0], slot_floats, 0.0, _stream()), "delta_single")
+        return o
     qkv = torch.empty((t, c), dtype=torch.float32, device=dev)
     bd = torch.empty((t, 5 * heads), dtype=torch.float32, device=dev)
     item_start, slots = _i32(ctx.item_start, "item offsets"), _i32(ctx.slots, "slots")

@@ -230,6 +230,13 @@ _SIGNATURES: dict[str, list] = {
     # (qkv, bd, decay, proj, dtype, ld, state, item_start, slots, records, o_out, items, chunks, G, H, dim, vdim, K, num_slots,
     #  slot_floats, stream)
     "psb_channel_delta_chunks": [P, P, P, P, I, L, P, P, P, P, P, I, I, I, I, I, I, I, I, L, P],
+    # (G, H, dim, vdim, K) -> 1 if psb_delta_single is built for the sizes
+    "psb_delta_single_supported": [I, I, I, I, I],
+    # (proj, dtype, ld, beta_at, ba, decay, taps, a_log, dt_bias, state, positions, item_start, slots, gain, out, items, G, H, dim, vdim, K,
+    #  num_slots, slot_floats, eps, stream)
+    "psb_delta_single": [P, I, L, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, L, F, P],
+    # () -> 0 while no bounded wait of that kernel has ever run out
+    "psb_delta_single_status": [],
     # (o, proj, dtype, gain, out, T, G, H, dim, vdim, eps, stream)
     "psb_delta_finish": [P, P, I, P, P, I, I, I, I, I, F, P],
     # (z, ldz, correction, chosen, weight, T, E, top, groups, keep, scale, stream)
@@ -365,10 +372,11 @@ def tcgen05_status() -> int:
 
     The product's code sits in the low byte, prefill attention's in the next, the TMA-fed decode attention's in the
     third, the few-row product's in the fourth, prefill attention's over rows in the fifth,
-    decode attention's over rows in the sixth."""
+    decode attention's over rows in the sixth, that of the delta rules over single tokens in the seventh."""
     return (int(lib().psb_tcgen05_status()) | (int(lib().psb_attention_tcgen05_status()) << 8)
             | (int(lib().psb_attention_decode_tma_status()) << 16) | (int(lib().psb_gemm_fewrows_status()) << 24)
-            | (int(lib().psb_attention_rows_tcgen05_status()) << 32) | (int(lib().psb_attention_rows_decode_status()) << 40))
+            | (int(lib().psb_attention_rows_tcgen05_status()) << 32) | (int(lib().psb_attention_rows_decode_status()) << 40)
+            | (int(lib().psb_delta_single_status()) << 48))
 
 
 def declare(name: str, argtypes: list) -> None:

@@ -6,6 +6,7 @@ stream.  Everything here refuses CPU tensors: there is no CPU path.
 
 from __future__ import annotations
 
+import functools
 import math
 
 import torch
@@ -44,6 +45,18 @@ def _stream() -> int:
 
 def _ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
+
+
+def _scratch(device: torch.device, *sizes: int) -> tuple[torch.Tensor, list[int]]:
+    """One allocation for several buffers of so many bytes: the tensor that holds them, to be kept until the last kernel that takes one is
+    launched, and their addresses, multiples of 256.  (An allocation of torch's costs the host 2 to 3 us, as much as a launch.)"""
+    at, total = [], 0
+    for n in sizes:
+        at.append(total)
+        total += (n + 255) & ~255
+    whole = torch.empty((total,), dtype=torch.uint8, device=device)
+    base = whole.data_ptr()
+    return whole, [base + a for a in at]
 
 
 def _rows_out(out: torch.Tensor | None, rows: int, cols: int, dtype: torch.dtype, device: torch.device) -> tuple[torch.Tensor, int]:
@@ -713,7 +726,9 @@ def latent_attention(q_lat: torch.Tensor, cache: torch.Tensor, table: torch.Tens
         banded = [(it.first_token, it.end - it.start, it.start) for it in items if it.end - it.start >= BAND_MIN_TOKENS]
     at = 0
     for first, n, _ in banded + [(t, 0, 0)]:   # the tokens between the banded portions: runs for the kernel that walks the keys
-        if first > at:
+        if at == 0 and first == t > 0:  # all of them, as they are
+            _latent_attention_walk(q_lat, cache, table, positions, token_item, gate, out, rank, page_size, window, scale, key_hint=int(window or key_hint), sink=sink)
+        elif first > at:
             _latent_attention_walk(q_lat[at:first], cache, table, positions[at:first], token_item[at:first],
                                    None if gate is None else gate[at:first], out[at:first], rank, page_size, window, scale,
                                    key_hint=int(window or key_hint), sink=sink)
@@ -748,6 +763,7 @@ LATENT_MMA_BLOCK_SHARE = 64
 LATENT_MMA_KEYS_PER_SPLIT = 64
 
 
+@functools.lru_cache(maxsize=4096)
 def _rows_splits(blocks: int, keys: int, slots: int, most: int = 8, least_keys: int = ROWS_KEYS_PER_SPLIT,
                  share: int = ROWS_BLOCK_SHARE) -> int:
     most = max(1, min(most, keys // least_keys))
@@ -1239,31 +1255,31 @@ def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: 
     chunked = proj.dtype == torch.bfloat16 and ctx.max_new_tokens >= DELTA_CHUNKED and not _delta_one_by_one(_portion_lengths(ctx))
     record = int(lib().psb_delta_chunk_record(dim, vdim)) if chunked else 0
     short = not record or _has_portions_below(ctx, DELTA_CHUNKED)
-    qkv = torch.empty((t, c), dtype=torch.float32, device=dev)
-    bd = torch.empty((t, 5 * heads), dtype=torch.float32, device=dev)   # beta, decay and three state-free dot products per head
+    portions = chunks = 0
+    if record:
+        portions, chunks = _portions_from(ctx, DELTA_CHUNKED), _portion_tiles(ctx, t, DELTA_CHUNKED, lib().psb_delta_chunk_tokens())
+    # (bd: beta, decay and three state-free dot products per head; the chunks' records)
+    held, (qkv, bd, o, records) = _scratch(dev, 4 * t * c, 4 * t * 5 * heads, 4 * t * heads * vdim, 4 * chunks * heads * record)
     positions, token_item = _i32(ctx.positions, "positions"), _i32(ctx.token_item, "token-to-item map")
     item_start, slots = _i32(ctx.item_start, "item offsets"), _i32(ctx.slots, "slots")
     check(lib().psb_delta_prepare(proj.data_ptr(), _code(proj, "projection output"), proj.shape[1], 0, ba.data_ptr(), None, taps.data_ptr(), a_log.data_ptr(),
                                   dt_bias.data_ptr(), state.data_ptr(), positions.data_ptr(), token_item.data_ptr(),
-                                  item_start.data_ptr(), slots.data_ptr(), qkv.data_ptr(), bd.data_ptr(), t, groups, heads, dim, vdim,
+                                  item_start.data_ptr(), slots.data_ptr(), qkv, bd, t, groups, heads, dim, vdim,
                                   k, state.shape[0], slot_floats, 1 if short else 0, _stream()), "delta_prepare")
-    o = torch.empty((t, heads, vdim), dtype=torch.float32, device=dev)
     most = 0x7fffffff  # tokens of the longest portion left to the kernel that goes token by token
     if record:
         most = DELTA_CHUNKED - 1
-        portions, chunks = _portions_from(ctx, DELTA_CHUNKED), _portion_tiles(ctx, t, DELTA_CHUNKED, lib().psb_delta_chunk_tokens())
-        records = torch.empty((chunks, heads, record), dtype=torch.float32, device=dev)
-        check(lib().psb_delta_chunks(qkv.data_ptr(), bd.data_ptr(), proj.data_ptr(), proj.shape[1],
-                                     state.data_ptr(), item_start.data_ptr(), slots.data_ptr(), records.data_ptr(), o.data_ptr(),
+        check(lib().psb_delta_chunks(qkv, bd, proj.data_ptr(), proj.shape[1],
+                                     state.data_ptr(), item_start.data_ptr(), slots.data_ptr(), records, o,
                                      ctx.num_items, portions, chunks, DELTA_CHUNKED, groups, heads, dim, vdim, k, state.shape[0], slot_floats,
                                      _stream()), "delta_chunks")
     if short:
         lanes = DELTA_LONG_LANES if min(ctx.max_new_tokens, most) >= DELTA_LONG_PORTION and dim >= DELTA_LONG_LANES else 4
-        check(lib().psb_delta_rule(qkv.data_ptr(), bd.data_ptr(), proj.data_ptr(), _code(proj, "projection output"), state.data_ptr(),
-                                   item_start.data_ptr(), slots.data_ptr(), o.data_ptr(), ctx.num_items, groups, heads, dim, vdim, k,
+        check(lib().psb_delta_rule(qkv, bd, proj.data_ptr(), _code(proj, "projection output"), state.data_ptr(),
+                                   item_start.data_ptr(), slots.data_ptr(), o, ctx.num_items, groups, heads, dim, vdim, k,
                                    state.shape[0], slot_floats, lanes, most, _stream()), "delta_rule")
     out = torch.empty((t, heads * vdim), dtype=proj.dtype, device=dev)
-    check(lib().psb_delta_finish(o.data_ptr(), proj.data_ptr(), _code(proj, "projection output"), gain.data_ptr(), out.data_ptr(), t,
+    check(lib().psb_delta_finish(o, proj.data_ptr(), _code(proj, "projection output"), gain.data_ptr(), out.data_ptr(), t,
                                  groups, heads, dim, vdim, float(eps), _stream()), "delta_finish")
     return out
 
@@ -1332,46 +1348,40 @@ def moe_experts(x: torch.Tensor, chosen: torch.Tensor, weight: torch.Tensor, w_u
                and h % 8 == 0 and ff % 8 == 0 and pairs >= MOE_TCGEN05_MIN_PAIRS)
     pad = 128 if grouped else 1
     room = -(-(pairs + e * (pad - 1)) // pad) * pad
-    offsets = torch.empty((e + 1,), dtype=torch.int32, device=dev)
-    row_pair = torch.empty((max(room, 1),), dtype=torch.int32, device=dev)
-    pair_row = torch.empty((max(pairs, 1),), dtype=torch.int32, device=dev)
-    tile_expert = torch.empty((room // pad,), dtype=torch.int32, device=dev) if grouped else None
-    row_weight = torch.empty((max(room, 1),), dtype=torch.float32, device=dev) if weight_on_input else None
-    check(lib().psb_moe_group(chosen.data_ptr(), offsets.data_ptr(), row_pair.data_ptr(), pair_row.data_ptr(), _ptr(tile_expert),
-                              pairs, e, pad, room, weight.data_ptr() if weight_on_input else None, _ptr(row_weight), _stream()), "moe_group")
+    # what lies between the two products: activations, gated already where the tcgen05 product's epilogue does it
+    between, size = ff if grouped else ff_in, x.element_size()
+    held, (offsets, row_pair, pair_row, tile_expert, row_weight, rows, mid, y) = _scratch(
+        dev, 4 * (e + 1), 4 * room, 4 * pairs, 4 * (room // pad) if grouped else 0, 4 * room if weight_on_input else 0, 2 * room * h if grouped else 0,
+        size * room * between, (2 if grouped else 4) * room * h)
+    row_weight = row_weight if weight_on_input else None
+    check(lib().psb_moe_group(chosen.data_ptr(), offsets, row_pair, pair_row, tile_expert if grouped else None, pairs, e, pad, room,
+                              weight.data_ptr() if weight_on_input else None, row_weight, _stream()), "moe_group")
     if grouped:
         from .tensorcore import _sms
         sms = _sms(dev)
-        rows = torch.empty((room, h), dtype=torch.bfloat16, device=dev)
-        check(lib().psb_moe_gather(x.data_ptr(), row_pair.data_ptr(), rows.data_ptr(), room, h, top, _stream()), "moe_gather")
+        check(lib().psb_moe_gather(x.data_ptr(), row_pair, rows, room, h, top, _stream()), "moe_gather")
         if silu_gate:
-            mid = torch.empty((room, ff), dtype=torch.bfloat16, device=dev)
-            check(lib().psb_gemm_tcgen05_grouped_gated_silu(rows.data_ptr(), w_up.data_ptr(), mid.data_ptr(), room, ff, h, e,
-                                                            tile_expert.data_ptr(), _ptr(row_weight), sms, _stream()),
+            check(lib().psb_gemm_tcgen05_grouped_gated_silu(rows, w_up.data_ptr(), mid, room, ff, h, e,
+                                                            tile_expert, row_weight, sms, _stream()),
                   "gemm_tcgen05_grouped_gated_silu")
         elif glu is not None:  # both branches and the gate in one product's epilogue
-            mid = torch.empty((room, ff), dtype=torch.bfloat16, device=dev)
-            check(lib().psb_gemm_tcgen05_grouped_gated_clipped(rows.data_ptr(), w_up.data_ptr(), mid.data_ptr(), room, ff, h, e,
-                                                               tile_expert.data_ptr(), float(glu[0]), float(glu[1]), float(glu[2]),
+            check(lib().psb_gemm_tcgen05_grouped_gated_clipped(rows, w_up.data_ptr(), mid, room, ff, h, e,
+                                                               tile_expert, float(glu[0]), float(glu[1]), float(glu[2]),
                                                                sms, _stream()), "gemm_tcgen05_grouped_gated_clipped")
         else:
-            mid = torch.empty((room, ff_in), dtype=torch.bfloat16, device=dev)
-            check(lib().psb_gemm_tcgen05_grouped(rows.data_ptr(), w_up.data_ptr(), mid.data_ptr(), room, ff_in, h, e, tile_expert.data_ptr(),
+            check(lib().psb_gemm_tcgen05_grouped(rows, w_up.data_ptr(), mid, room, ff_in, h, e, tile_expert,
                                                  MOE_ACTIVATIONS[activation], sms, _stream()), "gemm_tcgen05_grouped")
-        y = torch.empty((room, h), dtype=torch.bfloat16, device=dev)
-        check(lib().psb_gemm_tcgen05_grouped(mid.data_ptr(), w_down.data_ptr(), y.data_ptr(), room, h, ff, e, tile_expert.data_ptr(),
+        check(lib().psb_gemm_tcgen05_grouped(mid, w_down.data_ptr(), y, room, h, ff, e, tile_expert,
                                              0, sms, _stream()), "gemm_tcgen05_grouped")
     else:
-        mid = torch.empty((room, ff_in), dtype=x.dtype, device=dev)
-        check(lib().psb_moe_gemm(x.data_ptr(), _code(x, "expert input"), w_up.data_ptr(), _code(w_up, "expert up matrices"), mid.data_ptr(),
-                                 _code(mid, "expert activations"), offsets.data_ptr(), row_pair.data_ptr(), room, e, ff_in, h, top, 1,
+        check(lib().psb_moe_gemm(x.data_ptr(), _code(x, "expert input"), w_up.data_ptr(), _code(w_up, "expert up matrices"), mid,
+                                 _code(x, "expert input"), offsets, row_pair, room, e, ff_in, h, top, 1,
                                  MOE_ACTIVATIONS[activation], 0, 0.0, 0.0, 0.0, None, _stream()), "moe_gemm")
         # gated experts: the second product takes the gate of a row's two halves as it reads the row
         lim, alpha, off = (float(v) for v in glu) if glu is not None and not silu_gate else (0.0, 0.0, 0.0)
-        y = torch.empty((room, h), dtype=torch.float32, device=dev)
-        check(lib().psb_moe_gemm(mid.data_ptr(), _code(mid, "expert activations"), w_down.data_ptr(), _code(w_down, "expert down matrices"),
-                                 y.data_ptr(), F32, offsets.data_ptr(), row_pair.data_ptr(), room, e, h, ff, top, 0, 0,
-                                 2 if silu_gate else 1 if glu is not None else 0, lim, alpha, off, _ptr(row_weight), _stream()), "moe_gemm")
+        check(lib().psb_moe_gemm(mid, _code(x, "expert input"), w_down.data_ptr(), _code(w_down, "expert down matrices"),
+                                 y, F32, offsets, row_pair, room, e, h, ff, top, 0, 0,
+                                 2 if silu_gate else 1 if glu is not None else 0, lim, alpha, off, row_weight, _stream()), "moe_gemm")
     out = torch.empty((t, h), dtype=out_dtype or x.dtype, device=dev)
     ldg = 0
     if shared is not None:
@@ -1382,7 +1392,7 @@ def moe_experts(x: torch.Tensor, chosen: torch.Tensor, weight: torch.Tensor, w_u
             if shared_gate.dtype != torch.float32 or shared_gate.shape[0] != t or not shared_gate.is_cuda:
                 raise KernelError("experts: the shared expert's gate must be a float32 column on the device")
             ldg = shared_gate.stride(0)
-    check(lib().psb_moe_combine(y.data_ptr(), _code(y, "experts' outputs"), pair_row.data_ptr(), None if weight_on_input else weight.data_ptr(), _ptr(shared),
+    check(lib().psb_moe_combine(y, BF16 if grouped else F32, pair_row, None if weight_on_input else weight.data_ptr(), _ptr(shared),
                                 _code(shared, "shared expert output") if shared is not None else F32,
                                 _ptr(shared_gate) if shared is not None else None, ldg, out.data_ptr(), _code(out, "experts' sum"),
                                 t, h, top, _stream()), "moe_combine")
@@ -1594,8 +1604,6 @@ def channel_delta_rule(proj: torch.Tensor, beta_at: int, decay: torch.Tensor, ta
                                      _i32(ctx.item_start, "item offsets").data_ptr(), _i32(ctx.slots, "slots").data_ptr(), None, o.data_ptr(),
                                      ctx.num_items, groups, heads, dim, vdim, k, state.shape[0], slot_floats, 0.0, _stream()), "delta_single")
         return o
-    qkv = torch.empty((t, c), dtype=torch.float32, device=dev)
-    bd = torch.empty((t, 5 * heads), dtype=torch.float32, device=dev)
     item_start, slots = _i32(ctx.item_start, "item offsets"), _i32(ctx.slots, "slots")
     code, ld = _code(proj, "projection output"), proj.shape[1]
     from .tensorcore import _sms
@@ -1606,33 +1614,34 @@ def channel_delta_rule(proj: torch.Tensor, beta_at: int, decay: torch.Tensor, ta
         tokens = lib().psb_delta_chunk_tokens() if narrow else 16
         least = CHANNEL_DELTA_LEAST if narrow and _channel_delta_apart(ctx, heads * -(-vdim // 32), _sms(dev)) else 1
     short = not record or (least > 1 and _has_portions_below(ctx, least))
+    chunks = 0
+    if record:
+        chunks = _portion_tiles(ctx, t, least, tokens) if narrow else t // tokens + ctx.num_items
+    held, (qkv, bd, records) = _scratch(dev, 4 * t * c, 4 * t * 5 * heads, 4 * chunks * heads * record)
     check(lib().psb_delta_prepare(proj.data_ptr(), code, ld, beta_at, None, decay.data_ptr() if short else None, taps.data_ptr(), None, None,
                                   state.data_ptr(), _i32(ctx.positions, "positions").data_ptr(),
                                   _i32(ctx.token_item, "token-to-item map").data_ptr(), item_start.data_ptr(), slots.data_ptr(),
-                                  qkv.data_ptr(), bd.data_ptr(), t, groups, heads, dim, vdim, k, state.shape[0], slot_floats, 1, _stream()),
+                                  qkv, bd, t, groups, heads, dim, vdim, k, state.shape[0], slot_floats, 1, _stream()),
           "delta_prepare")
     o = torch.empty((t, heads, vdim), dtype=torch.float32, device=dev)
     most = 0x7fffffff  # tokens of the longest portion left to the kernel that goes token by token
-    if record and dim <= 128:
+    if record and narrow:
         most = least - 1
-        portions, chunks = _portions_from(ctx, least), _portion_tiles(ctx, t, least, tokens)
-        records = torch.empty((chunks, heads, record), dtype=torch.float32, device=dev)
-        check(lib().psb_channel_delta_chunks32(qkv.data_ptr(), bd.data_ptr(), decay.data_ptr(), proj.data_ptr(), code, ld, state.data_ptr(),
-                                               item_start.data_ptr(), slots.data_ptr(), records.data_ptr(), o.data_ptr(), ctx.num_items, portions,
+        portions = _portions_from(ctx, least)
+        check(lib().psb_channel_delta_chunks32(qkv, bd, decay.data_ptr(), proj.data_ptr(), code, ld, state.data_ptr(),
+                                               item_start.data_ptr(), slots.data_ptr(), records, o.data_ptr(), ctx.num_items, portions,
                                                chunks, least, groups, heads, dim, vdim, k, state.shape[0], slot_floats, _stream()),
               "channel_delta_chunks")
     elif record:
-        chunks = t // tokens + ctx.num_items
-        records = torch.empty((chunks, heads, record), dtype=torch.float32, device=dev)
-        check(lib().psb_channel_delta_chunks(qkv.data_ptr(), bd.data_ptr(), decay.data_ptr(), proj.data_ptr(), code, ld, state.data_ptr(),
-                                             item_start.data_ptr(), slots.data_ptr(), records.data_ptr(), o.data_ptr(), ctx.num_items,
+        check(lib().psb_channel_delta_chunks(qkv, bd, decay.data_ptr(), proj.data_ptr(), code, ld, state.data_ptr(),
+                                             item_start.data_ptr(), slots.data_ptr(), records, o.data_ptr(), ctx.num_items,
                                              chunks, groups, heads, dim, vdim, k, state.shape[0], slot_floats, _stream()),
               "channel_delta_chunks")
     if short:
         lanes = CHANNEL_DELTA_LONG_LANES if min(ctx.max_new_tokens, most) >= CHANNEL_DELTA_CHUNKED and dim >= CHANNEL_DELTA_LONG_LANES else 4
         while dim > 32 * lanes and lanes < 32:
             lanes *= 2
-        check(lib().psb_channel_delta_rule(qkv.data_ptr(), bd.data_ptr(), decay.data_ptr(), proj.data_ptr(), code, ld, state.data_ptr(),
+        check(lib().psb_channel_delta_rule(qkv, bd, decay.data_ptr(), proj.data_ptr(), code, ld, state.data_ptr(),
                                            item_start.data_ptr(), slots.data_ptr(), o.data_ptr(), ctx.num_items, groups, heads, dim, vdim, k,
                                            state.shape[0], slot_floats, lanes, most, _stream()), "channel_delta_rule")
     return o

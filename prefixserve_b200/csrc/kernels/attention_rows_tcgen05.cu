@@ -22,8 +22,8 @@
 // A launch takes as many rounds over the SMs as it has CTAs for, and a last round that is nearly empty costs as much as a full
 // one.  The units (128 tokens, two heads) of such a round are therefore cut into ranges of keys, a CTA each, which leave
 // unnormalised results for attention_rows_merge_kernel; so are those of a step that is small to begin with (two portions of
-// 1,500 and 1,200 tokens, 176 units for 148 SMs: 91 -> 76 us, 80 since masked scores have no say in the form of the cap and the
-// gate is exact; 256 tokens behind 2,000: 49 -> 24).
+// 1,500 and 1,200 tokens, 176 units for 148 SMs: 91 -> 76 us, 79 since masked scores have no say in the form of the cap and the
+// gate is exact, 76 since results leave by whole rows; 256 tokens behind 2,000: 49 -> 24, 22).
 //
 // Every wait on an mbarrier is bounded (tcgen05.cuh).
 #include "tcgen05.cuh"
@@ -557,22 +557,38 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
         ok = mbar_wait(&bars->o_full[t], (nblk - 1) & 1, abort, 3);
         ok = __all_sync(0xffffffffu, ok);
       }
+      // Results leave by whole rows: a thread has a row, and 32 rows at a time touch 32 lines an instruction.  The warp's 32 rows go through shared memory (the
+      // place of the tile's queries, which nobody reads any more), 64 columns at a time: [32][16] pieces of 16 bytes, piece j of row r at j ^ (r % 16).
+      // (Two portions of 1,500 and 1,200 tokens with gates 79 us -> 76, 300 tokens behind 1,500 23 -> 21.)
+      float4* const staging = reinterpret_cast<float4*>(smem + t * Q_TILE_BYTES) + quarter * 32 * 16;
+      auto staged = [&](int row, int piece) { return staging[row * 16 + (piece ^ (row & 15))]; };
+      auto stage_results = [&](int pass, float factor) {
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+          uint32_t v[32];
+          tmem_ld32(o_addr + pass * 64 + cc * 32, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            staging[lane * 16 + ((8 * cc + k) ^ (lane & 15))] = make_float4(__uint_as_float(v[4 * k]) * factor, __uint_as_float(v[4 * k + 1]) * factor,
+                                                                            __uint_as_float(v[4 * k + 2]) * factor, __uint_as_float(v[4 * k + 3]) * factor);
+        }
+        __syncwarp();
+      };
       if (ok && cut) {
         fence_after();
         const size_t slot = (((size_t)(unit - args.whole) * args.ranges + range) * ntiles + t) * TILE_M + r;
         const bool some = nblk > 0 && m_run != -INFINITY;
         *reinterpret_cast<float2*>(args.part_ml + slot * 2) = make_float2(some ? m_run * c : -INFINITY, some ? l_run : 0.f);
         if (nblk > 0) {
-          float* dst = args.part_o + slot * D;
+          float* dst = args.part_o + (slot - lane) * D;  // of the warp's first row
 #pragma unroll 1
-          for (int cc = 0; cc < D / 32; ++cc) {
-            uint32_t v[32];
-            tmem_ld32(o_addr + cc * 32, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int k = 0; k < 32; k += 4)
-              *reinterpret_cast<float4*>(dst + cc * 32 + k) = make_float4(__uint_as_float(v[k]), __uint_as_float(v[k + 1]),
-                                                                          __uint_as_float(v[k + 2]), __uint_as_float(v[k + 3]));
+          for (int pass = 0; pass < D / 64; ++pass) {
+            stage_results(pass, 1.f);
+#pragma unroll 4
+            for (int at = lane; at < 32 * 16; at += 32)
+              *reinterpret_cast<float4*>(dst + (size_t)(at >> 4) * D + 64 * pass + 4 * (at & 15)) = staged(at >> 4, at & 15);
+            __syncwarp();
           }
         }
         fence_before();
@@ -580,36 +596,36 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
         fence_after();
         // a sink joins the denominator here, where the row's sum is complete
         const float inv = (l_run > 0.f ? (args.sink ? sink_quotient2(m_run * c, l_run, args.sink[head] * PSB_LOG2E) : 1.f / l_run) : 0.f) * args.out_scale;
-        __nv_bfloat16* dst = args.out + (size_t)(t0 + r) * args.ldo + (size_t)head * D;
-        const __nv_bfloat16* gates = args.gate ? args.gate + (size_t)(t0 + r) * args.ldg + (size_t)head * D : nullptr;
+        const int row0 = t0 + quarter * 32, column = head * D + 8 * (lane & 7);
 #pragma unroll 1
-        for (int cc = 0; cc < D / 32; ++cc) {
-          uint32_t v[32];
-          tmem_ld32(o_addr + cc * 32, v);
-          uint4 g[4];
-          if (gates && valid) {
+        for (int pass = 0; pass < D / 64; ++pass) {
+          uint4 g[8];  // the gates this lane needs: rows lane / 8 + 4 i
+          if (args.gate) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) g[k] = *reinterpret_cast<const uint4*>(gates + cc * 32 + k * 8);
-          }
-          tmem_ld_wait();
-          if (valid) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              uint32_t packed[4];
-              const uint32_t gw[4] = {g[k].x, g[k].y, g[k].z, g[k].w};
-#pragma unroll
-              for (int w = 0; w < 4; ++w) {
-                float a = __uint_as_float(v[k * 8 + 2 * w]) * inv, b = __uint_as_float(v[k * 8 + 2 * w + 1]) * inv;
-                if (gates) {
-                  const float2 f = gates_of(gw[w]);
-                  a *= f.x;
-                  b *= f.y;
-                }
-                packed[w] = pack2(a, b);
-              }
-              *reinterpret_cast<uint4*>(dst + cc * 32 + k * 8) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            for (int i = 0; i < 8; ++i) {
+              const int row = 4 * i + (lane >> 3);
+              if (quarter * 32 + row < n) g[i] = *reinterpret_cast<const uint4*>(args.gate + (size_t)(row0 + row) * args.ldg + column + 64 * pass);
             }
           }
+          stage_results(pass, inv);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int row = 4 * i + (lane >> 3);
+            const float4 a = staged(row, 2 * (lane & 7)), b = staged(row, 2 * (lane & 7) + 1);
+            float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            if (quarter * 32 + row >= n) continue;
+            if (args.gate) {
+              const uint32_t gw[4] = {g[i].x, g[i].y, g[i].z, g[i].w};
+#pragma unroll
+              for (int w = 0; w < 4; ++w) {
+                const float2 f = gates_of(gw[w]);
+                v[2 * w] *= f.x;
+                v[2 * w + 1] *= f.y;
+              }
+            }
+            *reinterpret_cast<uint4*>(args.out + (size_t)(row0 + row) * args.ldo + column + 64 * pass) = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+          }
+          __syncwarp();
         }
         fence_before();
       }

@@ -2,12 +2,12 @@
 // [latent of RANK numbers | rotated key part of ROT], so a block takes 16 or 32 heads of one token and a run of its keys,
 // and every row it brings in serves all of them.
 //
-// A block (eight warps) walks its run 32 rows at a time; the rows come in with cp.async, STAGES tiles deep.  Per tile:
+// A block walks its run 32 rows at a time; the rows come in with cp.async, STAGES tiles deep.  Eight warps make the products of a tile:
 //   S = Q K^T   four groups of warps take a quarter of the row's 576 numbers each (144: nine steps of mma.sync m16n8k16) and
 //               leave their partial scores in shared memory; the queries stay in registers for the whole run;
-//   softmax     a thread adds the quarters of a few scores of one head, in float32, and keeps the head's maximum and sum;
-//   O += P V    every warp takes 64 of the 512 value columns.
-// S of the next tile is computed together with P V of this one, so that the tensor cores wait for the softmax only.
+//   O += P V    every warp takes 64 of the 512 value columns;
+// and four more bring the rows in and do the softmax between the two: a thread adds the quarters of a few scores of one head, in float32, and keeps the
+// head's maximum and sum.  While they work on one tile, the others make S of the next and P V of the one before.
 // Queries and weights are float32 and stay so: each goes in as three bfloat16 terms whose sum is the number to its last bit
 // (8 + 8 + 8 bits), against rows that are bfloat16 to begin with, so every product is exact.  The instruction cuts its sums off
 // instead of rounding them, so its accumulators hold 32 numbers' (or keys') terms at a time, the smallest terms first, and what
@@ -15,10 +15,10 @@
 // keys; 1.6e-7 on the CUDA cores).  A block that shares a token's keys with others leaves maximum, sum and unscaled result for
 // the merge kernel.
 //
-// What bounds it: the tensor cores' legacy path (three terms: 108 + 96 instructions a warp and tile, 1,024 multiply-adds a
-// clock and SM; busy 48 % of the time).  The kernel on the CUDA cores beside it (latent_attention_rows_kernel, still used for
-// other sizes) reads every row once for each pair of heads: 16 tokens of 32 heads over up to 3,500 keys took it 402 us a call, this
-// one and its merge 50 (61 with the same number of blocks for every token).
+// What bounds it: the tensor cores' legacy path (three terms: 108 + 96 instructions a warp and tile, 1,024 multiply-adds a clock and SM: 1.7 us a tile of
+// 32 heads, of which it takes 3.4; two chains of instructions a warp side by side are what the registers hold).  16 tokens of 32 heads over up to 3,500 keys and the
+// merge 41 us on the device, 32 tokens 77, 16 tokens of 16 heads 26; with the softmax on the products' own warps, which waited for it, 47, 91 and 31.  The kernel on the CUDA
+// cores beside it (latent_attention_rows_kernel, still used for other sizes) reads every row once for each pair of heads: 402 us.
 #include "common.cuh"
 
 #include <cfloat>
@@ -26,7 +26,7 @@
 namespace {
 
 constexpr int RANK = 512, ROT = 64, D = RANK + ROT;
-constexpr int WARPS = 8, THREADS = 32 * WARPS;
+constexpr int WARPS = 8, SOFTMAX = 128, THREADS = 32 * WARPS + SOFTMAX;  // warps of the products; threads of the softmax, behind them
 constexpr int QUARTERS = 4, STEPS = D / 16 / QUARTERS;   // steps of 16 numbers a group of warps takes of a row
 constexpr int PITCH = D + 8;                             // elements from row to row: an odd number of 16-byte pieces
 constexpr int KEYS = 32;                                 // of a tile
@@ -37,16 +37,22 @@ static_assert(D % (16 * QUARTERS) == 0 && RANK == 64 * WARPS, "shares of the war
 template <int HEADS>
 struct LatentShape {
   static constexpr int MG = HEADS / 16;
+  // A block is launched with 168 registers a thread, of which the softmax's threads hand some to the products' warps (32 heads with 224 and 56: 42 us
+  // instead of 41).
+  static constexpr int PRODUCT_REGISTERS = MG == 2 ? 232 : 224, SOFTMAX_REGISTERS = MG == 2 ? 40 : 56;
+  static_assert(32 * WARPS * PRODUCT_REGISTERS + SOFTMAX * SOFTMAX_REGISTERS <= THREADS * 168, "more registers than the block is launched with");
   static constexpr int KT = KEYS, STAGES = 4;
-  static constexpr int SPT = HEADS * KT / THREADS;  // scores a thread has in the softmax
+  static constexpr int SPT = HEADS * KT / SOFTMAX;  // scores a thread has in the softmax
   static constexpr int S_PITCH = KT + 8, P_PITCH = KT + 8;
   static constexpr int TILE_BYTES = KT * PITCH * 2;
   static constexpr int S_OFF = STAGES * TILE_BYTES;
-  static constexpr int P_OFF = S_OFF + QUARTERS * HEADS * S_PITCH * 4;
-  static constexpr int A_OFF = P_OFF + 3 * HEADS * P_PITCH * 2;   // per head: the factor of this tile, at the end the sum
-  static constexpr int L_OFF = A_OFF + HEADS * 4;                 // per stage and row: whether the row counts
+  // scores, weights and factors of two tiles, in turn
+  static constexpr int S_FLOATS = QUARTERS * HEADS * S_PITCH, P_WORDS = 3 * HEADS * P_PITCH / 2;
+  static constexpr int P_OFF = S_OFF + 2 * S_FLOATS * 4;
+  static constexpr int A_OFF = P_OFF + 2 * P_WORDS * 4;          // per head: the factor of the tile, at the end the result's
+  static constexpr int L_OFF = A_OFF + 2 * HEADS * 4;            // per stage and row: whether the row counts
   static constexpr int BYTES = L_OFF + STAGES * KT * 4;
-  static_assert(KT == 4 * WARPS && KT % SPT == 0, "rows of a tile");
+  static_assert(KT % (SOFTMAX / 32) == 0 && KT % SPT == 0 && BYTES <= 227 * 1024, "rows of a tile");
 };
 
 __device__ __forceinline__ void latent_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -181,181 +187,85 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const __nv_bfloat16
   const int end = p + 1 - first > per * KT ? first + per * KT : p + 1;
   const int ntiles = max(0, (end - first + KT - 1) / KT);
 
-  // A warp brings in four neighbouring rows of a tile; where they lie is looked up one tile earlier (lane r: row r), so that
-  // the copies never wait for the page table.
-  constexpr int MINE = KT / WARPS;
-  auto look_up = [&](int i) -> long long {
-    const int key = first + i * KT + warp * MINE + (lane & (MINE - 1));
-    if (i >= ntiles || key >= end) return -1;
-    const int page = pages[key / page_size];
-    return page >= 0 && page < num_pages ? ((long long)page * page_size + key % page_size) * D : -1;
-  };
-  auto bring = [&](int i, long long rows) {
-    const int stage = i % Sh::STAGES;
-    if (i < ntiles) {
-      if (lane < MINE) counts[stage * KT + warp * MINE + lane] = rows >= 0;
+  // Tile i's scores are made in turn i - 1, its weights in turn i and its part of the result in turn i + 1, so that products and softmax always have
+  // something to do; it is asked for in turn i - 2 and its stage is free again behind turn i + 1.
+  if (warp < WARPS) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Sh::PRODUCT_REGISTERS));
+    const int quarter = warp & 3, half = warp >> 2;        // half: of the heads (32) or of a tile's keys (16)
+    const int gr = lane >> 2, gc = 2 * (lane & 3);
+    uint32_t q[STEPS][3][4];
+    {
+      const float* rows = q_lat + ((size_t)t * heads + h0 + (MG == 2 ? 16 * half : 0) + gr) * D + quarter * STEPS * 16 + gc;
 #pragma unroll
-      for (int j = 0; j < MINE; ++j) {
-        const long long at = __shfl_sync(0xffffffffu, rows, j);
-        const __nv_bfloat16* src = cache + (at < 0 ? 0 : at);
-        const uint32_t dst = tiles_at + stage * Sh::TILE_BYTES + (warp * MINE + j) * PITCH * 2;
+      for (int k = 0; k < STEPS; ++k) {
 #pragma unroll
-        for (int c = 0; c < D / 8; c += 32)
-          if (c + lane < D / 8) latent_copy16(dst + (c + lane) * 16, src + (c + lane) * 8, at >= 0);
+        for (int j = 0; j < 4; ++j) {
+          const float2 x = *reinterpret_cast<const float2*>(rows + (size_t)(j & 1) * 8 * D + k * 16 + (j >> 1) * 8);
+          uint32_t terms[3];
+          three_terms(x.x, x.y, terms);
+#pragma unroll
+          for (int e = 0; e < 3; ++e) q[k][e][j] = terms[e];
+        }
       }
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
+    float o[MG][8][4];
 #pragma unroll
-  for (int i = 0; i < Sh::STAGES - 1; ++i) bring(i, look_up(i));
-  long long next_rows = look_up(Sh::STAGES - 1);
-
-  const int quarter = warp & 3, half = warp >> 2;        // half: of the heads (32) or of a tile's keys (16)
-  const int gr = lane >> 2, gc = 2 * (lane & 3);
-  uint32_t q[STEPS][3][4];
-  {
-    const float* rows = q_lat + ((size_t)t * heads + h0 + (MG == 2 ? 16 * half : 0) + gr) * D + quarter * STEPS * 16 + gc;
+    for (int m = 0; m < MG; ++m)
 #pragma unroll
-    for (int k = 0; k < STEPS; ++k) {
+      for (int n = 0; n < 8; ++n)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 x = *reinterpret_cast<const float2*>(rows + (size_t)(j & 1) * 8 * D + k * 16 + (j >> 1) * 8);
-        uint32_t terms[3];
-        three_terms(x.x, x.y, terms);
+        for (int e = 0; e < 4; ++e) o[m][n][e] = 0.f;
+    auto products = [&](int i) {  // this warp's share of the scores of tile i
+      constexpr int NT = MG == 2 ? KT / 8 : KT / 16;
+      const uint32_t tile = tiles_at + (i % Sh::STAGES) * Sh::TILE_BYTES;
+      const int key0 = MG == 2 ? 0 : KT / 2 * half;
+      float s[NT][4];
 #pragma unroll
-        for (int e = 0; e < 3; ++e) q[k][e][j] = terms[e];
-      }
-    }
-  }
-  float o[MG][8][4];
+      for (int n = 0; n < NT; ++n)
 #pragma unroll
-  for (int m = 0; m < MG; ++m)
+        for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
+      const uint32_t at = tile + ((key0 + (lane & 7) + 8 * (lane >> 4)) * PITCH + quarter * STEPS * 16 + 8 * ((lane >> 3) & 1)) * 2;
 #pragma unroll
-    for (int n = 0; n < 8; ++n)
+      for (int k = 0; k < STEPS; k += 2) {
+        constexpr int LAST = STEPS - 1;
+        const int steps = k < LAST ? 2 : 1;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) o[m][n][e] = 0.f;
-  // the softmax's share of a thread: SPT neighbouring keys of one head
-  constexpr int SPT = Sh::SPT, PER_HEAD = KT / SPT;
-  const int head = threadIdx.x / PER_HEAD, key_at = (threadIdx.x % PER_HEAD) * SPT;
-  float m_run = -FLT_MAX, l_run = 0.f;
-
-  auto products = [&](int i) {  // this warp's share of the scores of tile i
-    constexpr int NT = MG == 2 ? KT / 8 : KT / 16;
-    const uint32_t tile = tiles_at + (i % Sh::STAGES) * Sh::TILE_BYTES;
-    const int key0 = MG == 2 ? 0 : KT / 2 * half;
-    float s[NT][4];
+        for (int n = 0; n < NT; n += 2) {
+          uint32_t b[2][4];
+          float d0[4], d1[4];
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
+          for (int x = 0; x < steps; ++x) latent_ldmatrix(b[x], at + (n * 8 * PITCH + (k + x) * 16) * 2);
+          latent_mma_first(d0, q[k][2], b[0][0], b[0][1]);
+          latent_mma_first(d1, q[k][2], b[0][2], b[0][3]);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
-    const uint32_t at = tile + ((key0 + (lane & 7) + 8 * (lane >> 4)) * PITCH + quarter * STEPS * 16 + 8 * ((lane >> 3) & 1)) * 2;
+          for (int e = 2; e >= 0; --e)
 #pragma unroll
-    for (int k = 0; k < STEPS; k += 2) {
-      constexpr int LAST = STEPS - 1;
-      const int steps = k < LAST ? 2 : 1;
+            for (int x = e == 2 ? 1 : 0; x < steps; ++x) {
+              latent_mma(d0, q[k + x][e], b[x][0], b[x][1]);
+              latent_mma(d1, q[k + x][e], b[x][2], b[x][3]);
+            }
 #pragma unroll
-      for (int n = 0; n < NT; n += 2) {
-        uint32_t b[2][4];
-        float d0[4], d1[4];
-#pragma unroll
-        for (int x = 0; x < steps; ++x) latent_ldmatrix(b[x], at + (n * 8 * PITCH + (k + x) * 16) * 2);
-        latent_mma_first(d0, q[k][2], b[0][0], b[0][1]);
-        latent_mma_first(d1, q[k][2], b[0][2], b[0][3]);
-#pragma unroll
-        for (int e = 2; e >= 0; --e)
-#pragma unroll
-          for (int x = e == 2 ? 1 : 0; x < steps; ++x) {
-            latent_mma(d0, q[k + x][e], b[x][0], b[x][1]);
-            latent_mma(d1, q[k + x][e], b[x][2], b[x][3]);
+          for (int x = 0; x < 4; ++x) {
+            s[n][x] += d0[x];
+            s[n + 1][x] += d1[x];
           }
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          s[n][x] += d0[x];
-          s[n + 1][x] += d1[x];
         }
       }
-    }
-    float* dst = scores + (quarter * HEADS + (MG == 2 ? 16 * half : 0) + gr) * Sh::S_PITCH + key0 + gc;
+      float* dst = scores + (i & 1) * Sh::S_FLOATS + (quarter * HEADS + (MG == 2 ? 16 * half : 0) + gr) * Sh::S_PITCH + key0 + gc;
 #pragma unroll
-    for (int n = 0; n < NT; ++n) {
-      *reinterpret_cast<float2*>(dst + n * 8) = make_float2(s[n][0], s[n][1]);
-      *reinterpret_cast<float2*>(dst + 8 * Sh::S_PITCH + n * 8) = make_float2(s[n][2], s[n][3]);
-    }
-  };
-
-  asm volatile("cp.async.wait_group %0;" ::"n"(Sh::STAGES - 2) : "memory");
-  __syncthreads();
-  if (ntiles > 0) products(0);
-  for (int i = 0; i < ntiles; ++i) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(Sh::STAGES - 3) : "memory");
-    __syncthreads();  // the scores of tile i are there, tile i + 1 too, and everybody has left the stage of tile i - 1
-    bring(i + Sh::STAGES - 1, next_rows);
-    next_rows = look_up(i + Sh::STAGES);
-    {
-      float s[SPT];
-#pragma unroll
-      for (int j = 0; j < SPT; ++j) s[j] = 0.f;
-      bool on[SPT];
-#pragma unroll
-      for (int j = 0; j < SPT; j += 2) {
-#pragma unroll
-        for (int e = 0; e < QUARTERS; ++e) {
-          const float2 part = *reinterpret_cast<const float2*>(scores + (e * HEADS + head) * Sh::S_PITCH + key_at + j);
-          s[j] += part.x;
-          s[j + 1] += part.y;
-        }
-        const int2 live = *reinterpret_cast<const int2*>(counts + (i % Sh::STAGES) * KT + key_at + j);
-        on[j] = live.x != 0;
-        on[j + 1] = live.y != 0;
+      for (int n = 0; n < NT; ++n) {
+        *reinterpret_cast<float2*>(dst + n * 8) = make_float2(s[n][0], s[n][1]);
+        *reinterpret_cast<float2*>(dst + 8 * Sh::S_PITCH + n * 8) = make_float2(s[n][2], s[n][3]);
       }
-      // An infinity of the row times a term that is 0 is NaN, and so is a query beyond bfloat16's range: such a score is made again
-      // from the numbers themselves, and -inf drops out as it should.  (A value that is infinite may still come out as NaN.)
-#pragma unroll
-      for (int j = 0; j < SPT; ++j) {
-        if (!on[j] || s[j] == s[j]) continue;
-        const float* query = q_lat + ((size_t)t * heads + h0 + head) * D;
-        const __nv_bfloat16* row = reinterpret_cast<const __nv_bfloat16*>(latent_smem + (i % Sh::STAGES) * Sh::TILE_BYTES) + (key_at + j) * PITCH;
-        float sum = 0.f;
-#pragma unroll 1
-        for (int d = 0; d < D; ++d) sum = fmaf(query[d], __bfloat162float(row[d]), sum);
-        s[j] = sum;
-      }
-      float m_new = m_run;
-#pragma unroll
-      for (int e = 0; e < SPT; ++e) {
-        s[e] *= scale;
-        if (on[e]) m_new = fmaxf(m_new, s[e]);
-      }
-#pragma unroll
-      for (int off = 1; off < PER_HEAD; off <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, off));
-      const float alpha = expf(m_run - m_new);  // first tile: exp(-huge) = 0; no key that counts so far: 1, of nothing
-      float w[SPT], add = 0.f;
-#pragma unroll
-      for (int e = 0; e < SPT; ++e) {
-        w[e] = on[e] ? expf(s[e] - m_new) : 0.f;
-        add += w[e];
-      }
-      l_run = fmaf(l_run, alpha, add);
-      m_run = m_new;
-#pragma unroll
-      for (int j = 0; j < SPT; j += 2) {
-        uint32_t a[3];
-        three_terms(w[j], w[j + 1], a);
-#pragma unroll
-        for (int e = 0; e < 3; ++e) weights[((e * HEADS + head) * Sh::P_PITCH + key_at + j) / 2] = a[e];
-      }
-      if (key_at == 0) factors[head] = alpha;
-    }
-    __syncthreads();
-    if (i + 1 < ntiles) products(i + 1);
-    {
+    };
+    auto weighted = [&](int i) {  // O += P V of tile i
       const uint32_t tile = tiles_at + (i % Sh::STAGES) * Sh::TILE_BYTES;
       static_assert(KT == 32, "two steps of keys");
       const uint32_t at = tile + ((lane & 15) * PITCH + 64 * warp + 8 * (lane >> 4)) * 2;
-      const uint32_t wat = weights_at + ((lane & 15) * Sh::P_PITCH + 8 * (lane >> 4)) * 2;
+      const uint32_t wat = weights_at + (i & 1) * Sh::P_WORDS * 4 + ((lane & 15) * Sh::P_PITCH + 8 * (lane >> 4)) * 2;
 #pragma unroll
       for (int m = 0; m < MG; ++m) {
-        const float f0 = factors[16 * m + gr], f1 = factors[16 * m + gr + 8];
+        const float f0 = factors[(i & 1) * HEADS + 16 * m + gr], f1 = factors[(i & 1) * HEADS + 16 * m + gr + 8];
         uint32_t a[2][3][4];
 #pragma unroll
         for (int k = 0; k < 2; ++k)
@@ -383,44 +293,158 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const __nv_bfloat16
           }
         }
       }
+    };
+    __syncthreads();  // tile 0 is there
+    if (ntiles > 0) products(0);
+    __syncthreads();
+    for (int i = 0; i <= ntiles; ++i) {
+      if (i + 1 < ntiles) products(i + 1);
+      if (i > 0) weighted(i - 1);
+      if (i < ntiles) __syncthreads();
     }
-  }
+    if (shares > tokens) {  // a token's shares together: [heads, splits, RANK + 2]
+      float* mine = partial + ((size_t)run.first * heads + (size_t)h0 * splits + split) * (RANK + 2);
 #pragma unroll
-  for (int off = 1; off < PER_HEAD; off <<= 1) l_run += __shfl_xor_sync(0xffffffffu, l_run, off);
-  if (shares > tokens) {  // a token's shares together: [heads, splits, RANK + 2]; where they are stands in its rows of the result, if that's to be found
-    float* mine = partial + ((size_t)run.first * heads + (size_t)h0 * splits + split) * (RANK + 2);
-    if (each == 0 && split == 0 && threadIdx.x < HEADS) *reinterpret_cast<int2*>(out + ((size_t)t * heads + h0 + threadIdx.x) * RANK) = make_int2(run.first, splits);
-    if (key_at == 0) *reinterpret_cast<float2*>(mine + (size_t)head * splits * (RANK + 2)) = make_float2(m_run, l_run);
+      for (int m = 0; m < MG; ++m)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          float* row = mine + (size_t)(16 * m + gr + 8 * r) * splits * (RANK + 2) + 2 + 64 * warp + gc;
+#pragma unroll
+          for (int n = 0; n < 8; ++n) *reinterpret_cast<float2*>(row + n * 8) = make_float2(o[m][n][2 * r], o[m][n][2 * r + 1]);
+        }
+      return;
+    }
+    __syncthreads();  // the results' factors are there
 #pragma unroll
     for (int m = 0; m < MG; ++m)
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        float* row = mine + (size_t)(16 * m + gr + 8 * r) * splits * (RANK + 2) + 2 + 64 * warp + gc;
+        const int h = 16 * m + gr + 8 * r;
+        const float f = factors[(ntiles & 1) * HEADS + h];
+        __nv_bfloat16* row = out + ((size_t)t * heads + h0 + h) * RANK + 64 * warp + gc;
 #pragma unroll
-        for (int n = 0; n < 8; ++n) *reinterpret_cast<float2*>(row + n * 8) = make_float2(o[m][n][2 * r], o[m][n][2 * r + 1]);
+        for (int n = 0; n < 8; ++n) *reinterpret_cast<__nv_bfloat162*>(row + n * 8) = __floats2bfloat162_rn(o[m][n][2 * r] * f, o[m][n][2 * r + 1] * f);
       }
-    return;
-  }
-  __syncthreads();  // the last tile's factors have been read
-  if (key_at == 0) {
-    float by = 1.f / l_run;
-    if (sink) {
-      const float sk = sink[h0 + head], top = fmaxf(m_run, sk), down = expf(m_run - top);
-      by = down / fmaf(l_run, down, expf(sk - top));
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Sh::SOFTMAX_REGISTERS));
+    // A warp brings in eight neighbouring rows of a tile; where they lie is looked up one tile earlier (lane r: row r), so that
+    // the copies never wait for the page table.
+    constexpr int MINE = KT / (SOFTMAX / 32);
+    const int first_row = (warp - WARPS) * MINE;
+    auto look_up = [&](int i) -> long long {
+      const int key = first + i * KT + first_row + (lane & (MINE - 1));
+      if (i >= ntiles || key >= end) return -1;
+      const int page = pages[key / page_size];
+      return page >= 0 && page < num_pages ? ((long long)page * page_size + key % page_size) * D : -1;
+    };
+    auto bring = [&](int i, long long rows) {
+      const int stage = i % Sh::STAGES;
+      if (i < ntiles) {
+        if (lane < MINE) counts[stage * KT + first_row + lane] = rows >= 0;
+#pragma unroll
+        for (int j = 0; j < MINE; ++j) {
+          const long long at = __shfl_sync(0xffffffffu, rows, j);
+          const __nv_bfloat16* src = cache + (at < 0 ? 0 : at);
+          const uint32_t dst = tiles_at + stage * Sh::TILE_BYTES + (first_row + j) * PITCH * 2;
+#pragma unroll
+          for (int c = 0; c < D / 8; c += 32)
+            if (c + lane < D / 8) latent_copy16(dst + (c + lane) * 16, src + (c + lane) * 8, at >= 0);
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    bring(0, look_up(0));
+    bring(1, look_up(1));
+    long long next_rows = look_up(2);
+    // the softmax's share of a thread: SPT neighbouring keys of one head
+    constexpr int SPT = Sh::SPT, PER_HEAD = KT / SPT;
+    const int head = (threadIdx.x - 32 * WARPS) / PER_HEAD, key_at = ((threadIdx.x - 32 * WARPS) % PER_HEAD) * SPT;
+    float m_run = -FLT_MAX, l_run = 0.f;
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // tile 0 is there
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // its scores and tile 1 are
+    for (int i = 0; i < ntiles; ++i) {
+      bring(i + 2, next_rows);
+      next_rows = look_up(i + 3);
+      {
+        float s[SPT];
+#pragma unroll
+        for (int j = 0; j < SPT; ++j) s[j] = 0.f;
+        bool on[SPT];
+#pragma unroll
+        for (int j = 0; j < SPT; j += 2) {
+#pragma unroll
+          for (int e = 0; e < QUARTERS; ++e) {
+            const float2 part = *reinterpret_cast<const float2*>(scores + (i & 1) * Sh::S_FLOATS + (e * HEADS + head) * Sh::S_PITCH + key_at + j);
+            s[j] += part.x;
+            s[j + 1] += part.y;
+          }
+          const int2 live = *reinterpret_cast<const int2*>(counts + (i % Sh::STAGES) * KT + key_at + j);
+          on[j] = live.x != 0;
+          on[j + 1] = live.y != 0;
+        }
+        // An infinity of the row times a term that is 0 is NaN, and so is a query beyond bfloat16's range: such a score is made again
+        // from the numbers themselves, and -inf drops out as it should.  (A value that is infinite may still come out as NaN.)
+#pragma unroll
+        for (int j = 0; j < SPT; ++j) {
+          if (!on[j] || s[j] == s[j]) continue;
+          const float* query = q_lat + ((size_t)t * heads + h0 + head) * D;
+          const __nv_bfloat16* row = reinterpret_cast<const __nv_bfloat16*>(latent_smem + (i % Sh::STAGES) * Sh::TILE_BYTES) + (key_at + j) * PITCH;
+          float sum = 0.f;
+#pragma unroll 1
+          for (int d = 0; d < D; ++d) sum = fmaf(query[d], __bfloat162float(row[d]), sum);
+          s[j] = sum;
+        }
+        float m_new = m_run;
+#pragma unroll
+        for (int e = 0; e < SPT; ++e) {
+          s[e] *= scale;
+          if (on[e]) m_new = fmaxf(m_new, s[e]);
+        }
+#pragma unroll
+        for (int off = 1; off < PER_HEAD; off <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, off));
+        const float alpha = expf(m_run - m_new);  // first tile: exp(-huge) = 0; no key that counts so far: 1, of nothing
+        float w[SPT], add = 0.f;
+#pragma unroll
+        for (int e = 0; e < SPT; ++e) {
+          w[e] = on[e] ? expf(s[e] - m_new) : 0.f;
+          add += w[e];
+        }
+        l_run = fmaf(l_run, alpha, add);
+        m_run = m_new;
+#pragma unroll
+        for (int j = 0; j < SPT; j += 2) {
+          uint32_t a[3];
+          three_terms(w[j], w[j + 1], a);
+#pragma unroll
+          for (int e = 0; e < 3; ++e) weights[(i & 1) * Sh::P_WORDS + ((e * HEADS + head) * Sh::P_PITCH + key_at + j) / 2] = a[e];
+        }
+        if (key_at == 0) factors[(i & 1) * HEADS + head] = alpha;
+      }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
     }
-    factors[head] = by * (gate ? gate[(size_t)t * heads + h0 + head] : 1.f);
-  }
-  __syncthreads();
 #pragma unroll
-  for (int m = 0; m < MG; ++m)
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const int h = 16 * m + gr + 8 * r;
-      const float f = factors[h];
-      __nv_bfloat16* row = out + ((size_t)t * heads + h0 + h) * RANK + 64 * warp + gc;
-#pragma unroll
-      for (int n = 0; n < 8; ++n) *reinterpret_cast<__nv_bfloat162*>(row + n * 8) = __floats2bfloat162_rn(o[m][n][2 * r] * f, o[m][n][2 * r + 1] * f);
+    for (int off = 1; off < PER_HEAD; off <<= 1) l_run += __shfl_xor_sync(0xffffffffu, l_run, off);
+    if (shares > tokens) {
+      float* mine = partial + ((size_t)run.first * heads + (size_t)h0 * splits + split) * (RANK + 2);
+      // where a token's shares are stands in its rows of the result, if that's to be found
+      const int at = threadIdx.x - 32 * WARPS;
+      if (each == 0 && split == 0 && at < HEADS) *reinterpret_cast<int2*>(out + ((size_t)t * heads + h0 + at) * RANK) = make_int2(run.first, splits);
+      if (key_at == 0) *reinterpret_cast<float2*>(mine + (size_t)head * splits * (RANK + 2)) = make_float2(m_run, l_run);
+      return;
     }
+    if (key_at == 0) {
+      float by = 1.f / l_run;
+      if (sink) {
+        const float sk = sink[h0 + head], top = fmaxf(m_run, sk), down = expf(m_run - top);
+        by = down / fmaf(l_run, down, expf(sk - top));
+      }
+      factors[(ntiles & 1) * HEADS + head] = by * (gate ? gate[(size_t)t * heads + h0 + head] : 1.f);  // (not the last tile's place)
+    }
+    __syncthreads();
+  }
 }
 
 // A block per (token, head): the shares of the blocks that split its keys, every other one a group of threads, asked for before

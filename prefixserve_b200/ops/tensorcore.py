@@ -36,6 +36,12 @@ FEWROWS_MAX = {"plain": 64, "gated": 64, "rope": 64}
 WIDE_BELOW_TILES = 600   # matrices with fewer 16-row tiles than this get 16 warps per CTA instead of 8
 TCGEN05_PREFILL_MIN_TOKENS = 64   # steps whose longest prompt portion has at least this many tokens run prefill attention
                                   # on the tcgen05 kernel (tiles of 128 rows); shorter portions fill too little of a tile
+# ... and shorter ones too where their CTAs fit in one round over the SMs and they see at least so many keys (by head size): the other kernel
+# (mma.sync, all heads of a group in one tile) walks a portion's keys in one chain, 20 to 26 us a 1,024 of them, this one takes 17 (64) and 18 (128) and cuts
+# them into ranges besides.  32 heads over 8, one portion of 24 tokens, us by keys 512, 1,024, 2,048, 4,000: 15.0 25.5 46.6 85.9 there, 14.7 22.8 19.0
+# 25.5 here (heads of 64); 19.3 32.6 59.0 109 and 15.1 14.4 18.8 26.6 (128); three portions of eight 14.9 25.3 46.1 84.9 and 15.3 23.6 40.3 71.2; 17.4 30.2
+# 55.8 104 and 15.5 24.3 41.8 74.0.  In two rounds it loses up to 16 tokens (eight portions of eight, 4,000 keys 91.9 and 123.9).
+TCGEN05_SHORT_MIN_KEYS = {64: 1024, 128: 512}
 USE_TMA_DECODE = True     # decode attention: the kernel whose keys and values the TMA unit brings in (pages of 16 tokens
                           # or more), for key ranges of at least TMA_DECODE_MIN_RANGE keys; otherwise the one in which
                           # every lane copies its own pieces.  Measured at Llama-1B sizes, context 4,096, ms a decode step
@@ -445,6 +451,14 @@ def _decode_key_range(pairs: int, longest: int, sms: int, tma_kernel: bool, ctas
     return best[2]
 
 
+def _short_portions_in_tiles(portions: Sequence[int], kv_lens: Sequence[int], window: int, heads: int, d: int, sms: int, static_kv_len: int | None) -> bool:
+    """Whether portions shorter than TCGEN05_PREFILL_MIN_TOKENS are over sooner on the kernel of 128-row tiles."""
+    keys = static_kv_len if static_kv_len is not None else max(kv_lens)
+    if window:
+        keys = min(keys, window + max(portions))
+    return heads * len(portions) <= sms and keys >= TCGEN05_SHORT_MIN_KEYS.get(d, 1 << 30)
+
+
 def _attention_plan(new_tokens: Sequence[int], kv_lens: Sequence[int], window: int, group: int, hkv: int, d: int, page: int,
                     sms: int, static_kv_len: int | None) -> dict:
     """Launch shapes of a step's attention, from the host copies of the items' lengths.  The same for every layer with
@@ -470,8 +484,10 @@ def _attention_plan(new_tokens: Sequence[int], kv_lens: Sequence[int], window: i
         plan["max_splits"] = -(-longest // plan["chunk"])
         plan["all_single"] = 1 if len(singles) == b else 0
     portions = [n for n in new_tokens if not (plan["use_decode"] and n == 1)]
-    plan["tcgen05"] = bool(USE_TCGEN05 and portions and max(portions) >= TCGEN05_PREFILL_MIN_TOKENS
-                           and lib().psb_attention_prefill_tcgen05_supported(d, page))
+    plan["tcgen05"] = bool(USE_TCGEN05 and portions and lib().psb_attention_prefill_tcgen05_supported(d, page)
+                           and (max(portions) >= TCGEN05_PREFILL_MIN_TOKENS
+                                or _short_portions_in_tiles(portions, [kvl for n, kvl in zip(new_tokens, kv_lens) if not (plan["use_decode"] and n == 1)],
+                                                            window, hq_total, d, sms, static_kv_len)))
     if plan["tcgen05"]:
         # a CTA takes 256 rows of one head as two tiles that fill each other's waits; when that leaves more than half
         # of the SMs without a CTA (a few hundred new tokens), one tile each and twice the CTAs (measured at 32 heads:

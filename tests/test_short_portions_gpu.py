@@ -1,0 +1,43 @@
+"""Short prompt portions behind long contexts: which kernel attends for them, and that both agree with the general one to what bfloat16 weights and results
+give (2e-2 of numbers of about one, the bound of the other attention tests)."""
+
+import pytest
+import torch
+
+from prefixserve_b200 import ops
+from prefixserve_b200.engine import StepItem  # noqa: F401  (the engine's package loads)
+from prefixserve_b200.ops import library
+from prefixserve_b200.parts.base import ItemView, StepContext
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("d,hq,hkv,window,portions,taken", [
+    (64, 32, 8, None, [(31, 2000)], True), (64, 32, 8, None, [(2, 1022)], True), (64, 32, 8, None, [(2, 1021)], False),       # 1,024 keys
+    (128, 32, 8, None, [(63, 449), (1, 700), (5, 100)], True), (128, 32, 8, None, [(63, 448)], False),                         # 512 keys; beside a decoded token
+    (64, 32, 8, None, [(9, 1500)] * 4, True), (64, 32, 8, None, [(9, 1500)] * 5, False),                                       # 128 and 160 CTAs on 148 SMs
+    (128, 8, 8, 300, [(20, 3000)], False), (128, 8, 4, 500, [(20, 3000), (1, 2000)], True), (128, 6, 1, None, [(3, 4000)], True)])
+def test_short_portions(d, hq, hkv, window, portions, taken):
+    page, gen = 16, torch.Generator(device="cuda").manual_seed(d + len(portions))
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    starts, views = [0], []
+    for i, (n, held) in enumerate(portions):
+        views.append(ItemView(slot=i, start=held, end=held + n, first_token=starts[-1]))
+        starts.append(starts[-1] + n)
+    width = max(-(-(n + held) // page) for n, held in portions)
+    table = torch.randperm(len(portions) * width, generator=gen, device="cuda").to(torch.int32).view(len(portions), width)
+    ctx = StepContext(
+        num_tokens=starts[-1], num_items=len(portions), compute_dtype=torch.bfloat16, device=torch.device("cuda"), items=views,
+        token_ids=i32([0] * starts[-1]), positions=i32([p for n, held in portions for p in range(held, held + n)]),
+        token_item=i32([i for i, (n, _) in enumerate(portions) for _ in range(n)]), item_start=i32(starts), kv_len=i32([n + held for n, held in portions]),
+        slots=i32(list(range(len(portions)))), block_tables={0: table}, max_new_tokens=max(n for n, _ in portions),
+        max_kv_len=max(n + held for n, held in portions), all_decode=False)
+    q = torch.randn(starts[-1], hq, d, generator=gen, device="cuda").to(torch.bfloat16)
+    kv = torch.randn(len(portions) * width, 2, hkv, page, d, generator=gen, device="cuda").to(torch.bfloat16)
+    before = library.launch_counts.copy()
+    out = ops.attention(q, kv, table, ctx.positions, ctx.token_item, window=window, ctx=ctx)
+    counts = library.launch_counts - before
+    assert counts["attention_prefill_tcgen05"] == taken and counts["attention_prefill"] == (not taken)
+    want = ops.attention(q, kv, table, ctx.positions, ctx.token_item, window=window)  # (without the step: the general kernel)
+    assert library.tcgen05_status() == 0
+    assert torch.allclose(out.float(), want.float().view_as(out), atol=2e-2, rtol=2e-2), float((out.float() - want.float().view_as(out)).abs().max())

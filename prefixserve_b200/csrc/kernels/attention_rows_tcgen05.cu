@@ -401,6 +401,13 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
         return true;
       };
       if (nblk > 0) ok = request_scores(0);
+      // Left to themselves both tiles make the same step of a block at the same time: the products of both, then the caps (or biases) of both, then the
+      // exponentials, each on a unit of its own that is idle meanwhile.  A start half a block apart keeps them apart: 1,500 and 1,200 capped tokens 76.2 us ->
+      // 72.0 (1,200 to 1,600 clocks; 800 73.9, 2,000 73.0), with a bias 71.6 -> 69.6; plain scores, whose steps are the products and the exponentials, no difference.
+      if (MODE != PLAIN && t == 1) {
+        const long long from = clock64();
+        while (clock64() - from < 1300) {}
+      }
       for (int i = 0; ok && i < nblk; ++i) {
         const bool kept = is_kept(i);
         const int key0 = base_of(i);

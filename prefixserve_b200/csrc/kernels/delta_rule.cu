@@ -222,7 +222,7 @@ delta_prepare_run_kernel(const T* __restrict__ proj, const float* __restrict__ b
 // sizes): a warp takes a unit and a run of eight tokens, four neighbouring channels a lane, so that the inputs come in 8 (16) bytes a
 // lane, the results leave in 16 and the sums of squares need no barrier.  What a token's place in its portion decides is asked for once
 // a warp, and only a run at a portion's start looks at the slot.  Bound by what its warps issue (the taps and the SiLU of every
-// channel).  2,000 tokens of 16 heads over 8 groups of 128: 26 us, with a channel a thread 47.
+// channel).  2,000 tokens of 16 heads over 8 groups of 128: 21 us (28 with a division for every SiLU and each sum of squares by itself), with a channel a thread 47.
 template <typename T>
 __device__ __forceinline__ void load_four(const T* p, float (&v)[4]) {
   if constexpr (sizeof(T) == 2) {
@@ -294,7 +294,7 @@ delta_prepare_wide_kernel(const T* __restrict__ proj, const float* __restrict__ 
         float acc = 0.f;
 #pragma unroll
         for (int k = RUN_TAPS - 1; k >= 0; --k) acc = fmaf(w[j][k], x[i + RUN_TAPS - 1 - k][j], acc);
-        y[i][j] = siluf_(acc);  // (zero where there is no channel)
+        y[i][j] = acc;  // (zero where there is no channel)
       }
   } else {
 #pragma unroll
@@ -311,19 +311,35 @@ delta_prepare_wide_kernel(const T* __restrict__ proj, const float* __restrict__ 
             v = mine && k <= pos_i ? state[(size_t)slot_i * slot_floats + (size_t)(K - 1 - (k - own_i)) * C + c + j] : 0.f;
           acc = fmaf(w[j][k], v, acc);
         }
-        y[i][j] = mine ? siluf_(acc) : 0.f;
+        y[i][j] = mine ? acc : 0.f;
       }
     }
   }
+  silu_all(y);
   if (there && unit < 2 * G) {  // unit vectors; queries also times dim^-1/2
+    float ss[RUN_TOKENS];
 #pragma unroll
     for (int i = 0; i < RUN_TOKENS; ++i) {
-      float ss = 0.f;
+      ss[i] = 0.f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) ss = fmaf(y[i][j], y[i][j], ss);
-      const float factor = unit_factor(warp_sum(ss), unit < G ? dim : 1);
+      for (int j = 0; j < 4; ++j) ss[i] = fmaf(y[i][j], y[i][j], ss[i]);
+    }
+    // all tokens' sums over the warp at a time: four lanes end up with each, and make its factor
+    static_assert(RUN_TOKENS == 8, "a token per four lanes");
 #pragma unroll
-      for (int j = 0; j < 4; ++j) y[i][j] *= factor;
+    for (int m = 4, off = 16; m > 0; m >>= 1, off >>= 1) {
+      const bool up = lane & off;
+#pragma unroll
+      for (int e = 0; e < m; ++e) ss[e] = (up ? ss[e + m] : ss[e]) + __shfl_xor_sync(0xffffffffu, up ? ss[e] : ss[e + m], off);
+    }
+    ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 2);
+    ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
+    const float factor = unit_factor(ss[0], unit < G ? dim : 1);
+#pragma unroll
+    for (int i = 0; i < RUN_TOKENS; ++i) {
+      const float f = __shfl_sync(0xffffffffu, factor, 4 * i);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) y[i][j] *= f;
     }
   }
 #pragma unroll
@@ -1081,6 +1097,7 @@ delta_finish_wide_kernel(const float* __restrict__ o, const T* __restrict__ proj
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) g[j] = mine ? gain[4 * lane + j] : 0.f;
+  silu_all(z);
 #pragma unroll
   for (int u = 0; u < FINISH_UNITS; ++u) {
     float ss = 0.f;
@@ -1090,7 +1107,7 @@ delta_finish_wide_kernel(const float* __restrict__ o, const T* __restrict__ proj
     if (!mine || first + u >= units) continue;
     float v[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = x[u][j] * inv * g[j] * siluf_(z[u][j]);
+    for (int j = 0; j < 4; ++j) v[j] = x[u][j] * inv * g[j] * z[u][j];
     T* dst = out + (size_t)(first + u) * vdim + 4 * lane;
     if constexpr (sizeof(T) == 2) {
       __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);

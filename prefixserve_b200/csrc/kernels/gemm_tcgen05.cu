@@ -41,6 +41,8 @@ __host__ __device__ constexpr int part_columns(int bn, int parts) { return (bn /
 constexpr int TMEM_COLS = 512;              // two accumulator buffers, 256 float32 columns apart
 constexpr int ACC_STRIDE = 256;
 constexpr int MAX_STAGES = 6;
+// What a storing warp of two CTAs' tiles has of shared memory: 32 rows of 32 results, on their way out (see leave_rows).
+constexpr int LEAVING_WARP = 32 * 32 * 2, LEAVING_BYTES = 8 * LEAVING_WARP;
 
 // The output tile is 128 rows by BN columns: 256 where that fills the SMs evenly, 192 where it does not (a product of
 // 192 tiles of 256 columns takes 148 CTAs two rounds, as 256 tiles of 192 columns two rounds of three quarters the size),
@@ -182,8 +184,37 @@ __device__ __forceinline__ float divided(float n, float d) {
   return fmaf(fmaf(-q, d, n), r, q);
 }
 
-// One thread's row of a tile of sums: what the epilogue does, in two parts around the wait for the sums.
-template <int BN, int HB>
+// 32 columns of the warp's rows, a thread a row, from ``col`` on as far as there are columns (``limit``); rows from M on stay.  They go through shared memory
+// (pieces of 16 bytes, piece j of row r at j ^ (r / 2 % 4)) to where four lanes have a row's 64 bytes: stored by the thread that has the row, every 16 bytes are
+// half a sector on a line of their own.  Where a CTA's tiles follow one another and their stores are in the way, as in two CTAs a tile: routed experts on 2,037
+// tokens (8,148 rows of 2,048 by 1,024 in the second product: 50 us -> 42) 159 us a call -> 154, 142 -> 133 without gates, 1,979 tokens of feed-forward up to 1 % less.
+// A CTA's only tile leaves sooner straight from the registers (300 rows of 8,192 gated and 2,048 columns 44.0 us instead of 43.5).
+__device__ __forceinline__ void leave_rows(uint4* leaving, const uint32_t (&packed)[4][4], __nv_bfloat16* __restrict__ C, int row, int M, int col, int limit, int ldc) {
+  const int lane = threadIdx.x & 31, row0 = row - lane;
+  if (col + 32 <= limit && (ldc & 7) == 0) {
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) leaving[lane * 4 + (j ^ ((lane >> 1) & 3))] = make_uint4(packed[j][0], packed[j][1], packed[j][2], packed[j][3]);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int in = 8 * i + (lane >> 2), piece = lane & 3;
+      if (row0 + in < M) *reinterpret_cast<uint4*>(C + (size_t)(row0 + in) * ldc + col + 8 * piece) = leaving[in * 4 + (piece ^ ((in >> 1) & 3))];
+    }
+    __syncwarp();
+  } else if (row < M) {
+    __nv_bfloat16* crow = C + (size_t)row * ldc;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(packed[j]);
+      for (int q = 0; q < 8; ++q)
+        if (col + 8 * j + q < limit) crow[col + 8 * j + q] = e[q];
+    }
+  }
+}
+
+// One thread's row of a tile of sums: what the epilogue does, in two parts around the wait for the sums.  LEAVE: results go through shared memory.
+template <int BN, int HB, bool LEAVE = false>
 struct Epilogue {
   static constexpr int BN_HALF = BN / 2, PARTS = store_warps(HB) / 4;
   int pos = 0, page = -1;
@@ -205,6 +236,17 @@ struct Epilogue {
         }
       }
     }
+  }
+  // two results of a plain product with an activation
+  __device__ __forceinline__ static uint32_t activated(float v0, float v1, int mode) {
+    if (mode == MODE_RELU2) {
+      v0 = fmaxf(v0, 0.f), v1 = fmaxf(v1, 0.f);
+      v0 *= v0, v1 *= v1;
+    } else if (mode == MODE_SILU || mode == MODE_GELU) {
+      const int act = mode == MODE_SILU ? PSB_ACT_SILU : PSB_ACT_GELU_TANH;
+      v0 = quick_act(v0, act), v1 = quick_act(v1, act);
+    }
+    return pack2(v0, v1);
   }
   // ``value``: of the two rounded sums; ``quick`` the same where every |gate sum| * ``rate`` of the 32 is at most QUICK_UP_TO
   template <typename Quick, typename Value>
@@ -246,16 +288,52 @@ struct Epilogue {
       else columns(value);
     }
   }
+  // the same, through shared memory
+  template <typename Quick, typename Value>
+  __device__ __forceinline__ static void gated_columns_leave(uint32_t taddr, int row, int M, int n0, __nv_bfloat16* __restrict__ C, int N_out, int ldc, int part, float rate,
+                                                             uint4* leaving, Quick quick, Value value) {
+#pragma unroll 1
+    for (int c = part * (BN_HALF / PARTS); c < (part + 1) * (BN_HALF / PARTS); c += 32) {
+      uint32_t g[32], u[32];
+      tmem_ld32(taddr + c, g);
+      tmem_ld32(taddr + BN_HALF + c, u);
+      tmem_ld_wait();
+      if (row - (int)(threadIdx.x & 31) >= M) continue;
+      uint32_t packed[4][4] = {};
+      auto columns = [&](auto of) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t gb = pack2(__uint_as_float(g[8 * j + 2 * q]), __uint_as_float(g[8 * j + 2 * q + 1]));
+            const uint32_t ub = pack2(__uint_as_float(u[8 * j + 2 * q]), __uint_as_float(u[8 * j + 2 * q + 1]));
+            packed[j][q] = pack2(of(__uint_as_float(gb << 16), __uint_as_float(ub << 16)),
+                                 of(__uint_as_float(gb & 0xffff0000u), __uint_as_float(ub & 0xffff0000u)));
+          }
+      };
+      if (row < M) {
+        float top = 0.f;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) top = fmaxf(top, fabsf(__uint_as_float(g[j])));
+        if (top * rate <= QUICK_UP_TO) columns(quick);
+        else columns(value);
+      }
+      leave_rows(leaving, packed, C, row, M, n0 + c, N_out, ldc);
+    }
+  }
   // (M: rows there are; the tile's columns start at n0; part: which half of the columns, where two warps share the rows)
   __device__ __forceinline__ void store(uint32_t taddr, int row, int M, int n0, __nv_bfloat16* __restrict__ C, int N_out, int ldc, int mode, bool gated,
-                                        const RopeArgs& rope, const GluArgs& glu, const float* __restrict__ row_scale, int part) const {
+                                        const RopeArgs& rope, const GluArgs& glu, const float* __restrict__ row_scale, int part, uint4* leaving = nullptr) const {
     __nv_bfloat16* crow = C + (size_t)row * ldc;
     if (mode == MODE_ROPE) {
       rope_store_row<BN, HB>(taddr, row, M, n0, N_out, rope, pos, page, cs, sn, part);
     } else if (gated) {
       // the activation is chosen once a tile, not once a number
       const float rs = mode == MODE_GATED_SCALED && row < M ? row_scale[row] : 1.f;
-      auto gate = [&](float rate, auto quick, auto value) { gated_columns(taddr, row, M, n0, crow, N_out, ldc, part, rate, quick, value); };
+      auto gate = [&](float rate, auto quick, auto value) {
+        if constexpr (LEAVE) gated_columns_leave(taddr, row, M, n0, C, N_out, ldc, part, rate, leaving, quick, value);
+        else gated_columns(taddr, row, M, n0, crow, N_out, ldc, part, rate, quick, value);
+      };
       if (mode == MODE_GATED) {
         gate(1.f, [](float g, float u) { return divided(g, 1.f + __expf(-g)) * u; }, [](float g, float u) { return g / (1.f + __expf(-g)) * u; });
       } else if (mode == MODE_GATED_SCALED) {
@@ -277,24 +355,23 @@ struct Epilogue {
         uint32_t v[32];
         tmem_ld32(taddr + c, v);  // (a tile of 240 columns: the last load reads 16 columns beyond it, which nobody stores)
         tmem_ld_wait();
-        if (row < M) {
+        if constexpr (LEAVE) {
+          static_assert(BN % 32 == 0, "whole runs of columns");
+          if (row - (int)(threadIdx.x & 31) >= M) continue;
+          uint32_t packed[4][4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) packed[j][q] = activated(__uint_as_float(v[8 * j + 2 * q]), __uint_as_float(v[8 * j + 2 * q + 1]), mode);
+          leave_rows(leaving, packed, C, row, M, n0 + c, N_out, ldc);
+        } else if (row < M) {
 #pragma unroll
           for (int j = 0; j < 32; j += 8) {
             if (BN % 32 != 0 && c + j >= BN) break;
             const int col = n0 + c + j;
             uint32_t packed[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              float v0 = __uint_as_float(v[j + 2 * q]), v1 = __uint_as_float(v[j + 2 * q + 1]);
-              if (mode == MODE_RELU2) {
-                v0 = fmaxf(v0, 0.f), v1 = fmaxf(v1, 0.f);
-                v0 *= v0, v1 *= v1;
-              } else if (mode == MODE_SILU || mode == MODE_GELU) {
-                const int act = mode == MODE_SILU ? PSB_ACT_SILU : PSB_ACT_GELU_TANH;
-                v0 = quick_act(v0, act), v1 = quick_act(v1, act);
-              }
-              packed[q] = pack2(v0, v1);
-            }
+            for (int q = 0; q < 4; ++q) packed[q] = activated(__uint_as_float(v[j + 2 * q]), __uint_as_float(v[j + 2 * q + 1]), mode);
             if (col + 8 <= N_out && (ldc & 7) == 0) {
               *reinterpret_cast<uint4*>(crow + col) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
             } else {
@@ -465,7 +542,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // 1,979 tokens, K 4,096, 14,336 gated columns: 305 us on a cool GPU and 312 with one CTA a tile; in a loop, where power is the limit, both products of
 // the feed-forward take 557 us instead of 580.
 constexpr int PAIR_STAGES = 6, PAIR_STAGE = A_BYTES + 128 * BK * 2, MAX_UNITS = 2048;
-constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE + 1024 + 256 + MAX_UNITS * 2;
+constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE + 1024 + 256 + MAX_UNITS * 2 + LEAVING_BYTES;
 constexpr int ALONE = 1 << 15;  // the unit's second row tile is another expert's
 static_assert(PAIR_STAGES <= MAX_STAGES && PAIR_SMEM <= 227 * 1024, "beyond a CTA's shared memory");
 
@@ -617,12 +694,13 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       ++local;
       const Where w = where(tile);
       const int row = w.m0 + rank * BM + quarter * 32 + lane, rows = rank && !w.both ? 0 : M;
-      Epilogue<BN, HB> epilogue;
+      Epilogue<BN, HB, true> epilogue;
       epilogue.before(row, rows, mode, rope);
       ok = mbar_wait(&bars->acc_full[buf], use & 1, abort, 3);
       if (!ok) break;
       fence_after();
-      epilogue.store(tmem_base + buf * ACC_STRIDE + ((uint32_t)(quarter * 32) << 16), row, rows, w.n0, C, N_out, ldc, mode, gated, rope, glu, row_scale, (warp - 2) >> 2);
+      epilogue.store(tmem_base + buf * ACC_STRIDE + ((uint32_t)(quarter * 32) << 16), row, rows, w.n0, C, N_out, ldc, mode, gated, rope, glu, row_scale, (warp - 2) >> 2,
+                     reinterpret_cast<uint4*>(tiles + PAIR_STAGES * PAIR_STAGE + 256 + MAX_UNITS * 2 + (warp - 2) * LEAVING_WARP));
       fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(cluster_address(&bars->acc_empty[buf], 0));

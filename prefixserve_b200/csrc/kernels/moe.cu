@@ -622,68 +622,83 @@ __global__ void moe_combine_kernel(const TY* __restrict__ Y, const int32_t* __re
   }
 }
 
+// Eight numbers as they lie in memory.
 template <typename T>
-__device__ __forceinline__ void comb8(const T* p, float (&o)[8]);
+struct Eight;
 template <>
-__device__ __forceinline__ void comb8<float>(const float* p, float (&o)[8]) {
-  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
-  o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
-}
-template <>
-__device__ __forceinline__ void comb8<__nv_bfloat16>(const __nv_bfloat16* p, float (&o)[8]) {
-  const uint4 raw = *reinterpret_cast<const uint4*>(p);
-  const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float2 f = __bfloat1622float2(h2[k]);
-    o[2 * k] = f.x;
-    o[2 * k + 1] = f.y;
+struct Eight<float> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const float* p) { a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4); }
+  __device__ __forceinline__ void add_to(float (&v)[8], float w) const {
+    v[0] = fmaf(w, a.x, v[0]); v[1] = fmaf(w, a.y, v[1]); v[2] = fmaf(w, a.z, v[2]); v[3] = fmaf(w, a.w, v[3]);
+    v[4] = fmaf(w, b.x, v[4]); v[5] = fmaf(w, b.y, v[5]); v[6] = fmaf(w, b.z, v[6]); v[7] = fmaf(w, b.w, v[7]);
   }
-}
+};
+template <>
+struct Eight<__nv_bfloat16> {
+  uint4 raw;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { raw = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ void add_to(float (&v)[8], float w) const {
+    const uint32_t x[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = fmaf(w, __uint_as_float(x[i] << 16), v[2 * i]);
+      v[2 * i + 1] = fmaf(w, __uint_as_float(x[i] & 0xffff0000u), v[2 * i + 1]);
+    }
+  }
+};
 
-// The same with eight columns a thread; the rows of four slots are asked for together.  H % 8 == 0, rows on 16 bytes.
-template <typename TY, typename TS, typename TO>
+// The same with eight columns a thread; the rows of four slots, of TOKENS tokens each, and the shared expert's are asked for together.  H % 8 == 0, rows on 16
+// bytes.  Bound by how much is under way: 2,037 tokens of four slots and 2,048 columns 16 to 18 us a token at a time, the shared row behind the others, 12 so.
+template <int TOKENS, typename TY, typename TS, typename TO>
 __global__ void __launch_bounds__(256)
 moe_combine_vec_kernel(const TY* __restrict__ Y, const int32_t* __restrict__ pair_row, const float* __restrict__ weight,
-                       const TS* __restrict__ shared, const float* __restrict__ gate, int ldg, TO* __restrict__ out, int H, int top) {
+                       const TS* __restrict__ shared, const float* __restrict__ gate, int ldg, TO* __restrict__ out, int T, int H, int top) {
   pdl_trigger();
   pdl_wait();
-  const int t = blockIdx.x;
-  const float sg = shared ? sigmoidf_(gate ? gate[(size_t)t * ldg] : FLT_MAX) : 0.f;
+  const int t0 = blockIdx.x * TOKENS;
   for (int j = threadIdx.x * 8; j < H; j += blockDim.x * 8) {
-    float v[8] = {};
-    for (int k0 = 0; k0 < top; k0 += 4) {
-      float y[4][8], w[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (k0 + k >= top) break;
-        const size_t at = (size_t)t * top + k0 + k;
-        w[k] = weight ? weight[at] : 1.f;
-        comb8<TY>(Y + (size_t)pair_row[at] * H + j, y[k]);
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (k0 + k >= top) break;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = fmaf(w[k], y[k][i], v[i]);
-      }
-    }
+    float v[TOKENS][8] = {};
+    Eight<TS> of_shared[TOKENS];
     if (shared) {
-      float y[8];
-      comb8<TS>(shared + (size_t)t * H + j, y);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = fmaf(sg, y[i], v[i]);
+      for (int u = 0; u < TOKENS; ++u)
+        if (t0 + u < T) of_shared[u].load(shared + (size_t)(t0 + u) * H + j);
     }
-    TO* o = out + (size_t)t * H + j;
-    if constexpr (sizeof(TO) == 4) {
-      *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
-      *reinterpret_cast<float4*>(o + 4) = make_float4(v[4], v[5], v[6], v[7]);
-    } else {
-      uint4 raw;
-      __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&raw);
+    for (int k0 = 0; k0 < top; k0 += 4) {
+      Eight<TY> y[TOKENS][4];
+      float w[TOKENS][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) h2[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-      *reinterpret_cast<uint4*>(o) = raw;
+      for (int u = 0; u < TOKENS; ++u)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (k0 + k >= top || t0 + u >= T) continue;
+          const size_t at = (size_t)(t0 + u) * top + k0 + k;
+          w[u][k] = weight ? weight[at] : 1.f;
+          y[u][k].load(Y + (size_t)pair_row[at] * H + j);
+        }
+#pragma unroll
+      for (int u = 0; u < TOKENS; ++u)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (k0 + k < top && t0 + u < T) y[u][k].add_to(v[u], w[u][k]);
+    }
+#pragma unroll
+    for (int u = 0; u < TOKENS; ++u) {
+      const int t = t0 + u;
+      if (t >= T) break;
+      if (shared) of_shared[u].add_to(v[u], sigmoidf_(gate ? gate[(size_t)t * ldg] : FLT_MAX));
+      TO* o = out + (size_t)t * H + j;
+      if constexpr (sizeof(TO) == 4) {
+        *reinterpret_cast<float4*>(o) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+        *reinterpret_cast<float4*>(o + 4) = make_float4(v[u][4], v[u][5], v[u][6], v[u][7]);
+      } else {
+        uint4 raw;
+        __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&raw);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) h2[i] = __floats2bfloat162_rn(v[u][2 * i], v[u][2 * i + 1]);
+        *reinterpret_cast<uint4*>(o) = raw;
+      }
     }
   }
 }
@@ -814,8 +829,12 @@ PSB_API int psb_moe_combine(const void* y, int y_dtype, const void* pair_row, co
     PSB_DISPATCH_DTYPE(shared_dtype, TS, {
       PSB_DISPATCH_DTYPE(out_dtype, TO, {
         if (vec) {
-          psb_launch(moe_combine_vec_kernel<TY, TS, TO>, dim3(T), dim3(H >= 2048 ? 256 : 128), 0, stream, (const TY*)y, (const int32_t*)pair_row,
-                     (const float*)weight, (const TS*)shared, (const float*)gate, ldg, (TO*)out, H, top);
+          // two tokens a block where there are enough of them for every place on the SMs (four blocks each) and the rows are of 16 bits
+          constexpr int PAIR = sizeof(TY) == 2 ? 2 : 1;
+          const bool pairs = PAIR == 2 && T >= 8 * psb_current_sms();
+          auto kernel = pairs ? moe_combine_vec_kernel<PAIR, TY, TS, TO> : moe_combine_vec_kernel<1, TY, TS, TO>;
+          psb_launch(kernel, dim3(pairs ? (T + 1) / 2 : T), dim3(H >= 2048 ? 256 : 128), 0, stream, (const TY*)y, (const int32_t*)pair_row,
+                     (const float*)weight, (const TS*)shared, (const float*)gate, ldg, (TO*)out, T, H, top);
           PSB_LAUNCH_CHECK("moe_combine");
           return 0;
         }

@@ -117,7 +117,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                                  const int32_t* __restrict__ table, int table_width, const int32_t* __restrict__ item_start,
                                  const int32_t* __restrict__ kv_len, __nv_bfloat16* __restrict__ out, int num_items, int hq,
                                  int hkv, int page_shift, int window, float scale, int skip_single, int rows_per_cta,
-                                 int kv_splits, float* __restrict__ part_o, float* __restrict__ part_ml,
+                                 int whole, int longest_first, int kv_splits, float* __restrict__ part_o, float* __restrict__ part_ml,
                                  const float* __restrict__ sink) {
   using Sh = Shape<D>;
   constexpr int KB = Sh::KB, NB = Sh::S_BUFS, STAGES = Sh::STAGES;
@@ -131,8 +131,28 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   // which request and which 256 rows of it?  (lengths are inputs of the step: readable before the wait)
   const int head = blockIdx.x;
   int item = -1, pair = 0, n = 0;
-  {
-    int left = blockIdx.y;  // block 0 takes the last (longest) rows of the last request
+  // row groups from ``whole`` on are two CTAs' of half the rows each
+  const int by_half = max(0, (int)blockIdx.y - whole), group = min((int)blockIdx.y, whole) + (by_half >> 1);
+  const bool half = (int)blockIdx.y >= whole;
+  if (longest_first) {  // (at most 32 requests) by the keys the requests hold, a lane a request; a request's last rows first
+    int mine = 0, keys = 0, pairs = 0, before = 0;
+    if (lane < num_items) {
+      mine = item_start[lane + 1] - item_start[lane];
+      keys = kv_len[lane];
+      pairs = skip_single && mine == 1 ? 0 : (mine + rows_per_cta - 1) / rows_per_cta;
+    }
+    for (int i = 0; i < num_items; ++i) {
+      const int other = __shfl_sync(0xffffffffu, keys, i), its = __shfl_sync(0xffffffffu, pairs, i);
+      if (other > keys || (other == keys && i > lane)) before += its;
+    }
+    const unsigned found = __ballot_sync(0xffffffffu, group >= before && group < before + pairs);
+    if (found) {
+      item = __ffs(found) - 1;
+      pair = __shfl_sync(0xffffffffu, pairs - 1 - (group - before), item);
+      n = __shfl_sync(0xffffffffu, mine, item);
+    }
+  } else {
+    int left = group;  // block 0 takes the last (longest) rows of the last request
     for (int i = num_items - 1; i >= 0; --i) {
       const int ni = item_start[i + 1] - item_start[i];
       if (skip_single && ni == 1) continue;
@@ -142,6 +162,9 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     }
   }
   if (item < 0) return;  // uniform for the CTA, before anything is allocated
+  const int row0 = pair * rows_per_cta + (by_half & 1) * (rows_per_cta / 2);  // first of this CTA's rows among the new tokens
+  const int rows_here = min(half ? rows_per_cta / 2 : rows_per_cta, n - row0);
+  if (rows_here <= 0) return;
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, 1);
@@ -169,8 +192,6 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   const int t0 = item_start[item];
   const int kvl = kv_len[item];
   const int first_pos = kvl - n;                      // position of the request's first new token
-  const int row0 = pair * rows_per_cta;               // first of this CTA's rows among the new tokens
-  const int rows_here = min(rows_per_cta, n - row0);
   const int ntiles = rows_here > TILE_M ? 2 : 1;
   int p_first[TILES], p_last[TILES], bend[TILES];
 #pragma unroll
@@ -650,7 +671,7 @@ __global__ void attention_prefill_merge_kernel(const float* __restrict__ part_o,
 template <int D>
 int launch(const CUtensorMap& map_q, const CUtensorMap& map_kv, const void* table, int table_width, const void* item_start,
            const void* kv_len, void* out, int num_items, int num_pairs, int hq, int hkv, int page_shift, int window,
-           float scale, int skip_single, int rows_per_cta, int kv_splits, void* part_o, void* part_ml, const void* token_item,
+           float scale, int skip_single, int rows_per_cta, int whole, int longest_first, int kv_splits, void* part_o, void* part_ml, const void* token_item,
            int T, const float* sink, cudaStream_t stream) {
   static PsbPerDevice configured; 
   if (!configured.get()) {
@@ -658,9 +679,9 @@ int launch(const CUtensorMap& map_q, const CUtensorMap& map_kv, const void* tabl
     if (e != cudaSuccess) PSB_REFUSE("attention_prefill_tcgen05: cannot reserve %d bytes of shared memory: %s", smem_bytes<D>(), cudaGetErrorString(e));
     configured.set(); 
   }
-  psb_launch(attention_prefill_tcgen05_kernel<D>, dim3(hq, num_pairs, kv_splits), dim3(THREADS), (size_t)smem_bytes<D>(), stream, map_q, map_kv,
+  psb_launch(attention_prefill_tcgen05_kernel<D>, dim3(hq, whole + 2 * (num_pairs - whole), kv_splits), dim3(THREADS), (size_t)smem_bytes<D>(), stream, map_q, map_kv,
              (const int32_t*)table, table_width, (const int32_t*)item_start, (const int32_t*)kv_len, (__nv_bfloat16*)out,
-             num_items, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, kv_splits, (float*)part_o, (float*)part_ml,
+             num_items, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, whole, longest_first, kv_splits, (float*)part_o, (float*)part_ml,
              kv_splits > 1 ? (const float*)nullptr : sink);
   if (kv_splits > 1) {
     const long long units = (long long)T * hq;
@@ -686,13 +707,14 @@ PSB_API int psb_attention_prefill_tcgen05_rows_per_cta() { return ROWS_PER_CTA; 
 // q [T, hq*D] and out [T, hq*D] bfloat16; kv [num_pages, 2, hkv, page_size, D] bfloat16; table [num_items, table_width]
 // int32; item_start [num_items+1], kv_len [num_items] int32 on the device.  rows_per_cta: 256 or 128.  num_pairs: the sum
 // over the requests this kernel owns (all, or those with more than one new token when skip_single) of
-// ceil(new tokens / rows_per_cta).  kv_splits > 1: the keys are cut into that many ranges; part_o (float32
+// ceil(new tokens / rows_per_cta); the first ``whole`` of them are a CTA's for every head, the others two CTAs' of half the rows each.
+// longest_first (up to 32 requests): the requests' row groups by the keys that these hold, otherwise the last request's first.  kv_splits > 1: the keys are cut into that many ranges; part_o (float32
 // [T, hq, kv_splits, D]) and part_ml ([T, hq, kv_splits, 2]) take the ranges' partial results, token_item ([T] int32)
 // tells the merge which request a row belongs to.
 PSB_API int psb_attention_prefill_tcgen05(const void* q, const void* kv, const void* table, int table_width, const void* item_start,
                                           const void* kv_len, void* out, int num_items, int num_pairs, int T, int hq, int hkv,
                                           int D, int page_size, long long num_pages, int window, float scale, int skip_single,
-                                          int rows_per_cta, int kv_splits, void* part_o, void* part_ml, const void* token_item,
+                                          int rows_per_cta, int whole, int longest_first, int kv_splits, void* part_o, void* part_ml, const void* token_item,
                                           const void* sink, cudaStream_t stream) {
   if (kv_splits < 1 || kv_splits > 32 || (kv_splits > 1 && (!part_o || !part_ml || !token_item)))
     PSB_REFUSE("attention_prefill_tcgen05: %d key ranges (1 to 32), or their scratch is missing", kv_splits);
@@ -702,7 +724,10 @@ PSB_API int psb_attention_prefill_tcgen05(const void* q, const void* kv, const v
   if (hq < 1 || hkv < 1 || hq % hkv) PSB_REFUSE("attention_prefill_tcgen05: %d query heads over %d key heads", hq, hkv);
   if (window < 0 || table_width < 1 || T < 1 || num_pages < 1) PSB_REFUSE("attention_prefill_tcgen05: bad sizes (window=%d table_width=%d T=%d)", window, table_width, T);
   if (num_items <= 0 || num_pairs <= 0) return 0;
-  if (num_pairs > 65535) PSB_REFUSE("attention_prefill_tcgen05: %d row groups in one step (at most 65535)", num_pairs);
+  if (whole < 0 || whole > num_pairs || (whole < num_pairs && (rows_per_cta != ROWS_PER_CTA || kv_splits > 1)))
+    PSB_REFUSE("attention_prefill_tcgen05: %d of %d row groups whole (with key ranges, or groups of %d, all are)", whole, num_pairs, TILE_M);
+  if (longest_first && num_items > 32) PSB_REFUSE("attention_prefill_tcgen05: %d requests by length (at most 32)", num_items);
+  if (whole + 2LL * (num_pairs - whole) > 65535) PSB_REFUSE("attention_prefill_tcgen05: %d row groups in one step (at most 65535)", num_pairs);
   const long long kv_rows = num_pages * 2 * hkv * page_size;
   if (kv_rows > 0x7fffffffLL) PSB_REFUSE("attention_prefill_tcgen05: the cache entry has %lld rows, beyond a TMA coordinate", kv_rows);
   if (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)out) & 15) PSB_REFUSE("attention_prefill_tcgen05: operands must be 16-byte aligned");
@@ -714,8 +739,8 @@ PSB_API int psb_attention_prefill_tcgen05(const void* q, const void* kv, const v
   if (r == -1) PSB_REFUSE("attention_prefill_tcgen05: the driver does not export cuTensorMapEncodeTiled");
   if (r != 0) PSB_REFUSE("attention_prefill_tcgen05: cuTensorMapEncodeTiled failed with code %d", r);
   int rc;
-  if (D == 64) rc = launch<64>(map_q, map_kv, table, table_width, item_start, kv_len, out, num_items, num_pairs, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, kv_splits, part_o, part_ml, token_item, T, (const float*)sink, stream);
-  else rc = launch<128>(map_q, map_kv, table, table_width, item_start, kv_len, out, num_items, num_pairs, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, kv_splits, part_o, part_ml, token_item, T, (const float*)sink, stream);
+  if (D == 64) rc = launch<64>(map_q, map_kv, table, table_width, item_start, kv_len, out, num_items, num_pairs, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, whole, longest_first, kv_splits, part_o, part_ml, token_item, T, (const float*)sink, stream);
+  else rc = launch<128>(map_q, map_kv, table, table_width, item_start, kv_len, out, num_items, num_pairs, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, whole, longest_first, kv_splits, part_o, part_ml, token_item, T, (const float*)sink, stream);
   if (rc) return rc;
   PSB_LAUNCH_CHECK("attention_prefill_tcgen05");
   return 0;

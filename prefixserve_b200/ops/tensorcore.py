@@ -451,6 +451,17 @@ def _decode_key_range(pairs: int, longest: int, sms: int, tma_kernel: bool, ctas
     return best[2]
 
 
+def _whole_row_groups(groups: int, heads: int, d: int, sms: int) -> int:
+    """Row groups (256 rows of a head a CTA) before those that two CTAs of 128 rows take: of a second round over the SMs that is at most half full, where the
+    halves fit in one round.  Half the rows take a CTA 0.87 of the time (heads of 64) or 0.73 (128), so heads of 64 are halved up to a quarter of a round only.
+    32 heads, the longest request first, us whole and halved: 640 and 512 rows behind 1,500 55.1 and 53.9 (heads of 64), 66.4 and 61.2 (128); 500, 434
+    and 367 behind 100 28.8 and 27.2 (128); 1,300 behind 1,300 69.1 and 71.1 (64), 82.6 and 78.9 (128).  In a third round (900, 780 and 660 behind 2,100), whose CTAs begin
+    as the shorter ones before them end, 115 and 138, 145 and 157."""
+    ctas = heads * groups
+    last = -(-(ctas - sms) // heads)  # groups of the second round
+    return groups - last if sms < ctas < 2 * sms and (2 if d == 128 else 4) * heads * last <= sms else groups
+
+
 def _short_portions_in_tiles(portions: Sequence[int], kv_lens: Sequence[int], window: int, heads: int, d: int, sms: int, static_kv_len: int | None) -> bool:
     """Whether portions shorter than TCGEN05_PREFILL_MIN_TOKENS are over sooner on the kernel of 128-row tiles."""
     keys = static_kv_len if static_kv_len is not None else max(kv_lens)
@@ -506,7 +517,12 @@ def _attention_plan(new_tokens: Sequence[int], kv_lens: Sequence[int], window: i
             else:
                 per_cta //= 2
         plan["rows_per_cta"] = per_cta
-        plan["pairs"] = sum(-(-n // per_cta) for n in portions)
+        plan["pairs"] = pairs = sum(-(-n // per_cta) for n in portions)
+        # The requests that see most first, where the CTAs are less than two rounds: what begins last then ends soon.  With more the shorter ones are as well
+        # first (32 heads, us by place in the step, shortest first here, and by length; heads of 64 and 128: 1,000 and 800 rows behind 1,000 68.1 and 58.9,
+        # 77.1 and 69.2; 660, 572 and 483 behind 400 46.1 and 42.1, 49.3 and 47.0; 900, 780 and 660 behind 2,100, 352 CTAs, 115.1 and 117.4, 145.5 and 143.4).
+        plan["longest_first"] = 1 if sms < hq_total * pairs < 2 * sms and 1 < b <= 32 else 0
+        plan["whole"] = _whole_row_groups(pairs, hq_total, d, sms) if plan["kv_splits"] == 1 and per_cta == lib().psb_attention_prefill_tcgen05_rows_per_cta() else pairs
     else:
         rows = lib().psb_attention_prefill_rows_per_cta(d)
         plan["tiles"] = sum(-(-(n * group) // rows) for n in portions)
@@ -575,7 +591,8 @@ def attention_bf16(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, item_
         check(lib().psb_attention_prefill_tcgen05(
             q.data_ptr(), kv.data_ptr(), table.data_ptr(), table.shape[1], item_start.data_ptr(), kv_len.data_ptr(),
             out.data_ptr(), b, plan["pairs"], t, hq, hkv, d, page, kv.shape[0], w, float(scale),
-            1 if plan["use_decode"] else 0, plan["rows_per_cta"], splits, po, pm,
+            1 if plan["use_decode"] else 0, plan["rows_per_cta"], plan["whole"] if splits == 1 else plan["pairs"],
+            plan["longest_first"], splits, po, pm,
             token_item.data_ptr() if token_item is not None else None, sk, stream), "attention_prefill_tcgen05")
         return out
     tiles = plan.get("tiles")

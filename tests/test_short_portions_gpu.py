@@ -1,4 +1,5 @@
-"""Short prompt portions behind long contexts: which kernel attends for them, and that both agree with the general one to what bfloat16 weights and results
+"""Prompt portions on the kernel of 128-row tiles where its launch is not the plain one (short portions behind long contexts, row groups of a second round halved):
+which kernel attends for them, and that it agrees with the general one to what bfloat16 weights and results
 give (2e-2 of numbers of about one, the bound of the other attention tests)."""
 
 import pytest
@@ -6,18 +7,13 @@ import torch
 
 from prefixserve_b200 import ops
 from prefixserve_b200.engine import StepItem  # noqa: F401  (the engine's package loads)
-from prefixserve_b200.ops import library
+from prefixserve_b200.ops import library, tensorcore
 from prefixserve_b200.parts.base import ItemView, StepContext
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("d,hq,hkv,window,portions,taken", [
-    (64, 32, 8, None, [(31, 2000)], True), (64, 32, 8, None, [(2, 1022)], True), (64, 32, 8, None, [(2, 1021)], False),       # 1,024 keys
-    (128, 32, 8, None, [(63, 449), (1, 700), (5, 100)], True), (128, 32, 8, None, [(63, 448)], False),                         # 512 keys; beside a decoded token
-    (64, 32, 8, None, [(9, 1500)] * 4, True), (64, 32, 8, None, [(9, 1500)] * 5, False),                                       # 128 and 160 CTAs on 148 SMs
-    (128, 8, 8, 300, [(20, 3000)], False), (128, 8, 4, 500, [(20, 3000), (1, 2000)], True), (128, 6, 1, None, [(3, 4000)], True)])
-def test_short_portions(d, hq, hkv, window, portions, taken):
+def _step(d, hq, hkv, portions):
     page, gen = 16, torch.Generator(device="cuda").manual_seed(d + len(portions))
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
     starts, views = [0], []
@@ -34,10 +30,35 @@ def test_short_portions(d, hq, hkv, window, portions, taken):
         max_kv_len=max(n + held for n, held in portions), all_decode=False)
     q = torch.randn(starts[-1], hq, d, generator=gen, device="cuda").to(torch.bfloat16)
     kv = torch.randn(len(portions) * width, 2, hkv, page, d, generator=gen, device="cuda").to(torch.bfloat16)
+    return ctx, table, q, kv
+
+
+@pytest.mark.parametrize("d,hq,hkv,window,portions,taken", [
+    (64, 32, 8, None, [(31, 2000)], True), (64, 32, 8, None, [(2, 1022)], True), (64, 32, 8, None, [(2, 1021)], False),       # 1,024 keys
+    (128, 32, 8, None, [(63, 449), (1, 700), (5, 100)], True), (128, 32, 8, None, [(63, 448)], False),                         # 512 keys; beside a decoded token
+    (64, 32, 8, None, [(9, 1500)] * 4, True), (64, 32, 8, None, [(9, 1500)] * 5, False),                                       # 128 and 160 CTAs on 148 SMs
+    (128, 8, 8, 300, [(20, 3000)], False), (128, 8, 4, 500, [(20, 3000), (1, 2000)], True), (128, 6, 1, None, [(3, 4000)], True)])
+def test_short_portions(d, hq, hkv, window, portions, taken):
+    ctx, table, q, kv = _step(d, hq, hkv, portions)
     before = library.launch_counts.copy()
     out = ops.attention(q, kv, table, ctx.positions, ctx.token_item, window=window, ctx=ctx)
     counts = library.launch_counts - before
     assert counts["attention_prefill_tcgen05"] == taken and counts["attention_prefill"] == (not taken)
     want = ops.attention(q, kv, table, ctx.positions, ctx.token_item, window=window)  # (without the step: the general kernel)
+    assert library.tcgen05_status() == 0
+    assert torch.allclose(out.float(), want.float().view_as(out), atol=2e-2, rtol=2e-2), float((out.float() - want.float().view_as(out)).abs().max())
+
+
+@pytest.mark.parametrize("d,portions,groups,whole", [(64, [(640, 300), (512, 40)], 5, 4), (128, [(641, 300), (513, 40)], 6, 4), (128, [(1152, 7)], 5, 4), (64, [(700, 0), (560, 90)], 6, 6),
+                                                     (64, [(1025, 500), (1, 900)], 5, 4), (128, [(2048, 0)], 8, 8)])
+def test_row_groups_of_a_second_round(d, portions, groups, whole):
+    hq, hkv, sms = 32, 8, torch.cuda.get_device_properties(0).multi_processor_count
+    if sms != 148:
+        pytest.skip("the numbers of groups are for 148 SMs")
+    plan = tensorcore._attention_plan([n for n, _ in portions], [n + held for n, held in portions], 0, hq // hkv, hkv, d, 16, sms, None)
+    assert plan["tcgen05"] and (plan["pairs"], plan["whole"]) == (groups, whole)
+    ctx, table, q, kv = _step(d, hq, hkv, portions)
+    out = ops.attention(q, kv, table, ctx.positions, ctx.token_item, ctx=ctx)
+    want = ops.attention(q, kv, table, ctx.positions, ctx.token_item)
     assert library.tcgen05_status() == 0
     assert torch.allclose(out.float(), want.float().view_as(out), atol=2e-2, rtol=2e-2), float((out.float() - want.float().view_as(out)).abs().max())

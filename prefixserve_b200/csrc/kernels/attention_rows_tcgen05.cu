@@ -177,8 +177,8 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
   volatile uint32_t* abort = &bars->abort;
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
 
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();  // (behind the wait: the kernel that joins the ranges reads the step's lengths and the gates before its own)
   const bool cut = (int)blockIdx.x >= args.whole;
   const int unit = cut ? args.whole + ((int)blockIdx.x - args.whole) / args.ranges : (int)blockIdx.x;
   const int range = cut ? ((int)blockIdx.x - args.whole) % args.ranges : 0;
@@ -656,16 +656,28 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
 __global__ void __launch_bounds__(128)
 attention_rows_merge_kernel(const RowsArgs args) {
   pdl_trigger();
-  pdl_wait();
   const int at = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int in_unit = at % (args.heads_here * TILE_M), t = in_unit / TILE_M, r = in_unit % TILE_M;
   const int rest = at / (args.heads_here * TILE_M);
   int item, t0, n, h0;
   unit_tokens(args, args.whole + rest, item, t0, n, h0);
-  if (r >= n) return;
   const int head = h0 + t;
+  uint2 g = make_uint2(0, 0);
+  if (args.gate && r < n) g = *reinterpret_cast<const uint2*>(args.gate + (size_t)(t0 + r) * args.ldg + (size_t)head * D + 4 * lane);
+  pdl_wait();
+  if (r >= n) return;
   const size_t step = (size_t)args.heads_here * TILE_M;  // from range to range
   const size_t slot0 = (size_t)rest * args.ranges * step + (size_t)t * TILE_M + r;
+  // four ranges' results at a time, asked for before their weights are known (28 units in five ranges 10 us, one behind the other; 300 tokens behind 1,500, the
+  // whole call, 21.1 -> 19.6)
+  constexpr int AHEAD = 4;
+  float4 v[AHEAD];
+  auto ask = [&](int s0) {
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k)
+      if (s0 + k < args.ranges) v[k] = *reinterpret_cast<const float4*>(args.part_o + (slot0 + (s0 + k) * step) * D + 4 * lane);
+  };
+  ask(0);
   const float2 ml = lane < args.ranges ? *reinterpret_cast<const float2*>(args.part_ml + (slot0 + lane * step) * 2) : make_float2(-INFINITY, 0.f);
   const float s2 = args.sink ? args.sink[head] * PSB_LOG2E : -INFINITY;
   const float top = fmaxf(warp_max(ml.x), s2);
@@ -673,18 +685,20 @@ attention_rows_merge_kernel(const RowsArgs args) {
   const float sum = warp_sum(w * ml.y) + (args.sink ? exp2f(s2 - top) : 0.f);
   const float inv = (sum > 0.f ? 1.f / sum : 0.f) * args.out_scale;
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-  for (int s = 0; s < args.ranges; ++s) {
-    const float ws = __shfl_sync(0xffffffffu, w, s);
-    if (ws == 0.f) continue;  // a range that saw nothing has left nothing
-    const float4 v = *reinterpret_cast<const float4*>(args.part_o + (slot0 + s * step) * D + 4 * lane);
-    acc[0] = fmaf(ws, v.x, acc[0]); acc[1] = fmaf(ws, v.y, acc[1]);
-    acc[2] = fmaf(ws, v.z, acc[2]); acc[3] = fmaf(ws, v.w, acc[3]);
+  for (int s0 = 0; s0 < args.ranges; s0 += AHEAD) {
+    if (s0) ask(s0);
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) {
+      if (s0 + k >= args.ranges) break;
+      const float ws = __shfl_sync(0xffffffffu, w, s0 + k);
+      if (ws == 0.f) continue;  // a range that saw nothing has left nothing
+      acc[0] = fmaf(ws, v[k].x, acc[0]); acc[1] = fmaf(ws, v[k].y, acc[1]);
+      acc[2] = fmaf(ws, v[k].z, acc[2]); acc[3] = fmaf(ws, v[k].w, acc[3]);
+    }
   }
 #pragma unroll
   for (int e = 0; e < 4; ++e) acc[e] *= inv;
   if (args.gate) {
-    const uint2 g = *reinterpret_cast<const uint2*>(args.gate + (size_t)(t0 + r) * args.ldg + (size_t)head * D + 4 * lane);
     const uint32_t gw[2] = {g.x, g.y};
 #pragma unroll
     for (int e = 0; e < 2; ++e) {

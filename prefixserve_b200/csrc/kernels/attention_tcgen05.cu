@@ -2,17 +2,18 @@
 //
 // One CTA owns up to 256 consecutive new tokens of one request for one query head, as two tiles of 128 rows (or, when the
 // step has too few such groups to give every SM one, up to 128 tokens as a single tile), and walks
-// the keys they may see in blocks of KB keys (128 for a head size of 64, 64 for 128).  352 threads:
+// the keys they may see in blocks of KB keys (128 for a head size of 64, 64 for 128).  608 threads
+// for a head size of 64, 352 for 128:
 //   warp 0      producer: TMA loads (cp.async.bulk.tensor.2d, 128-byte swizzle) of the two Q tiles once, and per block of
 //               the pages that hold its keys and values, one box per page, into a ring of four or five stages (one
 //               mbarrier per stage takes both, so the MMA warp waits once per block);
-//   warp 1      (and, with 64 keys a block, warp 10 for S) MMA: one lane issues tcgen05.mma (cta_group::1, kind::f16, M=128):  S = Q K^T  (A and B K-major, N=KB)
+//   two warps   MMA: one lane issues tcgen05.mma (cta_group::1, kind::f16, M=128):  S = Q K^T  (A and B K-major, N=KB)
 //               into tensor memory, and  O += P V  (A = P from tensor memory, B = V MN-major exactly as the
 //               cache stores it: keys x head dim, N = head dim).  S goes into three (128 keys a block) or four (64)
-//               buffers in turn, so it is computed while the softmax of the blocks before it still runs.  This warp
-//               sets the kernel's pace: what it waits on and issues per block and tile takes about as long as a
-//               softmax warp's work on the block;
-//   warps 2..5  softmax of tile 0, warps 6..9 of tile 1: one thread per row.  tcgen05.ld of the row of S, masks,
+//               buffers in turn, so it is computed while the softmax of the blocks before it still runs.  A warp per
+//               tile with 128 keys a block, a warp per product with 64 (see there);
+//   the others  softmax, four warps of tile 0, then as many of tile 1: one thread per row; with 128 keys a block eight
+//               warps a tile and two threads per row, half of its keys each.  tcgen05.ld of the scores, masks,
 //               maximum and sum in float32 (three-input maxima and arithmetic on register pairs: the loop is bound by
 //               the instructions it issues), P as bfloat16 into tensor memory over the scores it came from.  O
 //               accumulates in tensor memory over the blocks; the row's reference maximum only follows the true one
@@ -36,9 +37,7 @@ using namespace tc;
 constexpr int TILE_M = 128;
 constexpr int TILES = 2;
 constexpr int ROWS_PER_CTA = TILE_M * TILES;
-constexpr int SOFTMAX_WARPS = 4;                     // per tile: one thread per row, a warp per quarter of tensor-memory lanes
-constexpr int S_WARP = 2 + SOFTMAX_WARPS * TILES;         // the warp that issues S = Q K^T (warp 1 issues O += P V)
-constexpr int THREADS = 32 * (3 + SOFTMAX_WARPS * TILES);  // producer, two MMA warps, softmax
+constexpr int SOFTMAX_WARPS = 4;                     // per tile and thread of a row: a warp per quarter of tensor-memory lanes
 constexpr int MAX_STAGES = 5, MAX_S_BUFS = 4;
 constexpr int TMEM_COLS = 512;
 constexpr float LOG2E_F = 1.4426950408889634f;
@@ -52,6 +51,11 @@ struct Shape {
   // blocks of keys and values in shared memory at a time: S of one tile alone runs S_BUFS blocks ahead of its P V
   static constexpr int STAGES = S_BUFS + 1;
   static constexpr bool TWO_ISSUERS = KB == 64;           // S and P V issued by two warps (see the MMA warps)
+  // threads of a row: two with 128 keys a block, half of the keys (and of the row's results) each
+  static constexpr int HALVES = KB == 128 ? 2 : 1, PART = KB / HALVES;
+  // warp 0 is the producer, warp 1 issues products
+  static constexpr int FIRST_SOFTMAX_WARP = TWO_ISSUERS ? 2 : 3, S_WARP = TWO_ISSUERS ? 2 + SOFTMAX_WARPS * TILES : 2;
+  static constexpr int THREADS = 32 * (3 + SOFTMAX_WARPS * HALVES * TILES);
   static constexpr int DS = D / 64;                       // 64-element sub-tiles along the head dim
   static constexpr int Q_TILE_BYTES = TILE_M * D * 2;
   static constexpr int Q_SUB_BYTES = TILE_M * 128;        // one [128 x 64] sub-tile
@@ -75,8 +79,12 @@ struct Barriers {
   uint32_t abort;
 };
 
+// behind the barriers, with two threads a row: what either tells the other, block by block in turn: maxima; at the end the sums
+struct FromHalf {
+  float v[2][TILES][2][TILE_M];
+};
 template <int D>
-constexpr int smem_bytes() { return Shape<D>::BAR_OFF + 1024 /* alignment slack */ + (int)sizeof(Barriers); }
+constexpr int smem_bytes() { return Shape<D>::BAR_OFF + 1024 /* alignment slack */ + (int)sizeof(Barriers) + (Shape<D>::HALVES == 2 ? (int)sizeof(FromHalf) : 0); }
 
 // The softmax loops are bound by how many instructions they issue; sm_100 has float32 arithmetic on register pairs
 // (one instruction, two results, each rounded as the scalar instruction would) and a maximum of three.
@@ -112,7 +120,7 @@ __device__ __forceinline__ float ex2(float x) {
 
 // status codes: 1 producer, 2 MMA, 3 softmax
 template <int D>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(Shape<D>::THREADS, 1)
 attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                                  const int32_t* __restrict__ table, int table_width, const int32_t* __restrict__ item_start,
                                  const int32_t* __restrict__ kv_len, __nv_bfloat16* __restrict__ out, int num_items, int hq,
@@ -170,14 +178,16 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     mbar_init(&bars->q_full, 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&bars->kv_full[s], 1);
-      mbar_init(&bars->kv_empty[s], 1);
+      mbar_init(&bars->kv_empty[s], Sh::TWO_ISSUERS || rows_here <= TILE_M ? 1 : 2);
     }
     for (int j = 0; j < NB; ++j) {
       mbar_init(&bars->s_full[j], 1);
       mbar_init(&bars->p_used[j], 1);
     }
     for (int t = 0; t < TILES; ++t) {
-      mbar_init(&bars->p_ready[t], SOFTMAX_WARPS);  // one arrival per softmax warp of the tile (arrivals on one barrier serialise)
+      // one arrival per softmax warp of the tile (arrivals on one barrier serialise)
+      if constexpr (Sh::HALVES == 2) mbar_init(&bars->p_ready[t], 2 * SOFTMAX_WARPS);
+      else mbar_init(&bars->p_ready[t], SOFTMAX_WARPS);
       mbar_init(&bars->o_full[t], 1);
     }
     bars->abort = 0;
@@ -262,15 +272,21 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       }
       if (++stage == STAGES) { stage = 0; phase ^= 1; }
     }
-  } else if (warp == 1 || warp == S_WARP) {
+  } else if (warp == 1 || warp == Sh::S_WARP) {
     // --------------------------------------------------------------------------------------------------- MMA
-    // With 64 keys a block (heads of 128) two warps issue the tensor-core instructions, S = Q K^T from one and
-    // O += P V from the other: what one warp waits on and issues for both, per block and tile, took longer than a
-    // softmax warp's work on the block and set the kernel's pace (8,192 tokens: 724 -> 568 us).  With 128 keys a block
-    // the softmax takes twice as long per block and one warp keeps up; two were 5 % slower there (431 -> 452 us).
-    // S of event e + NB takes the buffer that holds P of event e: one warp issues it behind that P V; with two, the S
-    // warp waits until the P V has completed (p_used).  A block's keys are no longer needed once P V of its last tile
-    // has been issued, because that follows the block's S of every tile through s_full, the softmax and p_ready.
+    // With 64 keys a block (heads of 128) one warp issues S = Q K^T and the other O += P V: what one warp waits on and
+    // issues for both, per block and tile, took longer than a softmax warp's work on the block and set the kernel's
+    // pace (8,192 tokens: 724 -> 568 us).  With 128 keys a block that split was 5 % slower than one warp for everything;
+    // there either warp issues a tile's P V and the S that takes the buffer behind it, so that neither tile waits
+    // behind the other one's barriers.  That pays together with two softmax threads a row, and only together: 32 heads of
+    // 64, three portions of 900 and fewer tokens behind 2,100, 115.6 us as before with either alone, 110.3 with both (the
+    // scores a thread holds are 64, not 128, and four warps a scheduler hide each other's waits); two of 700 behind 3,000
+    // 93.6 -> 88.1, two of 1,000 behind 1,000 59.0 -> 55.3, one of 2,000 alone 48.9 -> 46.6.  With heads of 128 both made
+    // it slower (142 -> 150).
+    // S of event e + NB takes the buffer that holds P of event e: the warp of e's tile issues it behind that P V; with a
+    // warp per product, the S warp waits until the P V has completed (p_used).  A block's keys are no longer needed
+    // once P V of it has been issued for every tile, because that follows the tile's S of the block through s_full,
+    // the softmax and p_ready: kv_empty takes that of the last tile, or, with a warp per tile, one arrival of each.
     // All lanes follow the barriers; an elected lane issues each instruction (tcgen05.cuh says why).  All of them work
     // on the block that holds the request's last key: value rows behind it were never written by this request, and
     // 0 x (whatever an earlier owner of the page left there) must be 0, so those rows are cleared in shared memory
@@ -335,10 +351,14 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       return true;
     };
     if constexpr (!Sh::TWO_ISSUERS) {
-      if (warp == 1) {  // one warp issues both products, S of event e + NB behind P V of event e
+      const int mine = warp - 1;  // the tile whose P V this warp issues, and S of event e + NB behind it
+      if (mine < ntiles) {
+        const int my_blocks = mine == 0 ? n0 : nblk;
         bool ok = mbar_wait(&bars->q_full, 0, abort, 2);
         ok = __all_sync(0xffffffffu, ok);
-        for (int e = 0; ok && e < NB && e < total; ++e) {
+        // the first S all come from one warp, in order (a softmax warp that waits for its next event's S by parity relies on
+        // S of the event before it in that buffer having completed, and that event may be the other tile's)
+        for (int e = 0; ok && mine == 0 && e < NB && e < total; ++e) {
           ok = block_ready(block_of(e));
           if (ok && elect_one()) {
             issue_s(tile_of(e), block_of(e) % STAGES, e % NB);
@@ -346,20 +366,21 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           }
           __syncwarp();
         }
-        for (int e = 0; ok && e < total; ++e) {
-          const int t = tile_of(e), i = block_of(e);
+        for (int i = 0; ok && i < my_blocks; ++i) {
+          const int e = seq_of(mine, i);
           ok = values_ready(i);
-          const bool ahead = e + NB < total;  // S of the block NB steps on (it takes this block's buffer) goes out together with this P V
+          const bool ahead = e + NB < total;
           if (ok && ahead) ok = block_ready(block_of(e + NB));
           if (!ok) break;
-          ok = mbar_wait(&bars->p_ready[t], i & 1, abort, 2);  // P of this block is written (over its S)
+          ok = mbar_wait(&bars->p_ready[mine], i & 1, abort, 2);  // P of this block is written (over its S)
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           fence_after();
           if (elect_one()) {
-            issue_pv(t, i % STAGES, e % NB, i);
-            mma_commit(&bars->o_full[t]);
-            if (t == ntiles - 1) mma_commit(&bars->kv_empty[i % STAGES]);  // the last tile to use this block
+            issue_pv(mine, i % STAGES, e % NB, i);
+            mma_commit(&bars->o_full[mine]);
+            if (ntiles == 2 && i >= n0) mbar_arrive(&bars->kv_empty[i % STAGES]);  // for the tile that does not see it
+            mma_commit(&bars->kv_empty[i % STAGES]);
             if (ahead) {
               issue_s(tile_of(e + NB), block_of(e + NB) % STAGES, e % NB);
               mma_commit(&bars->s_full[e % NB]);
@@ -368,7 +389,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           __syncwarp();
         }
       }
-    } else if (warp == S_WARP) {
+    } else if (warp == Sh::S_WARP) {
       bool ok = mbar_wait(&bars->q_full, 0, abort, 2);
       ok = __all_sync(0xffffffffu, ok);
       for (int e = 0; ok && e < total; ++e) {
@@ -407,14 +428,15 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     }
   } else {
     // ----------------------------------------------------------------------------------------------- softmax
-    // One thread per row: it reads the row's scores of a block from tensor memory, finds the maximum, writes the
-    // probabilities over the scores and keeps the row's running maximum and sum; nothing is shared between threads.
-    // Measured per head size: with 128 keys a block the scores alone are 128 registers of the 168 a thread may have
-    // (three warps on a scheduler), and arithmetic on register pairs, which wants them aligned, costs more in spills
-    // than it saves in instructions; with 64 keys a block there is room and it pays.
+    // One thread per row, or two with half of its keys each: it reads its scores of a block from tensor memory, finds the
+    // maximum, writes the probabilities over the scores and keeps the running maximum and sum.  Two threads agree on
+    // the maximum of every block (both rescale their half of the row of O by it) and add their sums up at the end.
+    // Arithmetic on register pairs, which wants them aligned, pays with 352 threads; with 608 a thread has 96 registers
+    // for 64 scores and what goes with them.
     constexpr bool PAIRS = D == 128;
-    const int sw = warp - 2;  // 0 .. SOFTMAX_WARPS * TILES - 1
-    const int t = sw / SOFTMAX_WARPS;
+    constexpr int HALVES = Sh::HALVES, PART = Sh::PART;
+    const int sw = warp - Sh::FIRST_SOFTMAX_WARP;
+    const int t = sw / (SOFTMAX_WARPS * HALVES), half = HALVES == 2 ? (sw >> 2) & 1 : 0;
     const int quarter = warp & 3;  // a warp may only touch tensor-memory lanes [32*(warp%4), +32)
     const int r = quarter * 32 + lane;
     if (t < ntiles) {
@@ -425,7 +447,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       const bool partial = row0 + TILE_M * (t + 1) > n;
       const float c = scale * LOG2E_F;
       const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-      const uint32_t o_addr = lane_addr + Sh::O_COL + t * D;
+      const uint32_t o_addr = lane_addr + Sh::O_COL + t * D + half * (D / HALVES);  // this thread's part of the row of O
       // m_run is the maximum the row's exponentials refer to.  It follows the true maximum only when that has grown by
       // more than 2^8 (in the exponent), so that the accumulator in tensor memory is rescaled rarely; sums and
       // products use the same reference, and the quotient at the end does not depend on it.
@@ -436,11 +458,11 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       // asked for as early as they can be: a block's scores are computed blocks ahead, so as a rule the loads of
       // block i+1 go out as soon as the exponentials of block i have let go of the registers, and arrive while this
       // thread waits for its stores and hands block i over.
-      constexpr int NCH = KB / 32;
+      constexpr int NCH = PART / 32;
       float sv[NCH][32];
       auto load_scores = [&](int e) {
         fence_after();
-        const uint32_t s_addr = lane_addr + Sh::S_COL + (e % NB) * KB;
+        const uint32_t s_addr = lane_addr + Sh::S_COL + (e % NB) * KB + half * PART;
 #pragma unroll
         for (int cc = 0; cc < NCH; ++cc) tmem_ld32(s_addr + cc * 32, *reinterpret_cast<uint32_t(*)[32]>(&sv[cc][0]));
       };
@@ -458,12 +480,17 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         load_scores(e);
         return true;
       };
+      // Both threads of a row refer to the same maximum: their warps meet once a block.  A warp whose wait gave up keeps
+      // meeting the other one, as often as it would have, so that neither is left waiting.
+      FromHalf& from_half = *reinterpret_cast<FromHalf*>(bars + 1);
+      int met = 0;
+      auto meet = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + t * 4 + quarter) : "memory"); };
       if (my_blocks > 0) ok = request_scores(0);
       for (int i = 0; ok && i < my_blocks; ++i) {
-        const int key0 = (b0 + i) * KB;
+        const int key0 = (b0 + i) * KB + half * PART;
         const int e = seq_of(t, i);
-        const uint32_t s_addr = lane_addr + Sh::S_COL + (e % NB) * KB;
-        const bool need_mask = partial || key0 + KB - 1 > p_first[t] || (window > 0 && key0 < p_last[t] - window + 1);
+        const uint32_t s_addr = lane_addr + Sh::S_COL + (e % NB) * KB + half * PART;
+        const bool need_mask = partial || key0 + PART - 1 > p_first[t] || (window > 0 && key0 < p_last[t] - window + 1);
         float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
         tmem_ld_wait();
 #pragma unroll
@@ -482,7 +509,13 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             mx2 = max3(mx2, x[k + 4], x[k + 5]); mx3 = max3(mx3, x[k + 6], x[k + 7]);
           }
         }
-        const float m_new = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+        float m_new = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+        if constexpr (HALVES == 2) {
+          from_half.v[i & 1][t][half][r] = m_new;
+          meet();
+          m_new = fmaxf(m_new, from_half.v[i & 1][t][half ^ 1][r]);
+          ++met;
+        }
         const bool grow = (m_new - m_run) * c > 8.f;  // false while the row has seen nothing (-inf - -inf)
         // Each phase of o_full (P V of this tile's block i-1 has finished) is waited for exactly once, during block i:
         // a parity wait can only tell the phase in progress from the one before it.  If O has to be rescaled, before
@@ -504,14 +537,15 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           if (grow) { m_run = m_new; l_run *= alpha; }
           if (i > 0) {
             fence_after();
+            constexpr int CHUNK = HALVES == 2 ? 16 : 32;  // columns at a time (beside the scores, which are in registers)
 #pragma unroll 1
-            for (int cc = 0; cc < D / 32; ++cc) {
-              uint32_t v[32];
-              tmem_ld32(o_addr + cc * 32, v);
+            for (int cc = 0; cc < D / HALVES; cc += CHUNK) {
+              uint32_t v[CHUNK];
+              if constexpr (CHUNK == 16) tmem_ld16(o_addr + cc, v); else tmem_ld32(o_addr + cc, v);
               tmem_ld_wait();
 #pragma unroll
-              for (int k = 0; k < 32; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) * alpha);
-              tmem_st32(o_addr + cc * 32, v);
+              for (int k = 0; k < CHUNK; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) * alpha);
+              if constexpr (CHUNK == 16) tmem_st16(o_addr + cc, v); else tmem_st32(o_addr + cc, v);
             }
             tmem_st_wait();
           }
@@ -563,6 +597,12 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           if (!ok) break;
         }
       }
+      if constexpr (HALVES == 2) {
+        for (; met < my_blocks; ++met) meet();
+        from_half.v[my_blocks & 1][t][half][r] = l_run;
+        meet();
+        l_run += from_half.v[my_blocks & 1][t][half ^ 1][r];
+      }
       // the quotient
       if (ok && my_blocks > 0) {
         ok = mbar_wait(&bars->o_full[t], (my_blocks - 1) & 1, abort, 3);
@@ -572,14 +612,14 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         // one key range of several: the row's unnormalised output with the exponent it refers to and its sum
         fence_after();
         const size_t slot = ((size_t)(t0 + row) * hq + head) * kv_splits + blockIdx.z;
-        if (valid) {
+        if (valid && half == 0) {
           part_ml[slot * 2] = (my_blocks > 0 && m_run != -INFINITY) ? m_run * c : -INFINITY;
           part_ml[slot * 2 + 1] = my_blocks > 0 ? l_run : 0.f;
         }
         if (my_blocks > 0) {
-          float* dst = part_o + slot * D;
+          float* dst = part_o + slot * D + half * (D / HALVES);
 #pragma unroll 1
-          for (int cc = 0; cc < D / 32; ++cc) {
+          for (int cc = 0; cc < D / HALVES / 32; ++cc) {
             uint32_t v[32];
             tmem_ld32(o_addr + cc * 32, v);
             tmem_ld_wait();
@@ -596,9 +636,9 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         fence_after();
         // a sink (a score per head without a value) joins the denominator here, where the row's sum is complete
         const float inv = l_run > 0.f ? (sink ? sink_quotient2(m_run * c, l_run, sink[head] * PSB_LOG2E) : 1.f / l_run) : 0.f;
-        __nv_bfloat16* dst = out + ((size_t)(t0 + row) * hq + head) * D;
+        __nv_bfloat16* dst = out + ((size_t)(t0 + row) * hq + head) * D + half * (D / HALVES);
 #pragma unroll 1
-        for (int cc = 0; cc < D / 32; ++cc) {
+        for (int cc = 0; cc < D / HALVES / 32; ++cc) {
           uint32_t v[32];
           tmem_ld32(o_addr + cc * 32, v);
           tmem_ld_wait();
@@ -679,7 +719,7 @@ int launch(const CUtensorMap& map_q, const CUtensorMap& map_kv, const void* tabl
     if (e != cudaSuccess) PSB_REFUSE("attention_prefill_tcgen05: cannot reserve %d bytes of shared memory: %s", smem_bytes<D>(), cudaGetErrorString(e));
     configured.set(); 
   }
-  psb_launch(attention_prefill_tcgen05_kernel<D>, dim3(hq, whole + 2 * (num_pairs - whole), kv_splits), dim3(THREADS), (size_t)smem_bytes<D>(), stream, map_q, map_kv,
+  psb_launch(attention_prefill_tcgen05_kernel<D>, dim3(hq, whole + 2 * (num_pairs - whole), kv_splits), dim3(Shape<D>::THREADS), (size_t)smem_bytes<D>(), stream, map_q, map_kv,
              (const int32_t*)table, table_width, (const int32_t*)item_start, (const int32_t*)kv_len, (__nv_bfloat16*)out,
              num_items, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, whole, longest_first, kv_splits, (float*)part_o, (float*)part_ml,
              kv_splits > 1 ? (const float*)nullptr : sink);

@@ -37,9 +37,9 @@ WIDE_BELOW_TILES = 600   # matrices with fewer 16-row tiles than this get 16 war
 TCGEN05_PREFILL_MIN_TOKENS = 64   # steps whose longest prompt portion has at least this many tokens run prefill attention
                                   # on the tcgen05 kernel (tiles of 128 rows); shorter portions fill too little of a tile
 # ... and shorter ones too where their CTAs fit in one round over the SMs and they see at least so many keys (by head size): the other kernel
-# (mma.sync, all heads of a group in one tile) walks a portion's keys in one chain, 20 to 26 us a 1,024 of them, this one takes 17 (64) and 18 (128) and cuts
-# them into ranges besides.  32 heads over 8, one portion of 24 tokens, us by keys 512, 1,024, 2,048, 4,000: 15.0 25.5 46.6 85.9 there, 14.7 22.8 19.0
-# 25.5 here (heads of 64); 19.3 32.6 59.0 109 and 15.1 14.4 18.8 26.6 (128); three portions of eight 14.9 25.3 46.1 84.9 and 15.3 23.6 40.3 71.2; 17.4 30.2
+# (mma.sync, all heads of a group in one tile) walks a portion's keys in one chain, 20 to 26 us a 1,024 of them, this one takes 15 (64) and 18 (128) and cuts
+# them into ranges besides.  32 heads over 8, one portion of 24 tokens, us by keys 512, 1,024, 2,048, 4,000: 13.8 24.3 45.2 85.9 there, 11.6 19.0 14.6
+# 22.2 here (heads of 64); 19.3 32.6 59.0 109 and 15.1 14.4 18.8 26.6 (128); three portions of eight 13.8 24.1 44.8 84.8 and 12.3 19.2 34.3 64.6; 17.4 30.2
 # 55.8 104 and 15.5 24.3 41.8 74.0.  In two rounds it loses up to 16 tokens (eight portions of eight, 4,000 keys 91.9 and 123.9).
 TCGEN05_SHORT_MIN_KEYS = {64: 1024, 128: 512}
 USE_TMA_DECODE = True     # decode attention: the kernel whose keys and values the TMA unit brings in (pages of 16 tokens
@@ -453,10 +453,10 @@ def _decode_key_range(pairs: int, longest: int, sms: int, tma_kernel: bool, ctas
 
 def _whole_row_groups(groups: int, heads: int, d: int, sms: int) -> int:
     """Row groups (256 rows of a head a CTA) before those that two CTAs of 128 rows take: of a second round over the SMs that is at most half full, where the
-    halves fit in one round.  Half the rows take a CTA 0.87 of the time (heads of 64) or 0.73 (128), so heads of 64 are halved up to a quarter of a round only.
-    32 heads, the longest request first, us whole and halved: 640 and 512 rows behind 1,500 55.1 and 53.9 (heads of 64), 66.4 and 61.2 (128); 500, 434
-    and 367 behind 100 28.8 and 27.2 (128); 1,300 behind 1,300 69.1 and 71.1 (64), 82.6 and 78.9 (128).  In a third round (900, 780 and 660 behind 2,100), whose CTAs begin
-    as the shorter ones before them end, 115 and 138, 145 and 157."""
+    halves fit in one round.  Half the rows take a CTA 0.73 of the time with heads of 128 and more with 64, so heads of 64 are halved up to a quarter of a round only.
+    32 heads, the longest request first, us whole and halved: 640 and 512 rows behind 1,500 51.9 and 50.5 (heads of 64), 66.1 and 60.9 (128); 500, 434
+    and 367 behind 100 28.8 and 27.2 (128); 1,300 behind 1,300 66.7 and 67.6 (64), 82.9 and 78.4 (128).  In a third round (900, 780 and 660 behind 2,100), whose CTAs begin
+    as the shorter ones before them end, 110 and 118 or more, 145 and 157 (each as placed in the step)."""
     ctas = heads * groups
     last = -(-(ctas - sms) // heads)  # groups of the second round
     return groups - last if sms < ctas < 2 * sms and (2 if d == 128 else 4) * heads * last <= sms else groups
@@ -519,8 +519,8 @@ def _attention_plan(new_tokens: Sequence[int], kv_lens: Sequence[int], window: i
         plan["rows_per_cta"] = per_cta
         plan["pairs"] = pairs = sum(-(-n // per_cta) for n in portions)
         # The requests that see most first, where the CTAs are less than two rounds: what begins last then ends soon.  With more the shorter ones are as well
-        # first (32 heads, us by place in the step, shortest first here, and by length; heads of 64 and 128: 1,000 and 800 rows behind 1,000 68.1 and 58.9,
-        # 77.1 and 69.2; 660, 572 and 483 behind 400 46.1 and 42.1, 49.3 and 47.0; 900, 780 and 660 behind 2,100, 352 CTAs, 115.1 and 117.4, 145.5 and 143.4).
+        # first (32 heads, us by place in the step, shortest first here, and by length; heads of 64 and 128: 1,000 and 800 rows behind 1,000 66.2 and 55.0,
+        # 77.1 and 69.2; 660, 572 and 483 behind 400 44.9 and 40.3, 49.3 and 46.7; 900, 780 and 660 behind 2,100, 352 CTAs, 109.8 and 114.0, 141.6 and 142.0).
         plan["longest_first"] = 1 if sms < hq_total * pairs < 2 * sms and 1 < b <= 32 else 0
         plan["whole"] = _whole_row_groups(pairs, hq_total, d, sms) if plan["kv_splits"] == 1 and per_cta == lib().psb_attention_prefill_tcgen05_rows_per_cta() else pairs
     else:

@@ -41,7 +41,9 @@ TCGEN05_PREFILL_MIN_TOKENS = 64   # steps whose longest prompt portion has at le
 # them into ranges besides.  32 heads over 8, one portion of 24 tokens, us by keys 512, 1,024, 2,048, 4,000: 13.8 24.3 45.2 85.9 there, 11.6 19.0 14.6
 # 22.2 here (heads of 64); 19.3 32.6 59.0 109 and 15.1 14.4 18.8 26.6 (128); three portions of eight 13.8 24.1 44.8 84.8 and 12.3 19.2 34.3 64.6; 17.4 30.2
 # 55.8 104 and 15.5 24.3 41.8 74.0.  In two rounds it loses up to 16 tokens (eight portions of eight, 4,000 keys 91.9 and 123.9).
-TCGEN05_SHORT_MIN_KEYS = {64: 1024, 128: 512}
+# At 520 keys heads of 64 take 14.2 us there and 13.5 here (two tokens), 17.0 and 13.6 (63 tokens), 15.0 and 14.4 (four portions of eight and fewer); at 256 keys the
+# two are level (8.6 and 8.6).
+TCGEN05_SHORT_MIN_KEYS = {64: 512, 128: 512}
 USE_TMA_DECODE = True     # decode attention: the kernel whose keys and values the TMA unit brings in (pages of 16 tokens
                           # or more), for key ranges of at least TMA_DECODE_MIN_RANGE keys; otherwise the one in which
                           # every lane copies its own pieces.  Measured at Llama-1B sizes, context 4,096, ms a decode step

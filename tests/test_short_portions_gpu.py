@@ -34,7 +34,7 @@ def _step(d, hq, hkv, portions):
 
 
 @pytest.mark.parametrize("d,hq,hkv,window,portions,taken", [
-    (64, 32, 8, None, [(31, 2000)], True), (64, 32, 8, None, [(2, 1022)], True), (64, 32, 8, None, [(2, 1021)], False),       # 1,024 keys
+    (64, 32, 8, None, [(31, 2000)], True), (64, 32, 8, None, [(2, 510)], True), (64, 32, 8, None, [(2, 509)], False),       # 512 keys
     (128, 32, 8, None, [(63, 449), (1, 700), (5, 100)], True), (128, 32, 8, None, [(63, 448)], False),                         # 512 keys; beside a decoded token
     (64, 32, 8, None, [(9, 1500)] * 4, True), (64, 32, 8, None, [(9, 1500)] * 5, False),                                       # 128 and 160 CTAs on 148 SMs
     (128, 8, 8, 300, [(20, 3000)], False), (128, 8, 4, 500, [(20, 3000), (1, 2000)], True), (128, 6, 1, None, [(3, 4000)], True)])

@@ -30,6 +30,7 @@ struct SingleArgs {
   long long P, slot_floats;
   int beta_at, G, H, dim, vdim, K, num_slots;
   float eps;
+  int* gives_up;  // not null: the wait gives up at once and says so there
 };
 
 template <typename T, bool CHANNEL>
@@ -105,7 +106,10 @@ delta_single_kernel(const T* __restrict__ proj, const SingleArgs a) {
   __syncthreads();
   const float fq = unit_factor(sums[0], dim), fk = unit_factor(sums[1], 1);
   float4* const rows = reinterpret_cast<float4*>(held) + lane;  // row d: (vdim / 4) d further
-  if (!tc::mbar_wait(&arrived, 0, &abort, 1)) __nanosleep(200000);  // (never seen: the copy is given time to land, the state is left as it was)
+  // A wait that gives up (never seen) leaves the head's state, the slot's inputs that this CTA keeps and the result as they were, but for
+  // the copy, which is waited for once more: it must not land in another CTA's shared memory.
+  if (!tc::mbar_wait_limited(&arrived, 0, &abort, 1, a.gives_up ? 0 : tc::SPIN_LIMIT, a.gives_up ? a.gives_up : &tc::g_status))
+    for (uint32_t spin = 0; spin < tc::SPIN_LIMIT && !tc::mbar_try_wait(&arrived, 0); ++spin) {}
   const bool fine = __syncthreads_and(abort == 0);
   {
     float4 sk = make_float4(0.f, 0.f, 0.f, 0.f), sq = sk;
@@ -136,7 +140,7 @@ delta_single_kernel(const T* __restrict__ proj, const SingleArgs a) {
     us[c] = u;
     o = fmaf(sums[2] * fq * fk, u, dec * sq[0]);
     if constexpr (CHANNEL) {
-      if (c < vdim) static_cast<float*>(a.out)[((size_t)t * a.H + h) * vdim + c] = o;
+      if (fine && c < vdim) static_cast<float*>(a.out)[((size_t)t * a.H + h) * vdim + c] = o;
     } else {
       const float ss = warp_sum(c < vdim ? o * o : 0.f);
       if (lane == 0) squares[warp] = ss;
@@ -158,7 +162,7 @@ delta_single_kernel(const T* __restrict__ proj, const SingleArgs a) {
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;"
                  ::"l"(S), "r"(tc::smem_u32(held)), "r"(bytes) : "memory");
   if constexpr (!CHANNEL) {
-    if (threadIdx.x < vdim) {
+    if (fine && threadIdx.x < vdim) {
       const int c = threadIdx.x;
       const float inv = 1.f / sqrtf(((squares[0] + squares[1]) + (squares[2] + squares[3])) / (float)vdim + a.eps);
       const size_t at = (size_t)h * vdim + c;
@@ -168,7 +172,7 @@ delta_single_kernel(const T* __restrict__ proj, const SingleArgs a) {
   }
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   // the slot's convolution inputs move up by one; a group's queries and keys by its first head
-  for (int j = (h % each == 0 ? 0 : 2 * dim) + threadIdx.x; j < channels; j += THREADS) {
+  for (int j = (h % each == 0 ? 0 : 2 * dim) + threadIdx.x; fine && j < channels; j += THREADS) {
     const int c = column(j);
     float keep[MAX_TAPS];
 #pragma unroll
@@ -196,12 +200,12 @@ PSB_API int psb_delta_single_supported(int G, int H, int dim, int vdim, int K) {
 
 // Requests of one token each; others are left untouched.  The gated rule (gain given): proj of either type [T, ld] with q | k | v | gate in its first columns, ba
 // float32 [T, 2 H], out [T, H vdim] of proj's type.  The other: decay float32 [T, H, dim], the write strengths in proj's columns from beta_at on,
-// out float32 [T, H, vdim].
+// out float32 [T, H, vdim].  gives_up (an int32 on the device, null as a rule): the wait for the state gives up without a poll and leaves its code there.
 // (proj, dtype, ld, beta_at, ba, decay, taps, a_log, dt_bias, state, positions, item_start, slots, gain, out, items, G, H, dim, vdim, K, num_slots,
-//  slot_floats, eps, stream)
+//  slot_floats, eps, gives_up, stream)
 PSB_API int psb_delta_single(const void* proj, int dtype, long long ld, int beta_at, const void* ba, const void* decay, const void* taps, const void* a_log,
                              const void* dt_bias, void* state, const void* positions, const void* item_start, const void* slots, const void* gain, void* out,
-                             int items, int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats, float eps, cudaStream_t stream) {
+                             int items, int G, int H, int dim, int vdim, int K, int num_slots, long long slot_floats, float eps, void* gives_up, cudaStream_t stream) {
   if (!psb_delta_single_supported(G, H, dim, vdim, K)) PSB_REFUSE("delta_single: sizes G=%d H=%d dim=%d vdim=%d K=%d are not built", G, H, dim, vdim, K);
   const long long C = 2LL * G * dim + (long long)H * vdim;
   const bool gated = gain != nullptr;
@@ -214,7 +218,7 @@ PSB_API int psb_delta_single(const void* proj, int dtype, long long ld, int beta
   args.ba = (const float*)ba; args.taps = (const float*)taps; args.a_log = (const float*)a_log; args.dt_bias = (const float*)dt_bias;
   args.decay = (const float*)decay; args.gain = (const float*)gain; args.state = (float*)state; args.positions = (const int32_t*)positions;
   args.item_start = (const int32_t*)item_start; args.slots = (const int32_t*)slots; args.out = out; args.P = ld; args.slot_floats = slot_floats;
-  args.beta_at = beta_at; args.G = G; args.H = H; args.dim = dim; args.vdim = vdim; args.K = K; args.num_slots = num_slots; args.eps = eps;
+  args.beta_at = beta_at; args.G = G; args.H = H; args.dim = dim; args.vdim = vdim; args.K = K; args.num_slots = num_slots; args.eps = eps; args.gives_up = (int*)gives_up;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)items, (unsigned)H);
   cfg.blockDim = dim3(THREADS);

@@ -1248,7 +1248,7 @@ def delta_rule(proj: torch.Tensor, ba: torch.Tensor, taps: torch.Tensor, a_log: 
         check(lib().psb_delta_single(proj.data_ptr(), _code(proj, "projection output"), proj.shape[1], 0, ba.data_ptr(), None, taps.data_ptr(),
                                      a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), _i32(ctx.positions, "positions").data_ptr(),
                                      _i32(ctx.item_start, "item offsets").data_ptr(), _i32(ctx.slots, "slots").data_ptr(), gain.data_ptr(),
-                                     out.data_ptr(), ctx.num_items, groups, heads, dim, vdim, k, state.shape[0], slot_floats, float(eps), _stream()),
+                                     out.data_ptr(), ctx.num_items, groups, heads, dim, vdim, k, state.shape[0], slot_floats, float(eps), None, _stream()),
               "delta_single")
         return out
     # Long portions go in chunks; what is left, if anything can be, token by token.
@@ -1602,7 +1602,7 @@ def channel_delta_rule(proj: torch.Tensor, beta_at: int, decay: torch.Tensor, ta
         check(lib().psb_delta_single(proj.data_ptr(), _code(proj, "projection output"), proj.shape[1], beta_at, None, decay.data_ptr(), taps.data_ptr(),
                                      None, None, state.data_ptr(), _i32(ctx.positions, "positions").data_ptr(),
                                      _i32(ctx.item_start, "item offsets").data_ptr(), _i32(ctx.slots, "slots").data_ptr(), None, o.data_ptr(),
-                                     ctx.num_items, groups, heads, dim, vdim, k, state.shape[0], slot_floats, 0.0, _stream()), "delta_single")
+                                     ctx.num_items, groups, heads, dim, vdim, k, state.shape[0], slot_floats, 0.0, None, _stream()), "delta_single")
         return o
     item_start, slots = _i32(ctx.item_start, "item offsets"), _i32(ctx.slots, "slots")
     code, ld = _code(proj, "projection output"), proj.shape[1]

@@ -233,8 +233,8 @@ _SIGNATURES: dict[str, list] = {
     # (G, H, dim, vdim, K) -> 1 if psb_delta_single is built for the sizes
     "psb_delta_single_supported": [I, I, I, I, I],
     # (proj, dtype, ld, beta_at, ba, decay, taps, a_log, dt_bias, state, positions, item_start, slots, gain, out, items, G, H, dim, vdim, K,
-    #  num_slots, slot_floats, eps, stream)
-    "psb_delta_single": [P, I, L, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, L, F, P],
+    #  num_slots, slot_floats, eps, gives_up, stream)
+    "psb_delta_single": [P, I, L, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, L, F, P, P],
     # () -> 0 while no bounded wait of that kernel has ever run out
     "psb_delta_single_status": [],
     # (o, proj, dtype, gain, out, T, G, H, dim, vdim, eps, stream)

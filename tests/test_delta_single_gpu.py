@@ -95,3 +95,32 @@ def test_single_tokens(groups, heads, dim, vdim, k, dtype, gated, requests):
     assert far(out, want) < 1.5 * far(other, want) + 2e-7
     untouched = [s for s in range(requests + 2) if s not in slots]
     assert torch.equal(state[untouched], state0[untouched])
+
+
+@pytest.mark.parametrize("gated", [True, False])
+def test_a_wait_that_gives_up_leaves_everything_as_it_was(gated):
+    """The wait for a head's state gives up at once: its code stands in the word handed in, and neither state, inputs nor result are touched."""
+    groups, heads, dim, vdim, k, requests = 2, 4, 64, 32, 4, 3
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rand = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    c = 2 * groups * dim + heads * vdim
+    proj = rand(requests, c + heads * vdim if gated else c + heads)
+    ba, decay, taps, a_log, dt_bias, gain = rand(requests, 2 * heads), torch.rand(requests, heads * dim, device="cuda"), rand(c, k), rand(heads), rand(heads), rand(vdim)
+    state, out, word = rand(requests, (k - 1) * c + heads * dim * vdim), rand(requests, heads * vdim), i32([0])
+    positions, item_start, slots = i32([0, 5, 700]), i32([0, 1, 2, 3]), i32([2, 0, 1])
+    of = lambda x, there: x.data_ptr() if there else None
+
+    def call(state, out, word):
+        library.check(library.lib().psb_delta_single(
+            proj.data_ptr(), 0, proj.shape[1], 0 if gated else c, of(ba, gated), of(decay, not gated), taps.data_ptr(), of(a_log, gated), of(dt_bias, gated),
+            state.data_ptr(), positions.data_ptr(), item_start.data_ptr(), slots.data_ptr(), of(gain, gated), out.data_ptr(), requests, groups, heads, dim, vdim, k,
+            requests, state.shape[1], EPS, word, library.stream_handle()), "delta_single")
+
+    state2, out2 = state.clone(), out.clone()
+    call(state2, out2, word.data_ptr())
+    assert word.item() == 1 and torch.equal(state2, state) and torch.equal(out2, out)
+    assert library.tcgen05_status() == 0  # (the word of the kernel itself is another)
+    call(state2, out2, None)
+    changed = (state2 != state).view(requests, -1)
+    assert bool(changed.any(1).all()) and not torch.equal(out2, out) and library.tcgen05_status() == 0

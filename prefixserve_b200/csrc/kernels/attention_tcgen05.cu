@@ -125,7 +125,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                                  const int32_t* __restrict__ table, int table_width, const int32_t* __restrict__ item_start,
                                  const int32_t* __restrict__ kv_len, __nv_bfloat16* __restrict__ out, int num_items, int hq,
                                  int hkv, int page_shift, int window, float scale, int skip_single, int rows_per_cta,
-                                 int whole, int longest_first, int kv_splits, float* __restrict__ part_o, float* __restrict__ part_ml,
+                                 int whole, int longest_first, float lag, int kv_splits, float* __restrict__ part_o, float* __restrict__ part_ml,
                                  const float* __restrict__ sink) {
   using Sh = Shape<D>;
   constexpr int KB = Sh::KB, NB = Sh::S_BUFS, STAGES = Sh::STAGES;
@@ -449,8 +449,12 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
       const uint32_t o_addr = lane_addr + Sh::O_COL + t * D + half * (D / HALVES);  // this thread's part of the row of O
       // m_run is the maximum the row's exponentials refer to.  It follows the true maximum only when that has grown by
-      // more than 2^8 (in the exponent), so that the accumulator in tensor memory is rescaled rarely; sums and
-      // products use the same reference, and the quotient at the end does not depend on it.
+      // more than 2^lag (in the exponent), so that the accumulator in tensor memory is rescaled rarely; sums and
+      // products use the same reference, and the quotient at the end does not depend on it.  But a row's largest
+      // probability is 1, which bfloat16 holds exactly, only where the reference is the maximum itself: with a lag of 8
+      // results are 4 to 6 % further from float64 than with one of 0 (2.32e-3 and 2.21e-3, 24 rows behind 1,000 keys), which
+      // takes 2 to 13 % longer there (31 rows over 4,000 keys in ranges, heads of 128, 25.8 us and 29.4).  So steps of short
+      // portions, which another kernel would attend for with a reference that does not lag, are launched with 0, others with 8.
       float m_run = -INFINITY, l_run = 0.f;
       bool ok = true;
       const int my_blocks = max(0, bend[t] - b0 + 1);
@@ -516,7 +520,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           m_new = fmaxf(m_new, from_half.v[i & 1][t][half ^ 1][r]);
           ++met;
         }
-        const bool grow = (m_new - m_run) * c > 8.f;  // false while the row has seen nothing (-inf - -inf)
+        const bool grow = (m_new - m_run) * c > lag;  // false while the row has seen nothing (-inf - -inf)
         // Each phase of o_full (P V of this tile's block i-1 has finished) is waited for exactly once, during block i:
         // a parity wait can only tell the phase in progress from the one before it.  If O has to be rescaled, before
         // that.  Otherwise, with 128 keys a block, ahead of the exponentials too: P V of the block before has completed
@@ -711,7 +715,7 @@ __global__ void attention_prefill_merge_kernel(const float* __restrict__ part_o,
 template <int D>
 int launch(const CUtensorMap& map_q, const CUtensorMap& map_kv, const void* table, int table_width, const void* item_start,
            const void* kv_len, void* out, int num_items, int num_pairs, int hq, int hkv, int page_shift, int window,
-           float scale, int skip_single, int rows_per_cta, int whole, int longest_first, int kv_splits, void* part_o, void* part_ml, const void* token_item,
+           float scale, int skip_single, int rows_per_cta, int whole, int longest_first, float lag, int kv_splits, void* part_o, void* part_ml, const void* token_item,
            int T, const float* sink, cudaStream_t stream) {
   static PsbPerDevice configured; 
   if (!configured.get()) {
@@ -721,7 +725,7 @@ int launch(const CUtensorMap& map_q, const CUtensorMap& map_kv, const void* tabl
   }
   psb_launch(attention_prefill_tcgen05_kernel<D>, dim3(hq, whole + 2 * (num_pairs - whole), kv_splits), dim3(Shape<D>::THREADS), (size_t)smem_bytes<D>(), stream, map_q, map_kv,
              (const int32_t*)table, table_width, (const int32_t*)item_start, (const int32_t*)kv_len, (__nv_bfloat16*)out,
-             num_items, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, whole, longest_first, kv_splits, (float*)part_o, (float*)part_ml,
+             num_items, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, whole, longest_first, lag, kv_splits, (float*)part_o, (float*)part_ml,
              kv_splits > 1 ? (const float*)nullptr : sink);
   if (kv_splits > 1) {
     const long long units = (long long)T * hq;
@@ -748,13 +752,14 @@ PSB_API int psb_attention_prefill_tcgen05_rows_per_cta() { return ROWS_PER_CTA; 
 // int32; item_start [num_items+1], kv_len [num_items] int32 on the device.  rows_per_cta: 256 or 128.  num_pairs: the sum
 // over the requests this kernel owns (all, or those with more than one new token when skip_single) of
 // ceil(new tokens / rows_per_cta); the first ``whole`` of them are a CTA's for every head, the others two CTAs' of half the rows each.
-// longest_first (up to 32 requests): the requests' row groups by the keys that these hold, otherwise the last request's first.  kv_splits > 1: the keys are cut into that many ranges; part_o (float32
+// longest_first (up to 32 requests): the requests' row groups by the keys that these hold, otherwise the last request's first.  lag (0 to 8): how far, as a power of two, the
+// exponentials' reference may lag behind a row's maximum (0: results closer to the exact ones, 8: sooner).  kv_splits > 1: the keys are cut into that many ranges; part_o (float32
 // [T, hq, kv_splits, D]) and part_ml ([T, hq, kv_splits, 2]) take the ranges' partial results, token_item ([T] int32)
 // tells the merge which request a row belongs to.
 PSB_API int psb_attention_prefill_tcgen05(const void* q, const void* kv, const void* table, int table_width, const void* item_start,
                                           const void* kv_len, void* out, int num_items, int num_pairs, int T, int hq, int hkv,
                                           int D, int page_size, long long num_pages, int window, float scale, int skip_single,
-                                          int rows_per_cta, int whole, int longest_first, int kv_splits, void* part_o, void* part_ml, const void* token_item,
+                                          int rows_per_cta, int whole, int longest_first, float lag, int kv_splits, void* part_o, void* part_ml, const void* token_item,
                                           const void* sink, cudaStream_t stream) {
   if (kv_splits < 1 || kv_splits > 32 || (kv_splits > 1 && (!part_o || !part_ml || !token_item)))
     PSB_REFUSE("attention_prefill_tcgen05: %d key ranges (1 to 32), or their scratch is missing", kv_splits);
@@ -766,6 +771,7 @@ PSB_API int psb_attention_prefill_tcgen05(const void* q, const void* kv, const v
   if (num_items <= 0 || num_pairs <= 0) return 0;
   if (whole < 0 || whole > num_pairs || (whole < num_pairs && (rows_per_cta != ROWS_PER_CTA || kv_splits > 1)))
     PSB_REFUSE("attention_prefill_tcgen05: %d of %d row groups whole (with key ranges, or groups of %d, all are)", whole, num_pairs, TILE_M);
+  if (!(lag >= 0.f && lag <= 8.f)) PSB_REFUSE("attention_prefill_tcgen05: the reference may lag by 0 to 8, not %g", (double)lag);
   if (longest_first && num_items > 32) PSB_REFUSE("attention_prefill_tcgen05: %d requests by length (at most 32)", num_items);
   if (whole + 2LL * (num_pairs - whole) > 65535) PSB_REFUSE("attention_prefill_tcgen05: %d row groups in one step (at most 65535)", num_pairs);
   const long long kv_rows = num_pages * 2 * hkv * page_size;
@@ -779,8 +785,8 @@ PSB_API int psb_attention_prefill_tcgen05(const void* q, const void* kv, const v
   if (r == -1) PSB_REFUSE("attention_prefill_tcgen05: the driver does not export cuTensorMapEncodeTiled");
   if (r != 0) PSB_REFUSE("attention_prefill_tcgen05: cuTensorMapEncodeTiled failed with code %d", r);
   int rc;
-  if (D == 64) rc = launch<64>(map_q, map_kv, table, table_width, item_start, kv_len, out, num_items, num_pairs, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, whole, longest_first, kv_splits, part_o, part_ml, token_item, T, (const float*)sink, stream);
-  else rc = launch<128>(map_q, map_kv, table, table_width, item_start, kv_len, out, num_items, num_pairs, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, whole, longest_first, kv_splits, part_o, part_ml, token_item, T, (const float*)sink, stream);
+  if (D == 64) rc = launch<64>(map_q, map_kv, table, table_width, item_start, kv_len, out, num_items, num_pairs, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, whole, longest_first, lag, kv_splits, part_o, part_ml, token_item, T, (const float*)sink, stream);
+  else rc = launch<128>(map_q, map_kv, table, table_width, item_start, kv_len, out, num_items, num_pairs, hq, hkv, page_shift, window, scale, skip_single, rows_per_cta, whole, longest_first, lag, kv_splits, part_o, part_ml, token_item, T, (const float*)sink, stream);
   if (rc) return rc;
   PSB_LAUNCH_CHECK("attention_prefill_tcgen05");
   return 0;

@@ -36,14 +36,16 @@ FEWROWS_MAX = {"plain": 64, "gated": 64, "rope": 64}
 WIDE_BELOW_TILES = 600   # matrices with fewer 16-row tiles than this get 16 warps per CTA instead of 8
 TCGEN05_PREFILL_MIN_TOKENS = 64   # steps whose longest prompt portion has at least this many tokens run prefill attention
                                   # on the tcgen05 kernel (tiles of 128 rows); shorter portions fill too little of a tile
-# ... and shorter ones too where their CTAs fit in one round over the SMs and they see at least so many keys (by head size): the other kernel
-# (mma.sync, all heads of a group in one tile) walks a portion's keys in one chain, 20 to 26 us a 1,024 of them, this one takes 15 (64) and 18 (128) and cuts
-# them into ranges besides.  32 heads over 8, one portion of 24 tokens, us by keys 512, 1,024, 2,048, 4,000: 13.8 24.3 45.2 85.9 there, 11.6 19.0 14.6
-# 22.2 here (heads of 64); 19.3 32.6 59.0 109 and 15.1 14.4 18.8 26.6 (128); three portions of eight 13.8 24.1 44.8 84.8 and 12.3 19.2 34.3 64.6; 17.4 30.2
-# 55.8 104 and 15.5 24.3 41.8 74.0.  In two rounds it loses up to 16 tokens (eight portions of eight, 4,000 keys 91.9 and 123.9).
-# At 520 keys heads of 64 take 14.2 us there and 13.5 here (two tokens), 17.0 and 13.6 (63 tokens), 15.0 and 14.4 (four portions of eight and fewer); at 256 keys the
-# two are level (8.6 and 8.6).
-TCGEN05_SHORT_MIN_KEYS = {64: 512, 128: 512}
+# ... and shorter ones too where their CTAs fit in one round over the SMs and they see at least so many keys: the other kernel
+# (mma.sync, all heads of a group in one tile) walks a portion's keys in one chain, 21 to 32 us a 1,024 of them, this one takes 25 and cuts
+# them into ranges besides.  Its exponentials refer to the maximum itself there, so that results are as close to float64 as the other's (2.2053e-3 of
+# them and 2.2055e-3 over 520 keys; in ranges 2.15e-3 and 2.21e-3).  With heads of 64 only in ranges: blocks of 128 keys
+# instead of 64 leave fewer probabilities that are exactly 1 (2.234e-3 and 2.227e-3 without ranges, 2.20e-3 and 2.26e-3 in them).
+# us there and here, one portion of 24 tokens, 32 heads over 8: heads of 128, by keys 512, 640, 768, 2,048, 4,000: 18.0 21.2 24.5 57.6 109 and 14.9 17.5 13.1
+# 18.5 29.4; three portions of eight 16.2 19.4 22.6 54.6 104 and 15.2 17.8 20.4 44.4 79.8; heads of 64, 1,409 and 1,900 keys 33.4 42.4 and 14.9 17.0.  32 heads over
+# 32, 16 and 2, 8 over 8, 4 and 1, one to four portions of 2 to 63 tokens: from 512 keys on here sooner in every one (closest 15.1 and 14.2, 15.5 and 15.0; 8.2
+# and 8.6 at 256 keys).  In two rounds it loses up to 16 tokens (eight portions of eight, 4,000 keys 91.9 and 123.9).
+TCGEN05_SHORT_MIN_KEYS = 512
 USE_TMA_DECODE = True     # decode attention: the kernel whose keys and values the TMA unit brings in (pages of 16 tokens
                           # or more), for key ranges of at least TMA_DECODE_MIN_RANGE keys; otherwise the one in which
                           # every lane copies its own pieces.  Measured at Llama-1B sizes, context 4,096, ms a decode step
@@ -464,12 +466,24 @@ def _whole_row_groups(groups: int, heads: int, d: int, sms: int) -> int:
     return groups - last if sms < ctas < 2 * sms and (2 if d == 128 else 4) * heads * last <= sms else groups
 
 
+def _prefill_key_ranges(portions: Sequence[int], kv_lens: Sequence[int], window: int, heads: int, d: int, sms: int, static_kv_len: int | None) -> int:
+    """Ranges the keys are cut into where CTAs of 256 rows leave more than half of the SMs without one: at least PREFILL_MIN_KEY_RANGES
+    of PREFILL_MIN_BLOCKS_PER_RANGE blocks of keys each, else 1."""
+    ctas = heads * sum(-(-n // lib().psb_attention_prefill_tcgen05_rows_per_cta()) for n in portions)
+    if ctas > sms // 2:
+        return 1
+    longest = static_kv_len if static_kv_len is not None else max(kv_lens)
+    splits = min(PREFILL_MAX_KEY_RANGES, sms // ctas, -(-longest // (128 if d == 64 else 64)) // PREFILL_MIN_BLOCKS_PER_RANGE)
+    return splits if splits >= PREFILL_MIN_KEY_RANGES else 1
+
+
 def _short_portions_in_tiles(portions: Sequence[int], kv_lens: Sequence[int], window: int, heads: int, d: int, sms: int, static_kv_len: int | None) -> bool:
-    """Whether portions shorter than TCGEN05_PREFILL_MIN_TOKENS are over sooner on the kernel of 128-row tiles."""
+    """Whether portions shorter than TCGEN05_PREFILL_MIN_TOKENS are over sooner on the kernel of 128-row tiles, and no further from the exact result."""
     keys = static_kv_len if static_kv_len is not None else max(kv_lens)
     if window:
         keys = min(keys, window + max(portions))
-    return heads * len(portions) <= sms and keys >= TCGEN05_SHORT_MIN_KEYS.get(d, 1 << 30)
+    return (heads * len(portions) <= sms and keys >= TCGEN05_SHORT_MIN_KEYS
+            and (d == 128 or _prefill_key_ranges(portions, kv_lens, window, heads, d, sms, static_kv_len) > 1))
 
 
 def _attention_plan(new_tokens: Sequence[int], kv_lens: Sequence[int], window: int, group: int, hkv: int, d: int, page: int,
@@ -496,29 +510,21 @@ def _attention_plan(new_tokens: Sequence[int], kv_lens: Sequence[int], window: i
             DECODE_CTAS_PER_SM if d <= 64 else DECODE_CTAS_PER_SM_128)
         plan["max_splits"] = -(-longest // plan["chunk"])
         plan["all_single"] = 1 if len(singles) == b else 0
-    portions = [n for n in new_tokens if not (plan["use_decode"] and n == 1)]
+    taken = [(n, kvl) for n, kvl in zip(new_tokens, kv_lens) if not (plan["use_decode"] and n == 1)]
+    portions, held = [n for n, _ in taken], [kvl for _, kvl in taken]
     plan["tcgen05"] = bool(USE_TCGEN05 and portions and lib().psb_attention_prefill_tcgen05_supported(d, page)
                            and (max(portions) >= TCGEN05_PREFILL_MIN_TOKENS
-                                or _short_portions_in_tiles(portions, [kvl for n, kvl in zip(new_tokens, kv_lens) if not (plan["use_decode"] and n == 1)],
-                                                            window, hq_total, d, sms, static_kv_len)))
+                                or _short_portions_in_tiles(portions, held, window, hq_total, d, sms, static_kv_len)))
     if plan["tcgen05"]:
         # a CTA takes 256 rows of one head as two tiles that fill each other's waits; when that leaves more than half
         # of the SMs without a CTA (a few hundred new tokens), one tile each and twice the CTAs (measured at 32 heads:
         # 512-token portions 7.29 -> 7.04 ms per 2,048 tokens, 1,024-token portions would lose)
         per_cta = lib().psb_attention_prefill_tcgen05_rows_per_cta()
-        ctas = hq_total * sum(-(-n // per_cta) for n in portions)
-        plan["kv_splits"] = 1
-        if ctas <= sms // 2:
-            # few CTAs: cut the keys into ranges if the portions' contexts are long enough (at least
-            # PREFILL_MIN_BLOCKS_PER_RANGE blocks a range), else give every CTA one tile instead of two
-            longest = static_kv_len if static_kv_len is not None else max(kvl for n, kvl in zip(new_tokens, kv_lens) if not (plan["use_decode"] and n == 1))
-            blocks = -(-longest // (128 if d == 64 else 64))
-            splits = min(PREFILL_MAX_KEY_RANGES, sms // ctas, blocks // PREFILL_MIN_BLOCKS_PER_RANGE)
-            if splits >= PREFILL_MIN_KEY_RANGES:
-                plan["kv_splits"] = splits
-            else:
-                per_cta //= 2
+        plan["kv_splits"] = _prefill_key_ranges(portions, held, window, hq_total, d, sms, static_kv_len)
+        if plan["kv_splits"] == 1 and hq_total * sum(-(-n // per_cta) for n in portions) <= sms // 2:
+            per_cta //= 2  # few CTAs, and contexts too short for ranges of keys: every CTA one tile instead of two
         plan["rows_per_cta"] = per_cta
+        plan["lag"] = 8.0 if max(portions) >= TCGEN05_PREFILL_MIN_TOKENS else 0.0
         plan["pairs"] = pairs = sum(-(-n // per_cta) for n in portions)
         # The requests that see most first, where the CTAs are less than two rounds: what begins last then ends soon.  With more the shorter ones are as well
         # first (32 heads, us by place in the step, shortest first here, and by length; heads of 64 and 128: 1,000 and 800 rows behind 1,000 66.2 and 55.0,
@@ -594,7 +600,7 @@ def attention_bf16(q: torch.Tensor, kv: torch.Tensor, table: torch.Tensor, item_
             q.data_ptr(), kv.data_ptr(), table.data_ptr(), table.shape[1], item_start.data_ptr(), kv_len.data_ptr(),
             out.data_ptr(), b, plan["pairs"], t, hq, hkv, d, page, kv.shape[0], w, float(scale),
             1 if plan["use_decode"] else 0, plan["rows_per_cta"], plan["whole"] if splits == 1 else plan["pairs"],
-            plan["longest_first"], splits, po, pm,
+            plan["longest_first"], plan["lag"], splits, po, pm,
             token_item.data_ptr() if token_item is not None else None, sk, stream), "attention_prefill_tcgen05")
         return out
     tiles = plan.get("tiles")

@@ -165,6 +165,10 @@ __device__ __forceinline__ float2 gates_of(uint32_t pair) {
 __device__ __forceinline__ uint32_t bits_from(int at) { return at <= 0 ? ~0u : at > 31 ? 0u : ~0u << at; }
 __device__ __forceinline__ uint32_t bits_upto(int at) { return at < 0 ? 0u : at > 30 ? ~0u : (2u << at) - 1u; }
 
+// blocks of a CTA from which on its tiles start apart (see the softmax)
+template <int MODE>
+constexpr int FEWEST_APART = MODE == CAPPED ? 2 : 3;
+
 // status codes: 1 producer, 2 MMA, 3 softmax
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -404,9 +408,13 @@ attention_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
       // Left to themselves both tiles make the same step of a block at the same time: the products of both, then the caps (or biases) of both, then the
       // exponentials, each on a unit of its own that is idle meanwhile.  A start half a block apart keeps them apart: 1,500 and 1,200 capped tokens 76.2 us ->
       // 72.0 (1,200 to 1,600 clocks; 800 73.9, 2,000 73.0), with a bias 71.6 -> 69.6; plain scores, whose steps are the products and the exponentials, no difference.
+      // Only where there are blocks to keep apart: 8 units of 128 tokens, us without and with it by blocks 1, 2, 3, 4, 8 of a CTA, capped 13.8 16.5 18.6 20.5 28.1
+      // and 13.8 16.1 17.8 19.5 26.0, in two ranges 13.0 15.2 17.6 19.6 27.1 and 13.1 15.2 16.9 18.6 25.2; with a bias 12.0 14.2 16.1 17.7 23.6 and 12.3 14.2 15.5 17.0
+      // 22.8, in two ranges 13.9 15.7 17.7 19.4 25.6 and 14.4 15.9 17.3 18.7 24.5.
       if (MODE != PLAIN && t == 1) {
+        const int apart = nblk >= FEWEST_APART<MODE> ? 1300 : 0;
         const long long from = clock64();
-        while (clock64() - from < 1300) {}
+        while (clock64() - from < apart) {}
       }
       for (int i = 0; ok && i < nblk; ++i) {
         const bool kept = is_kept(i);

@@ -206,9 +206,13 @@ __device__ __forceinline__ void leave_rows(uint4* leaving, const uint32_t (&pack
     __nv_bfloat16* crow = C + (size_t)row * ldc;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(packed[j]);
-      for (int q = 0; q < 8; ++q)
-        if (col + 8 * j + q < limit) crow[col + 8 * j + q] = e[q];
+      if (col + 8 * j + 8 <= limit && (ldc & 7) == 0) {  // a last run of fewer than 32: its whole eights
+        *reinterpret_cast<uint4*>(crow + col + 8 * j) = make_uint4(packed[j][0], packed[j][1], packed[j][2], packed[j][3]);
+      } else {
+        const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(packed[j]);
+        for (int q = 0; q < 8; ++q)
+          if (col + 8 * j + q < limit) crow[col + 8 * j + q] = e[q];
+      }
     }
   }
 }

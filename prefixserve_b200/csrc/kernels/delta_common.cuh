@@ -12,8 +12,9 @@ constexpr int BD = 5;
 __device__ __forceinline__ float softplusf_(float x) { return log1pf(expf(-fabsf(x))) + fmaxf(x, 0.f); }
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + expf(-x)); }
 __device__ __forceinline__ float siluf_(float x) { return x / (1.f + expf(-x)); }
-// The same of several numbers: the quotient by a reciprocal and what it leaves over where neither can overflow, which is asked for once.  0.485 units of the last
-// place from float64 over [-80, 80], as with the division, which takes twice as many instructions (2,000 tokens of 16 heads: delta_prepare_wide_kernel 28 us -> 21).
+// The same of several numbers, each by its own size: up to QUICK_UP_TO without a division, which takes twice as many instructions (2,000 tokens of 16 heads:
+// delta_prepare_wide_kernel 28 us -> 21); whether one lies beyond is asked for once.  From float64 0.485 units of the last place (root of the mean square, evenly over
+// [-80, 80]), as with the division.
 template <int M, int N>
 __device__ __forceinline__ void silu_all(float (&x)[M][N]) {
   float top = 0.f;
@@ -21,22 +22,19 @@ __device__ __forceinline__ void silu_all(float (&x)[M][N]) {
   for (int i = 0; i < M; ++i)
 #pragma unroll
     for (int j = 0; j < N; ++j) top = fmaxf(top, fabsf(x[i][j]));
-  if (top <= 80.f) {
+  if (top <= QUICK_UP_TO) {
+#pragma unroll
+    for (int i = 0; i < M; ++i)
+#pragma unroll
+      for (int j = 0; j < N; ++j) x[i][j] = divided(x[i][j], 1.f + expf(-x[i][j]));
+  } else {
 #pragma unroll
     for (int i = 0; i < M; ++i)
 #pragma unroll
       for (int j = 0; j < N; ++j) {
         const float d = 1.f + expf(-x[i][j]);
-        float r;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-        const float q = x[i][j] * r;
-        x[i][j] = fmaf(fmaf(-d, q, x[i][j]), r, q);
+        x[i][j] = fabsf(x[i][j]) <= QUICK_UP_TO ? divided(x[i][j], d) : x[i][j] / d;
       }
-  } else {
-#pragma unroll
-    for (int i = 0; i < M; ++i)
-#pragma unroll
-      for (int j = 0; j < N; ++j) x[i][j] = siluf_(x[i][j]);
   }
 }
 // what makes a vector with this sum of squares a unit vector, over sqrt(dim) for queries (keys: 1).  (rsqrtf(dim) is off by up to two units of the last place,

@@ -173,17 +173,6 @@ __device__ __forceinline__ void rope_store_row(uint32_t taddr, int row, int M, i
   }
 }
 
-// n / d for d from 1 to 2^120: the quotient by an approximate reciprocal, put right by what it leaves over (Markstein 1990: with a reciprocal to the last place and
-// the remainder exact, as a fused multiply-add gives it, that rounds like the division; here to within an extra 2^-47 of it).  The epilogues of gated products are
-// bounded by what their warps issue: experts on 2,037 tokens 206 us with the division itself, 191 so (189 with a quick one).
-constexpr float QUICK_UP_TO = 80.f;  // of -log(d - 1): beyond it, and for what is not finite, the division itself
-__device__ __forceinline__ float divided(float n, float d) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  const float q = n * r;
-  return fmaf(fmaf(-q, d, n), r, q);
-}
-
 // 32 columns of the warp's rows, a thread a row, from ``col`` on as far as there are columns (``limit``); rows from M on stay.  They go through shared memory
 // (pieces of 16 bytes, piece j of row r at j ^ (r / 2 % 4)) to where four lanes have a row's 64 bytes: stored by the thread that has the row, every 16 bytes are
 // half a sector on a line of their own.  Where a CTA's tiles follow one another and their stores are in the way, as in two CTAs a tile: routed experts on 2,037

@@ -124,3 +124,52 @@ def test_a_wait_that_gives_up_leaves_everything_as_it_was(gated):
     call(state2, out2, None)
     changed = (state2 != state).view(requests, -1)
     assert bool(changed.any(1).all()) and not torch.equal(out2, out) and library.tcgen05_status() == 0
+
+
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("groups,heads,dim,vdim,k", [(2, 4, 64, 32, 4), (1, 2, 128, 128, 4), (1, 1, 9, 4, 1)])
+def test_numbers_that_are_not_finite(gated, groups, heads, dim, vdim, k):
+    """Infinite and NaN projections, states, inputs and gates, and decays of 0, one kind a request: finite numbers, infinities and NaN stand where the kernels that
+    take any portion leave them, the finite ones as close as ever, and a request beside them is untouched by them."""
+    gen = torch.Generator(device="cuda").manual_seed(dim + gated)
+    rand = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    c = 2 * groups * dim + heads * vdim
+    inf, nan, n = float("inf"), float("nan"), 14
+    proj = rand(n, c + heads * vdim if gated else c + heads)
+    ba, decay = rand(n, 2 * heads), torch.sigmoid(rand(n, heads * dim) + 2)
+    taps, a_log, dt_bias, gain = rand(c, k) * 0.5, rand(heads) * 0.3, rand(heads), rand(vdim)
+    state = rand(n, (k - 1) * c + heads * dim * vdim)
+    S = state[:, (k - 1) * c:].view(n, heads, dim, vdim)
+    proj[0, 1], proj[1, groups * dim], proj[2, 2 * groups * dim + 1], proj[3, 2 * groups * dim] = nan, inf, -inf, 1e30   # query, key, values
+    S[4, 0, 0, 1], S[5, -1, 3, 2], S[6, 0, 1, 0], S[7, 0, 2, 3] = inf, -inf, nan, 3e38  # (a whole column of the last overflows or not by the order of its sum)
+    if k > 1:
+        state[8, 0], state[9, 2 * groups * dim] = nan, inf                                                              # inputs kept from before
+    if gated:
+        ba[10, 0], ba[11, heads], ba[12, heads] = inf, 3e4, nan                                                         # strength; a decay of 0
+        proj[13, c] = nan                                                                                               # the output gate
+        S[11, 0, 0, 0] = inf                                                                                            # 0 times that
+    else:
+        proj[10, c] = -inf
+        decay[11], decay[12, 1], decay[13, 0] = 0.0, nan, inf
+        S[11, 0, 0, 0] = inf
+    positions, token_item, starts, slots = i32([5] * n), i32(list(range(n))), i32(list(range(n + 1))), i32(list(range(n)))
+
+    def call(longest):
+        ctx = types.SimpleNamespace(positions=positions, token_item=token_item, item_start=starts, slots=slots, num_items=n, max_new_tokens=longest)
+        mine = state.clone()
+        if gated:
+            out = ops.delta_rule(proj, ba, taps, a_log, dt_bias, gain, mine, ctx, groups=groups, heads=heads, dim=dim, vdim=vdim, eps=EPS)
+        else:
+            out = ops.channel_delta_rule(proj, c, decay, taps, mine, ctx, groups=groups, heads=heads, dim=dim, vdim=vdim)
+        return out.view(n, -1), mine
+
+    (out, mine), (other, theirs) = call(1), call(2)
+    for got, want in ((out, other), (mine, theirs)):
+        for r in range(n):
+            assert torch.equal(got[r].isnan(), want[r].isnan()), r
+            assert torch.equal(got[r].nan_to_num(0.0, 7.0, -7.0)[got[r].isinf()], want[r].nan_to_num(0.0, 7.0, -7.0)[want[r].isinf()]), r
+            fine = got[r].isfinite()
+            if bool(fine.any()):
+                far = (got[r][fine].double() - want[r][fine].double()).abs().max()
+                assert float(far) <= 8e-6 * float(want[r][fine].double().abs().max()), r

@@ -17,8 +17,8 @@
 //               maximum and sum in float32 (three-input maxima and arithmetic on register pairs: the loop is bound by
 //               the instructions it issues), P as bfloat16 into tensor memory over the scores it came from.  O
 //               accumulates in tensor memory over the blocks; the row's reference maximum only follows the true one
-//               when that has grown by more than 2^8, and only then is the row of O rescaled (tcgen05.ld, multiply,
-//               tcgen05.st), which is rare.
+//               when that has grown by more than 2^lag (8 as a rule, see there), and only then is the row of O rescaled
+//               (tcgen05.ld, multiply, tcgen05.st), which is rare.
 // The two tiles alternate on the tensor cores: while one tile's rows are in the softmax, the other's products run.
 // A step with few such CTAs and long cached prefixes (a prompt portion of a few hundred tokens) may also cut the keys
 // into ranges: CTA (head, rows, range) then walks its share of the blocks and leaves an unnormalised partial result
@@ -452,8 +452,8 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       // more than 2^lag (in the exponent), so that the accumulator in tensor memory is rescaled rarely; sums and
       // products use the same reference, and the quotient at the end does not depend on it.  But a row's largest
       // probability is 1, which bfloat16 holds exactly, only where the reference is the maximum itself: with a lag of 8
-      // results are 4 to 6 % further from float64 than with one of 0 (2.32e-3 and 2.21e-3, 24 rows behind 1,000 keys), which
-      // takes 2 to 13 % longer there (31 rows over 4,000 keys in ranges, heads of 128, 25.8 us and 29.4).  So steps of short
+      // results are 3 to 9 % further from float64 than with one of 0 (2.34e-3 and 2.21e-3, 24 rows over 520 keys, heads of 128), which
+      // takes 1 to 14 % longer there (24 rows over 4,000 keys in ranges, heads of 128, 25.8 us and 29.4).  So steps of short
       // portions, which another kernel would attend for with a reference that does not lag, are launched with 0, others with 8.
       float m_run = -INFINITY, l_run = 0.f;
       bool ok = true;

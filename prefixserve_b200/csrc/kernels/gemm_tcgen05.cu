@@ -176,7 +176,7 @@ __device__ __forceinline__ void rope_store_row(uint32_t taddr, int row, int M, i
 // 32 columns of the warp's rows, a thread a row, from ``col`` on as far as there are columns (``limit``); rows from M on stay.  They go through shared memory
 // (pieces of 16 bytes, piece j of row r at j ^ (r / 2 % 4)) to where four lanes have a row's 64 bytes: stored by the thread that has the row, every 16 bytes are
 // half a sector on a line of their own.  Where a CTA's tiles follow one another and their stores are in the way, as in two CTAs a tile: routed experts on 2,037
-// tokens (8,148 rows of 2,048 by 1,024 in the second product: 50 us -> 42) 159 us a call -> 154, 142 -> 133 without gates, 1,979 tokens of feed-forward up to 1 % less.
+// tokens (8,148 rows of 2,048 by 1,024 in the second product: 50 us -> 42) 159 us a call -> 154, 142 -> 133 without gates; 1,979 tokens of feed-forward as before.
 // A CTA's only tile leaves sooner straight from the registers (300 rows of 8,192 gated and 2,048 columns 44.0 us instead of 43.5).
 __device__ __forceinline__ void leave_rows(uint4* leaving, const uint32_t (&packed)[4][4], __nv_bfloat16* __restrict__ C, int row, int M, int col, int limit, int ldc) {
   const int lane = threadIdx.x & 31, row0 = row - lane;

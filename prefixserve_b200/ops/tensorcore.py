@@ -38,8 +38,8 @@ TCGEN05_PREFILL_MIN_TOKENS = 64   # steps whose longest prompt portion has at le
                                   # on the tcgen05 kernel (tiles of 128 rows); shorter portions fill too little of a tile
 # ... and shorter ones too where their CTAs fit in one round over the SMs and they see at least so many keys: the other kernel
 # (mma.sync, all heads of a group in one tile) walks a portion's keys in one chain, 21 to 32 us a 1,024 of them, this one takes 25 and cuts
-# them into ranges besides.  Its exponentials refer to the maximum itself there, so that results are as close to float64 as the other's (2.2053e-3 of
-# them and 2.2055e-3 over 520 keys; in ranges 2.15e-3 and 2.21e-3).  With heads of 64 only in ranges: blocks of 128 keys
+# them into ranges besides.  Its exponentials refer to the maximum itself there, so that results are as close to float64 as the other's (2.2054e-3 of
+# them and 2.2056e-3 over 520 keys; in ranges 2.15e-3 and 2.21e-3).  With heads of 64 only in ranges: blocks of 128 keys
 # instead of 64 leave fewer probabilities that are exactly 1 (2.234e-3 and 2.227e-3 without ranges, 2.20e-3 and 2.26e-3 in them).
 # us there and here, one portion of 24 tokens, 32 heads over 8: heads of 128, by keys 512, 640, 768, 2,048, 4,000: 18.0 21.2 24.5 57.6 109 and 14.9 17.5 13.1
 # 18.5 29.4; three portions of eight 16.2 19.4 22.6 54.6 104 and 15.2 17.8 20.4 44.4 79.8; heads of 64, 1,409 and 1,900 keys 33.4 42.4 and 14.9 17.0.  32 heads over
@@ -460,7 +460,7 @@ def _whole_row_groups(groups: int, heads: int, d: int, sms: int) -> int:
     halves fit in one round.  Half the rows take a CTA 0.73 of the time with heads of 128 and more with 64, so heads of 64 are halved up to a quarter of a round only.
     32 heads, the longest request first, us whole and halved: 640 and 512 rows behind 1,500 51.9 and 50.5 (heads of 64), 66.1 and 60.9 (128); 500, 434
     and 367 behind 100 28.8 and 27.2 (128); 1,300 behind 1,300 66.7 and 67.6 (64), 82.9 and 78.4 (128).  In a third round (900, 780 and 660 behind 2,100), whose CTAs begin
-    as the shorter ones before them end, 110 and 118 or more, 145 and 157 (each as placed in the step)."""
+    as the shorter ones before them end, 110 and 118 or more, 145 and 157 (each as placed in the step).  The same with 1, 4, 8 and 32 heads a key head, within 2 %."""
     ctas = heads * groups
     last = -(-(ctas - sms) // heads)  # groups of the second round
     return groups - last if sms < ctas < 2 * sms and (2 if d == 128 else 4) * heads * last <= sms else groups
@@ -468,7 +468,9 @@ def _whole_row_groups(groups: int, heads: int, d: int, sms: int) -> int:
 
 def _prefill_key_ranges(portions: Sequence[int], kv_lens: Sequence[int], window: int, heads: int, d: int, sms: int, static_kv_len: int | None) -> int:
     """Ranges the keys are cut into where CTAs of 256 rows leave more than half of the SMs without one: at least PREFILL_MIN_KEY_RANGES
-    of PREFILL_MIN_BLOCKS_PER_RANGE blocks of keys each, else 1."""
+    of PREFILL_MIN_BLOCKS_PER_RANGE blocks of the longest context each, else 1.  A window's rows see less of it, and ranges by what they see would be
+    fewer and take longer: 8 heads of 128, 20 tokens behind 3,900, 8 ranges 10.4 us and none 15.9 (window 500), 8 ranges 12.0 and 4 13.8 (1,024); 8 heads of 64,
+    200 tokens, 8 ranges 12.4 and none 15.7 (500), 8 ranges 18.0 and 4 22.3 (2,048); 32 heads of 128, 200 tokens, 4 ranges 18.2 and none 16.7 (500)."""
     ctas = heads * sum(-(-n // lib().psb_attention_prefill_tcgen05_rows_per_cta()) for n in portions)
     if ctas > sms // 2:
         return 1
@@ -528,7 +530,7 @@ def _attention_plan(new_tokens: Sequence[int], kv_lens: Sequence[int], window: i
         plan["pairs"] = pairs = sum(-(-n // per_cta) for n in portions)
         # The requests that see most first, where the CTAs are less than two rounds: what begins last then ends soon.  With more the shorter ones are as well
         # first (32 heads, us by place in the step, shortest first here, and by length; heads of 64 and 128: 1,000 and 800 rows behind 1,000 66.2 and 55.0,
-        # 77.1 and 69.2; 660, 572 and 483 behind 400 44.9 and 40.3, 49.3 and 46.7; 900, 780 and 660 behind 2,100, 352 CTAs, 109.8 and 114.0, 141.6 and 142.0).
+        # 77.1 and 69.2; 660, 572 and 483 behind 400 44.9 and 40.3, 49.3 and 46.7; 900, 780 and 660 behind 2,100, 352 CTAs, 109.8 and 114.0, 141.6 and 142.0; over 8, 32, 4 and 1 key heads alike).
         plan["longest_first"] = 1 if sms < hq_total * pairs < 2 * sms and 1 < b <= 32 else 0
         plan["whole"] = _whole_row_groups(pairs, hq_total, d, sms) if plan["kv_splits"] == 1 and per_cta == lib().psb_attention_prefill_tcgen05_rows_per_cta() else pairs
     else:
